@@ -109,6 +109,13 @@ RUBIX_API int rubix_spaxel_sort(const int32_t* idx, const uint8_t* keep, int64_t
 RUBIX_API size_t rubix_cube_workspace_size(int64_t n, int32_t n_segments, int32_t n_wave_t,
                                            int32_t n_met, int32_t n_age, int32_t n_wave);
 
+/* Kernels that rubix_cube_fwd (general = 0), or rubix_cube_fwd_general and
+ * rubix_cube_fwd_dust (general = 1), launch for these sizes with a workspace of
+ * workspace_bytes. */
+RUBIX_API int rubix_cube_fwd_launches(int64_t n, int32_t n_segments, int32_t n_wave_t,
+                                      int32_t n_met, int32_t n_age, int32_t n_wave,
+                                      int32_t general, size_t workspace_bytes);
+
 /*
  * cube[s][0..n_wave_t) = sum over kept particles p of spaxel s of
  *   resample(mass_p * interp2d_linear(Z_p, age_p), wave_z*exp(v_p/c), wave_t).
@@ -126,6 +133,26 @@ RUBIX_API size_t rubix_cube_workspace_size(int64_t n, int32_t n_segments, int32_
  * same time.
  */
 RUBIX_API int rubix_cube_fwd(const float* ssp_flux, const float* ssp_metallicity,
+                   const float* ssp_age, const float* ssp_wave_z, int32_t n_met,
+                   int32_t n_age, int32_t n_wave, const float* wave_t, int32_t n_wave_t,
+                   const float* mass, const float* metallicity, const float* age,
+                   const float* velocity, int64_t vel_stride, int32_t vel_component,
+                   const int32_t* perm, const int32_t* seg_offsets, int32_t n_segments,
+                   int64_t n, const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop,
+                   float* cube, int64_t spaxel_stride, void* workspace,
+                   size_t workspace_bytes, void* stream);
+
+/*
+ * rubix_cube_fwd with every particle evaluated at every telescope wavelength, as
+ * rubix_cube_fwd itself does where the template grid does not qualify for the sums over
+ * SSP nodes (csrc/cube_nodes.cu).  The two agree to float32 rounding; this one keeps the
+ * summation order that the gradients' float64 sums over the cube have been recorded with.
+ * Workspace: rubix_cube_general_workspace_size.
+ */
+RUBIX_API size_t rubix_cube_general_workspace_size(int64_t n, int32_t n_segments,
+                                                   int32_t n_wave_t, int32_t n_met,
+                                                   int32_t n_age, int32_t n_wave);
+RUBIX_API int rubix_cube_fwd_general(const float* ssp_flux, const float* ssp_metallicity,
                    const float* ssp_age, const float* ssp_wave_z, int32_t n_met,
                    int32_t n_age, int32_t n_wave, const float* wave_t, int32_t n_wave_t,
                    const float* mass, const float* metallicity, const float* age,
@@ -335,11 +362,12 @@ RUBIX_API int rubix_gauss_taps(const double* sigma, const double* x, int32_t m, 
  * rubix_cube_fwd without the workspace argument, for callers that cannot allocate
  * device memory when they render: hosts that own all GPU memory through their own
  * pool and forbid cudaMalloc from plugins, or loops that must never enter an
- * allocator.  Same inputs, output and results as rubix_cube_fwd (bit-identical); the
- * scratch is a static device array of RUBIX_CUBE_NOALLOC_SCRATCH_BYTES that every GPU
+ * allocator.  Same inputs, output and results as rubix_cube_fwd: bit-identical where the
+ * array holds the node path's tables (coarse template grids), else those of the general
+ * path, equal to float32 rounding.  The scratch is a static device array of RUBIX_CUBE_NOALLOC_SCRATCH_BYTES that every GPU
  * loading this part of the library keeps until process exit.  Arguments are checked
- * as rubix_cube_fwd checks them (same codes); then problems needing more scratch
- * (rubix_cube_workspace_size) return RUBIX_E_WORKSPACE.  The first call in a CUDA
+ * as rubix_cube_fwd checks them (same codes); then problems whose general path needs more
+ * scratch return RUBIX_E_WORKSPACE.  The first call in a CUDA
  * context looks up the array's address (cudaGetSymbolAddress, cached per context)
  * and should come before any stream capture.  All calls share the array: calls whose
  * GPU work overlaps race.

@@ -106,9 +106,12 @@ class DatacubeFunction(torch.autograd.Function):
         r = renderer
         nseg = r.sbin * r.sbin
         dust_e = None if dust_av is None else r.dust_exponent
+        # the general path: the float64 sigma gradients are sums over this cube, and a
+        # recorded fit reproduces them bit for bit
         A = ops.cube_forward(r.ssp_flux, r.ssp_metallicity, r.ssp_age, r.ssp_wave_z, r.wave_t,
                              mass, metallicity, age, velocity, r.velocity_axis, perm,
-                             seg_offsets, nseg, dust_av=dust_av, dust_exponent=dust_e)
+                             seg_offsets, nseg, dust_av=dust_av, dust_exponent=dust_e,
+                             general=True)
         lsf_t = _lsf_taps(sigma_lsf, wave_res)
         psf_t = _psf_taps(sigma_psf, int(psf_size))
         crop = (len(lsf_t[0]) - 1) // 2

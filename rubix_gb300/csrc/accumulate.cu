@@ -35,6 +35,7 @@
 //   * Optional epilogue: the LSF convolution along wavelength of the finished spectrum
 //     (rubix/telescope/lsf/lsf.py:29-105), which commutes with the PSF.
 #include "cube_common.cuh"
+#include "cube_nodes.cuh"
 #include "tma.cuh"
 
 namespace rubix {
@@ -64,6 +65,10 @@ struct MainArgs {
   int lsf_k, lsf_crop;  // lsf_k = 0: no LSF epilogue
   float lsf[kMaxLsfTaps + 1];
   const float* dust_e2;  // per telescope wavelength: -0.4 log2(10) A(lambda)/A(V)
+  // not null: the spaxels that the node path leaves, gate[0] items of several-chunk
+  // spaxels at items[0..) and gate[1] others at items[split..)
+  const int* gate;
+  int split;
 };
 
 // Shared-memory carve-up of the main kernel (byte offsets, 16-byte aligned): the TMA
@@ -609,6 +614,8 @@ __device__ __forceinline__ void lsf_epilogue_k(const MainArgs& a,
 
 template <int R, bool kDust, bool kStaged>
 __global__ void __launch_bounds__(kAccThreads, 2) cube_main_kernel(MainArgs a) {
+  const int* gate = kDust ? nullptr : a.gate;
+  if (gate && gate[0] + gate[1] == 0) return;
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemLayout SL = smem_layout(kStaged ? a.n_wave : 0, kStaged ? a.pool : 0, a.pool);
   float* s_wz = reinterpret_cast<float*>(smem + SL.wz);
@@ -651,7 +658,7 @@ __global__ void __launch_bounds__(kAccThreads, 2) cube_main_kernel(MainArgs a) {
   // wavelength before the first one (dlambda_0 = 0: rubix's prepend-diff)
   const float lam_prev = a.wave_t[t0 == 0 ? 0 : min(t0 - 1, n_t - 1)];
   const float A0 = a.At[t0 < n_t ? t0 : n_t - 1];
-  const int n_items = a.ctrl->n_items;
+  const int n_items = gate ? gate[0] + gate[1] : a.ctrl->n_items;
   uint32_t phase = 0;
   int step = 0;
   __syncthreads();
@@ -659,8 +666,9 @@ __global__ void __launch_bounds__(kAccThreads, 2) cube_main_kernel(MainArgs a) {
   for (;;) {
     if (tid == 0) s_item = atomicAdd(&a.ctrl->next_item, 1);
     __syncthreads();
-    const int item = s_item;
+    int item = s_item;
     if (item >= n_items) break;
+    if (gate && item >= gate[0]) item += a.split - gate[0];
     const int2 it = a.items[item];
     const int s = it.x, chunk = it.y;
     const int seg_b = a.seg_off[s], seg_e = a.seg_off[s + 1];
@@ -906,8 +914,8 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                   const float* metallicity, const float* age, const float* velocity,
                   int64_t vel_stride, int32_t vel_component, const int32_t* perm,
                   const int32_t* seg_offsets, int32_t n_segments, int64_t n,
-                  const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop, const float* av,
-                  const float* dust_e2, float* cube, int64_t spaxel_stride, void* workspace,
+                  const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop, bool nodes,
+                  const float* av, const float* dust_e2, float* cube, int64_t spaxel_stride, void* workspace,
                   size_t workspace_bytes, void* stream);
 
 }  // namespace
@@ -915,12 +923,31 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
 
 using namespace rubix;
 
-extern "C" size_t rubix_cube_workspace_size(int64_t n, int32_t n_segments, int32_t n_wave_t,
-                                            int32_t n_met, int32_t n_age, int32_t n_wave) {
-  if (n < 0 || n_segments < 0 || n_wave_t < 0 || n_met < 0 || n_age < 0 || n_wave < 0) return 0;
+// Workspace of the general path, which every call can take.
+size_t rubix::cube_general_workspace(int64_t n, int32_t n_segments, int32_t n_wave_t,
+                                     int32_t n_met, int32_t n_age, int32_t n_wave) {
   return carve_cube(nullptr, n, n_segments, n_wave_t, n_met, n_age, n_wave,
                     cube_tuning_current().chunk)
       .bytes;
+}
+
+extern "C" size_t rubix_cube_workspace_size(int64_t n, int32_t n_segments, int32_t n_wave_t,
+                                            int32_t n_met, int32_t n_age, int32_t n_wave) {
+  if (n < 0 || n_segments < 0 || n_wave_t < 0 || n_met < 0 || n_age < 0 || n_wave < 0) return 0;
+  const size_t general = rubix::cube_general_workspace(n, n_segments, n_wave_t, n_met, n_age, n_wave);
+  if (n == 0 || !cube_nodes_supported(n_met, n_age, n_wave, n_wave_t)) return general;
+  return std::max(general, cube_nodes_bytes(n, n_segments, n_met, n_age, n_wave, n_wave_t));
+}
+
+extern "C" int rubix_cube_fwd_launches(int64_t n, int32_t n_segments, int32_t n_wave_t,
+                                       int32_t n_met, int32_t n_age, int32_t n_wave,
+                                       int32_t general, size_t workspace_bytes) {
+  if (n_segments <= 0) return 0;
+  if (!general && n > 0 && cube_nodes_supported(n_met, n_age, n_wave, n_wave_t) &&
+      cube_nodes_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes))
+    return cube_nodes_launches(n, n_segments, n_met, n_age, n_wave, workspace_bytes) + 1;
+  // setup, corner table, prefix, count, scans (one launch), fill, main (+ gather)
+  return 7 + (n > 0 ? 1 : 0);
 }
 
 namespace rubix {
@@ -972,8 +999,8 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                   const float* metallicity, const float* age, const float* velocity,
                   int64_t vel_stride, int32_t vel_component, const int32_t* perm,
                   const int32_t* seg_offsets, int32_t n_segments, int64_t n,
-                  const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop, const float* av,
-                  const float* dust_e2, float* cube, int64_t spaxel_stride, void* workspace,
+                  const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop, bool nodes,
+                  const float* av, const float* dust_e2, float* cube, int64_t spaxel_stride, void* workspace,
                   size_t workspace_bytes, void* stream) {
   {
     bool nothing_to_do = false;
@@ -984,7 +1011,9 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                                        lsf_crop, cube, spaxel_stride, &nothing_to_do);
     if (rc != RUBIX_OK || nothing_to_do) return rc;
   }
-  const size_t need = rubix_cube_workspace_size(n, n_segments, n_wave_t, n_met, n_age, n_wave);
+  const CubeTuning tune = cube_tuning_current();
+  const size_t need =
+      carve_cube(nullptr, n, n_segments, n_wave_t, n_met, n_age, n_wave, tune.chunk).bytes;
   RUBIX_REQUIRE(workspace != nullptr && workspace_bytes >= need, RUBIX_E_WORKSPACE,
                 "%s: workspace of %zu bytes needed, %zu given", who, need, workspace_bytes);
   RUBIX_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, RUBIX_E_INVALID,
@@ -1007,17 +1036,36 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                 who, n_wave, SL.total);
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const CubeTuning tune = cube_tuning_current();
-  const CubeLayout L =
+  CubeLayout L =
       carve_cube(workspace, n, n_segments, n_wave_t, n_met, n_age, n_wave, tune.chunk);
   const CubeInputs in{ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, n_met, n_age, n_wave,
                       wave_t, n_wave_t, mass, metallicity, age, velocity, vel_stride,
                       vel_component, perm, seg_offsets, n_segments, n, av};
-  {
+  MainArgs args;
+  args.gate = nullptr;
+  args.split = 0;
+  args.chunk = tune.chunk;
+  if (nodes && dust_e2 == nullptr && n > 0 && cube_nodes_supported(n_met, n_age, n_wave, n_wave_t) &&
+      cube_nodes_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes)) {
+    NodeFallback fb;
+    const int rc = cube_nodes_forward(in, lsf_taps, n_lsf_taps, lsf_crop, tune.big_item, cube,
+                                      spaxel_stride, workspace, workspace_bytes, &fb, st);
+    if (rc != RUBIX_OK) return rc;
+    args.gate = fb.gate;
+    args.split = fb.split;
+    args.chunk = fb.chunk;
+    L.At = fb.At;
+    L.bucket = fb.bucket;
+    L.ct = fb.ct;
+    L.rec = fb.rec;
+    L.slot_cnt = fb.slot_start;
+    L.items = fb.items;
+    L.done = fb.done;
+    L.partials = fb.partials;
+  } else {
     const int rc = cube_prepare(in, L, tune, /*with_grad=*/false, st);
     if (rc != RUBIX_OK) return rc;
   }
-  MainArgs args;
   args.ct = L.ct;
   args.wave_z = ssp_wave_z;
   args.nZ = n_met;
@@ -1039,7 +1087,6 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
   args.row_cap = row_cap;
   args.staged = staged;
   args.pool = pool;
-  args.chunk = tune.chunk;
   args.lsf_k = n_lsf_taps;
   args.lsf_crop = lsf_crop;
   for (int i = 0; i <= kMaxLsfTaps; ++i) args.lsf[i] = i < n_lsf_taps ? lsf_taps[i] : 0.f;
@@ -1070,7 +1117,7 @@ int cube_fwd_named(const char* who, const float* ssp_flux, const float* ssp_meta
   return cube_fwd_impl(who, ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, n_met, n_age,
                        n_wave, wave_t, n_wave_t, mass, metallicity, age, velocity, vel_stride,
                        vel_component, perm, seg_offsets, n_segments, n, lsf_taps, n_lsf_taps,
-                       lsf_crop, nullptr, nullptr, cube, spaxel_stride, workspace,
+                       lsf_crop, true, nullptr, nullptr, cube, spaxel_stride, workspace,
                        workspace_bytes, stream);
 }
 
@@ -1089,8 +1136,33 @@ extern "C" int rubix_cube_fwd(const float* ssp_flux, const float* ssp_metallicit
   return cube_fwd_impl("rubix_cube_fwd", ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, n_met,
                        n_age, n_wave, wave_t, n_wave_t, mass, metallicity, age, velocity,
                        vel_stride, vel_component, perm, seg_offsets, n_segments, n, lsf_taps,
-                       n_lsf_taps, lsf_crop, nullptr, nullptr, cube, spaxel_stride, workspace,
+                       n_lsf_taps, lsf_crop, true, nullptr, nullptr, cube, spaxel_stride, workspace,
                        workspace_bytes, stream);
+}
+
+extern "C" size_t rubix_cube_general_workspace_size(int64_t n, int32_t n_segments,
+                                                    int32_t n_wave_t, int32_t n_met,
+                                                    int32_t n_age, int32_t n_wave) {
+  if (n < 0 || n_segments < 0 || n_wave_t < 0 || n_met < 0 || n_age < 0 || n_wave < 0) return 0;
+  return cube_general_workspace(n, n_segments, n_wave_t, n_met, n_age, n_wave);
+}
+
+extern "C" int rubix_cube_fwd_general(const float* ssp_flux, const float* ssp_metallicity,
+                                      const float* ssp_age, const float* ssp_wave_z,
+                                      int32_t n_met, int32_t n_age, int32_t n_wave,
+                                      const float* wave_t, int32_t n_wave_t, const float* mass,
+                                      const float* metallicity, const float* age,
+                                      const float* velocity, int64_t vel_stride,
+                                      int32_t vel_component, const int32_t* perm,
+                                      const int32_t* seg_offsets, int32_t n_segments, int64_t n,
+                                      const float* lsf_taps, int32_t n_lsf_taps,
+                                      int32_t lsf_crop, float* cube, int64_t spaxel_stride,
+                                      void* workspace, size_t workspace_bytes, void* stream) {
+  return cube_fwd_impl("rubix_cube_fwd_general", ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z,
+                       n_met, n_age, n_wave, wave_t, n_wave_t, mass, metallicity, age, velocity,
+                       vel_stride, vel_component, perm, seg_offsets, n_segments, n, lsf_taps,
+                       n_lsf_taps, lsf_crop, false, nullptr, nullptr, cube, spaxel_stride,
+                       workspace, workspace_bytes, stream);
 }
 
 extern "C" int rubix_cube_fwd_dust(const float* ssp_flux, const float* ssp_metallicity,
@@ -1109,7 +1181,7 @@ extern "C" int rubix_cube_fwd_dust(const float* ssp_flux, const float* ssp_metal
   return cube_fwd_impl("rubix_cube_fwd_dust", ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z,
                        n_met, n_age, n_wave, wave_t, n_wave_t, mass, metallicity, age, velocity,
                        vel_stride, vel_component, perm, seg_offsets, n_segments, n, lsf_taps,
-                       n_lsf_taps, lsf_crop, av, ext_exponent, cube, spaxel_stride, workspace,
+                       n_lsf_taps, lsf_crop, false, av, ext_exponent, cube, spaxel_stride, workspace,
                        workspace_bytes, stream);
 }
 

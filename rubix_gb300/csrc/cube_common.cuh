@@ -17,19 +17,6 @@ struct CubeTuning {
 };
 CubeTuning cube_tuning_current();  // of the current device
 
-namespace {
-
-constexpr int kAccThreads = 384;  // forward kernel: 2 blocks of 12 warps per SM
-constexpr int kAccWarps = kAccThreads / 32;
-constexpr int kPB = 2;          // staging/row pools of the forward kernel: kPB full rows
-constexpr int kMaxChunk = 256;  // largest work item (particles); records staged per item
-constexpr int kMinChunk = 32;
-constexpr int kBuckets = 1024;  // log-wavelength bucket table entries
-constexpr double kVmaxKms = 10000.0;  // bucket table and one-step-walk check sized for this
-constexpr int kMaxWaveT = 4096;  // telescope wavelengths per spectrum
-constexpr int kGenericFlag = 1 << 30;  // in rec.b.z: particle needs the general walk
-constexpr int kMaxLsfTaps = 63;
-
 struct CubeCtrl {
   int next_item;
   int n_items;
@@ -48,6 +35,42 @@ struct ParticleRec {  // 48 bytes, three vector loads
   float4 c;  // T = in-range flux sum of the mixed template, dT/dZ, dT/dage (gradient
              // passes only), A_V of the dust in front of the particle (0 without dust)
 };
+
+// Everything the setup passes read: the SSP grid, the telescope grid and the
+// spaxel-sorted particles.
+struct CubeInputs {
+  const float* ssp_flux;
+  const float* ssp_met;
+  const float* ssp_age;
+  const float* ssp_wave_z;
+  int n_met, n_age, n_wave;
+  const float* wave_t;
+  int n_wave_t;
+  const float* mass;
+  const float* met;
+  const float* age;
+  const float* vel;
+  long long vel_stride;
+  int vel_comp;
+  const int* perm;
+  const int* seg_off;
+  int n_seg;
+  long long n;
+  const float* av = nullptr;  // per-particle A_V (dust), input order; nullptr: none
+};
+
+namespace {
+
+constexpr int kAccThreads = 384;  // forward kernel: 2 blocks of 12 warps per SM
+constexpr int kAccWarps = kAccThreads / 32;
+constexpr int kPB = 2;          // staging/row pools of the forward kernel: kPB full rows
+constexpr int kMaxChunk = 256;  // largest work item (particles); records staged per item
+constexpr int kMinChunk = 32;
+constexpr int kBuckets = 1024;  // log-wavelength bucket table entries
+constexpr double kVmaxKms = 10000.0;  // bucket table and one-step-walk check sized for this
+constexpr int kMaxWaveT = 4096;  // telescope wavelengths per spectrum
+constexpr int kGenericFlag = 1 << 30;  // in rec.b.z: particle needs the general walk
+constexpr int kMaxLsfTaps = 63;
 
 __device__ __forceinline__ int count_le_scaled(const float* __restrict__ wz, int n, float alpha,
                                                float q) {
@@ -76,6 +99,21 @@ __device__ __forceinline__ void bucket_params(const float* wave_t, int n_t, doub
   const double hi = log((double)wave_t[n_t - 1]) + kVmaxKms / c;
   h = (hi - lnq0) / (double)(kBuckets - 2);
   if (!(h > 0.0)) h = 1e-6;
+}
+
+// Bucket b covers u in [b - 0.5, b + 0.5) (round-to-nearest lookup).
+__device__ __forceinline__ int2 bucket_entry(const float* __restrict__ wave_z, int n_wave,
+                                             double lnq0, double h, int b) {
+  const double q = exp(lnq0 + ((double)b - 0.5) * h);
+  int lo = 0, hi = n_wave;
+  while (lo < hi) {
+    int mid = (lo + hi) >> 1;
+    if ((double)wave_z[mid] <= q) lo = mid + 1; else hi = mid;
+  }
+  const int k0 = lo - 1;
+  float thr = 3.0e38f;
+  if (k0 + 1 < n_wave) thr = (float)((log((double)wave_z[k0 + 1]) - lnq0) / h);
+  return make_int2(k0, __float_as_int(thr));
 }
 
 // Bucket table over log(q), per-wavelength bucket coordinates A_t, and the spacing
@@ -115,25 +153,13 @@ __global__ void cube_setup_kernel(const float* __restrict__ wave_z, int n_wave,
       atomicMin(&ctrl->dz_min_bits, __float_as_uint(d));
     }
   }
-  for (int b = gtid; b < kBuckets; b += gsz) {
-    // Bucket b covers u in [b - 0.5, b + 0.5) (round-to-nearest lookup).
-    const double q = exp(lnq0 + ((double)b - 0.5) * h);
-    int lo = 0, hi = n_wave;
-    while (lo < hi) {
-      int mid = (lo + hi) >> 1;
-      if ((double)wave_z[mid] <= q) lo = mid + 1; else hi = mid;
-    }
-    const int k0 = lo - 1;
-    float thr = 3.0e38f;
-    if (k0 + 1 < n_wave) thr = (float)((log((double)wave_z[k0 + 1]) - lnq0) / h);
-    bucket[b] = make_int2(k0, __float_as_int(thr));
-  }
+  for (int b = gtid; b < kBuckets; b += gsz) bucket[b] = bucket_entry(wave_z, n_wave, lnq0, h, b);
 }
 
 // Corner table: ct[(iz*(nA-1) + ia)*nW + k] = (F[iz][ia][k], F[iz+1][ia][k],
 // F[iz][ia+1][k], F[iz+1][ia+1][k]).
-__global__ void cube_corner_table_kernel(const float* __restrict__ flux, int nZ, int nA,
-                                         int nW, float4* __restrict__ ct) {
+__device__ __forceinline__ void corner_table(const float* __restrict__ flux, int nZ, int nA,
+                                             int nW, float4* __restrict__ ct) {
   const long long total = (long long)(nZ - 1) * (nA - 1) * nW;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -144,6 +170,11 @@ __global__ void cube_corner_table_kernel(const float* __restrict__ flux, int nZ,
     const long long b10 = b00 + (long long)nA * nW;
     ct[i] = make_float4(flux[b00], flux[b10], flux[b00 + nW], flux[b10 + nW]);
   }
+}
+
+__global__ void cube_corner_table_kernel(const float* __restrict__ flux, int nZ, int nA,
+                                         int nW, float4* __restrict__ ct) {
+  corner_table(flux, nZ, nA, nW, ct);
 }
 
 // prefix[r][k] = sum_{k'=1..k} F[r][k'] * (lambda_z,k' - lambda_z,k'-1) for every SSP row
@@ -157,55 +188,54 @@ constexpr int kPrefixThreads = 128;
 // Per SSP row r: prefix[r][k] = sum_{j=1..k} F[r][j] (lambda_z[j] - lambda_z[j-1]) in
 // float64.  One block per row: each thread sums a run of consecutive entries, a block
 // scan of the run totals gives each run's offset, and the run is written out.
-__global__ void __launch_bounds__(kPrefixThreads) cube_prefix_kernel(
-    const float* __restrict__ flux, int rows, int nW, const float* __restrict__ wave_z,
-    double* __restrict__ prefix) {
+__device__ __forceinline__ void prefix_row(const float* __restrict__ flux, int r, int nW,
+                                           const float* __restrict__ wave_z,
+                                           double* __restrict__ prefix) {
   __shared__ double s_warp[kPrefixThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int per = (nW + kPrefixThreads - 1) / kPrefixThreads;
   const int k0 = threadIdx.x * per;
   const int k1 = min(k0 + per, nW);
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    const float* f = flux + (long long)r * nW;
-    double* o = prefix + (long long)r * nW;
-    double sum = 0.0;
-    for (int k = max(k0, 1); k < k1; ++k) sum += (double)f[k] * (double)(wave_z[k] - wave_z[k - 1]);
-    double x = sum;  // inclusive scan over the block's runs
+  const float* f = flux + (long long)r * nW;
+  double* o = prefix + (long long)r * nW;
+  double sum = 0.0;
+  for (int k = max(k0, 1); k < k1; ++k) sum += (double)f[k] * (double)(wave_z[k] - wave_z[k - 1]);
+  double x = sum;  // inclusive scan over the block's runs
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const double y = __shfl_up_sync(0xffffffffu, x, d);
-      if (lane >= d) x += y;
-    }
-    if (lane == 31) s_warp[warp] = x;
-    __syncthreads();
-    double run = x - sum;
-    for (int w = 0; w < warp; ++w) run += s_warp[w];
-    for (int k = k0; k < k1; ++k) {
-      if (k >= 1) run += (double)f[k] * (double)(wave_z[k] - wave_z[k - 1]);
-      o[k] = run;
-    }
-    __syncthreads();  // s_warp is reused by the next row
+  for (int d = 1; d < 32; d <<= 1) {
+    const double y = __shfl_up_sync(0xffffffffu, x, d);
+    if (lane >= d) x += y;
   }
+  if (lane == 31) s_warp[warp] = x;
+  __syncthreads();
+  double run = x - sum;
+  for (int w = 0; w < warp; ++w) run += s_warp[w];
+  for (int k = k0; k < k1; ++k) {
+    if (k >= 1) run += (double)f[k] * (double)(wave_z[k] - wave_z[k - 1]);
+    o[k] = run;
+  }
+  __syncthreads();  // s_warp is reused by the next row
 }
 
-__global__ void cube_gather_kernel(const float* __restrict__ mass, const float* __restrict__ met,
-                                   const float* __restrict__ age, const float* __restrict__ vel,
-                                   long long vel_stride, int vel_comp,
-                                   const int* __restrict__ perm, const int* __restrict__ seg_off,
-                                   int n_seg, long long n, const float* __restrict__ zg, int nZ,
-                                   const float* __restrict__ ag, int nA,
-                                   const float* __restrict__ wave_z, int n_wave,
-                                   const float* __restrict__ wave_t, int n_t,
-                                   const double* __restrict__ prefix,
-                                   const CubeCtrl* __restrict__ ctrl,
-                                   ParticleRec* __restrict__ rec, int with_grad,
-                                   const float* __restrict__ av, float alo, float ahi) {
+__global__ void __launch_bounds__(kPrefixThreads) cube_prefix_kernel(
+    const float* __restrict__ flux, int rows, int nW, const float* __restrict__ wave_z,
+    double* __restrict__ prefix) {
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) prefix_row(flux, r, nW, wave_z, prefix);
+}
+
+// dz, dt: smallest SSP spacing near the telescope range and widest telescope bin.
+__device__ __forceinline__ void gather_records(
+    const float* __restrict__ mass, const float* __restrict__ met,
+    const float* __restrict__ age, const float* __restrict__ vel, long long vel_stride,
+    int vel_comp, const int* __restrict__ perm, const int* __restrict__ seg_off, int n_seg,
+    long long n, const float* __restrict__ zg, int nZ, const float* __restrict__ ag, int nA,
+    const float* __restrict__ wave_z, int n_wave, const float* __restrict__ wave_t, int n_t,
+    const double* __restrict__ prefix, double inv_h, float bmax, float dz, float dt,
+    ParticleRec* __restrict__ rec, int with_grad, const float* __restrict__ av, float alo,
+    float ahi) {
   const long long n_valid = seg_off[n_seg];
   const float t_lo = wave_t[0], t_hi = wave_t[n_t - 1];
-  const double inv_h = ctrl->inv_h;
-  const float bmax = ctrl->bmax;
   // lambda' spacing >= alpha*dz minus two float32 roundings of lambda' (|lambda'| < 2^14)
-  const float dz = __uint_as_float(ctrl->dz_min_bits), dt = __uint_as_float(ctrl->dt_max_bits);
   const bool coarse_ok = dz * alo - 4.0e-3f > dt;
   for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n && j < n_valid;
        j += (long long)gridDim.x * blockDim.x) {
@@ -267,6 +297,24 @@ __global__ void cube_gather_kernel(const float* __restrict__ mass, const float* 
     r.c = make_float4(T, (float)TZ, (float)TA, av ? av[i] : 0.f);
     rec[j] = r;
   }
+}
+
+__global__ void cube_gather_kernel(const float* __restrict__ mass, const float* __restrict__ met,
+                                   const float* __restrict__ age, const float* __restrict__ vel,
+                                   long long vel_stride, int vel_comp,
+                                   const int* __restrict__ perm, const int* __restrict__ seg_off,
+                                   int n_seg, long long n, const float* __restrict__ zg, int nZ,
+                                   const float* __restrict__ ag, int nA,
+                                   const float* __restrict__ wave_z, int n_wave,
+                                   const float* __restrict__ wave_t, int n_t,
+                                   const double* __restrict__ prefix,
+                                   const CubeCtrl* __restrict__ ctrl,
+                                   ParticleRec* __restrict__ rec, int with_grad,
+                                   const float* __restrict__ av, float alo, float ahi) {
+  gather_records(mass, met, age, vel, vel_stride, vel_comp, perm, seg_off, n_seg, n, zg, nZ, ag,
+                 nA, wave_z, n_wave, wave_t, n_t, prefix, ctrl->inv_h, ctrl->bmax,
+                 __uint_as_float(ctrl->dz_min_bits), __uint_as_float(ctrl->dt_max_bits), rec,
+                 with_grad, av, alo, ahi);
 }
 
 // Per spaxel: chunk count.  Multi-chunk spaxels get one item (and partial slot) per
@@ -344,32 +392,6 @@ CubeLayout carve_cube(void* ws, long long n, int n_seg, int n_t, int nZ, int nA,
   L.bytes = c.off;
   return L;
 }
-
-// Work-item tuning of the cube kernels (set per device through rubix_cube_tuning_set;
-// defined in tuning.cu).
-
-// Everything the setup passes read: the SSP grid, the telescope grid and the
-// spaxel-sorted particles.
-struct CubeInputs {
-  const float* ssp_flux;
-  const float* ssp_met;
-  const float* ssp_age;
-  const float* ssp_wave_z;
-  int n_met, n_age, n_wave;
-  const float* wave_t;
-  int n_wave_t;
-  const float* mass;
-  const float* met;
-  const float* age;
-  const float* vel;
-  long long vel_stride;
-  int vel_comp;
-  const int* perm;
-  const int* seg_off;
-  int n_seg;
-  long long n;
-  const float* av = nullptr;  // per-particle A_V (dust), input order; nullptr: none
-};
 
 // Launches the setup passes into the carved workspace: bucket table, corner table,
 // prefix sums, particle records (with dT/dZ, dT/dage when with_grad) and the work-item

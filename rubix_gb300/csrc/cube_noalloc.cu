@@ -29,7 +29,7 @@
 //   * rubix_cube_noalloc_status reads the device error word of the last call (a bounded
 //     shared-memory copy wait that gave up leaves an invalid cube).
 //   * No call here allocates or frees device memory.
-#include "common.cuh"
+#include "cube_nodes.cuh"
 
 #include <cuda.h>  // CUcontext / CUresult types; the functions come through the runtime
 
@@ -158,7 +158,7 @@ extern "C" int rubix_cube_fwd_noalloc(const float* ssp_flux, const float* ssp_me
                                       lsf_crop, cube, spaxel_stride, &nothing_to_do);
   if (rc != RUBIX_OK || nothing_to_do) return rc;
   const size_t need =
-      rubix_cube_workspace_size(n, n_segments, n_wave_t, n_met, n_age, n_wave);
+      rubix::cube_general_workspace(n, n_segments, n_wave_t, n_met, n_age, n_wave);
   RUBIX_REQUIRE(need <= (size_t)RUBIX_CUBE_NOALLOC_SCRATCH_BYTES, RUBIX_E_WORKSPACE,
                 "%s: this problem needs %zu bytes of scratch but the static array holds "
                 "%zu; use rubix_cube_fwd with a caller workspace",

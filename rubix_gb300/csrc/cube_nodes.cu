@@ -1,0 +1,1372 @@
+// The datacube accumulated node by node: the forward of kernel (b) for template grids
+// that fit an SM's shared memory, wavelength slice by wavelength slice.
+//
+// A particle adds beta * I(x_t) to its spaxel, with I the piecewise-linear interpolant of
+// its mixed template on the shifted grid lambda'_k = fl32(lambda_z,k * alpha) and
+// beta = m T / T' (rubix/spectra/ifu.py:224-266).  Two properties of the path make the
+// work per particle proportional to the SSP nodes inside the telescope range (737 at
+// MUSE's 3721 bins on a 1221-node template) instead of to the telescope bins:
+//
+//   * T' = sum_t I_t dlambda_t is linear in the template, T' = sum_c w_c H_c(alpha) over
+//     the four corners c, and H_c(alpha) is smooth in alpha.  H is tabulated at
+//     alpha_i = 1 + i 2^-18 (1.1 km/s apart, exact in float32) for every template by one
+//     small matrix product and interpolated linearly: 2e-8 of T' rms on the synthetic
+//     templates (lines of 45 % depth, 2-8 A wide), below float32 rounding.  beta is then
+//     known before any spectrum is formed.
+//   * Inside one SSP interval the particle's spectrum is A + B (x - x_j).  A lane owns an
+//     SSP node; while alpha moves by less than one telescope bin the samples strictly
+//     between two nodes stay the same, so the lane sums (A, B) of its interval over all
+//     particles in registers and only the sample at the node itself needs a choice of
+//     side.  The sums are spread over the 4-5 samples of the interval once per group of
+//     particles instead of once per particle.
+//
+// Measured (221 x 6 x 1221 templates, 3721 samples, LSF fused, one GB300): 10^7 particles on
+// 300 x 300 spaxels, whole render 12.9 ms against 40.2 ms with every particle evaluated at
+// every sample (this file's slice kernel ~8.5 ms of it, cube_main_kernel 38.5 ms); 10^6 on
+// 150 x 150, 1.75 ms against 4.46 ms.  Relative 2-norm error against float64 7.6e-8, as before.
+//
+// Stages (one launch each): grid extrema and the velocity range; prefix sums of the
+// templates and the resampling weights at alpha_i; H; the work-item list; records of
+// every item sorted by alpha; the slice kernel; the merge of the slices (and chunks) of a
+// spaxel with the optional LSF.  A spaxel with any particle that the tables do not cover
+// (a shifted grid that does not span the telescope range, |v| above 2300 km/s, values
+// that are not finite or that may overflow) is flagged and left to cube_main_kernel, as
+// is everything when the grids themselves do not qualify.  Every decision depends on the
+// configuration and the spaxel's own particles only, so a spaxel's result does not depend
+// on what else is rendered with it.
+#include "cube_nodes.cuh"
+
+#include <type_traits>
+
+namespace rubix {
+namespace {
+
+constexpr int kExt = 512;        // virtual telescope samples on either side
+constexpr int kMaxBins = 224;    // samples of one (item, slice) row: 7 per lane
+constexpr int kWin = 768;        // samples of a slice's window over all alpha
+constexpr int kMaxSlices = 128;
+constexpr int kMaxWaves = 64;
+constexpr int kSub = 256;        // particles sorted together
+constexpr int kItem = 4 * kSub;  // particles of a work item
+constexpr int kAlphaBits = 18;
+constexpr float kAlphaStep = 1.0f / (1 << kAlphaBits);
+constexpr int kAlphaHalf = 2048;                       // alpha rows on either side of 1
+constexpr float kAlphaMax = 2040.f * kAlphaStep;       // |alpha - 1| covered (2333 km/s)
+constexpr int kAlphaTile = 64;                         // rows computed together
+constexpr int kAlphaTiles = 2 * kAlphaHalf / kAlphaTile + 1;
+constexpr int kAlphaRows = kAlphaTiles * kAlphaTile;
+constexpr int kNodeWarps = 20;
+constexpr int kNodeThreads = 32 * kNodeWarps;
+constexpr int kStage = 33;       // staged records of a warp: 32 and one of weight zero
+constexpr int kRuns = 4;
+
+struct NodeCtrl {
+  int flagged;                  // some spaxel is left to cube_main_kernel
+  int left[2];                  // its work items there: of several-chunk spaxels, of others
+  unsigned tile_mask[(kAlphaTiles + 31) / 32];
+  unsigned dz_inv, dt_inv;      // ~bits of the smallest SSP / telescope spacing
+  unsigned dz_max, dt_max;      // bits of the largest (3e38: not ascending)
+  unsigned run_max[kRuns], run_min_inv[kRuns];  // extent of own_nodes(r) + 1, + 0 intervals
+  int k_first;                  // 1 + node below the telescope range at any alpha
+  int k_last_inv;               // n_wave - node above it
+  unsigned fmax;                // bits of max |flux| (above inf: NaN)
+  int n_items, n_multi;         // work items with particles; those of several-item spaxels
+  int next[kMaxWaves][kMaxSlices];
+};
+
+// A slice has 32, 16, 8 or 4 nodes; all but its first and last are its own.
+__host__ __device__ constexpr int own_nodes(int r) { return (32 >> r) - 2; }
+
+// Slices that the workspace provides rows for.
+__host__ __device__ inline int max_slices_of(int n_wave) {
+  const int s = (n_wave + 30) / 31 + 1;
+  return s > kMaxSlices ? kMaxSlices : (s < 48 ? 48 : s);
+}
+
+struct NodePlan {
+  int ok;
+  int k_first, n_own, n_slices;  // first node, nodes of a slice
+  int w;                         // samples that a node may cross within a group of particles
+  float dt_min, window;          // samples that an item's alpha range may span
+};
+
+// How the grids are cut into slices, from the extrema; every block derives the same plan.
+__device__ __forceinline__ NodePlan node_plan(const NodeCtrl* c, int n_wave, float x_last) {
+  NodePlan p;
+  const float dz = __uint_as_float(~c->dz_inv), dt = __uint_as_float(~c->dt_inv);
+  const float dtm = __uint_as_float(c->dt_max), fm = __uint_as_float(c->fmax);
+  p.k_first = max(c->k_first - 1, 0);
+  const int k_last = min(n_wave - c->k_last_inv, n_wave - 1);
+  p.dt_min = dt;
+  p.ok = 0;
+  p.n_own = 0;
+  p.w = 1;
+  p.n_slices = 0;
+  p.window = 0.f;
+  // lambda' spacing >= alpha*dz minus two roundings of lambda' (|lambda'| < 2^14): at
+  // least one sample between two nodes; float32 exact enough to order samples and nodes
+  if (!(dz * (1.f - kAlphaMax) - 4.0e-3f > dtm) || !(dt > 2.0e-2f) || !(dtm < 1e30f) ||
+      !(__uint_as_float(c->dz_max) < 1e30f) || !(x_last < 16384.f) || !(fm < 1e30f) ||
+      k_last <= p.k_first)
+    return p;
+  const float ratio = (dz * (1.f - kAlphaMax) - 4.0e-3f) / dtm;
+  p.w = ratio > 2.f ? 2 : 1;
+  const float swing = 2.f * kAlphaMax * x_last / dt;  // samples a node moves over all alpha
+  for (int r = 0; r < kRuns; ++r) {
+    const float hi = __uint_as_float(c->run_max[r]) * (1.f + kAlphaMax) / dt;
+    const float lo = __uint_as_float(~c->run_min_inv[r]) * (1.f - kAlphaMax) / dtm;
+    const float win = fminf((float)kMaxBins - hi, lo) - 4.f;
+    if (win < 24.f || hi + swing + 8.f > (float)(kExt - 16) ||
+        hi + swing + 8.f > (float)(kWin - 8))
+      continue;
+    p.n_own = own_nodes(r);
+    p.window = win;
+    p.n_slices = (k_last - p.k_first + p.n_own - 1) / p.n_own;
+    p.ok = p.n_slices <= max_slices_of(n_wave);
+    return p;
+  }
+  return p;
+}
+
+// SSP wavelength k, continued with the end spacings beyond the grid.
+__device__ __forceinline__ float lam_ext(const float* __restrict__ wz, int n, int k) {
+  if (k < 0) return wz[0] + (float)k * (wz[1] - wz[0]);
+  if (k >= n) return wz[n - 1] + (float)(k - n + 1) * (wz[n - 1] - wz[n - 2]);
+  return wz[k];
+}
+
+// Telescope sample e of the extended grid (e = t + kExt), continued with the end spacings.
+__device__ __forceinline__ float x_ext(const float* __restrict__ wt, int n, int e) {
+  const int t = e - kExt;
+  if (t < 0) return wt[0] + (float)t * (wt[1] - wt[0]);
+  if (t >= n) return wt[n - 1] + (float)(t - n + 1) * (wt[n - 1] - wt[n - 2]);
+  return wt[t];
+}
+
+// Grid extrema, and the rows of alpha that the particles' velocities fall on.
+__global__ void __launch_bounds__(256) node_setup_kernel(
+    const float* __restrict__ wz, int n_wave, const float* __restrict__ wt, int n_t,
+    const float* __restrict__ vel, long long vel_stride, int vel_comp, long long n,
+    NodeCtrl* __restrict__ ctrl) {
+  const long long gtid = blockIdx.x * 256LL + threadIdx.x, gsz = gridDim.x * 256LL;
+  if (gtid < n_t - 1) {
+    float d = wt[gtid + 1] - wt[gtid];
+    const bool bad = !(d > 0.f);
+    atomicMax(&ctrl->dt_max, bad ? __float_as_uint(3e38f) : __float_as_uint(d));
+    if (!bad) atomicMax(&ctrl->dt_inv, ~__float_as_uint(d));
+  }
+  const float x0 = wt[0], x1 = wt[n_t - 1];
+  const float hi = 1.f + kAlphaMax, lo = 1.f - kAlphaMax;
+  if (gtid < n_wave - 1) {
+    const int k = (int)gtid;
+    const float a = wz[k], b = wz[k + 1];
+    if (a * hi <= x0 && !(b * hi <= x0)) ctrl->k_first = k + 1;
+    if (!(a * lo > x1) && b * lo > x1) ctrl->k_last_inv = n_wave - (k + 1);
+    const float d = b - a;
+    const bool bad = !(d > 0.f);
+    const bool seen = bad || (b * 1.05f >= x0 && a * 0.95f <= x1);
+    if (seen) {
+      atomicMax(&ctrl->dz_max, bad ? __float_as_uint(3e38f) : __float_as_uint(d));
+      atomicMax(&ctrl->dz_inv, ~__float_as_uint(bad ? 0.f : d));
+    }
+#pragma unroll
+    for (int r = 0; r < kRuns; ++r) {
+      const float e0 = lam_ext(wz, n_wave, k + own_nodes(r)) - a;
+      const float e1 = lam_ext(wz, n_wave, k + own_nodes(r) + 1) - a;
+      if (seen && e0 >= 0.f && e1 >= 0.f) {
+        atomicMax(&ctrl->run_max[r], __float_as_uint(e1));
+        atomicMax(&ctrl->run_min_inv[r], ~__float_as_uint(e0));
+      }
+    }
+  }
+  __shared__ unsigned s_mask[(kAlphaTiles + 31) / 32];
+  if (threadIdx.x < (kAlphaTiles + 31) / 32) s_mask[threadIdx.x] = 0u;
+  __syncthreads();
+  int last = -1;
+  for (long long i = gtid; i < n; i += gsz) {
+    // alpha - 1 to ~1e-7: the rows on either side of it are marked
+    const float z = vel[i * vel_stride + vel_comp] * (float)(1.0 / kSpeedOfLight);
+    const float am1 = z * (1.f + 0.5f * z * (1.f + (1.f / 3.f) * z));
+    if (!(fabsf(am1) <= kAlphaMax)) continue;
+    const int r = (int)floorf(am1 * (float)(1 << kAlphaBits)) + kAlphaHalf;
+    const int a = max(r - 1, 0) / kAlphaTile, b = min(r + 2, kAlphaRows - 1) / kAlphaTile;
+    if (a != last) atomicOr(&s_mask[a >> 5], 1u << (a & 31));
+    if (b != a) atomicOr(&s_mask[b >> 5], 1u << (b & 31));
+    last = a;
+  }
+  __syncthreads();
+  if (threadIdx.x < (kAlphaTiles + 31) / 32 && s_mask[threadIdx.x])
+    atomicOr(&ctrl->tile_mask[threadIdx.x], s_mask[threadIdx.x]);
+}
+
+__device__ __forceinline__ bool tile_used(const NodeCtrl* c, int tile) {
+  return (c->tile_mask[tile >> 5] >> (tile & 31)) & 1u;
+}
+
+// The two resampling weights that interval [k, k + 1] gives its nodes at one alpha: the
+// samples x_t inside it at distance d from node k weigh dx_t (1 - d / len) and dx_t d / len.
+// The nodes are lambda_z * alpha unrounded, as float pairs; the few samples of an interval
+// are summed directly.
+__device__ __forceinline__ float2 interval_weights(const float* __restrict__ wz,
+                                                   const float* __restrict__ wt, int n_t, int k,
+                                                   float alpha, float x0, float inv) {
+  const float z0 = wz[k], z1 = wz[k + 1];
+  const float ah = __fmul_rn(z0, alpha), al = fmaf(z0, alpha, -ah);
+  const float bh = __fmul_rn(z1, alpha), bl = fmaf(z1, alpha, -bh);
+  int t = min(max((int)((ah - x0) * inv), 0), n_t - 1);
+  while (t > 0 && (wt[t - 1] - ah) - al >= 0.f) --t;
+  while (t < n_t && (wt[t] - ah) - al < 0.f) ++t;
+  float s0 = 0.f, s1 = 0.f, prev = t > 0 ? wt[t - 1] : x0;
+  for (; t < n_t; ++t) {
+    const float x = wt[t];
+    if ((x - bh) - bl >= 0.f) break;
+    const float dx = t > 0 ? x - prev : 0.f;
+    s0 += dx;
+    s1 = fmaf(dx, (x - ah) - al, s1);
+    prev = x;
+  }
+  const float rise = s1 / ((bh - ah) + (bl - al));
+  return make_float2(s0 - rise, rise);
+}
+
+constexpr int kWeightBlocks = 1024;
+
+// Per template: float64 prefix sums (block b < rows, as cube_prefix_kernel) and max |F|.
+// The remaining blocks: the resampling weights of T' at alpha_i, h_k = sum_t dlambda_t
+// hat_k(x_t) with hat_k the hat function of node k, one alpha row of a used tile at a time.
+// Nodes are stored from k_first on, kpad to a row, zero beyond the last.
+__global__ void __launch_bounds__(kPrefixThreads) node_tables_kernel(
+    const float* __restrict__ flux, int rows, int n_wave, const float* __restrict__ wz,
+    const float* __restrict__ wt, int n_t, double* __restrict__ prefix, float* __restrict__ h,
+    int kpad, NodeCtrl* __restrict__ ctrl) {
+  if ((int)blockIdx.x < rows) {
+    prefix_row(flux, blockIdx.x, n_wave, wz, prefix);
+    const float* f = flux + (long long)blockIdx.x * n_wave;
+    unsigned m = 0u;
+    for (int k = threadIdx.x; k < n_wave; k += kPrefixThreads)
+      m = max(m, __float_as_uint(f[k]) & 0x7fffffffu);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) atomicMax(&ctrl->fmax, m);
+    return;
+  }
+  __shared__ float s_rise[kPrefixThreads + 1];
+  const int tid = threadIdx.x;
+  // the grid's node range (fmax, still being formed, only decides whether it is used)
+  const int k_first = max(ctrl->k_first - 1, 0);
+  const int count = min(n_wave - ctrl->k_last_inv, n_wave - 1) - k_first + 1;
+  const float x0 = wt[0], inv = (float)(n_t - 1) / (wt[n_t - 1] - x0);
+  for (int u = blockIdx.x - rows;; u += kWeightBlocks) {
+    // row u of the used tiles
+    int tile = 0, left = u / kAlphaTile;
+    while (tile < kAlphaTiles && (!tile_used(ctrl, tile) || left-- > 0)) ++tile;
+    if (tile == kAlphaTiles) return;
+    const int row = tile * kAlphaTile + u % kAlphaTile;
+    const float alpha = 1.f + (float)(row - kAlphaHalf) * kAlphaStep;  // exact
+    if (tid == 0) s_rise[0] = 0.f;
+    for (int q0 = 0; q0 < kpad; q0 += kPrefixThreads) {
+      const int q = q0 + tid;
+      float2 w = make_float2(0.f, 0.f);
+      if (q < count - 1) w = interval_weights(wz, wt, n_t, k_first + q, alpha, x0, inv);
+      s_rise[tid + 1] = w.y;
+      __syncthreads();
+      if (q < kpad) h[(long long)row * kpad + q] = w.x + s_rise[tid];
+      __syncthreads();
+      if (tid == kPrefixThreads - 1) s_rise[0] = w.y;
+    }
+    __syncthreads();
+  }
+}
+
+// H[i][c] = sum_k h[i][k] F[c][k]: 64 alpha rows x 32 templates per block of 128 threads,
+// 4 x 4 per thread, 32 nodes staged at a time.  Sums of 32 products are added with Kahan's
+// compensation: a plain float32 sum over ~740 nodes would be 5e-7 off, this one is 1e-8.
+// Bound by FMA issue: 1 GFMA for 1025 rows of a 1326-template grid, 40 TFMA/s on the chip.
+__global__ void __launch_bounds__(128) node_table_product_kernel(
+    const float* __restrict__ h, int kpad, const float* __restrict__ flux, int n_templ,
+    int n_wave, const float* __restrict__ wt, int n_t, const NodeCtrl* __restrict__ ctrl,
+    float* __restrict__ H) {
+  constexpr int BK = 32, BM = kAlphaTile, BN = 32;
+  const int tile = blockIdx.y;
+  if (!tile_used(ctrl, tile)) return;
+  const NodePlan p = node_plan(ctrl, n_wave, wt[n_t - 1]);
+  if (!p.ok) return;
+  const int k_last = min(n_wave - ctrl->k_last_inv, n_wave - 1);
+  const int K = min(k_last - p.k_first + 1, kpad);
+  __shared__ float sa[2][BK][BM + 4];
+  __shared__ float sb[2][BK][BN + 4];
+  const int tid = threadIdx.x;
+  const int r0 = tile * BM, c0 = blockIdx.x * BN;
+  const int tr = (tid >> 3) * 4, tc = (tid & 7) * 4;
+  // loads: a thread takes 4 consecutive nodes of h in 4 rows, and of F node `lane` in 8
+  const int lr = tid >> 3, lk = (tid & 7) * 4, lane = tid & 31, warp = tid >> 5;
+  float4 ra[4];
+  float rb[8];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      ra[i] = *reinterpret_cast<const float4*>(h + (long long)(r0 + lr + 16 * i) * kpad + k0 + lk);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int c = c0 + warp * 8 + j;
+      rb[j] = (k0 + lane < K && c < n_templ)
+                  ? flux[(long long)c * n_wave + p.k_first + k0 + lane] : 0.f;
+    }
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      sa[buf][lk][lr + 16 * i] = ra[i].x;
+      sa[buf][lk + 1][lr + 16 * i] = ra[i].y;
+      sa[buf][lk + 2][lr + 16 * i] = ra[i].z;
+      sa[buf][lk + 3][lr + 16 * i] = ra[i].w;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sb[buf][lane][warp * 8 + j] = rb[j];
+  };
+  float sum[4][4], comp[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum[i][j] = comp[i][j] = 0.f;
+  const int steps = (K + BK - 1) / BK;  // kpad is a multiple of BK
+  load(0);
+  store(0);
+  __syncthreads();
+  for (int s = 0; s < steps; ++s) {
+    if (s + 1 < steps) load((s + 1) * BK);
+    float acc[4][4];
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      const float4 a = *reinterpret_cast<const float4*>(&sa[s & 1][k][tr]);
+      const float4 b = *reinterpret_cast<const float4*>(&sb[s & 1][k][tc]);
+      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          acc[i][j] = k == 0 ? av[i] * bv[j] : fmaf(av[i], bv[j], acc[i][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float y = acc[i][j] - comp[i][j];
+        const float t = sum[i][j] + y;
+        comp[i][j] = (t - sum[i][j]) - y;
+        sum[i][j] = t;
+      }
+    if (s + 1 < steps) store((s + 1) & 1);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (c0 + tc + j < n_templ) H[(long long)(r0 + tr + i) * n_templ + c0 + tc + j] = sum[i][j];
+}
+
+// Work items: ranges of up to kItem particles of one spaxel; empty spaxels have none.
+// Spaxels of several items first (item index = row), then those with many particles.
+__global__ void node_count_kernel(const int* __restrict__ seg_off, int n_seg, int big,
+                                  int* __restrict__ multi, int* __restrict__ large,
+                                  int* __restrict__ small) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += gridDim.x * blockDim.x) {
+    const int cnt = seg_off[s + 1] - seg_off[s];
+    multi[s] = cnt > kItem ? (cnt + kItem - 1) / kItem : 0;
+    large[s] = (cnt <= kItem && cnt >= big) ? 1 : 0;
+    small[s] = (cnt < big && cnt > 0) ? 1 : 0;
+  }
+}
+
+// Item index of chunk 0 of a spaxel (its chunks follow one another).
+__device__ __forceinline__ int first_item(int s, int cnt, int big, int n_seg,
+                                          const int* __restrict__ multi,
+                                          const int* __restrict__ large,
+                                          const int* __restrict__ small) {
+  if (cnt > kItem) return multi[s];
+  if (cnt >= big) return multi[n_seg] + large[s];
+  return multi[n_seg] + large[n_seg] + small[s];
+}
+
+__global__ void node_fill_items_kernel(const int* __restrict__ seg_off, int n_seg, int big,
+                                       const int* __restrict__ multi,
+                                       const int* __restrict__ large,
+                                       const int* __restrict__ small, int2* __restrict__ items,
+                                       NodeCtrl* __restrict__ ctrl) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += gridDim.x * blockDim.x) {
+    const int cnt = seg_off[s + 1] - seg_off[s];
+    if (cnt == 0) continue;
+    const int i0 = first_item(s, cnt, big, n_seg, multi, large, small);
+    for (int c = 0; c * kItem < cnt; ++c) items[i0 + c] = make_int2(s, c);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctrl->n_multi = multi[n_seg];
+    ctrl->n_items = multi[n_seg] + large[n_seg] + small[n_seg];
+  }
+}
+
+struct GatherArgs {
+  CubeInputs in;
+  const double* prefix;
+  const float* H;
+  NodeCtrl* ctrl;
+  const int2* items;
+  float4* rec_w;
+  float2* rec_a;
+  int* flags;
+  int4* desc;
+};
+
+// One block per work item: the record of each particle (beta times the four corner
+// weights; alpha and the byte offset of its first corner row in the slice table), sorted
+// by alpha within runs of kSub (ties by input order: the order is a function of the
+// spaxel's particles alone).  Latency-bound on the gathers through the permutation.
+__global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
+  __shared__ __align__(16) unsigned s_key[kSub];
+  __shared__ float s_lo[kSub / 32], s_hi[kSub / 32];
+  __shared__ NodePlan s_plan;
+  __shared__ int s_flag;
+  const CubeInputs& in = a.in;
+  const int tid = threadIdx.x;
+  const float x0 = in.wave_t[0], x1 = in.wave_t[in.n_wave_t - 1];
+  if (tid == 0) s_plan = node_plan(a.ctrl, in.n_wave, x1);
+  __syncthreads();
+  const NodePlan plan = s_plan;
+  const float fmax = __uint_as_float(a.ctrl->fmax);
+  const int n_items = a.ctrl->n_items;
+  const int n_templ = in.n_met * in.n_age;
+  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+    const int2 it = a.items[item];
+    const int seg_b = in.seg_off[it.x], seg_e = in.seg_off[it.x + 1];
+    const int jb = seg_b + it.y * kItem;
+    const int je = min(jb + kItem, seg_e);
+    float amin = 2.f, amax = 0.f;
+    if (tid == 0) s_flag = !plan.ok;
+    __syncthreads();
+    for (int j0 = jb; j0 < je && plan.ok; j0 += kSub) {
+      const int m = min(kSub, je - j0);
+      float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+      float alpha = 1.f;
+      int row = 0;
+      bool bad = false;
+      if (tid < m) {
+        const long long i = in.perm[j0 + tid];
+        const float Z = in.met[i], A = in.age[i], mass = in.mass[i];
+        alpha = doppler_factor(in.vel[i * in.vel_stride + in.vel_comp]);
+        const bool outside = (Z < in.ssp_met[0]) || (Z > in.ssp_met[in.n_met - 1]) ||
+                             (A < in.ssp_age[0]) || (A > in.ssp_age[in.n_age - 1]);
+        if (!(fabsf(alpha - 1.f) <= kAlphaMax)) {
+          bad = true;
+          alpha = 1.f;
+        } else if (outside) {
+          bad = !isfinite(mass);  // an all-zero spectrum unless 0 * mass is not 0
+        } else {
+          const int iz = min(max(count_le(in.ssp_met, in.n_met, Z), 1), in.n_met - 1);
+          const int ia = min(max(count_le(in.ssp_age, in.n_age, A), 1), in.n_age - 1);
+          const float dzg = in.ssp_met[iz] - in.ssp_met[iz - 1];
+          const float dag = in.ssp_age[ia] - in.ssp_age[ia - 1];
+          const float tz = dzg == 0.f ? 0.f : (Z - in.ssp_met[iz - 1]) / dzg;
+          const float ta = dag == 0.f ? 0.f : (A - in.ssp_age[ia - 1]) / dag;
+          const int ks = count_le_scaled(in.ssp_wave_z, in.n_wave, alpha, x0) - 1;
+          const int ke = count_le_scaled(in.ssp_wave_z, in.n_wave, alpha, x1) - 1;
+          row = (iz - 1) * in.n_age + (ia - 1);
+          if (ks < 0 || ke + 1 > in.n_wave - 1) {
+            bad = true;
+          } else {
+            const float wc[4] = {(1.f - tz) * (1.f - ta), tz * (1.f - ta), (1.f - tz) * ta,
+                                 tz * ta};
+            const int rr[4] = {row, row + in.n_age, row + 1, row + in.n_age + 1};
+            // T: in-range flux sum, entries ka..kb with x0 <= lambda'_k <= x1, k >= 1
+            int ka = __fmul_rn(in.ssp_wave_z[ks], alpha) >= x0 ? ks : ks + 1;
+            ka = max(ka, 1);
+            float T = 0.f, Tp = 0.f;
+            const float u = (alpha - 1.f) * (float)(1 << kAlphaBits);  // exact
+            const int r = (int)floorf(u) + kAlphaHalf;
+            const float fr = u - floorf(u);
+            const float* h0 = a.H + (long long)r * n_templ;
+            const float* h1 = h0 + n_templ;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const double* pf = a.prefix + (long long)rr[c] * in.n_wave;
+              if (ka <= ke) T = fmaf(wc[c], (float)(pf[ke] - pf[ka - 1]), T);
+              Tp = fmaf(wc[c], fmaf(fr, h1[rr[c]] - h0[rr[c]], h0[rr[c]]), Tp);
+            }
+            T *= alpha;
+            const float sc = T / Tp;
+            const float beta = mass != 0.f ? mass * sc : 0.f;
+            const float top = fabsf(beta) * fmax;
+            // what the general kernel treats specially, or what may leave float32's range
+            bad = !(sc > 0.25f && sc < 4.f) || !(top < 1e30f) || (beta != 0.f && !(top > 1e-25f));
+            w = make_float4(beta * wc[0], beta * wc[1], beta * wc[2], beta * wc[3]);
+          }
+        }
+      }
+      if (bad) s_flag = 1;
+      s_key[tid] = tid < m ? __float_as_uint(alpha) : 0xffffffffu;
+      __syncthreads();
+      if (tid < m) {
+        amin = fminf(amin, alpha);
+        amax = fmaxf(amax, alpha);
+        const unsigned key = s_key[tid];
+        int rank = 0;
+        for (int q = 0; q < m; q += 4) {
+          const uint4 v = *reinterpret_cast<const uint4*>(&s_key[q]);
+          rank += (v.x < key || (v.x == key && q < tid)) + (v.y < key || (v.y == key && q + 1 < tid)) +
+                  (v.z < key || (v.z == key && q + 2 < tid)) +
+                  (v.w < key || (v.w == key && q + 3 < tid));
+        }
+        a.rec_w[j0 + rank] = w;
+        a.rec_a[j0 + rank] = make_float2(alpha, __int_as_float(row * 128));
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      amin = fminf(amin, __shfl_xor_sync(0xffffffffu, amin, o));
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    }
+    if ((tid & 31) == 0) {
+      s_lo[tid >> 5] = amin;
+      s_hi[tid >> 5] = amax;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      for (int q = 1; q < kSub / 32; ++q) {
+        amin = fminf(amin, s_lo[q]);
+        amax = fmaxf(amax, s_hi[q]);
+      }
+      a.desc[item] = make_int4(jb, je - jb, __float_as_int(amin), __float_as_int(amax));
+      // the samples a node crosses within the item must fit the row
+      if (s_flag || (amax - amin) * x1 / (1.f - kAlphaMax) > plan.window * plan.dt_min) {
+        a.flags[it.x] = 1;
+        a.ctrl->flagged = 1;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+struct SliceArgs {
+  const float* flux;
+  const float* wz;
+  const float* wt;
+  int n_templ, n_age, n_wave, n_t;
+  const int4* desc;  // per item: first record, records, smallest and largest alpha
+  const float4* rec_w;
+  const float2* rec_a;
+  float* rows;    // [row][slice][kMaxBins]
+  int2* row_pos;  // [row][slice]: first extended sample, samples
+  NodeCtrl* ctrl;
+  int wave, multi_rows, n_seg;
+  long long slice_rows;  // rows of kMaxBins samples in the workspace
+};
+
+// Single-item spaxels of a wave: as many as the rows left by the others hold.
+__device__ __forceinline__ int wave_size(long long slice_rows, int n_slices, int multi_rows,
+                                         int n_seg) {
+  return (int)min((long long)n_seg, slice_rows / n_slices - multi_rows);
+}
+
+// Items [i0, i1) of a wave: wave 0 holds every item of a several-item spaxel and the first
+// wave_items others, wave w the next wave_items.  Item i uses row i when it is one of
+// several, else the row of its place in the wave.
+__device__ __forceinline__ void wave_range(const NodeCtrl* c, int wave, int wave_items, int& i0,
+                                           int& i1) {
+  const int s0 = c->n_multi + wave * wave_items;
+  i0 = wave == 0 ? 0 : min(s0, c->n_items);
+  i1 = min(s0 + wave_items, c->n_items);
+}
+__device__ __forceinline__ int item_row(int item, int n_multi, int wave, int wave_items,
+                                        int multi_rows) {
+  return item < n_multi ? item : multi_rows + (item - n_multi - wave * wave_items);
+}
+
+// 1 / x by the hardware's reciprocal (relative error about 2^-23); x is a positive normal.
+__device__ __forceinline__ float fast_rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// The records that a warp has staged, one array per value: a step reads one word of NPL
+// records at a time, one wavefront each (16-byte loads of the same take four).
+struct StagedRecs {
+  float w[4][kStage];  // corner weights times beta
+  float alpha[kStage];
+  int row[kStage];     // byte offset of the first corner's row in the slice table
+};
+
+struct SliceShared {
+  const float* tab;  // [template][32]
+  const float* xw;   // window of the extended telescope grid, kWin samples
+  StagedRecs* st;    // this warp's staged records
+  float* f;          // this warp's samples, kMaxBins
+  float inv;         // samples per Angstrom over the window
+};
+
+// Smallest window index j with xw[j] >= x: a linear guess, right to one sample on a uniform
+// grid and corrected by steps on others.
+__device__ __forceinline__ int sample_at(const SliceShared& s, float x) {
+  int j = min(max((int)((x - s.xw[0]) * s.inv), 1), kWin - 2);
+  const float x0 = s.xw[j - 1], x1 = s.xw[j], x2 = s.xw[j + 1];
+  if (x0 < x && x <= x2) return x <= x1 ? j : j + 1;
+  while (j > 1 && s.xw[j - 1] >= x) --j;
+  while (j < kWin - 1 && s.xw[j] < x) ++j;
+  return j;
+}
+
+// One item by one warp on one slice: NPL nodes per lane (two or four, in packed pairs), NPL
+// particles at a time, each on 32 / NPL lanes.
+//
+// A group holds particles whose alpha differ by less than W telescope bins.  With j the
+// first sample at or right of node l at the group's first alpha, node l (1..n_own of the
+// slice) fills the samples from j to the next node's; with t = x_j - lambda'_l it sums
+//   A = sum (G_l + s_l t), B = sum s_l    the right interval's line, the value from j+W on
+//   D_m = sum (s_{l-1} - s_l) min(t, -d_m), m < W, d_m = x_{j+m} - x_j: the samples that the
+//         node crosses lie on the left line (slope sum B of node l - 1) while t < -d_m, so
+//         f_{j+m} = A + D_m + d_m B_{l-1}.
+// The groups are the same for every slice: neighbours agree on who fills a sample.
+template <int NPL, int W>
+struct SliceItem {
+  static constexpr int LPG = 32 / NPL;  // lanes of a particle
+  static constexpr int PR = NPL / 2;    // packed pairs of nodes
+  const SliceShared& sh;
+  const int lane, i, g, own, nxt_lane, prv_lane;
+  const bool mine;
+  const float lam_own;
+  float2 nlam[PR];  // minus the wavelengths: -lambda' comes from one packed product
+  float nlam_r;
+  const char* tab;
+
+  __device__ __forceinline__ SliceItem(const SliceShared& s, int lane_, int n_own,
+                                       const float* __restrict__ lam)
+      : sh(s), lane(lane_), i(lane_ & (LPG - 1)), g(lane_ / LPG), own(i * NPL + g),
+        nxt_lane((((own + 1) % NPL) * LPG + (own + 1) / NPL) & 31),
+        prv_lane(own == 0 ? 0 : ((own - 1) % NPL) * LPG + (own - 1) / NPL),
+        mine(own >= 1 && own <= n_own), lam_own(lam[own]) {
+#pragma unroll
+    for (int q = 0; q < PR; ++q)
+      nlam[q] = make_float2(-lam[i * NPL + 2 * q], -lam[i * NPL + 2 * q + 1]);
+    nlam_r = -lam[i * NPL + NPL];
+    tab = reinterpret_cast<const char*>(s.tab) + i * (4 * NPL);
+  }
+
+  int j;
+  float xo, xo1;                   // samples j and (W > 1) j + 1 of the node this lane collects
+  float2 xj[PR], dm[PR], A[PR], B[PR], D[W][PR];
+
+  // Reduction over the particle groups; lane (g, i) ends with the sum of node i*NPL + g.
+  __device__ __forceinline__ float collect(const float2 (&v)[PR]) const {
+    if constexpr (NPL == 2) {
+      return (g ? v[0].y : v[0].x) + __shfl_xor_sync(0xffffffffu, g ? v[0].x : v[0].y, 16);
+    } else {
+      const bool h = g & 2, l = g & 1;
+      const float a0 =
+          (h ? v[1].x : v[0].x) + __shfl_xor_sync(0xffffffffu, h ? v[0].x : v[1].x, 16);
+      const float a1 =
+          (h ? v[1].y : v[0].y) + __shfl_xor_sync(0xffffffffu, h ? v[0].y : v[1].y, 16);
+      return (l ? a1 : a0) + __shfl_xor_sync(0xffffffffu, l ? a0 : a1, 8);
+    }
+  }
+  // The owner lanes' value for every node of this lane.
+  __device__ __forceinline__ void spread(float v, float2 (&o)[PR]) const {
+#pragma unroll
+    for (int q = 0; q < PR; ++q) {
+      o[q].x = __shfl_sync(0xffffffffu, v, 2 * q * LPG + i);
+      o[q].y = __shfl_sync(0xffffffffu, v, (2 * q + 1) * LPG + i);
+    }
+  }
+
+  __device__ __forceinline__ void open(float alpha) {
+    j = sample_at(sh, __fmul_rn(lam_own, alpha));
+    xo = sh.xw[j];
+    spread(xo, xj);
+    if constexpr (W > 1) {
+      xo1 = sh.xw[j + 1];
+      spread(xo - xo1, dm);
+    }
+#pragma unroll
+    for (int q = 0; q < PR; ++q) {
+      A[q] = B[q] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int m = 0; m < W; ++m) D[m][q] = make_float2(0.f, 0.f);
+    }
+  }
+
+  // The group's sums to this warp's samples.  Every sample has one lane.
+  __device__ __forceinline__ void flush(int jb) {
+    const float s0 = collect(A), s1 = collect(B);
+    const float p0 = s0 + collect(D[0]);
+    float p1 = 0.f;
+    if constexpr (W > 1) p1 = s0 + collect(D[1]);
+    const int jn = __shfl_sync(0xffffffffu, j, nxt_lane);
+    if constexpr (W > 1) {
+      const float left = __shfl_sync(0xffffffffu, s1, prv_lane);
+      p1 = fmaf(xo1 - xo, left, p1);
+    }
+    if (mine) {
+      float* f = sh.f - jb;
+      const int e1 = min(jn, jb + kMaxBins);  // the window checks keep every sample inside
+      constexpr int U = 4;                    // samples inside the interval taken together
+      float v[U], x[U];
+      const bool in = j + W <= e1;
+      const float f0 = in ? f[j] : 0.f;
+      const float f1 = in && W > 1 ? f[j + 1] : 0.f;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = j + W + u;
+        v[u] = e < e1 ? f[e] : 0.f;
+        x[u] = e < e1 ? sh.xw[e] : 0.f;
+      }
+      if (in) {
+        f[j] = f0 + p0;
+        if (W > 1) f[j + 1] = f1 + p1;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = j + W + u;
+        if (e < e1) f[e] = v[u] + fmaf(s1, x[u] - xo, s0);
+      }
+      for (int e = j + W + U; e < e1; ++e) f[e] += fmaf(s1, sh.xw[e] - xo, s0);
+    }
+    __syncwarp();
+  }
+
+  // What a step reads of its NPL particles, loaded a step ahead; r: this lane's record.
+  struct Loaded {
+    float2 c[4][PR];
+    float w[4], alpha;
+  };
+  __device__ __forceinline__ void load(int r, int zoff, Loaded& v) const {
+    const StagedRecs& st = *sh.st;
+    const char* t0 = tab + st.row[r];
+    const char* t1 = t0 + zoff;
+    const char* tc[4] = {t0, t1, t0 + 128, t1 + 128};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v.w[k] = st.w[k][r];
+      if constexpr (NPL == 2) {
+        v.c[k][0] = *reinterpret_cast<const float2*>(tc[k]);
+      } else {
+        const float4 x = *reinterpret_cast<const float4*>(tc[k]);
+        v.c[k][0] = make_float2(x.x, x.y);
+        v.c[k][PR - 1] = make_float2(x.z, x.w);
+      }
+    }
+    v.alpha = st.alpha[r];
+  }
+  __device__ __forceinline__ void step(const Loaded& v) {
+    float2 G[PR];
+    const float2 w0 = make_float2(v.w[0], v.w[0]), w1 = make_float2(v.w[1], v.w[1]);
+    const float2 w2 = make_float2(v.w[2], v.w[2]), w3 = make_float2(v.w[3], v.w[3]);
+    const float2 al = make_float2(v.alpha, v.alpha);
+    const auto& c = v.c;
+    float2 nlp[PR], s[PR];
+#pragma unroll
+    for (int q = 0; q < PR; ++q) {
+      G[q] = __fmul2_rn(w0, c[0][q]);
+      G[q] = __ffma2_rn(w1, c[1][q], G[q]);
+      G[q] = __ffma2_rn(w2, c[2][q], G[q]);
+      G[q] = __ffma2_rn(w3, c[3][q], G[q]);
+      nlp[q] = __fmul2_rn(nlam[q], al);
+    }
+    const float G_r = __shfl_down_sync(0xffffffffu, G[0].x, 1, LPG);
+    const float nlp_r = __fmul_rn(nlam_r, al.x);
+#pragma unroll
+    for (int q = 0; q < PR; ++q) {
+      const float Gn = q + 1 < PR ? G[q + 1 < PR ? q + 1 : 0].x : G_r;
+      const float ln = q + 1 < PR ? nlp[q + 1 < PR ? q + 1 : 0].x : nlp_r;
+      const float2 r = make_float2(fast_rcp(nlp[q].x - nlp[q].y), fast_rcp(nlp[q].y - ln));
+      s[q] = __fmul2_rn(make_float2(G[q].y - G[q].x, Gn - G[q].y), r);
+    }
+    const float s_l = __shfl_up_sync(0xffffffffu, s[PR - 1].y, 1, LPG);
+#pragma unroll
+    for (int q = 0; q < PR; ++q) {
+      const float2 t = __fadd2_rn(xj[q], nlp[q]);
+      const float sp = q > 0 ? s[q > 0 ? q - 1 : 0].y : s_l;
+      const float2 d = make_float2(sp - s[q].x, s[q].x - s[q].y);
+      D[0][q] = __ffma2_rn(d, make_float2(fminf(t.x, 0.f), fminf(t.y, 0.f)), D[0][q]);
+      if constexpr (W > 1)
+        D[1][q] = __ffma2_rn(d, make_float2(fminf(t.x, dm[q].x), fminf(t.y, dm[q].y)), D[1][q]);
+      A[q] = __fadd2_rn(A[q], __ffma2_rn(s[q], t, G[q]));
+      B[q] = __fadd2_rn(B[q], s[q]);
+    }
+  }
+};
+
+// Item of a warp: its first record and record count, its smallest and largest alpha.
+struct ItemDesc {
+  int p0, np;
+  float lo, hi;
+};
+
+// The slice kernel: a block holds one slice (32 nodes) of every template in shared memory
+// and its warps take the work items in turn, so a particle's corners cost four shared
+// loads per 32 nodes (13 KB per particle in all, 40 TB/s over the chip) instead of the same
+// bytes from L2.  Bound by shared-memory wavefronts (63 % of the pipe) and issue (0.65 per
+// cycle) together at 409 us for 4 10^5 particles on 60 x 60 spaxels; a step's operands are
+// loaded one step ahead (483 us without), 20 warps hide more latency than 16 or 12 (+2 %,
+// +15 %), four nodes a lane beat two by 6 % and one by 8 %, W = 2 needs half the flushes of
+// W = 1, W = 3 costs more per step than it saves.  A warp's next item, its description and its first records are fetched while the one before
+// is processed.  A block whose slice has no items left takes the slice with the most.
+template <int NPL, int W>
+__device__ __forceinline__ void slice_items(const SliceArgs& a, const SliceShared& sh,
+                                            const float* s_lam, int n_own, int lane, int slice,
+                                            int n_slices, int i0, int total, int e0, float w_seg,
+                                            int n_multi, int wave_items, int* __restrict__ next) {
+  SliceItem<NPL, W> w(sh, lane, n_own, s_lam);
+  const int zoff = a.n_age * 128;
+  const float lam_lo = s_lam[1], lam_hi = s_lam[n_own + 1];
+  auto take = [&]() { return lane == 0 ? atomicAdd(next, 1) : 0; };
+  auto describe = [&](int cur) {
+    ItemDesc d{0, 0, 1.f, 1.f};
+    if (cur < total) {
+      const int4 v = a.desc[i0 + cur];
+      d = ItemDesc{v.x, v.y, __int_as_float(v.z), __int_as_float(v.w)};
+    }
+    return d;
+  };
+  float4 rw = make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 ra = make_float2(1.f, 0.f);
+  auto fetch = [&](int p, int n) {
+    rw = make_float4(0.f, 0.f, 0.f, 0.f);
+    ra = make_float2(1.f, 0.f);
+    if (lane < n) {
+      rw = a.rec_w[(long long)p + lane];
+      ra = a.rec_a[(long long)p + lane];
+    }
+  };
+  int cur = __shfl_sync(0xffffffffu, take(), 0);
+  int nxt = __shfl_sync(0xffffffffu, take(), 0);
+  ItemDesc d = describe(cur), dn = describe(nxt);
+  int nxt2_raw = take();
+  fetch(d.p0, d.np);
+  while (d.np > 0) {
+    const int nxt2 = __shfl_sync(0xffffffffu, nxt2_raw, 0);
+    const ItemDesc dn2 = describe(nxt2);
+    nxt2_raw = take();
+    const int jb = sample_at(sh, __fmul_rn(lam_lo, d.lo));
+    bool open = false;
+    float a_lim = 0.f;  // alpha at which the sample windows have to move
+    for (int base = 0; base < d.np; base += 32) {
+      const int cnt = min(32, d.np - base);
+      __syncwarp();
+      sh.st->w[0][lane] = rw.x;
+      sh.st->w[1][lane] = rw.y;
+      sh.st->w[2][lane] = rw.z;
+      sh.st->w[3][lane] = rw.w;
+      sh.st->alpha[lane] = ra.x;
+      sh.st->row[lane] = __float_as_int(ra.y);
+      const float al = ra.x;
+      __syncwarp();
+      if (base + 32 < d.np) fetch(d.p0 + base + 32, d.np - base - 32);
+      else fetch(dn.p0, dn.np);
+      bool fresh = (base & (kSub - 1)) == 0;  // a new sorted run
+      int pos = 0;
+      while (pos < cnt) {
+        const float a0 = __shfl_sync(0xffffffffu, al, pos);
+        if (!open || a0 >= a_lim || fresh) {
+          if (open) w.flush(jb);
+          w.open(a0);
+          a_lim = a0 + w_seg;
+          open = true;
+          fresh = false;
+        }
+        const unsigned past =
+            __ballot_sync(0xffffffffu, lane > pos && lane < cnt && al >= a_lim);
+        const int end = past ? __ffs(past) - 1 : cnt;
+        typename SliceItem<NPL, W>::Loaded v;
+        w.load(pos + w.g < end ? pos + w.g : 32, zoff, v);  // 32: a record of weight zero
+        for (int p = pos + NPL; p < end; p += NPL) {
+          const typename SliceItem<NPL, W>::Loaded u = v;
+          w.load(p + w.g < end ? p + w.g : 32, zoff, v);
+          w.step(u);
+        }
+        w.step(v);
+        pos = end;
+      }
+    }
+    if (open) w.flush(jb);
+    const int nb = min(sample_at(sh, __fmul_rn(lam_hi, d.hi)) - jb, kMaxBins);
+    const long long row =
+        (long long)item_row(i0 + cur, n_multi, a.wave, wave_items, a.multi_rows) * n_slices +
+        slice;
+    float* out = a.rows + row * kMaxBins;
+    for (int b = lane; b < nb; b += 32) {
+      out[b] = sh.f[b];
+      sh.f[b] = 0.f;
+    }
+    if (lane == 0) a.row_pos[row] = make_int2(e0 + jb, nb);
+    __syncwarp();
+    cur = nxt;
+    nxt = nxt2;
+    d = dn;
+    dn = dn2;
+  }
+}
+
+__global__ void __launch_bounds__(kNodeThreads, 1) node_slice_kernel(SliceArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  float* s_tab = reinterpret_cast<float*>(smem);
+  float* s_xw = s_tab + (size_t)a.n_templ * 32;
+  StagedRecs* s_st = reinterpret_cast<StagedRecs*>(s_xw + kWin);
+  float* s_f = reinterpret_cast<float*>(s_st + kNodeWarps);
+  __shared__ float s_lam[36];
+  __shared__ NodePlan s_plan;
+  __shared__ int s_slice, s_e0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const float x_last = a.wt[a.n_t - 1];
+  if (tid == 0) s_plan = node_plan(a.ctrl, a.n_wave, x_last);
+  __syncthreads();
+  const NodePlan plan = s_plan;
+  if (!plan.ok) return;
+  int i0, i1;
+  const int wave_items = wave_size(a.slice_rows, plan.n_slices, a.multi_rows, a.n_seg);
+  wave_range(a.ctrl, a.wave, wave_items, i0, i1);
+  const int total = i1 - i0;
+  if (total <= 0) return;
+  SliceShared sh;
+  sh.tab = s_tab;
+  sh.xw = s_xw;
+  sh.st = s_st + warp;
+  sh.f = s_f + warp * kMaxBins;
+  if (lane == 0) {
+    for (int k = 0; k < 4; ++k) sh.st->w[k][32] = 0.f;
+    sh.st->alpha[32] = 1.f;
+    sh.st->row[32] = 0;
+  }
+  for (int b = lane; b < kMaxBins; b += 32) sh.f[b] = 0.f;
+  int* next = a.ctrl->next[a.wave];
+  int slice = (int)((long long)blockIdx.x * plan.n_slices / gridDim.x);
+  const float w_seg =
+      (float)plan.w * 0.98f * plan.dt_min * (1.f - kAlphaMax) / x_last - 2.4e-7f;
+
+  for (;;) {
+    const int k0 = plan.k_first - 1 + slice * plan.n_own;  // node of lane 0
+    for (int r = warp; r < a.n_templ; r += kNodeWarps) {
+      const int k = k0 + lane;
+      s_tab[r * 32 + lane] =
+          (lane <= plan.n_own + 1 && k >= 0 && k < a.n_wave)
+              ? a.flux[(long long)r * a.n_wave + k] : 0.f;
+    }
+    if (tid < 36) s_lam[tid] = lam_ext(a.wz, a.n_wave, k0 + tid);
+    if (tid == 0) {
+      const float x = lam_ext(a.wz, a.n_wave, k0) * (1.f - kAlphaMax);
+      int lo = 0, hi = a.n_t + 2 * kExt - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (x_ext(a.wt, a.n_t, mid) < x) lo = mid + 1; else hi = mid;
+      }
+      s_e0 = max(lo - 3, 0);
+    }
+    __syncthreads();
+    const int e0 = s_e0;
+    for (int q = tid; q < kWin; q += kNodeThreads) s_xw[q] = x_ext(a.wt, a.n_t, e0 + q);
+    __syncthreads();
+    sh.inv = (float)(kWin - 1) / (s_xw[kWin - 1] - s_xw[0]);
+    if (plan.w == 1)
+      slice_items<2, 1>(a, sh, s_lam, plan.n_own, lane, slice, plan.n_slices, i0, total, e0,
+                        w_seg, a.ctrl->n_multi, wave_items, next + slice);
+    else
+      slice_items<4, 2>(a, sh, s_lam, plan.n_own, lane, slice, plan.n_slices, i0, total, e0,
+                        w_seg, a.ctrl->n_multi, wave_items, next + slice);
+    __syncthreads();
+    if (tid == 0) {
+      int best = -1, most = 2 * kNodeWarps;
+      for (int q = 0; q < plan.n_slices; ++q) {
+        const int left = total - *(volatile int*)&next[q];
+        if (left > most) {
+          most = left;
+          best = q;
+        }
+      }
+      s_slice = best;
+    }
+    __syncthreads();
+    slice = s_slice;
+    if (slice < 0) return;
+  }
+}
+
+struct MergeArgs {
+  const int* seg_off;
+  const int* multi;
+  const int* large;
+  const int* small;
+  int n_seg, big, n_t, n_wave;
+  const float* wt;
+  const int* flags;
+  const float* rows;
+  const int2* row_pos;
+  const NodeCtrl* ctrl;
+  int wave, multi_rows;
+  long long slice_rows;
+  float* cube;
+  long long stride;
+  int lsf_k, lsf_crop;
+  float lsf[kMaxLsfTaps + 1];
+};
+
+constexpr int kMergeThreads = 256;
+
+// One block per spaxel: the slices of its items summed (neighbouring slices share only the
+// samples around their common node: even slices first, then odd ones; items with Kahan's
+// compensation), then the LSF (rubix/telescope/lsf/lsf.py:29-105) and the store.  Empty
+// spaxels are zero.  Bound by HBM: the rows once, the cube once.
+template <int R>
+__global__ void __launch_bounds__(kMergeThreads) node_merge_kernel(MergeArgs a) {
+  extern __shared__ float s_buf[];
+  __shared__ NodePlan s_plan;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) s_plan = node_plan(a.ctrl, a.n_wave, a.wt[a.n_t - 1]);
+  __syncthreads();
+  const int n_slices = s_plan.n_slices;
+  const int K = a.lsf_k, n_t = a.n_t;
+  const int lead = K > 0 ? K - 1 - a.lsf_crop : 0;
+  const int pad = R * kMergeThreads + (K > 0 ? K : 0);  // s_spec: lead + n_t + zeros
+  float* s_spec = s_buf;
+  float* s_comp = s_buf + pad;
+  int i0 = 0, i1 = 0, wave_items = 0;
+  if (s_plan.ok) {
+    wave_items = wave_size(a.slice_rows, n_slices, a.multi_rows, a.n_seg);
+    wave_range(a.ctrl, a.wave, wave_items, i0, i1);
+  }
+  const int n_multi = a.ctrl->n_multi;
+  for (int s = blockIdx.x; s < a.n_seg; s += gridDim.x) {
+    const int cnt = a.seg_off[s + 1] - a.seg_off[s];
+    float* out = a.cube + (long long)s * a.stride;
+    if (cnt == 0) {
+      if (a.wave == 0)
+        for (int t = tid; t < n_t; t += kMergeThreads) out[t] = 0.f;
+      continue;
+    }
+    const int it0 = first_item(s, cnt, a.big, a.n_seg, a.multi, a.large, a.small);
+    if (it0 < i0 || it0 >= i1 || a.flags[s]) continue;
+    const int chunks = (cnt + kItem - 1) / kItem;
+    for (int i = tid; i < pad; i += kMergeThreads) s_spec[i] = 0.f;
+    if (chunks > 1)
+      for (int i = tid; i < n_t; i += kMergeThreads) s_comp[i] = 0.f;
+    __syncthreads();
+    for (int c = 0; c < chunks; ++c) {
+      const long long row0 =
+          (long long)item_row(it0 + c, n_multi, a.wave, wave_items, a.multi_rows) * n_slices;
+#pragma unroll
+      for (int parity = 0; parity < 2; ++parity) {
+        for (int q = 2 * warp + parity; q < n_slices; q += 2 * (kMergeThreads / 32)) {
+          const int2 pos = a.row_pos[row0 + q];
+          const float* src = a.rows + (row0 + q) * kMaxBins;
+          float v[kMaxBins / 32];
+#pragma unroll
+          for (int u = 0; u < kMaxBins / 32; ++u)
+            v[u] = 32 * u + lane < pos.y ? src[32 * u + lane] : 0.f;
+#pragma unroll
+          for (int u = 0; u < kMaxBins / 32; ++u) {
+            const int t = pos.x - kExt + 32 * u + lane;
+            if (32 * u + lane < pos.y && t >= 0 && t < n_t) {
+              float* d = s_spec + lead + t;
+              if (chunks == 1) {
+                *d += v[u];
+              } else {
+                const float y = v[u] - s_comp[t];
+                const float z = *d + y;
+                s_comp[t] = (z - *d) - y;
+                *d = z;
+              }
+            }
+          }
+        }
+        __syncthreads();
+      }
+    }
+    if (K > 0) {
+      float o[R];
+      const int t0 = tid * R;
+      if (K == 25) {  // rubix's LSF: 2 * 12 + 1 taps (telescope/lsf/lsf.py:12-26)
+        float win[R + 24];
+#pragma unroll
+        for (int i = 0; i < R + 24; ++i) win[i] = s_spec[t0 + i];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          o[r] = 0.f;
+#pragma unroll
+          for (int j = 0; j < 25; ++j) o[r] = fmaf(a.lsf[j], win[r + 24 - j], o[r]);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) o[r] = 0.f;
+        for (int j = 0; j < K; ++j) {
+          const float w = a.lsf[j];
+#pragma unroll
+          for (int r = 0; r < R; ++r) o[r] = fmaf(w, s_spec[t0 + r + K - 1 - j], o[r]);
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < R; ++r) s_spec[t0 + r] = o[r];
+      __syncthreads();
+    }
+    for (int t = tid; t < n_t; t += kMergeThreads) out[t] = s_spec[t];
+    __syncthreads();
+  }
+}
+
+size_t slice_smem(int n_templ) {
+  return sizeof(float) * ((size_t)n_templ * 32 + kWin + kNodeWarps * kMaxBins) +
+         sizeof(StagedRecs) * kNodeWarps;
+}
+
+size_t row_bytes(int n_wave) {
+  return (size_t)max_slices_of(n_wave) * (kMaxBins * sizeof(float) + sizeof(int2));
+}
+
+// Rows of the items of spaxels with more than kItem particles: at most n / kItem full ones
+// and one partial one for each such spaxel.
+long long multi_row_count(long long n) { return 2 * n / kItem + 1; }
+
+struct NodeLayout {
+  NodeCtrl* ctrl;
+  int* flags;
+  int *multi, *large, *small;
+  int2* items;
+  int4* desc;
+  double* prefix;
+  // not used before the last merge by the fallback, nor after it by the slices
+  float* h;
+  float* H;
+  float4* rec_w;
+  float2* rec_a;
+  float* rows;
+  int2* row_pos;
+  size_t shared_off, fixed;  // start of the shared region; bytes without rows
+};
+
+int kpad_of(int n_wave) { return (n_wave + 31) / 32 * 32; }
+
+NodeLayout carve_nodes(void* ws, long long n, int n_seg, int nZ, int nA, int nW) {
+  Carve c(ws);
+  NodeLayout L;
+  c.take<CubeCtrl>(1);
+  L.ctrl = c.take<NodeCtrl>(1);
+  L.flags = c.take<int>((size_t)n_seg);
+  L.multi = c.take<int>((size_t)n_seg + 1);
+  L.large = c.take<int>((size_t)n_seg + 1);
+  L.small = c.take<int>((size_t)n_seg + 1);
+  L.items = c.take<int2>((size_t)(multi_row_count(n) + n_seg));
+  L.desc = c.take<int4>((size_t)(multi_row_count(n) + n_seg));
+  L.prefix = c.take<double>((size_t)nZ * nA * nW);
+  L.shared_off = c.off;
+  L.h = c.take<float>((size_t)kAlphaRows * kpad_of(nW));
+  L.H = c.take<float>((size_t)kAlphaRows * nZ * nA);
+  L.rec_w = c.take<float4>((size_t)n);
+  L.rec_a = c.take<float2>((size_t)n);
+  L.fixed = c.off;
+  L.rows = nullptr;
+  L.row_pos = nullptr;
+  return L;
+}
+
+NodeFallback carve_fallback(Carve& c, const CubeInputs& in) {
+  NodeFallback f{};
+  f.At = c.take<float>((size_t)in.n_wave_t);
+  f.bucket = c.take<int2>(kBuckets);
+  f.ct = c.take<float4>((size_t)(in.n_met - 1) * (in.n_age - 1) * in.n_wave);
+  f.rec = c.take<ParticleRec>((size_t)in.n);
+  f.done = c.take<int>((size_t)in.n_seg);
+  f.slot_start = c.take<int>((size_t)in.n_seg);
+  f.chunk = kMaxChunk;
+  f.split = (int)max_slots(in.n, kMaxChunk);
+  f.items = c.take<int2>((size_t)f.split + in.n_seg);
+  f.partials = c.take<float>((size_t)f.split * in.n_wave_t);
+  return f;
+}
+
+size_t fallback_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
+  CubeInputs in{};
+  in.n_met = nZ;
+  in.n_age = nA;
+  in.n_wave = nW;
+  in.n_wave_t = n_t;
+  in.n_seg = n_seg;
+  in.n = n;
+  Carve c(nullptr);
+  carve_fallback(c, in);
+  return c.off;
+}
+
+// What cube_main_kernel reads (cube_prepare's setup passes), when a spaxel is flagged.
+__global__ void __launch_bounds__(256) node_fallback_kernel(CubeInputs in, NodeFallback f,
+                                                            const double* __restrict__ prefix,
+                                                            const int* __restrict__ flags,
+                                                            NodeCtrl* __restrict__ nc) {
+  if (!nc->flagged) return;
+  const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
+  double lnq0, h;
+  bucket_params(in.wave_t, in.n_wave_t, lnq0, h);
+  for (int t = gtid; t < in.n_wave_t; t += gsz)
+    f.At[t] = (float)((log((double)in.wave_t[t]) - lnq0) / h);
+  for (int b = gtid; b < kBuckets; b += gsz)
+    f.bucket[b] = bucket_entry(in.ssp_wave_z, in.n_wave, lnq0, h, b);
+  for (int s = gtid; s < in.n_seg; s += gsz) {
+    if (!flags[s]) continue;
+    const int cnt = in.seg_off[s + 1] - in.seg_off[s];
+    const int nch = (cnt + f.chunk - 1) / f.chunk;
+    const int at = nch > 1 ? atomicAdd(&nc->left[0], nch) : f.split + atomicAdd(&nc->left[1], 1);
+    f.slot_start[s] = at;
+    f.done[s] = 0;
+    for (int c = 0; c < nch; ++c) f.items[at + c] = make_int2(s, c);
+  }
+  corner_table(in.ssp_flux, in.n_met, in.n_age, in.n_wave, f.ct);
+  gather_records(in.mass, in.met, in.age, in.vel, in.vel_stride, in.vel_comp, in.perm,
+                 in.seg_off, in.n_seg, in.n, in.ssp_met, in.n_met, in.ssp_age, in.n_age,
+                 in.ssp_wave_z, in.n_wave, in.wave_t, in.n_wave_t, prefix, 1.0 / h,
+                 (float)(kVmaxKms / kSpeedOfLight / h), __uint_as_float(~nc->dz_inv),
+                 __uint_as_float(nc->dt_max), f.rec, 0, nullptr,
+                 (float)exp(-kVmaxKms / kSpeedOfLight), (float)exp(kVmaxKms / kSpeedOfLight));
+}
+
+constexpr size_t kRowBudget = (size_t)2 << 30;  // rows of single-item spaxels at a time
+
+long long min_wave_items(int n_seg) {
+  return std::max<long long>((n_seg + kMaxWaves - 1) / kMaxWaves, std::min(n_seg, 256));
+}
+
+}  // namespace
+
+bool cube_nodes_supported(int nZ, int nA, int nW, int n_t) {
+  return n_t >= 2 && nW >= 2 && slice_smem(nZ * nA) <= 227 * 1024;
+}
+
+size_t cube_nodes_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
+  const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
+  const long long wave = std::max(
+      min_wave_items(n_seg), std::min<long long>(n_seg, (long long)(kRowBudget / row_bytes(nW))));
+  return std::max(L.fixed + (size_t)(multi_row_count(n) + wave) * row_bytes(nW),
+                  L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t));
+}
+
+bool cube_nodes_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, size_t bytes) {
+  const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
+  return bytes >= L.fixed + (size_t)(multi_row_count(n) + min_wave_items(n_seg)) * row_bytes(nW) &&
+         bytes >= L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t);
+}
+
+int cube_nodes_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t bytes) {
+  const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
+  const long long fit = (long long)((bytes - L.fixed) / row_bytes(nW)) - multi_row_count(n);
+  const long long wave = std::min<long long>(n_seg, fit);
+  return 8 + 2 * (int)((n_seg + wave - 1) / wave);
+}
+
+int cube_nodes_forward(const CubeInputs& in, const float* lsf_taps, int n_lsf, int lsf_crop,
+                       int big_item, float* cube, long long stride, void* ws, size_t ws_bytes,
+                       NodeFallback* fb, cudaStream_t st) {
+  NodeLayout L = carve_nodes(ws, in.n, in.n_seg, in.n_met, in.n_age, in.n_wave);
+  const int n_templ = in.n_met * in.n_age, nW = in.n_wave;
+  const size_t rb = row_bytes(nW);
+  const long long multi_rows = multi_row_count(in.n);
+  const long long fit = (long long)((ws_bytes - L.fixed) / rb) - multi_rows;
+  const int wave_items = (int)std::min<long long>(in.n_seg, fit);
+  const int waves = (in.n_seg + wave_items - 1) / wave_items;
+  const size_t total_rows = (size_t)(multi_rows + wave_items) * max_slices_of(nW);
+  char* base = static_cast<char*>(ws) + L.fixed;
+  L.rows = reinterpret_cast<float*>(base);
+  L.row_pos = reinterpret_cast<int2*>(base + total_rows * kMaxBins * sizeof(float));
+
+  // control block, counters and flags are contiguous
+  RUBIX_CUDA_TRY(cudaMemsetAsync(ws, 0, (size_t)((char*)(L.flags + in.n_seg) - (char*)ws), st));
+  {
+    const long long work = std::max<long long>(std::max(in.n_wave_t, nW), in.n);
+    const int g = (int)std::min<long long>((work + 255) / 256, (long long)sm_count() * 8);
+    const int need = (std::max(in.n_wave_t, nW) + 255) / 256;
+    node_setup_kernel<<<std::max(g, need), 256, 0, st>>>(in.ssp_wave_z, nW, in.wave_t,
+                                                         in.n_wave_t, in.vel, in.vel_stride,
+                                                         in.vel_comp, in.n, L.ctrl);
+    RUBIX_LAUNCH_CHECK("node_setup_kernel");
+  }
+  const int kpad = kpad_of(nW);
+  {
+    node_tables_kernel<<<n_templ + kWeightBlocks, kPrefixThreads, 0, st>>>(
+        in.ssp_flux, n_templ, nW, in.ssp_wave_z, in.wave_t, in.n_wave_t, L.prefix, L.h, kpad,
+        L.ctrl);
+    RUBIX_LAUNCH_CHECK("node_tables_kernel");
+    node_table_product_kernel<<<dim3((n_templ + 31) / 32, kAlphaTiles), 128, 0, st>>>(
+        L.h, kpad, in.ssp_flux, n_templ, nW, in.wave_t, in.n_wave_t, L.ctrl, L.H);
+    RUBIX_LAUNCH_CHECK("node_table_product_kernel");
+  }
+  {
+    const int g = (int)std::min<long long>((in.n_seg + 255) / 256, (long long)sm_count() * 8);
+    node_count_kernel<<<g, 256, 0, st>>>(in.seg_off, in.n_seg, big_item, L.multi, L.large,
+                                         L.small);
+    RUBIX_LAUNCH_CHECK("node_count_kernel");
+    scan_exclusive_3<<<3, 1024, 0, st>>>(L.multi, L.large, L.small, in.n_seg);
+    RUBIX_LAUNCH_CHECK("scan_exclusive_3");
+    node_fill_items_kernel<<<g, 256, 0, st>>>(in.seg_off, in.n_seg, big_item, L.multi, L.large,
+                                              L.small, L.items, L.ctrl);
+    RUBIX_LAUNCH_CHECK("node_fill_items_kernel");
+  }
+  const long long items_max = multi_rows + std::min<long long>(in.n_seg, in.n);
+  {
+    GatherArgs g{in, L.prefix, L.H, L.ctrl, L.items, L.rec_w, L.rec_a, L.flags, L.desc};
+    const int blocks = (int)std::min<long long>(items_max, (long long)sm_count() * 8);
+    node_gather_kernel<<<blocks, kSub, 0, st>>>(g);
+    RUBIX_LAUNCH_CHECK("node_gather_kernel");
+  }
+  const size_t smem = slice_smem(n_templ);
+  RUBIX_CUDA_TRY(cudaFuncSetAttribute(node_slice_kernel,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  MergeArgs m;
+  m.seg_off = in.seg_off;
+  m.multi = L.multi;
+  m.large = L.large;
+  m.small = L.small;
+  m.n_seg = in.n_seg;
+  m.big = big_item;
+  m.n_t = in.n_wave_t;
+  m.n_wave = nW;
+  m.wt = in.wave_t;
+  m.flags = L.flags;
+  m.rows = L.rows;
+  m.row_pos = L.row_pos;
+  m.ctrl = L.ctrl;
+  m.multi_rows = (int)multi_rows;
+  m.slice_rows = (long long)total_rows;
+  m.cube = cube;
+  m.stride = stride;
+  m.lsf_k = n_lsf;
+  m.lsf_crop = lsf_crop;
+  for (int i = 0; i <= kMaxLsfTaps; ++i) m.lsf[i] = i < n_lsf ? lsf_taps[i] : 0.f;
+  for (int w = 0; w < waves; ++w) {
+    const SliceArgs a{in.ssp_flux, in.ssp_wave_z, in.wave_t, n_templ, in.n_age, nW, in.n_wave_t,
+                      L.desc, L.rec_w, L.rec_a, L.rows, L.row_pos, L.ctrl, w, (int)multi_rows, in.n_seg, (long long)total_rows};
+    node_slice_kernel<<<sm_count(), kNodeThreads, smem, st>>>(a);
+    RUBIX_LAUNCH_CHECK("node_slice_kernel");
+    m.wave = w;
+    const int blocks = (int)std::min<long long>(in.n_seg, (long long)sm_count() * 8);
+    auto launch = [&](auto r) -> int {
+      constexpr int R = decltype(r)::value;
+      const size_t ms = sizeof(float) * ((size_t)R * kMergeThreads + std::max(n_lsf, 0) + in.n_wave_t);
+      RUBIX_CUDA_TRY(cudaFuncSetAttribute(node_merge_kernel<R>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ms));
+      node_merge_kernel<R><<<blocks, kMergeThreads, ms, st>>>(m);
+      RUBIX_LAUNCH_CHECK("node_merge_kernel");
+      return RUBIX_OK;
+    };
+    const int need = (in.n_wave_t + kMergeThreads - 1) / kMergeThreads;
+    int rc;
+    if (need <= 4) rc = launch(std::integral_constant<int, 4>{});
+    else if (need <= 8) rc = launch(std::integral_constant<int, 8>{});
+    else if (need <= 15) rc = launch(std::integral_constant<int, 15>{});
+    else rc = launch(std::integral_constant<int, 16>{});
+    if (rc != RUBIX_OK) return rc;
+  }
+  // The flagged spaxels, if any, in the region that the slices no longer need.
+  Carve c(static_cast<char*>(ws) + L.shared_off);
+  *fb = carve_fallback(c, in);
+  fb->gate = L.ctrl->left;
+  const int blocks = sm_count() * 8;
+  node_fallback_kernel<<<blocks, 256, 0, st>>>(in, *fb, L.prefix, L.flags, L.ctrl);
+  RUBIX_LAUNCH_CHECK("node_fallback_kernel");
+  return RUBIX_OK;
+}
+
+}  // namespace rubix

@@ -124,13 +124,16 @@ def spaxel_sort(idx: torch.Tensor, n_segments: int, keep: torch.Tensor | None = 
 
 def cube_forward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, metallicity,
                  age, velocity, vel_component, perm, seg_offsets, n_segments, out=None,
-                 lsf_taps=None, lsf_crop=0, check=False, dust_av=None, dust_exponent=None):
+                 lsf_taps=None, lsf_crop=0, check=False, dust_av=None, dust_exponent=None,
+                 general=False):
     """Fused lookup + mass + Doppler/resample + per-spaxel sum -> cube [n_segments, L].
 
     ``lsf_taps`` (optional) adds the LSF convolution along wavelength of every finished
     spectrum.  ``dust_av`` ([n], A_V per particle) with ``dust_exponent`` ([L],
     -0.4 log2(10) A(lambda)/A(V)) multiplies every resampled spectrum by its dust
-    transmission before the sum.  ``check=True`` synchronises the stream and raises if
+    transmission before the sum.  ``general=True`` evaluates every particle at every
+    wavelength (``rubix_cube_fwd_general``) instead of summing over SSP nodes where the
+    template grid allows that; the two agree to float32 rounding.  ``check=True`` synchronises the stream and raises if
     the kernel reported a device error (a timed-out shared-memory copy wait)."""
     ssp_flux = _contig("ssp_flux", ssp_flux, torch.float32)
     if ssp_flux.dim() != 3:
@@ -161,14 +164,16 @@ def cube_forward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, m
         if out.dim() != 2 or out.shape[0] != n_segments or out.shape[1] < L or out.stride(1) != 1:
             raise ValueError("out must be [n_segments, >=L] with unit stride along wavelength")
     lsf = None if lsf_taps is None else _host_taps(lsf_taps)
-    nbytes = _lib.query("rubix_cube_workspace_size", n, int(n_segments), L, nz, na, nw)
+    general = general or dust_av is not None
+    nbytes = _lib.query("rubix_cube_general_workspace_size" if general
+                        else "rubix_cube_workspace_size", n, int(n_segments), L, nz, na, nw)
     ws = workspace(nbytes, dev)
     lsf_args = (None if lsf is None else lsf.ctypes.data, 0 if lsf is None else lsf.size,
                 int(lsf_crop))
     if (dust_av is None) != (dust_exponent is None):
         raise ValueError("dust_av and dust_exponent go together")
     if dust_av is None:
-        _lib.call("rubix_cube_fwd", _ptr(ssp_flux), _ptr(ssp_metallicity), _ptr(ssp_age),
+        _lib.call("rubix_cube_fwd_general" if general else "rubix_cube_fwd", _ptr(ssp_flux), _ptr(ssp_metallicity), _ptr(ssp_age),
                   _ptr(ssp_wave_z), nz, na, nw, _ptr(wave_t), L, _ptr(mass), _ptr(metallicity),
                   _ptr(age), _ptr(velocity), vstride, int(vel_component), _ptr(perm),
                   _ptr(seg_offsets), int(n_segments), n, *lsf_args, _ptr(out), out.stride(0),
@@ -184,8 +189,8 @@ def cube_forward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, m
                   _ptr(dust_av), _ptr(dust_exponent), _ptr(perm), _ptr(seg_offsets),
                   int(n_segments), n, *lsf_args, _ptr(out), out.stride(0), _ptr(ws),
                   ws.numel(), _stream(dev))
-    # setup, corner table, prefix, count, scans (one launch), fill, main (+ gather)
-    _count((7 + (1 if n > 0 else 0)) if n_segments > 0 else 0)
+    _count(_lib.query("rubix_cube_fwd_launches", n, int(n_segments), L, nz, na, nw,
+                      1 if general else 0, ws.numel()))
     if check and n_segments > 0:
         import ctypes
 

@@ -184,12 +184,14 @@ class RaggedBatch:
     def sort(self, idx, keep):
         return ops.spaxel_sort(idx, self.n_segments, keep)
 
-    def accumulate(self, mass, metallicity, age, velocity, perm, offs, with_lsf=True, out=None):
+    def accumulate(self, mass, metallicity, age, velocity, perm, offs, with_lsf=True, out=None,
+                   general=False):
         r = self.r
         return ops.cube_forward(r.ssp_flux, r.ssp_metallicity, r.ssp_age, r.ssp_wave_z, r.wave_t,
                                 mass, metallicity, age, velocity, r.velocity_axis, perm, offs,
                                 self.n_segments, out=out,
-                                lsf_taps=self.lsf_t if with_lsf else None, lsf_crop=self.lsf_crop)
+                                lsf_taps=self.lsf_t if with_lsf else None, lsf_crop=self.lsf_crop,
+                                general=general)
 
     def psf(self, cube: torch.Tensor, table: Optional[torch.Tensor] = None, out=None):
         table = self.tab_fwd if table is None else table
@@ -247,7 +249,9 @@ class RaggedBatch:
         r = self.r
         idx, keep = self.assign(coords)
         perm, offs = self.sort(idx, keep)
-        A = self.accumulate(mass, metallicity, age, velocity, perm, offs, with_lsf=False)
+        # the general path, as in DatacubeFunction
+        A = self.accumulate(mass, metallicity, age, velocity, perm, offs, with_lsf=False,
+                            general=True)
         Q = self.lsf(A)
         cube = self.psf(Q)
         g = cube - target if keep_cube else cube.sub_(target)
