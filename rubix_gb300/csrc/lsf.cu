@@ -1,10 +1,9 @@
 // Kernel (d): 1-D convolution of every spectrum of a datacube along wavelength,
 // the full convolution cropped to [crop, n + crop) (rubix/telescope/lsf/lsf.py:29-105).
 //
-// A block stages one spectrum in shared memory with K-1 zeros of halo and each
-// thread produces 4 consecutive outputs from float4 loads of its window, so the
-// shared-memory traffic is (K+3)/4 vector loads per 4 outputs and the kernel stays
-// bound by the one read and one write of the cube in HBM.
+// A block stages one spectrum in shared memory with K-1 zeros of halo.  Up to 28 taps a
+// thread produces 12 consecutive outputs (4 in the fused dot) from float4 loads of its
+// window; longer kernels take one output at a time.
 #include "common.cuh"
 #include "dot_reduce.cuh"
 
@@ -97,6 +96,112 @@ __global__ void __launch_bounds__(kLsfThreads)
   }
 }
 
+// The same products in the same order (bit-identical outputs) with the traffic of the
+// store path and of the weights spread over more outputs.  One group of 12 outputs per
+// thread: the window costs (12 + 4 KC) / 4 vector loads, 40 wavefronts per 384 outputs where
+// 4 outputs a thread need 96, the weights one broadcast load per 12 outputs, and a lane
+// stride of 48 bytes keeps the 16-byte loads free of bank conflicts.  The outputs return to
+// shared memory and leave as whole 128-byte lines; the next row waits in registers
+// behind the arithmetic (178 us; as 4-byte asynchronous copies into a second buffer, 187).  Bound by FMA issue and shared memory together, then HBM: 84 M outputs
+// (150 x 150 x 3721, 25 taps) take 178 us, where the 4-output kernel took 246 us, bound
+// by shared-memory wavefronts; one read and one write at the copy rate are 98 us.
+constexpr int kLsfOut = 12;
+constexpr int kLsfRowThreads = 320;  // 320 * 12 = 3840 outputs at a time
+constexpr int kLsfPre = 13;           // rows of up to 13 * 320 staged floats
+
+__device__ __forceinline__ void cp_async_word(float* dst, const float* src, bool valid) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  const int n = valid ? 4 : 0;  // 0: zero-fill, nothing read
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(n)
+               : "memory");
+}
+
+// Floats of one staged row: the last group's window ends 4 KC past a multiple of 12.
+__host__ __device__ constexpr int lsf_row_floats(int n, int KC) {
+  return (n + kLsfOut - 1) / kLsfOut * kLsfOut + 4 * KC;
+}
+
+template <int KC>
+__global__ void __launch_bounds__(kLsfRowThreads) lsf_row_kernel(LsfArgs a) {
+  extern __shared__ __align__(16) float s_buf[];
+  __shared__ __align__(16) float s_w[KC * 4];
+  const int tid = threadIdx.x;
+  const int span = lsf_row_floats(a.n, KC);
+  const int groups = (a.n + kLsfOut - 1) / kLsfOut;
+  const int lead = a.K - 1 - a.crop;  // zeros before in[0]
+  const float* tp = a.taps_dev ? a.taps_dev : a.taps;
+  for (int q = tid; q < KC * 4; q += kLsfRowThreads) s_w[q] = (q < a.K) ? tp[a.K - 1 - q] : 0.f;
+  float pre[kLsfPre];  // the next row's values at places tid, tid + 320, ...
+  auto fetch = [&](long long row) {
+    const float* src = a.in + row * a.sin + tid - lead;
+#pragma unroll
+    for (int k = 0; k < kLsfPre; ++k) {
+      const int g = tid - lead + k * kLsfRowThreads;
+      pre[k] = (unsigned)g < (unsigned)a.n ? __ldcs(src + k * kLsfRowThreads) : 0.f;
+    }
+  };
+  if (blockIdx.x < a.rows) fetch(blockIdx.x);
+  for (long long row = blockIdx.x; row < a.rows; row += gridDim.x) {
+    float* cur = s_buf;
+    __syncthreads();  // the row before is stored
+#pragma unroll
+    for (int k = 0; k < kLsfPre; ++k)
+      if (tid + k * kLsfRowThreads < span) cur[tid + k * kLsfRowThreads] = pre[k];
+    __syncthreads();
+    if (row + gridDim.x < a.rows) fetch(row + gridDim.x);
+    float* dst = a.out + row * a.sout;
+    for (int u0 = 0; u0 < groups; u0 += kLsfRowThreads) {
+      const int u = u0 + tid;
+      float2 o[kLsfOut / 2];
+      if (u < groups) {
+        // the window in pairs from even and from odd places: one packed FMA per tap and
+        // two outputs
+        constexpr int NP = (kLsfOut + KC * 4) / 2;
+        float2 even[NP];
+        const float4* p = reinterpret_cast<const float4*>(cur + kLsfOut * u);
+#pragma unroll
+        for (int c = 0; c < NP / 2; ++c) {
+          const float4 v = p[c];
+          even[2 * c] = make_float2(v.x, v.y);
+          even[2 * c + 1] = make_float2(v.z, v.w);
+        }
+#pragma unroll
+        for (int r = 0; r < kLsfOut / 2; ++r) o[r] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < KC; ++c) {
+          const float4 w4 = *reinterpret_cast<const float4*>(s_w + 4 * c);
+          const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float2 wq = make_float2(w[q], w[q]);
+#pragma unroll
+            for (int r = 0; r < kLsfOut / 2; ++r) {
+              const int m = 2 * c + q / 2 + r;  // pair of window places 4c + q + 2r, + 1
+              o[r] = __ffma2_rn(
+                  wq, (q & 1) ? make_float2(even[m].y, even[m + 1 < NP ? m + 1 : m].x) : even[m],
+                  o[r]);
+            }
+          }
+        }
+      }
+      // a window reaches 4 KC past its outputs, into the next groups': store only when
+      // every window of this round has been read, and the next round's first are safe
+      // because its outputs start after them
+      __syncthreads();
+      if (u < groups) {
+        float4* p = reinterpret_cast<float4*>(cur + kLsfOut * u);
+#pragma unroll
+        for (int c = 0; c < kLsfOut / 4; ++c)
+          p[c] = make_float4(o[2 * c].x, o[2 * c].y, o[2 * c + 1].x, o[2 * c + 1].y);
+      }
+      __syncthreads();
+      const int t1 = min(a.n, (u0 + kLsfRowThreads) * kLsfOut);
+#pragma unroll 4
+      for (int t = u0 * kLsfOut + tid; t < t1; t += kLsfRowThreads) dst[t] = cur[t];
+    }
+  }
+}
+
 // Generic path for long kernels: one output per thread iteration.
 __global__ void __launch_bounds__(kLsfThreads) lsf_scalar_kernel(LsfArgs a) {
   extern __shared__ __align__(16) float s_row[];
@@ -124,16 +229,31 @@ __global__ void __launch_bounds__(kLsfThreads) lsf_scalar_kernel(LsfArgs a) {
 }
 
 template <int KC>
-int launch_vec(const LsfArgs& a, cudaStream_t st) {
-  const int n4 = (a.n + 3) / 4;
-  const size_t smem = sizeof(float) * ((size_t)n4 * 4 + KC * 4 + 4);
-  cudaError_t e = cudaFuncSetAttribute(lsf_vec_kernel<KC>,
+int launch_row(const LsfArgs& a, cudaStream_t st) {
+  const size_t smem = sizeof(float) * (size_t)lsf_row_floats(a.n, KC);
+  if (lsf_row_floats(a.n, KC) > kLsfPre * kLsfRowThreads) {  // a longer row
+    const size_t one = sizeof(float) * ((size_t)(a.n + 3) / 4 * 4 + KC * 4 + 4);
+    cudaError_t e = cudaFuncSetAttribute(lsf_vec_kernel<KC>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one);
+    if (e != cudaSuccess)
+      return set_error(RUBIX_E_CUDA, "cudaFuncSetAttribute(lsf_vec_kernel): %s",
+                       cudaGetErrorString(e));
+    const long long grid = std::min<long long>(a.rows, (long long)sm_count() * 8);
+    lsf_vec_kernel<KC><<<(int)grid, kLsfThreads, one, st>>>(a);
+    RUBIX_LAUNCH_CHECK("lsf_vec_kernel");
+    return RUBIX_OK;
+  }
+  cudaError_t e = cudaFuncSetAttribute(lsf_row_kernel<KC>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess)
-    return set_error(RUBIX_E_CUDA, "cudaFuncSetAttribute(lsf_vec_kernel): %s", cudaGetErrorString(e));
-  long long grid = std::min<long long>(a.rows, (long long)sm_count() * 8);
-  lsf_vec_kernel<KC><<<(int)grid, kLsfThreads, smem, st>>>(a);
-  RUBIX_LAUNCH_CHECK("lsf_vec_kernel");
+    return set_error(RUBIX_E_CUDA, "cudaFuncSetAttribute(lsf_row_kernel): %s",
+                     cudaGetErrorString(e));
+  int per_sm = 0;
+  RUBIX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lsf_row_kernel<KC>,
+                                                               kLsfRowThreads, smem));
+  const long long grid = std::min<long long>(a.rows, (long long)sm_count() * std::max(per_sm, 1));
+  lsf_row_kernel<KC><<<(int)grid, kLsfRowThreads, smem, st>>>(a);
+  RUBIX_LAUNCH_CHECK("lsf_row_kernel");
   return RUBIX_OK;
 }
 
@@ -191,13 +311,13 @@ int lsf_fwd_impl(const float* in, float* out, int64_t n_rows, int32_t n_wave_t,
   // KC = ceil(K/4) weight chunks; each thread's window is KC+1 float4 loads.
   switch ((n_taps + 3) / 4) {
     case 0:
-    case 1: return launch_vec<1>(a, st);
-    case 2: return launch_vec<2>(a, st);
-    case 3: return launch_vec<3>(a, st);
-    case 4: return launch_vec<4>(a, st);
-    case 5: return launch_vec<5>(a, st);
-    case 6: return launch_vec<6>(a, st);
-    case 7: return launch_vec<7>(a, st);
+    case 1: return launch_row<1>(a, st);
+    case 2: return launch_row<2>(a, st);
+    case 3: return launch_row<3>(a, st);
+    case 4: return launch_row<4>(a, st);
+    case 5: return launch_row<5>(a, st);
+    case 6: return launch_row<6>(a, st);
+    case 7: return launch_row<7>(a, st);
     default: break;
   }
   const size_t smem = sizeof(float) * ((size_t)n_wave_t + n_taps + 4);
