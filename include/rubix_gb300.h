@@ -109,8 +109,8 @@ RUBIX_API int rubix_spaxel_sort(const int32_t* idx, const uint8_t* keep, int64_t
 RUBIX_API size_t rubix_cube_workspace_size(int64_t n, int32_t n_segments, int32_t n_wave_t,
                                            int32_t n_met, int32_t n_age, int32_t n_wave);
 
-/* Kernels that rubix_cube_fwd (general = 0), or rubix_cube_fwd_general and
- * rubix_cube_fwd_dust (general = 1), launch for these sizes with a workspace of
+/* Kernels that rubix_cube_fwd and rubix_cube_fwd_dust (general = 0), or
+ * rubix_cube_fwd_general (general = 1), launch for these sizes with a workspace of
  * workspace_bytes. */
 RUBIX_API int rubix_cube_fwd_launches(int64_t n, int32_t n_segments, int32_t n_wave_t,
                                       int32_t n_met, int32_t n_age, int32_t n_wave,
@@ -143,10 +143,11 @@ RUBIX_API int rubix_cube_fwd(const float* ssp_flux, const float* ssp_metallicity
                    size_t workspace_bytes, void* stream);
 
 /*
- * rubix_cube_fwd with every particle evaluated at every telescope wavelength, as
- * rubix_cube_fwd itself does where the template grid does not qualify for the sums over
- * SSP nodes (csrc/cube_nodes.cu).  The two agree to float32 rounding; this one keeps the
- * summation order that the gradients' float64 sums over the cube have been recorded with.
+ * rubix_cube_fwd (av and ext_exponent NULL) or rubix_cube_fwd_dust with every particle
+ * evaluated at every telescope wavelength, as those themselves do where the template grid
+ * does not qualify for sums over SSP nodes (csrc/cube_nodes.cu).  The results agree to
+ * float32 rounding; this one keeps the summation order that float64 sums over the cube (the
+ * gradients of the instrument widths) have been recorded with.
  * Workspace: rubix_cube_general_workspace_size.
  */
 RUBIX_API size_t rubix_cube_general_workspace_size(int64_t n, int32_t n_segments,
@@ -157,8 +158,9 @@ RUBIX_API int rubix_cube_fwd_general(const float* ssp_flux, const float* ssp_met
                    int32_t n_age, int32_t n_wave, const float* wave_t, int32_t n_wave_t,
                    const float* mass, const float* metallicity, const float* age,
                    const float* velocity, int64_t vel_stride, int32_t vel_component,
-                   const int32_t* perm, const int32_t* seg_offsets, int32_t n_segments,
-                   int64_t n, const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop,
+                   const float* av, const float* ext_exponent, const int32_t* perm,
+                   const int32_t* seg_offsets, int32_t n_segments, int64_t n,
+                   const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop,
                    float* cube, int64_t spaxel_stride, void* workspace,
                    size_t workspace_bytes, void* stream);
 

@@ -50,7 +50,7 @@ SIGNATURES = {
     "rubix_cube_fwd_general": (
         _c.c_int,
         [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp, _i32,
-         _vp, _vp, _vp, _vp, _i64, _i32,
+         _vp, _vp, _vp, _vp, _i64, _i32, _vp, _vp,
          _vp, _vp, _i32, _i64, _vp, _i32, _i32, _vp, _i64, _vp, _sz, _vp],
     ),
     "rubix_cube_general_workspace_size": (_sz, [_i64, _i32, _i32, _i32, _i32, _i32]),

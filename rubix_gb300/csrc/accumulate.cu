@@ -65,10 +65,6 @@ struct MainArgs {
   int lsf_k, lsf_crop;  // lsf_k = 0: no LSF epilogue
   float lsf[kMaxLsfTaps + 1];
   const float* dust_e2;  // per telescope wavelength: -0.4 log2(10) A(lambda)/A(V)
-  // not null: the spaxels that the node path leaves, gate[0] items of several-chunk
-  // spaxels at items[0..) and gate[1] others at items[split..)
-  const int* gate;
-  int split;
 };
 
 // Shared-memory carve-up of the main kernel (byte offsets, 16-byte aligned): the TMA
@@ -614,8 +610,6 @@ __device__ __forceinline__ void lsf_epilogue_k(const MainArgs& a,
 
 template <int R, bool kDust, bool kStaged>
 __global__ void __launch_bounds__(kAccThreads, 2) cube_main_kernel(MainArgs a) {
-  const int* gate = kDust ? nullptr : a.gate;
-  if (gate && gate[0] + gate[1] == 0) return;
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemLayout SL = smem_layout(kStaged ? a.n_wave : 0, kStaged ? a.pool : 0, a.pool);
   float* s_wz = reinterpret_cast<float*>(smem + SL.wz);
@@ -658,7 +652,7 @@ __global__ void __launch_bounds__(kAccThreads, 2) cube_main_kernel(MainArgs a) {
   // wavelength before the first one (dlambda_0 = 0: rubix's prepend-diff)
   const float lam_prev = a.wave_t[t0 == 0 ? 0 : min(t0 - 1, n_t - 1)];
   const float A0 = a.At[t0 < n_t ? t0 : n_t - 1];
-  const int n_items = gate ? gate[0] + gate[1] : a.ctrl->n_items;
+  const int n_items = a.ctrl->n_items;
   uint32_t phase = 0;
   int step = 0;
   __syncthreads();
@@ -666,9 +660,8 @@ __global__ void __launch_bounds__(kAccThreads, 2) cube_main_kernel(MainArgs a) {
   for (;;) {
     if (tid == 0) s_item = atomicAdd(&a.ctrl->next_item, 1);
     __syncthreads();
-    int item = s_item;
+    const int item = s_item;
     if (item >= n_items) break;
-    if (gate && item >= gate[0]) item += a.split - gate[0];
     const int2 it = a.items[item];
     const int s = it.x, chunk = it.y;
     const int seg_b = a.seg_off[s], seg_e = a.seg_off[s + 1];
@@ -915,8 +908,8 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                   int64_t vel_stride, int32_t vel_component, const int32_t* perm,
                   const int32_t* seg_offsets, int32_t n_segments, int64_t n,
                   const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop, bool nodes,
-                  const float* av, const float* dust_e2, float* cube, int64_t spaxel_stride, void* workspace,
-                  size_t workspace_bytes, void* stream);
+                  const float* av, const float* dust_e2, float* cube, int64_t spaxel_stride,
+                  void* workspace, size_t workspace_bytes, void* stream);
 
 }  // namespace
 }  // namespace rubix
@@ -1000,8 +993,8 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                   int64_t vel_stride, int32_t vel_component, const int32_t* perm,
                   const int32_t* seg_offsets, int32_t n_segments, int64_t n,
                   const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop, bool nodes,
-                  const float* av, const float* dust_e2, float* cube, int64_t spaxel_stride, void* workspace,
-                  size_t workspace_bytes, void* stream) {
+                  const float* av, const float* dust_e2, float* cube, int64_t spaxel_stride,
+                  void* workspace, size_t workspace_bytes, void* stream) {
   {
     bool nothing_to_do = false;
     const int rc = cube_fwd_check_args(who, ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z,
@@ -1042,17 +1035,14 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                       wave_t, n_wave_t, mass, metallicity, age, velocity, vel_stride,
                       vel_component, perm, seg_offsets, n_segments, n, av};
   MainArgs args;
-  args.gate = nullptr;
-  args.split = 0;
   args.chunk = tune.chunk;
-  if (nodes && dust_e2 == nullptr && n > 0 && cube_nodes_supported(n_met, n_age, n_wave, n_wave_t) &&
+  if (nodes && n > 0 && cube_nodes_supported(n_met, n_age, n_wave, n_wave_t) &&
       cube_nodes_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes)) {
     NodeFallback fb;
-    const int rc = cube_nodes_forward(in, lsf_taps, n_lsf_taps, lsf_crop, tune.big_item, cube,
-                                      spaxel_stride, workspace, workspace_bytes, &fb, st);
+    const int rc = cube_nodes_forward(in, dust_e2, lsf_taps, n_lsf_taps, lsf_crop,
+                                      tune.big_item, cube, spaxel_stride, workspace,
+                                      workspace_bytes, &fb, st);
     if (rc != RUBIX_OK) return rc;
-    args.gate = fb.gate;
-    args.split = fb.split;
     args.chunk = fb.chunk;
     L.At = fb.At;
     L.bucket = fb.bucket;
@@ -1153,15 +1143,18 @@ extern "C" int rubix_cube_fwd_general(const float* ssp_flux, const float* ssp_me
                                       const float* wave_t, int32_t n_wave_t, const float* mass,
                                       const float* metallicity, const float* age,
                                       const float* velocity, int64_t vel_stride,
-                                      int32_t vel_component, const int32_t* perm,
+                                      int32_t vel_component, const float* av,
+                                      const float* ext_exponent, const int32_t* perm,
                                       const int32_t* seg_offsets, int32_t n_segments, int64_t n,
                                       const float* lsf_taps, int32_t n_lsf_taps,
                                       int32_t lsf_crop, float* cube, int64_t spaxel_stride,
                                       void* workspace, size_t workspace_bytes, void* stream) {
+  RUBIX_REQUIRE(n == 0 || (av != nullptr) == (ext_exponent != nullptr), RUBIX_E_INVALID,
+                "rubix_cube_fwd_general: A_V and extinction exponent go together");
   return cube_fwd_impl("rubix_cube_fwd_general", ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z,
                        n_met, n_age, n_wave, wave_t, n_wave_t, mass, metallicity, age, velocity,
                        vel_stride, vel_component, perm, seg_offsets, n_segments, n, lsf_taps,
-                       n_lsf_taps, lsf_crop, false, nullptr, nullptr, cube, spaxel_stride,
+                       n_lsf_taps, lsf_crop, false, av, ext_exponent, cube, spaxel_stride,
                        workspace, workspace_bytes, stream);
 }
 
@@ -1181,7 +1174,7 @@ extern "C" int rubix_cube_fwd_dust(const float* ssp_flux, const float* ssp_metal
   return cube_fwd_impl("rubix_cube_fwd_dust", ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z,
                        n_met, n_age, n_wave, wave_t, n_wave_t, mass, metallicity, age, velocity,
                        vel_stride, vel_component, perm, seg_offsets, n_segments, n, lsf_taps,
-                       n_lsf_taps, lsf_crop, false, av, ext_exponent, cube, spaxel_stride, workspace,
+                       n_lsf_taps, lsf_crop, true, av, ext_exponent, cube, spaxel_stride, workspace,
                        workspace_bytes, stream);
 }
 

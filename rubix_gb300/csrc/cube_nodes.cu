@@ -59,10 +59,11 @@ constexpr int kNodeWarps = 20;
 constexpr int kNodeThreads = 32 * kNodeWarps;
 constexpr int kStage = 33;       // staged records of a warp: 32 and one of weight zero
 constexpr int kRuns = 4;
+constexpr int kDustMost = 8;     // samples between two nodes that a lane holds with dust
 
 struct NodeCtrl {
   int flagged;                  // some spaxel is left to cube_main_kernel
-  int left[2];                  // its work items there: of several-chunk spaxels, of others
+  unsigned e_lo, e_hi;          // bits of max(-e), max(e) of the dust exponents, >= 0
   unsigned tile_mask[(kAlphaTiles + 31) / 32];
   unsigned dz_inv, dt_inv;      // ~bits of the smallest SSP / telescope spacing
   unsigned dz_max, dt_max;      // bits of the largest (3e38: not ascending)
@@ -88,10 +89,12 @@ struct NodePlan {
   int k_first, n_own, n_slices;  // first node, nodes of a slice
   int w;                         // samples that a node may cross within a group of particles
   float dt_min, window;          // samples that an item's alpha range may span
+  int most;                      // samples between two nodes at most
 };
 
 // How the grids are cut into slices, from the extrema; every block derives the same plan.
-__device__ __forceinline__ NodePlan node_plan(const NodeCtrl* c, int n_wave, float x_last) {
+__device__ __forceinline__ NodePlan node_plan(const NodeCtrl* c, int n_wave, float x_last,
+                                              bool dust) {
   NodePlan p;
   const float dz = __uint_as_float(~c->dz_inv), dt = __uint_as_float(~c->dt_inv);
   const float dtm = __uint_as_float(c->dt_max), fm = __uint_as_float(c->fmax);
@@ -101,6 +104,7 @@ __device__ __forceinline__ NodePlan node_plan(const NodeCtrl* c, int n_wave, flo
   p.ok = 0;
   p.n_own = 0;
   p.w = 1;
+  p.most = 0;
   p.n_slices = 0;
   p.window = 0.f;
   // lambda' spacing >= alpha*dz minus two roundings of lambda' (|lambda'| < 2^14): at
@@ -111,6 +115,10 @@ __device__ __forceinline__ NodePlan node_plan(const NodeCtrl* c, int n_wave, flo
     return p;
   const float ratio = (dz * (1.f - kAlphaMax) - 4.0e-3f) / dtm;
   p.w = ratio > 2.f ? 2 : 1;
+  p.most = (int)(__uint_as_float(c->dz_max) * (1.f + kAlphaMax) / dt + 1.01f);
+  // with dust every sample is evaluated: fewer than two of them between nodes, or more than
+  // a lane holds, are the general kernel's
+  if (dust && (p.w < 2 || p.most > kDustMost)) return p;
   const float swing = 2.f * kAlphaMax * x_last / dt;  // samples a node moves over all alpha
   for (int r = 0; r < kRuns; ++r) {
     const float hi = __uint_as_float(c->run_max[r]) * (1.f + kAlphaMax) / dt;
@@ -147,13 +155,19 @@ __device__ __forceinline__ float x_ext(const float* __restrict__ wt, int n, int 
 __global__ void __launch_bounds__(256) node_setup_kernel(
     const float* __restrict__ wz, int n_wave, const float* __restrict__ wt, int n_t,
     const float* __restrict__ vel, long long vel_stride, int vel_comp, long long n,
-    NodeCtrl* __restrict__ ctrl) {
+    const float* __restrict__ dust_e, NodeCtrl* __restrict__ ctrl) {
   const long long gtid = blockIdx.x * 256LL + threadIdx.x, gsz = gridDim.x * 256LL;
   if (gtid < n_t - 1) {
     float d = wt[gtid + 1] - wt[gtid];
     const bool bad = !(d > 0.f);
     atomicMax(&ctrl->dt_max, bad ? __float_as_uint(3e38f) : __float_as_uint(d));
     if (!bad) atomicMax(&ctrl->dt_inv, ~__float_as_uint(d));
+  }
+  if (dust_e && gtid < n_t) {
+    const float e = dust_e[gtid];
+    // a value that is not finite makes the limit infinite: every star is flagged
+    atomicMax(&ctrl->e_hi, __float_as_uint(isfinite(e) ? fmaxf(e, 0.f) : kFltMax));
+    atomicMax(&ctrl->e_lo, __float_as_uint(isfinite(e) ? fmaxf(-e, 0.f) : kFltMax));
   }
   const float x0 = wt[0], x1 = wt[n_t - 1];
   const float hi = 1.f + kAlphaMax, lo = 1.f - kAlphaMax;
@@ -283,12 +297,12 @@ __global__ void __launch_bounds__(kPrefixThreads) node_tables_kernel(
 // Bound by FMA issue: 1 GFMA for 1025 rows of a 1326-template grid, 40 TFMA/s on the chip.
 __global__ void __launch_bounds__(128) node_table_product_kernel(
     const float* __restrict__ h, int kpad, const float* __restrict__ flux, int n_templ,
-    int n_wave, const float* __restrict__ wt, int n_t, const NodeCtrl* __restrict__ ctrl,
-    float* __restrict__ H) {
+    int n_wave, const float* __restrict__ wt, int n_t, bool dust,
+    const NodeCtrl* __restrict__ ctrl, float* __restrict__ H) {
   constexpr int BK = 32, BM = kAlphaTile, BN = 32;
   const int tile = blockIdx.y;
   if (!tile_used(ctrl, tile)) return;
-  const NodePlan p = node_plan(ctrl, n_wave, wt[n_t - 1]);
+  const NodePlan p = node_plan(ctrl, n_wave, wt[n_t - 1], dust);
   if (!p.ok) return;
   const int k_last = min(n_wave - ctrl->k_last_inv, n_wave - 1);
   const int K = min(k_last - p.k_first + 1, kpad);
@@ -413,9 +427,17 @@ struct GatherArgs {
   const int2* items;
   float4* rec_w;
   float2* rec_a;
+  float* rec_av;  // dust only
   int* flags;
   int4* desc;
 };
+
+// Largest dust transmission that a column lets through (2^(e A_V) over all wavelengths).
+__device__ __forceinline__ float dust_top(const GatherArgs& a, float av) {
+  if (!a.rec_av) return 1.f;
+  const float up = fmaxf(__uint_as_float(a.ctrl->e_hi) * av, -__uint_as_float(a.ctrl->e_lo) * av);
+  return isfinite(av) ? exp2f(fmaxf(up, 0.f)) : kFltMax;
+}
 
 // One block per work item: the record of each particle (beta times the four corner
 // weights; alpha and the byte offset of its first corner row in the slice table), sorted
@@ -429,7 +451,7 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
   const CubeInputs& in = a.in;
   const int tid = threadIdx.x;
   const float x0 = in.wave_t[0], x1 = in.wave_t[in.n_wave_t - 1];
-  if (tid == 0) s_plan = node_plan(a.ctrl, in.n_wave, x1);
+  if (tid == 0) s_plan = node_plan(a.ctrl, in.n_wave, x1, a.rec_av != nullptr);
   __syncthreads();
   const NodePlan plan = s_plan;
   const float fmax = __uint_as_float(a.ctrl->fmax);
@@ -446,20 +468,22 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
     for (int j0 = jb; j0 < je && plan.ok; j0 += kSub) {
       const int m = min(kSub, je - j0);
       float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-      float alpha = 1.f;
+      float alpha = 1.f, av = 0.f;
       int row = 0;
       bool bad = false;
       if (tid < m) {
         const long long i = in.perm[j0 + tid];
         const float Z = in.met[i], A = in.age[i], mass = in.mass[i];
         alpha = doppler_factor(in.vel[i * in.vel_stride + in.vel_comp]);
+        if (a.rec_av) av = in.av[i];
         const bool outside = (Z < in.ssp_met[0]) || (Z > in.ssp_met[in.n_met - 1]) ||
                              (A < in.ssp_age[0]) || (A > in.ssp_age[in.n_age - 1]);
         if (!(fabsf(alpha - 1.f) <= kAlphaMax)) {
           bad = true;
           alpha = 1.f;
         } else if (outside) {
-          bad = !isfinite(mass);  // an all-zero spectrum unless 0 * mass is not 0
+          // an all-zero spectrum unless 0 times the mass or the transmission is not 0
+          bad = !isfinite(mass) || !(dust_top(a, av) < 1e30f);
         } else {
           const int iz = min(max(count_le(in.ssp_met, in.n_met, Z), 1), in.n_met - 1);
           const int ia = min(max(count_le(in.ssp_age, in.n_age, A), 1), in.n_age - 1);
@@ -494,9 +518,10 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
             T *= alpha;
             const float sc = T / Tp;
             const float beta = mass != 0.f ? mass * sc : 0.f;
-            const float top = fabsf(beta) * fmax;
+            const float top = fabsf(beta) * fmax;  // without dust dust_top is 1
             // what the general kernel treats specially, or what may leave float32's range
-            bad = !(sc > 0.25f && sc < 4.f) || !(top < 1e30f) || (beta != 0.f && !(top > 1e-25f));
+            bad = !(sc > 0.25f && sc < 4.f) || !(top * dust_top(a, av) < 1e30f) ||
+                  (beta != 0.f && !(top > 1e-25f));
             w = make_float4(beta * wc[0], beta * wc[1], beta * wc[2], beta * wc[3]);
           }
         }
@@ -517,6 +542,7 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
         }
         a.rec_w[j0 + rank] = w;
         a.rec_a[j0 + rank] = make_float2(alpha, __int_as_float(row * 128));
+        if (a.rec_av) a.rec_av[j0 + rank] = av;
       }
       __syncthreads();
     }
@@ -554,6 +580,8 @@ struct SliceArgs {
   const int4* desc;  // per item: first record, records, smallest and largest alpha
   const float4* rec_w;
   const float2* rec_a;
+  const float* rec_av;  // dust only, with the exponents per telescope wavelength
+  const float* dust_e;
   float* rows;    // [row][slice][kMaxBins]
   int2* row_pos;  // [row][slice]: first extended sample, samples
   NodeCtrl* ctrl;
@@ -599,7 +627,9 @@ struct StagedRecs {
 struct SliceShared {
   const float* tab;  // [template][32]
   const float* xw;   // window of the extended telescope grid, kWin samples
+  const float* ew;   // with dust: the exponents of the window's samples
   StagedRecs* st;    // this warp's staged records
+  float* st_av;      // with dust: their columns
   float* f;          // this warp's samples, kMaxBins
   float inv;         // samples per Angstrom over the window
 };
@@ -794,6 +824,95 @@ struct SliceItem {
   }
 };
 
+// The same with a dust column in front of every particle: its spectrum is multiplied by
+// 2^(e_t A_V) (spectra/dust/dust_baseclasses.py:163-164), so every sample is evaluated, one
+// node and its up to M samples per lane, one particle at a time.  The group's samples, their
+// exponents and sums stay in registers.  Bound by the 2^x rate (16 a cycle and SM) and issue:
+// about 60 instructions and 7 multi-function ones per particle and 32 nodes.
+template <int M>
+struct DustItem {
+  static constexpr int W = 2;
+  const SliceShared& sh;
+  const int lane;
+  const bool mine;
+  const float lam, lam_r;
+  const char* tab;
+  int j;
+  float xo, d[M], e[M], acc[M];
+
+  __device__ __forceinline__ DustItem(const SliceShared& s, int lane_, int n_own,
+                                      const float* __restrict__ l)
+      : sh(s), lane(lane_), mine(lane_ >= 1 && lane_ <= n_own), lam(l[lane_]),
+        lam_r(l[lane_ + 1]), tab(reinterpret_cast<const char*>(s.tab) + 4 * lane_) {}
+
+  __device__ __forceinline__ void open(float alpha) {
+    j = sample_at(sh, __fmul_rn(lam, alpha));
+    xo = sh.xw[j];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int q = min(j + m, kWin - 1);
+      d[m] = sh.xw[q] - xo;
+      e[m] = sh.ew[q];
+      acc[m] = 0.f;
+    }
+  }
+
+  __device__ __forceinline__ void flush(int jb) {
+    const int jn = __shfl_down_sync(0xffffffffu, j, 1);
+    if (mine) {
+      float* f = sh.f - jb;
+      const int e1 = min(jn, jb + kMaxBins);
+      float v[M];
+#pragma unroll
+      for (int m = 0; m < M; ++m) v[m] = j + m < e1 ? f[j + m] : 0.f;
+#pragma unroll
+      for (int m = 0; m < M; ++m)
+        if (j + m < e1) f[j + m] = v[m] + acc[m];
+    }
+    __syncwarp();
+  }
+
+  struct Loaded {
+    float c[4], w[4], alpha, av;
+  };
+  __device__ __forceinline__ void load(int r, int zoff, Loaded& v) const {
+    const StagedRecs& st = *sh.st;
+    const char* t0 = tab + st.row[r];
+    v.c[0] = *reinterpret_cast<const float*>(t0);
+    v.c[1] = *reinterpret_cast<const float*>(t0 + zoff);
+    v.c[2] = *reinterpret_cast<const float*>(t0 + 128);
+    v.c[3] = *reinterpret_cast<const float*>(t0 + zoff + 128);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v.w[k] = st.w[k][r];
+    v.alpha = st.alpha[r];
+    v.av = sh.st_av[r];
+  }
+  __device__ __forceinline__ void step(const Loaded& v) {
+    float G = v.w[0] * v.c[0];
+    G = fmaf(v.w[1], v.c[1], G);
+    G = fmaf(v.w[2], v.c[2], G);
+    G = fmaf(v.w[3], v.c[3], G);
+    const float lp = __fmul_rn(lam, v.alpha);
+    const float G_r = __shfl_down_sync(0xffffffffu, G, 1);
+    const float s = (G_r - G) * fast_rcp(__fmul_rn(lam_r, v.alpha) - lp);
+    const float s_l = __shfl_up_sync(0xffffffffu, s, 1);
+    const float t = xo - lp;
+    const float base = fmaf(s, t, G);
+    const float c = s_l - s;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      float y = fmaf(s, d[m], base);
+      if (m < W) y = fmaf(c, fminf(t + d[m], 0.f), y);
+      acc[m] = fmaf(y, dust_transmission(e[m], v.av), acc[m]);
+    }
+  }
+};
+
+template <class T>
+struct TypeOf {
+  using type = T;
+};
+
 // Item of a warp: its first record and record count, its smallest and largest alpha.
 struct ItemDesc {
   int p0, np;
@@ -809,12 +928,13 @@ struct ItemDesc {
 // +15 %), four nodes a lane beat two by 6 % and one by 8 %, W = 2 needs half the flushes of
 // W = 1, W = 3 costs more per step than it saves.  A warp's next item, its description and its first records are fetched while the one before
 // is processed.  A block whose slice has no items left takes the slice with the most.
-template <int NPL, int W>
+template <class Item, int NPL, bool kDust>
 __device__ __forceinline__ void slice_items(const SliceArgs& a, const SliceShared& sh,
                                             const float* s_lam, int n_own, int lane, int slice,
                                             int n_slices, int i0, int total, int e0, float w_seg,
                                             int n_multi, int wave_items, int* __restrict__ next) {
-  SliceItem<NPL, W> w(sh, lane, n_own, s_lam);
+  Item w(sh, lane, n_own, s_lam);
+  const int grp = lane / (32 / NPL);  // the lane's particle of a step
   const int zoff = a.n_age * 128;
   const float lam_lo = s_lam[1], lam_hi = s_lam[n_own + 1];
   auto take = [&]() { return lane == 0 ? atomicAdd(next, 1) : 0; };
@@ -828,10 +948,12 @@ __device__ __forceinline__ void slice_items(const SliceArgs& a, const SliceShare
   };
   float4 rw = make_float4(0.f, 0.f, 0.f, 0.f);
   float2 ra = make_float2(1.f, 0.f);
+  float rv = 0.f;
   auto fetch = [&](int p, int n) {
     rw = make_float4(0.f, 0.f, 0.f, 0.f);
     ra = make_float2(1.f, 0.f);
     if (lane < n) {
+      if (kDust) rv = a.rec_av[(long long)p + lane];
       rw = a.rec_w[(long long)p + lane];
       ra = a.rec_a[(long long)p + lane];
     }
@@ -857,6 +979,7 @@ __device__ __forceinline__ void slice_items(const SliceArgs& a, const SliceShare
       sh.st->w[3][lane] = rw.w;
       sh.st->alpha[lane] = ra.x;
       sh.st->row[lane] = __float_as_int(ra.y);
+      if (kDust) sh.st_av[lane] = rv;
       const float al = ra.x;
       __syncwarp();
       if (base + 32 < d.np) fetch(d.p0 + base + 32, d.np - base - 32);
@@ -875,11 +998,11 @@ __device__ __forceinline__ void slice_items(const SliceArgs& a, const SliceShare
         const unsigned past =
             __ballot_sync(0xffffffffu, lane > pos && lane < cnt && al >= a_lim);
         const int end = past ? __ffs(past) - 1 : cnt;
-        typename SliceItem<NPL, W>::Loaded v;
-        w.load(pos + w.g < end ? pos + w.g : 32, zoff, v);  // 32: a record of weight zero
+        typename Item::Loaded v;
+        w.load(pos + grp < end ? pos + grp : 32, zoff, v);  // 32: a record of weight zero
         for (int p = pos + NPL; p < end; p += NPL) {
-          const typename SliceItem<NPL, W>::Loaded u = v;
-          w.load(p + w.g < end ? p + w.g : 32, zoff, v);
+          const typename Item::Loaded u = v;
+          w.load(p + grp < end ? p + grp : 32, zoff, v);
           w.step(u);
         }
         w.step(v);
@@ -905,18 +1028,21 @@ __device__ __forceinline__ void slice_items(const SliceArgs& a, const SliceShare
   }
 }
 
+template <bool kDust>
 __global__ void __launch_bounds__(kNodeThreads, 1) node_slice_kernel(SliceArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   float* s_tab = reinterpret_cast<float*>(smem);
   float* s_xw = s_tab + (size_t)a.n_templ * 32;
   StagedRecs* s_st = reinterpret_cast<StagedRecs*>(s_xw + kWin);
   float* s_f = reinterpret_cast<float*>(s_st + kNodeWarps);
+  float* s_ew = s_f + kNodeWarps * kMaxBins;  // dust only
+  float* s_av = s_ew + kWin;
   __shared__ float s_lam[36];
   __shared__ NodePlan s_plan;
   __shared__ int s_slice, s_e0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float x_last = a.wt[a.n_t - 1];
-  if (tid == 0) s_plan = node_plan(a.ctrl, a.n_wave, x_last);
+  if (tid == 0) s_plan = node_plan(a.ctrl, a.n_wave, x_last, kDust);
   __syncthreads();
   const NodePlan plan = s_plan;
   if (!plan.ok) return;
@@ -930,7 +1056,10 @@ __global__ void __launch_bounds__(kNodeThreads, 1) node_slice_kernel(SliceArgs a
   sh.xw = s_xw;
   sh.st = s_st + warp;
   sh.f = s_f + warp * kMaxBins;
+  sh.ew = s_ew;
+  sh.st_av = s_av + warp * kStage;
   if (lane == 0) {
+    if (kDust) sh.st_av[32] = 0.f;
     for (int k = 0; k < 4; ++k) sh.st->w[k][32] = 0.f;
     sh.st->alpha[32] = 1.f;
     sh.st->row[32] = 0;
@@ -961,15 +1090,28 @@ __global__ void __launch_bounds__(kNodeThreads, 1) node_slice_kernel(SliceArgs a
     }
     __syncthreads();
     const int e0 = s_e0;
-    for (int q = tid; q < kWin; q += kNodeThreads) s_xw[q] = x_ext(a.wt, a.n_t, e0 + q);
+    for (int q = tid; q < kWin; q += kNodeThreads) {
+      s_xw[q] = x_ext(a.wt, a.n_t, e0 + q);
+      if (kDust) s_ew[q] = a.dust_e[min(max(e0 + q - kExt, 0), a.n_t - 1)];
+    }
     __syncthreads();
     sh.inv = (float)(kWin - 1) / (s_xw[kWin - 1] - s_xw[0]);
-    if (plan.w == 1)
-      slice_items<2, 1>(a, sh, s_lam, plan.n_own, lane, slice, plan.n_slices, i0, total, e0,
-                        w_seg, a.ctrl->n_multi, wave_items, next + slice);
-    else
-      slice_items<4, 2>(a, sh, s_lam, plan.n_own, lane, slice, plan.n_slices, i0, total, e0,
-                        w_seg, a.ctrl->n_multi, wave_items, next + slice);
+    auto run = [&](auto item, auto npl) {
+      slice_items<typename decltype(item)::type, decltype(npl)::value, kDust>(
+          a, sh, s_lam, plan.n_own, lane, slice, plan.n_slices, i0, total, e0, w_seg,
+          a.ctrl->n_multi, wave_items, next + slice);
+    };
+    using I1 = std::integral_constant<int, 1>;
+    using I2 = std::integral_constant<int, 2>;
+    using I4 = std::integral_constant<int, 4>;
+    if constexpr (kDust) {
+      if (plan.most <= 4) run(TypeOf<DustItem<4>>{}, I1{});
+      else if (plan.most <= 6) run(TypeOf<DustItem<6>>{}, I1{});
+      else run(TypeOf<DustItem<kDustMost>>{}, I1{});
+    } else {
+      if (plan.w == 1) run(TypeOf<SliceItem<2, 1>>{}, I2{});
+      else run(TypeOf<SliceItem<4, 2>>{}, I4{});
+    }
     __syncthreads();
     if (tid == 0) {
       int best = -1, most = 2 * kNodeWarps;
@@ -1000,6 +1142,7 @@ struct MergeArgs {
   const int2* row_pos;
   const NodeCtrl* ctrl;
   int wave, multi_rows;
+  bool dust;
   long long slice_rows;
   float* cube;
   long long stride;
@@ -1018,7 +1161,7 @@ __global__ void __launch_bounds__(kMergeThreads) node_merge_kernel(MergeArgs a) 
   extern __shared__ float s_buf[];
   __shared__ NodePlan s_plan;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_plan = node_plan(a.ctrl, a.n_wave, a.wt[a.n_t - 1]);
+  if (tid == 0) s_plan = node_plan(a.ctrl, a.n_wave, a.wt[a.n_t - 1], a.dust);
   __syncthreads();
   const int n_slices = s_plan.n_slices;
   const int K = a.lsf_k, n_t = a.n_t;
@@ -1112,7 +1255,7 @@ __global__ void __launch_bounds__(kMergeThreads) node_merge_kernel(MergeArgs a) 
 
 size_t slice_smem(int n_templ) {
   return sizeof(float) * ((size_t)n_templ * 32 + kWin + kNodeWarps * kMaxBins) +
-         sizeof(StagedRecs) * kNodeWarps;
+         sizeof(StagedRecs) * kNodeWarps + sizeof(float) * (kWin + kNodeWarps * kStage);
 }
 
 size_t row_bytes(int n_wave) {
@@ -1135,6 +1278,7 @@ struct NodeLayout {
   float* H;
   float4* rec_w;
   float2* rec_a;
+  float* rec_av;
   float* rows;
   int2* row_pos;
   size_t shared_off, fixed;  // start of the shared region; bytes without rows
@@ -1159,6 +1303,7 @@ NodeLayout carve_nodes(void* ws, long long n, int n_seg, int nZ, int nA, int nW)
   L.H = c.take<float>((size_t)kAlphaRows * nZ * nA);
   L.rec_w = c.take<float4>((size_t)n);
   L.rec_a = c.take<float2>((size_t)n);
+  L.rec_av = c.take<float>((size_t)n);
   L.fixed = c.off;
   L.rows = nullptr;
   L.row_pos = nullptr;
@@ -1174,9 +1319,8 @@ NodeFallback carve_fallback(Carve& c, const CubeInputs& in) {
   f.done = c.take<int>((size_t)in.n_seg);
   f.slot_start = c.take<int>((size_t)in.n_seg);
   f.chunk = kMaxChunk;
-  f.split = (int)max_slots(in.n, kMaxChunk);
-  f.items = c.take<int2>((size_t)f.split + in.n_seg);
-  f.partials = c.take<float>((size_t)f.split * in.n_wave_t);
+  f.items = c.take<int2>((size_t)max_slots(in.n, kMaxChunk) + in.n_seg);
+  f.partials = c.take<float>((size_t)max_slots(in.n, kMaxChunk) * in.n_wave_t);
   return f;
 }
 
@@ -1197,7 +1341,8 @@ size_t fallback_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
 __global__ void __launch_bounds__(256) node_fallback_kernel(CubeInputs in, NodeFallback f,
                                                             const double* __restrict__ prefix,
                                                             const int* __restrict__ flags,
-                                                            NodeCtrl* __restrict__ nc) {
+                                                            const NodeCtrl* __restrict__ nc,
+                                                            CubeCtrl* __restrict__ ctrl) {
   if (!nc->flagged) return;
   const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
   double lnq0, h;
@@ -1206,21 +1351,36 @@ __global__ void __launch_bounds__(256) node_fallback_kernel(CubeInputs in, NodeF
     f.At[t] = (float)((log((double)in.wave_t[t]) - lnq0) / h);
   for (int b = gtid; b < kBuckets; b += gsz)
     f.bucket[b] = bucket_entry(in.ssp_wave_z, in.n_wave, lnq0, h, b);
-  for (int s = gtid; s < in.n_seg; s += gsz) {
-    if (!flags[s]) continue;
-    const int cnt = in.seg_off[s + 1] - in.seg_off[s];
-    const int nch = (cnt + f.chunk - 1) / f.chunk;
-    const int at = nch > 1 ? atomicAdd(&nc->left[0], nch) : f.split + atomicAdd(&nc->left[1], 1);
-    f.slot_start[s] = at;
-    f.done[s] = 0;
-    for (int c = 0; c < nch; ++c) f.items[at + c] = make_int2(s, c);
+  if (blockIdx.x == 0) {
+    // the flagged spaxels' items: those of several chunks first
+    __shared__ int s_multi, s_single;
+    if (threadIdx.x == 0) s_multi = s_single = 0;
+    __syncthreads();
+    for (int pass = 0; pass < 2; ++pass) {
+      for (int s = threadIdx.x; s < in.n_seg; s += blockDim.x) {
+        if (!flags[s]) continue;
+        const int cnt = in.seg_off[s + 1] - in.seg_off[s];
+        const int nch = (cnt + f.chunk - 1) / f.chunk;
+        if ((nch > 1) != (pass == 0)) continue;
+        const int at = atomicAdd(pass == 0 ? &s_multi : &s_single, nch);
+        f.slot_start[s] = at;
+        f.done[s] = 0;
+        for (int c = 0; c < nch; ++c) f.items[at + c] = make_int2(s, c);
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        if (pass == 0) s_single = s_multi;
+        else ctrl->n_items = s_single;
+      }
+      __syncthreads();
+    }
   }
   corner_table(in.ssp_flux, in.n_met, in.n_age, in.n_wave, f.ct);
   gather_records(in.mass, in.met, in.age, in.vel, in.vel_stride, in.vel_comp, in.perm,
                  in.seg_off, in.n_seg, in.n, in.ssp_met, in.n_met, in.ssp_age, in.n_age,
                  in.ssp_wave_z, in.n_wave, in.wave_t, in.n_wave_t, prefix, 1.0 / h,
                  (float)(kVmaxKms / kSpeedOfLight / h), __uint_as_float(~nc->dz_inv),
-                 __uint_as_float(nc->dt_max), f.rec, 0, nullptr,
+                 __uint_as_float(nc->dt_max), f.rec, 0, in.av,
                  (float)exp(-kVmaxKms / kSpeedOfLight), (float)exp(kVmaxKms / kSpeedOfLight));
 }
 
@@ -1257,7 +1417,7 @@ int cube_nodes_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t b
   return 8 + 2 * (int)((n_seg + wave - 1) / wave);
 }
 
-int cube_nodes_forward(const CubeInputs& in, const float* lsf_taps, int n_lsf, int lsf_crop,
+int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* lsf_taps, int n_lsf, int lsf_crop,
                        int big_item, float* cube, long long stride, void* ws, size_t ws_bytes,
                        NodeFallback* fb, cudaStream_t st) {
   NodeLayout L = carve_nodes(ws, in.n, in.n_seg, in.n_met, in.n_age, in.n_wave);
@@ -1280,7 +1440,7 @@ int cube_nodes_forward(const CubeInputs& in, const float* lsf_taps, int n_lsf, i
     const int need = (std::max(in.n_wave_t, nW) + 255) / 256;
     node_setup_kernel<<<std::max(g, need), 256, 0, st>>>(in.ssp_wave_z, nW, in.wave_t,
                                                          in.n_wave_t, in.vel, in.vel_stride,
-                                                         in.vel_comp, in.n, L.ctrl);
+                                                         in.vel_comp, in.n, dust_e, L.ctrl);
     RUBIX_LAUNCH_CHECK("node_setup_kernel");
   }
   const int kpad = kpad_of(nW);
@@ -1290,7 +1450,8 @@ int cube_nodes_forward(const CubeInputs& in, const float* lsf_taps, int n_lsf, i
         L.ctrl);
     RUBIX_LAUNCH_CHECK("node_tables_kernel");
     node_table_product_kernel<<<dim3((n_templ + 31) / 32, kAlphaTiles), 128, 0, st>>>(
-        L.h, kpad, in.ssp_flux, n_templ, nW, in.wave_t, in.n_wave_t, L.ctrl, L.H);
+        L.h, kpad, in.ssp_flux, n_templ, nW, in.wave_t, in.n_wave_t, dust_e != nullptr,
+        L.ctrl, L.H);
     RUBIX_LAUNCH_CHECK("node_table_product_kernel");
   }
   {
@@ -1306,14 +1467,16 @@ int cube_nodes_forward(const CubeInputs& in, const float* lsf_taps, int n_lsf, i
   }
   const long long items_max = multi_rows + std::min<long long>(in.n_seg, in.n);
   {
-    GatherArgs g{in, L.prefix, L.H, L.ctrl, L.items, L.rec_w, L.rec_a, L.flags, L.desc};
+    GatherArgs g{in, L.prefix, L.H, L.ctrl, L.items, L.rec_w, L.rec_a,
+                 dust_e ? L.rec_av : nullptr, L.flags, L.desc};
     const int blocks = (int)std::min<long long>(items_max, (long long)sm_count() * 8);
     node_gather_kernel<<<blocks, kSub, 0, st>>>(g);
     RUBIX_LAUNCH_CHECK("node_gather_kernel");
   }
   const size_t smem = slice_smem(n_templ);
-  RUBIX_CUDA_TRY(cudaFuncSetAttribute(node_slice_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const auto slice_kernel = dust_e ? node_slice_kernel<true> : node_slice_kernel<false>;
+  RUBIX_CUDA_TRY(cudaFuncSetAttribute(slice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
   MergeArgs m;
   m.seg_off = in.seg_off;
   m.multi = L.multi;
@@ -1329,6 +1492,7 @@ int cube_nodes_forward(const CubeInputs& in, const float* lsf_taps, int n_lsf, i
   m.row_pos = L.row_pos;
   m.ctrl = L.ctrl;
   m.multi_rows = (int)multi_rows;
+  m.dust = dust_e != nullptr;
   m.slice_rows = (long long)total_rows;
   m.cube = cube;
   m.stride = stride;
@@ -1337,8 +1501,8 @@ int cube_nodes_forward(const CubeInputs& in, const float* lsf_taps, int n_lsf, i
   for (int i = 0; i <= kMaxLsfTaps; ++i) m.lsf[i] = i < n_lsf ? lsf_taps[i] : 0.f;
   for (int w = 0; w < waves; ++w) {
     const SliceArgs a{in.ssp_flux, in.ssp_wave_z, in.wave_t, n_templ, in.n_age, nW, in.n_wave_t,
-                      L.desc, L.rec_w, L.rec_a, L.rows, L.row_pos, L.ctrl, w, (int)multi_rows, in.n_seg, (long long)total_rows};
-    node_slice_kernel<<<sm_count(), kNodeThreads, smem, st>>>(a);
+                      L.desc, L.rec_w, L.rec_a, L.rec_av, dust_e, L.rows, L.row_pos, L.ctrl, w, (int)multi_rows, in.n_seg, (long long)total_rows};
+    slice_kernel<<<sm_count(), kNodeThreads, smem, st>>>(a);
     RUBIX_LAUNCH_CHECK("node_slice_kernel");
     m.wave = w;
     const int blocks = (int)std::min<long long>(in.n_seg, (long long)sm_count() * 8);
@@ -1362,9 +1526,9 @@ int cube_nodes_forward(const CubeInputs& in, const float* lsf_taps, int n_lsf, i
   // The flagged spaxels, if any, in the region that the slices no longer need.
   Carve c(static_cast<char*>(ws) + L.shared_off);
   *fb = carve_fallback(c, in);
-  fb->gate = L.ctrl->left;
   const int blocks = sm_count() * 8;
-  node_fallback_kernel<<<blocks, 256, 0, st>>>(in, *fb, L.prefix, L.flags, L.ctrl);
+  node_fallback_kernel<<<blocks, 256, 0, st>>>(in, *fb, L.prefix, L.flags, L.ctrl,
+                                               static_cast<CubeCtrl*>(ws));
   RUBIX_LAUNCH_CHECK("node_fallback_kernel");
   return RUBIX_OK;
 }

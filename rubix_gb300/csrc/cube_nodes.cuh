@@ -5,12 +5,11 @@
 
 namespace rubix {
 
-// What the node path leaves for cube_main_kernel: the flagged spaxels and its inputs
-// (built only when some spaxel is flagged; all pointers are device memory).
+// What the node path leaves for cube_main_kernel: the work items of the flagged spaxels
+// (their number in the workspace's CubeCtrl, 0 when none is flagged) and its inputs.
 struct NodeFallback {
-  const int* gate;  // work items: of several-chunk spaxels, of the others
-  int2* items;      // the former from 0, the latter from split
-  int split, chunk;
+  int chunk;
+  int2* items;  // items of several-chunk spaxels (item index = partial slot), then others
   int* slot_start;
   float* At;
   int2* bucket;
@@ -21,7 +20,8 @@ struct NodeFallback {
 };
 
 // Runs the node path: the cube of every spaxel that is not flagged, and *fb for the rest.
-int cube_nodes_forward(const CubeInputs& in, const float* lsf_taps, int n_lsf, int lsf_crop,
+// dust_e: dust exponents per telescope wavelength (with in.av), or null.
+int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* lsf_taps, int n_lsf, int lsf_crop,
                        int big_item, float* cube, long long stride, void* ws, size_t ws_bytes,
                        NodeFallback* fb, cudaStream_t st);
 

@@ -164,7 +164,6 @@ def cube_forward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, m
         if out.dim() != 2 or out.shape[0] != n_segments or out.shape[1] < L or out.stride(1) != 1:
             raise ValueError("out must be [n_segments, >=L] with unit stride along wavelength")
     lsf = None if lsf_taps is None else _host_taps(lsf_taps)
-    general = general or dust_av is not None
     nbytes = _lib.query("rubix_cube_general_workspace_size" if general
                         else "rubix_cube_workspace_size", n, int(n_segments), L, nz, na, nw)
     ws = workspace(nbytes, dev)
@@ -172,23 +171,25 @@ def cube_forward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, m
                 int(lsf_crop))
     if (dust_av is None) != (dust_exponent is None):
         raise ValueError("dust_av and dust_exponent go together")
-    if dust_av is None:
-        _lib.call("rubix_cube_fwd_general" if general else "rubix_cube_fwd", _ptr(ssp_flux), _ptr(ssp_metallicity), _ptr(ssp_age),
-                  _ptr(ssp_wave_z), nz, na, nw, _ptr(wave_t), L, _ptr(mass), _ptr(metallicity),
-                  _ptr(age), _ptr(velocity), vstride, int(vel_component), _ptr(perm),
-                  _ptr(seg_offsets), int(n_segments), n, *lsf_args, _ptr(out), out.stride(0),
-                  _ptr(ws), ws.numel(), _stream(dev))
-    else:
+    ssp_args = (_ptr(ssp_flux), _ptr(ssp_metallicity), _ptr(ssp_age), _ptr(ssp_wave_z), nz, na,
+                nw, _ptr(wave_t), L)
+    star_args = (_ptr(mass), _ptr(metallicity), _ptr(age), _ptr(velocity), vstride,
+                 int(vel_component))
+    out_args = (_ptr(perm), _ptr(seg_offsets), int(n_segments), n, *lsf_args, _ptr(out),
+                out.stride(0), _ptr(ws), ws.numel(), _stream(dev))
+    if dust_av is not None:
         dust_av = _contig("dust_av", dust_av, torch.float32).reshape(-1)
         dust_exponent = _contig("dust_exponent", dust_exponent, torch.float32).reshape(-1)
         if dust_av.numel() != n or dust_exponent.numel() != L:
             raise ValueError("dust_av must be [n] and dust_exponent [L]")
-        _lib.call("rubix_cube_fwd_dust", _ptr(ssp_flux), _ptr(ssp_metallicity),
-                  _ptr(ssp_age), _ptr(ssp_wave_z), nz, na, nw, _ptr(wave_t), L, _ptr(mass),
-                  _ptr(metallicity), _ptr(age), _ptr(velocity), vstride, int(vel_component),
-                  _ptr(dust_av), _ptr(dust_exponent), _ptr(perm), _ptr(seg_offsets),
-                  int(n_segments), n, *lsf_args, _ptr(out), out.stride(0), _ptr(ws),
-                  ws.numel(), _stream(dev))
+    if general:
+        _lib.call("rubix_cube_fwd_general", *ssp_args, *star_args, _ptr(dust_av),
+                  _ptr(dust_exponent), *out_args)
+    elif dust_av is None:
+        _lib.call("rubix_cube_fwd", *ssp_args, *star_args, *out_args)
+    else:
+        _lib.call("rubix_cube_fwd_dust", *ssp_args, *star_args, _ptr(dust_av),
+                  _ptr(dust_exponent), *out_args)
     _count(_lib.query("rubix_cube_fwd_launches", n, int(n_segments), L, nz, na, nw,
                       1 if general else 0, ws.numel()))
     if check and n_segments > 0:

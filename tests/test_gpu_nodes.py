@@ -38,7 +38,7 @@ def _problem(counts, ssp=(12, 4, 400), wave=(4700.15, 9351.4), res=5.0, seed=0, 
     return s, tel.cosmological_doppler_shift(dist_z, s.wavelength), wt, p, offs
 
 
-def _run(lib, prob, general, lsf=None):
+def _run(lib, prob, general, lsf=None, av=None):
     import torch
 
     from rubix_gb300 import _lib
@@ -54,24 +54,31 @@ def _run(lib, prob, general, lsf=None):
     ws = torch.zeros(size, dtype=torch.uint8, device="cuda")
     out = torch.full((nseg, L), float("nan"), device="cuda")
     taps = None if lsf is None else np.asarray(lsf, np.float32)
-    _lib.call("rubix_cube_fwd_general" if general else "rubix_cube_fwd", *[t.data_ptr() for t in d[:4]], nz, na, nw, d[4].data_ptr(), L,
-              *[t.data_ptr() for t in d[5:9]], 1, 0, perm.data_ptr(), off.data_ptr(), nseg, n,
-              None if taps is None else taps.ctypes.data, 0 if taps is None else taps.size,
-              0 if taps is None else taps.size // 2, out.data_ptr(), L, ws.data_ptr(), size,
-              torch.cuda.current_stream().cuda_stream)
+    dust = []
+    if av is not None or general:
+        e = None if av is None else to_dev((-1.33 * (wt / 5500.0) ** -0.7).astype(np.float32))
+        v = None if av is None else to_dev(np.asarray(av, np.float32))
+        dust = [None if t is None else t.data_ptr() for t in (v, e)]
+    name = "rubix_cube_fwd_general" if general else (
+        "rubix_cube_fwd" if av is None else "rubix_cube_fwd_dust")
+    _lib.call(name, *[t.data_ptr() for t in d[:4]], nz, na, nw, d[4].data_ptr(), L,
+              *[t.data_ptr() for t in d[5:9]], 1, 0, *dust, perm.data_ptr(), off.data_ptr(),
+              nseg, n, None if taps is None else taps.ctypes.data,
+              0 if taps is None else taps.size, 0 if taps is None else taps.size // 2,
+              out.data_ptr(), L, ws.data_ptr(), size, torch.cuda.current_stream().cuda_stream)
     err = ctypes.c_int(0)
     _lib.call("rubix_cube_status", ws.data_ptr(), ctypes.byref(err),
               torch.cuda.current_stream().cuda_stream)
     return out.cpu().numpy()
 
 
-def _compare(lib, prob, lsf=None):
-    a, b = _run(lib, prob, False, lsf), _run(lib, prob, True, lsf)
+def _compare(lib, prob, lsf=None, av=None):
+    a, b = _run(lib, prob, False, lsf, av), _run(lib, prob, True, lsf, av)
     assert np.array_equal(np.isfinite(a), np.isfinite(b))
     assert np.array_equal(np.isnan(a), np.isnan(b))
     c = b
     if (prob[3]["mass"] < 0).any():  # the bound is on sums of one sign
-        c = _run(lib, prob[:3] + (dict(prob[3], mass=np.abs(prob[3]["mass"])), prob[4]), True, lsf)
+        c = _run(lib, prob[:3] + (dict(prob[3], mass=np.abs(prob[3]["mass"])), prob[4]), True, lsf, av)
     scale = np.nanmax(np.where(np.isfinite(c), np.abs(c), 0.0), axis=1, keepdims=True)
     with np.errstate(invalid="ignore"):
         err = np.abs(a - b) / np.maximum(scale, 1e-30)
@@ -178,3 +185,26 @@ def test_random_template_noise(rubix_lib):
     rng = np.random.default_rng(5)
     prob[0].flux[:] *= rng.uniform(0.5, 1.5, prob[0].flux.shape).astype(np.float32)
     _compare(rubix_lib, prob)
+
+
+@pytest.mark.parametrize("n_wave, res", [(400, 1.25), (1447, 1.25), (1221, 1.25), (1000, 1.25),
+                                         (400, 5.0), (800, 1.6)])
+@pytest.mark.parametrize("lsf", [None, 25])
+def test_dust(rubix_lib, n_wave, res, lsf):
+    """2 to 15 samples between two nodes (at most 4, 6, 8, or the general kernel's) behind
+    columns of 0 to 200 mag; the transmission 2^x adds an approximation of 2^-22 = 2.4e-7,
+    the same in both paths."""
+    prob = _problem(EDGES, ssp=(5, 3, n_wave), res=res)
+    n = prob[3]["mass"].size
+    av = np.random.default_rng(3).exponential(0.5, n)
+    av[::17] = 0.0
+    av[5::311] = 200.0
+    _compare(rubix_lib, prob, None if lsf is None else tel.gaussian_taps_1d(lsf, 1.3), av)
+
+
+def test_dust_outliers(rubix_lib):
+    """Columns that are not finite, or negative so that the transmission overflows."""
+    prob = _problem([40, 30, 70, 0, 300, 5])
+    av = np.random.default_rng(3).exponential(0.5, prob[3]["mass"].size)
+    av[3], av[45], av[100], av[200:220] = np.nan, -300.0, np.inf, -2.0
+    _compare(rubix_lib, prob, None, av)
