@@ -511,6 +511,11 @@ RUBIX_API int rubix_lsf_fwd(const float* in, float* out, int64_t n_rows, int32_t
  */
 RUBIX_API size_t rubix_cube_bwd_workspace_size(int64_t n, int32_t n_segments, int32_t n_wave_t,
                                                int32_t n_met, int32_t n_age, int32_t n_wave);
+/* Kernels that rubix_cube_bwd (dust = 0) or the dusty adjoints (dust = 1) launch. */
+RUBIX_API int rubix_cube_bwd_launches(int64_t n, int32_t n_segments, int32_t n_wave_t,
+                                      int32_t n_met, int32_t n_age, int32_t n_wave,
+                                      int32_t dust, size_t workspace_bytes);
+
 RUBIX_API int rubix_cube_bwd(const float* ssp_flux, const float* ssp_metallicity,
                              const float* ssp_age, const float* ssp_wave_z, int32_t n_met,
                              int32_t n_age, int32_t n_wave, const float* wave_t,

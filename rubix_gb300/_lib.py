@@ -39,6 +39,7 @@ SIGNATURES = {
     "rubix_spaxel_sort_workspace_size": (_sz, [_i64, _i32]),
     "rubix_spaxel_sort": (_c.c_int, [_vp, _vp, _i64, _i32, _vp, _vp, _vp, _sz, _vp]),
     "rubix_cube_workspace_size": (_sz, [_i64, _i32, _i32, _i32, _i32, _i32]),
+    "rubix_cube_bwd_launches": (_c.c_int, [_i64, _i32, _i32, _i32, _i32, _i32, _i32, _sz]),
     "rubix_cube_fwd_launches": (_c.c_int, [_i64, _i32, _i32, _i32, _i32, _i32, _i32, _sz]),
     "rubix_cube_status": (_c.c_int, [_vp, _c.POINTER(_c.c_int), _vp]),
     "rubix_cube_fwd": (

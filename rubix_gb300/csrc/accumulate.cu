@@ -610,6 +610,7 @@ __device__ __forceinline__ void lsf_epilogue_k(const MainArgs& a,
 
 template <int R, bool kDust, bool kStaged>
 __global__ void __launch_bounds__(kAccThreads, 2) cube_main_kernel(MainArgs a) {
+  if (a.ctrl->n_items == 0) return;  // the node path has left nothing
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemLayout SL = smem_layout(kStaged ? a.n_wave : 0, kStaged ? a.pool : 0, a.pool);
   float* s_wz = reinterpret_cast<float*>(smem + SL.wz);

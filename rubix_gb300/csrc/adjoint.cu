@@ -20,6 +20,7 @@
 // accumulates 8 partial sums over its wavelengths, the block reduces them in a fixed
 // order, and warp 0 writes the particle's gradients.  No atomics, deterministic.
 #include "cube_common.cuh"
+#include "cube_nodes.cuh"
 #include "tma.cuh"
 
 namespace rubix {
@@ -365,6 +366,7 @@ __device__ __forceinline__ float warp_reduce8(const float (&v)[8], int lane) {
 
 template <int R, bool kDust>
 __global__ void __launch_bounds__(kAdjThreads, 2) cube_adjoint_kernel(AdjArgs a) {
+  if (a.ctrl->n_items == 0) return;  // the node path has left nothing
   extern __shared__ __align__(16) unsigned char smem[];
   const AdjSmem SL = adj_smem_layout(a.n_wave, a.nZ + a.nA, a.row_cap, a.staged != 0);
   float* s_wz = reinterpret_cast<float*>(smem + SL.wz);
@@ -571,9 +573,21 @@ using namespace rubix;
 extern "C" size_t rubix_cube_bwd_workspace_size(int64_t n, int32_t n_segments, int32_t n_wave_t,
                                                 int32_t n_met, int32_t n_age, int32_t n_wave) {
   if (n < 0 || n_segments < 0 || n_wave_t < 0 || n_met < 0 || n_age < 0 || n_wave < 0) return 0;
-  return carve_cube(nullptr, n, n_segments, n_wave_t, n_met, n_age, n_wave,
-                    cube_tuning_current().chunk)
-      .bytes;
+  const size_t general =
+      cube_general_workspace(n, n_segments, n_wave_t, n_met, n_age, n_wave);
+  if (n == 0 || !cube_nodes_bwd_supported(n_met, n_age, n_wave, n_wave_t)) return general;
+  return std::max(general, cube_nodes_bwd_bytes(n, n_segments, n_met, n_age, n_wave, n_wave_t));
+}
+
+extern "C" int rubix_cube_bwd_launches(int64_t n, int32_t n_segments, int32_t n_wave_t,
+                                       int32_t n_met, int32_t n_age, int32_t n_wave, int32_t dust,
+                                       size_t workspace_bytes) {
+  if (n_segments <= 0 || n <= 0) return 0;
+  if (!dust && cube_nodes_bwd_supported(n_met, n_age, n_wave, n_wave_t) &&
+      cube_nodes_bwd_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes))
+    return cube_nodes_bwd_launches(n, n_segments, n_met, n_age, n_wave, workspace_bytes) + 1;
+  // setup, corner table, prefix, gather, count, scans (one launch), fill, adjoint
+  return 8;
 }
 
 namespace rubix {
@@ -607,7 +621,8 @@ int cube_bwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
   RUBIX_REQUIRE(ssp_flux && ssp_metallicity && ssp_age && ssp_wave_z && wave_t && seg_offsets &&
                     adj && mass && metallicity && age && velocity && perm,
                 RUBIX_E_INVALID, "%s: null pointer", who);
-  const size_t need = rubix_cube_bwd_workspace_size(n, n_segments, n_wave_t, n_met, n_age, n_wave);
+  const size_t need =
+      cube_general_workspace(n, n_segments, n_wave_t, n_met, n_age, n_wave);
   RUBIX_REQUIRE(workspace != nullptr && workspace_bytes >= need, RUBIX_E_WORKSPACE,
                 "%s: workspace of %zu bytes needed, %zu given", who, need, workspace_bytes);
   RUBIX_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, RUBIX_E_INVALID,
@@ -623,16 +638,29 @@ int cube_bwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                 who, n_wave, SL.total);
 
   const CubeTuning tune = cube_tuning_current();
-  const CubeLayout L =
+  CubeLayout L =
       carve_cube(workspace, n, n_segments, n_wave_t, n_met, n_age, n_wave, tune.chunk);
   const CubeInputs in{ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, n_met, n_age, n_wave,
                       wave_t, n_wave_t, mass, metallicity, age, velocity, vel_stride,
                       vel_component, perm, seg_offsets, n_segments, n, av};
-  {
+  AdjArgs args;
+  args.chunk = tune.chunk;
+  if (dust_e2 == nullptr && cube_nodes_bwd_supported(n_met, n_age, n_wave, n_wave_t) &&
+      cube_nodes_bwd_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes)) {
+    NodeFallback fb;
+    const int rc =
+        cube_nodes_backward(in, adj, adj_stride, grads, workspace, workspace_bytes, &fb, st);
+    if (rc != RUBIX_OK) return rc;
+    args.chunk = fb.chunk;
+    L.At = fb.At;
+    L.bucket = fb.bucket;
+    L.ct = fb.ct;
+    L.rec = fb.rec;
+    L.items = fb.items;
+  } else {
     const int rc = cube_prepare(in, L, tune, /*with_grad=*/true, st);
     if (rc != RUBIX_OK) return rc;
   }
-  AdjArgs args;
   args.ct = L.ct;
   args.wave_z = ssp_wave_z;
   args.nZ = n_met;
@@ -658,7 +686,6 @@ int cube_bwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
   args.bucket = L.bucket;
   args.row_cap = row_cap;
   args.staged = staged ? 1 : 0;
-  args.chunk = tune.chunk;
   args.dust_e2 = dust_e2;
   const int need_r = (n_wave_t + kAdjThreads - 1) / kAdjThreads;
   const size_t smem = SL.total;

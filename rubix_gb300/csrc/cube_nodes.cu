@@ -35,349 +35,14 @@
 // configuration and the spaxel's own particles only, so a spaxel's result does not depend
 // on what else is rendered with it.
 #include "cube_nodes.cuh"
+#include "node_tables.cuh"
 
 #include <type_traits>
 
 namespace rubix {
 namespace {
 
-constexpr int kExt = 512;        // virtual telescope samples on either side
-constexpr int kMaxBins = 224;    // samples of one (item, slice) row: 7 per lane
-constexpr int kWin = 768;        // samples of a slice's window over all alpha
-constexpr int kMaxSlices = 128;
-constexpr int kMaxWaves = 64;
-constexpr int kSub = 256;        // particles sorted together
 constexpr int kItem = 4 * kSub;  // particles of a work item
-constexpr int kAlphaBits = 18;
-constexpr float kAlphaStep = 1.0f / (1 << kAlphaBits);
-constexpr int kAlphaHalf = 2048;                       // alpha rows on either side of 1
-constexpr float kAlphaMax = 2040.f * kAlphaStep;       // |alpha - 1| covered (2333 km/s)
-constexpr int kAlphaTile = 64;                         // rows computed together
-constexpr int kAlphaTiles = 2 * kAlphaHalf / kAlphaTile + 1;
-constexpr int kAlphaRows = kAlphaTiles * kAlphaTile;
-constexpr int kNodeWarps = 20;
-constexpr int kNodeThreads = 32 * kNodeWarps;
-constexpr int kStage = 33;       // staged records of a warp: 32 and one of weight zero
-constexpr int kRuns = 4;
-constexpr int kDustMost = 8;     // samples between two nodes that a lane holds with dust
-
-struct NodeCtrl {
-  int flagged;                  // some spaxel is left to cube_main_kernel
-  unsigned e_lo, e_hi;          // bits of max(-e), max(e) of the dust exponents, >= 0
-  unsigned tile_mask[(kAlphaTiles + 31) / 32];
-  unsigned dz_inv, dt_inv;      // ~bits of the smallest SSP / telescope spacing
-  unsigned dz_max, dt_max;      // bits of the largest (3e38: not ascending)
-  unsigned run_max[kRuns], run_min_inv[kRuns];  // extent of own_nodes(r) + 1, + 0 intervals
-  int k_first;                  // 1 + node below the telescope range at any alpha
-  int k_last_inv;               // n_wave - node above it
-  unsigned fmax;                // bits of max |flux| (above inf: NaN)
-  int n_items, n_multi;         // work items with particles; those of several-item spaxels
-  int next[kMaxWaves][kMaxSlices];
-};
-
-// A slice has 32, 16, 8 or 4 nodes; all but its first and last are its own.
-__host__ __device__ constexpr int own_nodes(int r) { return (32 >> r) - 2; }
-
-// Slices that the workspace provides rows for.
-__host__ __device__ inline int max_slices_of(int n_wave) {
-  const int s = (n_wave + 30) / 31 + 1;
-  return s > kMaxSlices ? kMaxSlices : (s < 48 ? 48 : s);
-}
-
-struct NodePlan {
-  int ok;
-  int k_first, n_own, n_slices;  // first node, nodes of a slice
-  int w;                         // samples that a node may cross within a group of particles
-  float dt_min, window;          // samples that an item's alpha range may span
-  int most;                      // samples between two nodes at most
-};
-
-// How the grids are cut into slices, from the extrema; every block derives the same plan.
-__device__ __forceinline__ NodePlan node_plan(const NodeCtrl* c, int n_wave, float x_last,
-                                              bool dust) {
-  NodePlan p;
-  const float dz = __uint_as_float(~c->dz_inv), dt = __uint_as_float(~c->dt_inv);
-  const float dtm = __uint_as_float(c->dt_max), fm = __uint_as_float(c->fmax);
-  p.k_first = max(c->k_first - 1, 0);
-  const int k_last = min(n_wave - c->k_last_inv, n_wave - 1);
-  p.dt_min = dt;
-  p.ok = 0;
-  p.n_own = 0;
-  p.w = 1;
-  p.most = 0;
-  p.n_slices = 0;
-  p.window = 0.f;
-  // lambda' spacing >= alpha*dz minus two roundings of lambda' (|lambda'| < 2^14): at
-  // least one sample between two nodes; float32 exact enough to order samples and nodes
-  if (!(dz * (1.f - kAlphaMax) - 4.0e-3f > dtm) || !(dt > 2.0e-2f) || !(dtm < 1e30f) ||
-      !(__uint_as_float(c->dz_max) < 1e30f) || !(x_last < 16384.f) || !(fm < 1e30f) ||
-      k_last <= p.k_first)
-    return p;
-  const float ratio = (dz * (1.f - kAlphaMax) - 4.0e-3f) / dtm;
-  p.w = ratio > 2.f ? 2 : 1;
-  p.most = (int)(__uint_as_float(c->dz_max) * (1.f + kAlphaMax) / dt + 1.01f);
-  // with dust every sample is evaluated: fewer than two of them between nodes, or more than
-  // a lane holds, are the general kernel's
-  if (dust && (p.w < 2 || p.most > kDustMost)) return p;
-  const float swing = 2.f * kAlphaMax * x_last / dt;  // samples a node moves over all alpha
-  for (int r = 0; r < kRuns; ++r) {
-    const float hi = __uint_as_float(c->run_max[r]) * (1.f + kAlphaMax) / dt;
-    const float lo = __uint_as_float(~c->run_min_inv[r]) * (1.f - kAlphaMax) / dtm;
-    const float win = fminf((float)kMaxBins - hi, lo) - 4.f;
-    if (win < 24.f || hi + swing + 8.f > (float)(kExt - 16) ||
-        hi + swing + 8.f > (float)(kWin - 8))
-      continue;
-    p.n_own = own_nodes(r);
-    p.window = win;
-    p.n_slices = (k_last - p.k_first + p.n_own - 1) / p.n_own;
-    p.ok = p.n_slices <= max_slices_of(n_wave);
-    return p;
-  }
-  return p;
-}
-
-// SSP wavelength k, continued with the end spacings beyond the grid.
-__device__ __forceinline__ float lam_ext(const float* __restrict__ wz, int n, int k) {
-  if (k < 0) return wz[0] + (float)k * (wz[1] - wz[0]);
-  if (k >= n) return wz[n - 1] + (float)(k - n + 1) * (wz[n - 1] - wz[n - 2]);
-  return wz[k];
-}
-
-// Telescope sample e of the extended grid (e = t + kExt), continued with the end spacings.
-__device__ __forceinline__ float x_ext(const float* __restrict__ wt, int n, int e) {
-  const int t = e - kExt;
-  if (t < 0) return wt[0] + (float)t * (wt[1] - wt[0]);
-  if (t >= n) return wt[n - 1] + (float)(t - n + 1) * (wt[n - 1] - wt[n - 2]);
-  return wt[t];
-}
-
-// Grid extrema, and the rows of alpha that the particles' velocities fall on.
-__global__ void __launch_bounds__(256) node_setup_kernel(
-    const float* __restrict__ wz, int n_wave, const float* __restrict__ wt, int n_t,
-    const float* __restrict__ vel, long long vel_stride, int vel_comp, long long n,
-    const float* __restrict__ dust_e, NodeCtrl* __restrict__ ctrl) {
-  const long long gtid = blockIdx.x * 256LL + threadIdx.x, gsz = gridDim.x * 256LL;
-  if (gtid < n_t - 1) {
-    float d = wt[gtid + 1] - wt[gtid];
-    const bool bad = !(d > 0.f);
-    atomicMax(&ctrl->dt_max, bad ? __float_as_uint(3e38f) : __float_as_uint(d));
-    if (!bad) atomicMax(&ctrl->dt_inv, ~__float_as_uint(d));
-  }
-  if (dust_e && gtid < n_t) {
-    const float e = dust_e[gtid];
-    // a value that is not finite makes the limit infinite: every star is flagged
-    atomicMax(&ctrl->e_hi, __float_as_uint(isfinite(e) ? fmaxf(e, 0.f) : kFltMax));
-    atomicMax(&ctrl->e_lo, __float_as_uint(isfinite(e) ? fmaxf(-e, 0.f) : kFltMax));
-  }
-  const float x0 = wt[0], x1 = wt[n_t - 1];
-  const float hi = 1.f + kAlphaMax, lo = 1.f - kAlphaMax;
-  if (gtid < n_wave - 1) {
-    const int k = (int)gtid;
-    const float a = wz[k], b = wz[k + 1];
-    if (a * hi <= x0 && !(b * hi <= x0)) ctrl->k_first = k + 1;
-    if (!(a * lo > x1) && b * lo > x1) ctrl->k_last_inv = n_wave - (k + 1);
-    const float d = b - a;
-    const bool bad = !(d > 0.f);
-    const bool seen = bad || (b * 1.05f >= x0 && a * 0.95f <= x1);
-    if (seen) {
-      atomicMax(&ctrl->dz_max, bad ? __float_as_uint(3e38f) : __float_as_uint(d));
-      atomicMax(&ctrl->dz_inv, ~__float_as_uint(bad ? 0.f : d));
-    }
-#pragma unroll
-    for (int r = 0; r < kRuns; ++r) {
-      const float e0 = lam_ext(wz, n_wave, k + own_nodes(r)) - a;
-      const float e1 = lam_ext(wz, n_wave, k + own_nodes(r) + 1) - a;
-      if (seen && e0 >= 0.f && e1 >= 0.f) {
-        atomicMax(&ctrl->run_max[r], __float_as_uint(e1));
-        atomicMax(&ctrl->run_min_inv[r], ~__float_as_uint(e0));
-      }
-    }
-  }
-  __shared__ unsigned s_mask[(kAlphaTiles + 31) / 32];
-  if (threadIdx.x < (kAlphaTiles + 31) / 32) s_mask[threadIdx.x] = 0u;
-  __syncthreads();
-  int last = -1;
-  for (long long i = gtid; i < n; i += gsz) {
-    // alpha - 1 to ~1e-7: the rows on either side of it are marked
-    const float z = vel[i * vel_stride + vel_comp] * (float)(1.0 / kSpeedOfLight);
-    const float am1 = z * (1.f + 0.5f * z * (1.f + (1.f / 3.f) * z));
-    if (!(fabsf(am1) <= kAlphaMax)) continue;
-    const int r = (int)floorf(am1 * (float)(1 << kAlphaBits)) + kAlphaHalf;
-    const int a = max(r - 1, 0) / kAlphaTile, b = min(r + 2, kAlphaRows - 1) / kAlphaTile;
-    if (a != last) atomicOr(&s_mask[a >> 5], 1u << (a & 31));
-    if (b != a) atomicOr(&s_mask[b >> 5], 1u << (b & 31));
-    last = a;
-  }
-  __syncthreads();
-  if (threadIdx.x < (kAlphaTiles + 31) / 32 && s_mask[threadIdx.x])
-    atomicOr(&ctrl->tile_mask[threadIdx.x], s_mask[threadIdx.x]);
-}
-
-__device__ __forceinline__ bool tile_used(const NodeCtrl* c, int tile) {
-  return (c->tile_mask[tile >> 5] >> (tile & 31)) & 1u;
-}
-
-// The two resampling weights that interval [k, k + 1] gives its nodes at one alpha: the
-// samples x_t inside it at distance d from node k weigh dx_t (1 - d / len) and dx_t d / len.
-// The nodes are lambda_z * alpha unrounded, as float pairs; the few samples of an interval
-// are summed directly.
-__device__ __forceinline__ float2 interval_weights(const float* __restrict__ wz,
-                                                   const float* __restrict__ wt, int n_t, int k,
-                                                   float alpha, float x0, float inv) {
-  const float z0 = wz[k], z1 = wz[k + 1];
-  const float ah = __fmul_rn(z0, alpha), al = fmaf(z0, alpha, -ah);
-  const float bh = __fmul_rn(z1, alpha), bl = fmaf(z1, alpha, -bh);
-  int t = min(max((int)((ah - x0) * inv), 0), n_t - 1);
-  while (t > 0 && (wt[t - 1] - ah) - al >= 0.f) --t;
-  while (t < n_t && (wt[t] - ah) - al < 0.f) ++t;
-  float s0 = 0.f, s1 = 0.f, prev = t > 0 ? wt[t - 1] : x0;
-  for (; t < n_t; ++t) {
-    const float x = wt[t];
-    if ((x - bh) - bl >= 0.f) break;
-    const float dx = t > 0 ? x - prev : 0.f;
-    s0 += dx;
-    s1 = fmaf(dx, (x - ah) - al, s1);
-    prev = x;
-  }
-  const float rise = s1 / ((bh - ah) + (bl - al));
-  return make_float2(s0 - rise, rise);
-}
-
-constexpr int kWeightBlocks = 1024;
-
-// Per template: float64 prefix sums (block b < rows, as cube_prefix_kernel) and max |F|.
-// The remaining blocks: the resampling weights of T' at alpha_i, h_k = sum_t dlambda_t
-// hat_k(x_t) with hat_k the hat function of node k, one alpha row of a used tile at a time.
-// Nodes are stored from k_first on, kpad to a row, zero beyond the last.
-__global__ void __launch_bounds__(kPrefixThreads) node_tables_kernel(
-    const float* __restrict__ flux, int rows, int n_wave, const float* __restrict__ wz,
-    const float* __restrict__ wt, int n_t, double* __restrict__ prefix, float* __restrict__ h,
-    int kpad, NodeCtrl* __restrict__ ctrl) {
-  if ((int)blockIdx.x < rows) {
-    prefix_row(flux, blockIdx.x, n_wave, wz, prefix);
-    const float* f = flux + (long long)blockIdx.x * n_wave;
-    unsigned m = 0u;
-    for (int k = threadIdx.x; k < n_wave; k += kPrefixThreads)
-      m = max(m, __float_as_uint(f[k]) & 0x7fffffffu);
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) atomicMax(&ctrl->fmax, m);
-    return;
-  }
-  __shared__ float s_rise[kPrefixThreads + 1];
-  const int tid = threadIdx.x;
-  // the grid's node range (fmax, still being formed, only decides whether it is used)
-  const int k_first = max(ctrl->k_first - 1, 0);
-  const int count = min(n_wave - ctrl->k_last_inv, n_wave - 1) - k_first + 1;
-  const float x0 = wt[0], inv = (float)(n_t - 1) / (wt[n_t - 1] - x0);
-  for (int u = blockIdx.x - rows;; u += kWeightBlocks) {
-    // row u of the used tiles
-    int tile = 0, left = u / kAlphaTile;
-    while (tile < kAlphaTiles && (!tile_used(ctrl, tile) || left-- > 0)) ++tile;
-    if (tile == kAlphaTiles) return;
-    const int row = tile * kAlphaTile + u % kAlphaTile;
-    const float alpha = 1.f + (float)(row - kAlphaHalf) * kAlphaStep;  // exact
-    if (tid == 0) s_rise[0] = 0.f;
-    for (int q0 = 0; q0 < kpad; q0 += kPrefixThreads) {
-      const int q = q0 + tid;
-      float2 w = make_float2(0.f, 0.f);
-      if (q < count - 1) w = interval_weights(wz, wt, n_t, k_first + q, alpha, x0, inv);
-      s_rise[tid + 1] = w.y;
-      __syncthreads();
-      if (q < kpad) h[(long long)row * kpad + q] = w.x + s_rise[tid];
-      __syncthreads();
-      if (tid == kPrefixThreads - 1) s_rise[0] = w.y;
-    }
-    __syncthreads();
-  }
-}
-
-// H[i][c] = sum_k h[i][k] F[c][k]: 64 alpha rows x 32 templates per block of 128 threads,
-// 4 x 4 per thread, 32 nodes staged at a time.  Sums of 32 products are added with Kahan's
-// compensation: a plain float32 sum over ~740 nodes would be 5e-7 off, this one is 1e-8.
-// Bound by FMA issue: 1 GFMA for 1025 rows of a 1326-template grid, 40 TFMA/s on the chip.
-__global__ void __launch_bounds__(128) node_table_product_kernel(
-    const float* __restrict__ h, int kpad, const float* __restrict__ flux, int n_templ,
-    int n_wave, const float* __restrict__ wt, int n_t, bool dust,
-    const NodeCtrl* __restrict__ ctrl, float* __restrict__ H) {
-  constexpr int BK = 32, BM = kAlphaTile, BN = 32;
-  const int tile = blockIdx.y;
-  if (!tile_used(ctrl, tile)) return;
-  const NodePlan p = node_plan(ctrl, n_wave, wt[n_t - 1], dust);
-  if (!p.ok) return;
-  const int k_last = min(n_wave - ctrl->k_last_inv, n_wave - 1);
-  const int K = min(k_last - p.k_first + 1, kpad);
-  __shared__ float sa[2][BK][BM + 4];
-  __shared__ float sb[2][BK][BN + 4];
-  const int tid = threadIdx.x;
-  const int r0 = tile * BM, c0 = blockIdx.x * BN;
-  const int tr = (tid >> 3) * 4, tc = (tid & 7) * 4;
-  // loads: a thread takes 4 consecutive nodes of h in 4 rows, and of F node `lane` in 8
-  const int lr = tid >> 3, lk = (tid & 7) * 4, lane = tid & 31, warp = tid >> 5;
-  float4 ra[4];
-  float rb[8];
-  auto load = [&](int k0) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      ra[i] = *reinterpret_cast<const float4*>(h + (long long)(r0 + lr + 16 * i) * kpad + k0 + lk);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int c = c0 + warp * 8 + j;
-      rb[j] = (k0 + lane < K && c < n_templ)
-                  ? flux[(long long)c * n_wave + p.k_first + k0 + lane] : 0.f;
-    }
-  };
-  auto store = [&](int buf) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      sa[buf][lk][lr + 16 * i] = ra[i].x;
-      sa[buf][lk + 1][lr + 16 * i] = ra[i].y;
-      sa[buf][lk + 2][lr + 16 * i] = ra[i].z;
-      sa[buf][lk + 3][lr + 16 * i] = ra[i].w;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) sb[buf][lane][warp * 8 + j] = rb[j];
-  };
-  float sum[4][4], comp[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) sum[i][j] = comp[i][j] = 0.f;
-  const int steps = (K + BK - 1) / BK;  // kpad is a multiple of BK
-  load(0);
-  store(0);
-  __syncthreads();
-  for (int s = 0; s < steps; ++s) {
-    if (s + 1 < steps) load((s + 1) * BK);
-    float acc[4][4];
-#pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      const float4 a = *reinterpret_cast<const float4*>(&sa[s & 1][k][tr]);
-      const float4 b = *reinterpret_cast<const float4*>(&sb[s & 1][k][tc]);
-      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          acc[i][j] = k == 0 ? av[i] * bv[j] : fmaf(av[i], bv[j], acc[i][j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float y = acc[i][j] - comp[i][j];
-        const float t = sum[i][j] + y;
-        comp[i][j] = (t - sum[i][j]) - y;
-        sum[i][j] = t;
-      }
-    if (s + 1 < steps) store((s + 1) & 1);
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (c0 + tc + j < n_templ) H[(long long)(r0 + tr + i) * n_templ + c0 + tc + j] = sum[i][j];
-}
 
 // Work items: ranges of up to kItem particles of one spaxel; empty spaxels have none.
 // Spaxels of several items first (item index = row), then those with many particles.
@@ -450,13 +115,12 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
   __shared__ int s_flag;
   const CubeInputs& in = a.in;
   const int tid = threadIdx.x;
-  const float x0 = in.wave_t[0], x1 = in.wave_t[in.n_wave_t - 1];
+  const float x1 = in.wave_t[in.n_wave_t - 1];
   if (tid == 0) s_plan = node_plan(a.ctrl, in.n_wave, x1, a.rec_av != nullptr);
   __syncthreads();
   const NodePlan plan = s_plan;
   const float fmax = __uint_as_float(a.ctrl->fmax);
   const int n_items = a.ctrl->n_items;
-  const int n_templ = in.n_met * in.n_age;
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const int2 it = a.items[item];
     const int seg_b = in.seg_off[it.x], seg_e = in.seg_off[it.x + 1];
@@ -473,57 +137,21 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
       bool bad = false;
       if (tid < m) {
         const long long i = in.perm[j0 + tid];
-        const float Z = in.met[i], A = in.age[i], mass = in.mass[i];
-        alpha = doppler_factor(in.vel[i * in.vel_stride + in.vel_comp]);
+        const NodeParticle q = node_particle(in, a.prefix, a.H, i);
+        const float mass = in.mass[i];
         if (a.rec_av) av = in.av[i];
-        const bool outside = (Z < in.ssp_met[0]) || (Z > in.ssp_met[in.n_met - 1]) ||
-                             (A < in.ssp_age[0]) || (A > in.ssp_age[in.n_age - 1]);
-        if (!(fabsf(alpha - 1.f) <= kAlphaMax)) {
-          bad = true;
-          alpha = 1.f;
-        } else if (outside) {
-          // an all-zero spectrum unless 0 times the mass or the transmission is not 0
+        alpha = q.alpha;
+        row = q.row;
+        const float beta = mass != 0.f ? mass * (q.T / q.Tp) : 0.f;
+        const float top = fabsf(beta) * fmax;  // without dust dust_top is 1
+        // what the general kernel treats specially, or what may leave float32's range; a
+        // particle outside the templates has no spectrum unless 0 times its mass or its
+        // transmission is not 0
+        if (q.outside && !q.bad) {
           bad = !isfinite(mass) || !(dust_top(a, av) < 1e30f);
         } else {
-          const int iz = min(max(count_le(in.ssp_met, in.n_met, Z), 1), in.n_met - 1);
-          const int ia = min(max(count_le(in.ssp_age, in.n_age, A), 1), in.n_age - 1);
-          const float dzg = in.ssp_met[iz] - in.ssp_met[iz - 1];
-          const float dag = in.ssp_age[ia] - in.ssp_age[ia - 1];
-          const float tz = dzg == 0.f ? 0.f : (Z - in.ssp_met[iz - 1]) / dzg;
-          const float ta = dag == 0.f ? 0.f : (A - in.ssp_age[ia - 1]) / dag;
-          const int ks = count_le_scaled(in.ssp_wave_z, in.n_wave, alpha, x0) - 1;
-          const int ke = count_le_scaled(in.ssp_wave_z, in.n_wave, alpha, x1) - 1;
-          row = (iz - 1) * in.n_age + (ia - 1);
-          if (ks < 0 || ke + 1 > in.n_wave - 1) {
-            bad = true;
-          } else {
-            const float wc[4] = {(1.f - tz) * (1.f - ta), tz * (1.f - ta), (1.f - tz) * ta,
-                                 tz * ta};
-            const int rr[4] = {row, row + in.n_age, row + 1, row + in.n_age + 1};
-            // T: in-range flux sum, entries ka..kb with x0 <= lambda'_k <= x1, k >= 1
-            int ka = __fmul_rn(in.ssp_wave_z[ks], alpha) >= x0 ? ks : ks + 1;
-            ka = max(ka, 1);
-            float T = 0.f, Tp = 0.f;
-            const float u = (alpha - 1.f) * (float)(1 << kAlphaBits);  // exact
-            const int r = (int)floorf(u) + kAlphaHalf;
-            const float fr = u - floorf(u);
-            const float* h0 = a.H + (long long)r * n_templ;
-            const float* h1 = h0 + n_templ;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const double* pf = a.prefix + (long long)rr[c] * in.n_wave;
-              if (ka <= ke) T = fmaf(wc[c], (float)(pf[ke] - pf[ka - 1]), T);
-              Tp = fmaf(wc[c], fmaf(fr, h1[rr[c]] - h0[rr[c]], h0[rr[c]]), Tp);
-            }
-            T *= alpha;
-            const float sc = T / Tp;
-            const float beta = mass != 0.f ? mass * sc : 0.f;
-            const float top = fabsf(beta) * fmax;  // without dust dust_top is 1
-            // what the general kernel treats specially, or what may leave float32's range
-            bad = !(sc > 0.25f && sc < 4.f) || !(top * dust_top(a, av) < 1e30f) ||
-                  (beta != 0.f && !(top > 1e-25f));
-            w = make_float4(beta * wc[0], beta * wc[1], beta * wc[2], beta * wc[3]);
-          }
+          bad = q.bad || !(top * dust_top(a, av) < 1e30f) || (beta != 0.f && !(top > 1e-25f));
+          w = make_float4(beta * q.w[0], beta * q.w[1], beta * q.w[2], beta * q.w[3]);
         }
       }
       if (bad) s_flag = 1;
@@ -532,14 +160,7 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
       if (tid < m) {
         amin = fminf(amin, alpha);
         amax = fmaxf(amax, alpha);
-        const unsigned key = s_key[tid];
-        int rank = 0;
-        for (int q = 0; q < m; q += 4) {
-          const uint4 v = *reinterpret_cast<const uint4*>(&s_key[q]);
-          rank += (v.x < key || (v.x == key && q < tid)) + (v.y < key || (v.y == key && q + 1 < tid)) +
-                  (v.z < key || (v.z == key && q + 2 < tid)) +
-                  (v.w < key || (v.w == key && q + 3 < tid));
-        }
+        const int rank = run_rank(s_key, m, tid);
         a.rec_w[j0 + rank] = w;
         a.rec_a[j0 + rank] = make_float2(alpha, __int_as_float(row * 128));
         if (a.rec_av) a.rec_av[j0 + rank] = av;
@@ -607,42 +228,6 @@ __device__ __forceinline__ void wave_range(const NodeCtrl* c, int wave, int wave
 __device__ __forceinline__ int item_row(int item, int n_multi, int wave, int wave_items,
                                         int multi_rows) {
   return item < n_multi ? item : multi_rows + (item - n_multi - wave * wave_items);
-}
-
-// 1 / x by the hardware's reciprocal (relative error about 2^-23); x is a positive normal.
-__device__ __forceinline__ float fast_rcp(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// The records that a warp has staged, one array per value: a step reads one word of NPL
-// records at a time, one wavefront each (16-byte loads of the same take four).
-struct StagedRecs {
-  float w[4][kStage];  // corner weights times beta
-  float alpha[kStage];
-  int row[kStage];     // byte offset of the first corner's row in the slice table
-};
-
-struct SliceShared {
-  const float* tab;  // [template][32]
-  const float* xw;   // window of the extended telescope grid, kWin samples
-  const float* ew;   // with dust: the exponents of the window's samples
-  StagedRecs* st;    // this warp's staged records
-  float* st_av;      // with dust: their columns
-  float* f;          // this warp's samples, kMaxBins
-  float inv;         // samples per Angstrom over the window
-};
-
-// Smallest window index j with xw[j] >= x: a linear guess, right to one sample on a uniform
-// grid and corrected by steps on others.
-__device__ __forceinline__ int sample_at(const SliceShared& s, float x) {
-  int j = min(max((int)((x - s.xw[0]) * s.inv), 1), kWin - 2);
-  const float x0 = s.xw[j - 1], x1 = s.xw[j], x2 = s.xw[j + 1];
-  if (x0 < x && x <= x2) return x <= x1 ? j : j + 1;
-  while (j > 1 && s.xw[j - 1] >= x) --j;
-  while (j < kWin - 1 && s.xw[j] < x) ++j;
-  return j;
 }
 
 // One item by one warp on one slice: NPL nodes per lane (two or four, in packed pairs), NPL
@@ -1079,14 +664,9 @@ __global__ void __launch_bounds__(kNodeThreads, 1) node_slice_kernel(SliceArgs a
               ? a.flux[(long long)r * a.n_wave + k] : 0.f;
     }
     if (tid < 36) s_lam[tid] = lam_ext(a.wz, a.n_wave, k0 + tid);
-    if (tid == 0) {
-      const float x = lam_ext(a.wz, a.n_wave, k0) * (1.f - kAlphaMax);
-      int lo = 0, hi = a.n_t + 2 * kExt - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (x_ext(a.wt, a.n_t, mid) < x) lo = mid + 1; else hi = mid;
-      }
-      s_e0 = max(lo - 3, 0);
+    if (warp == 0) {
+      const int e = window_start(a.wt, a.n_t, lam_ext(a.wz, a.n_wave, k0), lane);
+      if (lane == 0) s_e0 = e;
     }
     __syncthreads();
     const int e0 = s_e0;
@@ -1113,17 +693,7 @@ __global__ void __launch_bounds__(kNodeThreads, 1) node_slice_kernel(SliceArgs a
       else run(TypeOf<SliceItem<4, 2>>{}, I4{});
     }
     __syncthreads();
-    if (tid == 0) {
-      int best = -1, most = 2 * kNodeWarps;
-      for (int q = 0; q < plan.n_slices; ++q) {
-        const int left = total - *(volatile int*)&next[q];
-        if (left > most) {
-          most = left;
-          best = q;
-        }
-      }
-      s_slice = best;
-    }
+    if (tid == 0) s_slice = busiest_slice(next, plan.n_slices, total, 2 * kNodeWarps);
     __syncthreads();
     slice = s_slice;
     if (slice < 0) return;
@@ -1284,8 +854,6 @@ struct NodeLayout {
   size_t shared_off, fixed;  // start of the shared region; bytes without rows
 };
 
-int kpad_of(int n_wave) { return (n_wave + 31) / 32 * 32; }
-
 NodeLayout carve_nodes(void* ws, long long n, int n_seg, int nZ, int nA, int nW) {
   Carve c(ws);
   NodeLayout L;
@@ -1310,80 +878,6 @@ NodeLayout carve_nodes(void* ws, long long n, int n_seg, int nZ, int nA, int nW)
   return L;
 }
 
-NodeFallback carve_fallback(Carve& c, const CubeInputs& in) {
-  NodeFallback f{};
-  f.At = c.take<float>((size_t)in.n_wave_t);
-  f.bucket = c.take<int2>(kBuckets);
-  f.ct = c.take<float4>((size_t)(in.n_met - 1) * (in.n_age - 1) * in.n_wave);
-  f.rec = c.take<ParticleRec>((size_t)in.n);
-  f.done = c.take<int>((size_t)in.n_seg);
-  f.slot_start = c.take<int>((size_t)in.n_seg);
-  f.chunk = kMaxChunk;
-  f.items = c.take<int2>((size_t)max_slots(in.n, kMaxChunk) + in.n_seg);
-  f.partials = c.take<float>((size_t)max_slots(in.n, kMaxChunk) * in.n_wave_t);
-  return f;
-}
-
-size_t fallback_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
-  CubeInputs in{};
-  in.n_met = nZ;
-  in.n_age = nA;
-  in.n_wave = nW;
-  in.n_wave_t = n_t;
-  in.n_seg = n_seg;
-  in.n = n;
-  Carve c(nullptr);
-  carve_fallback(c, in);
-  return c.off;
-}
-
-// What cube_main_kernel reads (cube_prepare's setup passes), when a spaxel is flagged.
-__global__ void __launch_bounds__(256) node_fallback_kernel(CubeInputs in, NodeFallback f,
-                                                            const double* __restrict__ prefix,
-                                                            const int* __restrict__ flags,
-                                                            const NodeCtrl* __restrict__ nc,
-                                                            CubeCtrl* __restrict__ ctrl) {
-  if (!nc->flagged) return;
-  const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
-  double lnq0, h;
-  bucket_params(in.wave_t, in.n_wave_t, lnq0, h);
-  for (int t = gtid; t < in.n_wave_t; t += gsz)
-    f.At[t] = (float)((log((double)in.wave_t[t]) - lnq0) / h);
-  for (int b = gtid; b < kBuckets; b += gsz)
-    f.bucket[b] = bucket_entry(in.ssp_wave_z, in.n_wave, lnq0, h, b);
-  if (blockIdx.x == 0) {
-    // the flagged spaxels' items: those of several chunks first
-    __shared__ int s_multi, s_single;
-    if (threadIdx.x == 0) s_multi = s_single = 0;
-    __syncthreads();
-    for (int pass = 0; pass < 2; ++pass) {
-      for (int s = threadIdx.x; s < in.n_seg; s += blockDim.x) {
-        if (!flags[s]) continue;
-        const int cnt = in.seg_off[s + 1] - in.seg_off[s];
-        const int nch = (cnt + f.chunk - 1) / f.chunk;
-        if ((nch > 1) != (pass == 0)) continue;
-        const int at = atomicAdd(pass == 0 ? &s_multi : &s_single, nch);
-        f.slot_start[s] = at;
-        f.done[s] = 0;
-        for (int c = 0; c < nch; ++c) f.items[at + c] = make_int2(s, c);
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        if (pass == 0) s_single = s_multi;
-        else ctrl->n_items = s_single;
-      }
-      __syncthreads();
-    }
-  }
-  corner_table(in.ssp_flux, in.n_met, in.n_age, in.n_wave, f.ct);
-  gather_records(in.mass, in.met, in.age, in.vel, in.vel_stride, in.vel_comp, in.perm,
-                 in.seg_off, in.n_seg, in.n, in.ssp_met, in.n_met, in.ssp_age, in.n_age,
-                 in.ssp_wave_z, in.n_wave, in.wave_t, in.n_wave_t, prefix, 1.0 / h,
-                 (float)(kVmaxKms / kSpeedOfLight / h), __uint_as_float(~nc->dz_inv),
-                 __uint_as_float(nc->dt_max), f.rec, 0, in.av,
-                 (float)exp(-kVmaxKms / kSpeedOfLight), (float)exp(kVmaxKms / kSpeedOfLight));
-}
-
 constexpr size_t kRowBudget = (size_t)2 << 30;  // rows of single-item spaxels at a time
 
 long long min_wave_items(int n_seg) {
@@ -1401,13 +895,13 @@ size_t cube_nodes_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t)
   const long long wave = std::max(
       min_wave_items(n_seg), std::min<long long>(n_seg, (long long)(kRowBudget / row_bytes(nW))));
   return std::max(L.fixed + (size_t)(multi_row_count(n) + wave) * row_bytes(nW),
-                  L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t));
+                  L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, false));
 }
 
 bool cube_nodes_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, size_t bytes) {
   const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
   return bytes >= L.fixed + (size_t)(multi_row_count(n) + min_wave_items(n_seg)) * row_bytes(nW) &&
-         bytes >= L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t);
+         bytes >= L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, false);
 }
 
 int cube_nodes_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t bytes) {
@@ -1435,24 +929,8 @@ int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* l
   // control block, counters and flags are contiguous
   RUBIX_CUDA_TRY(cudaMemsetAsync(ws, 0, (size_t)((char*)(L.flags + in.n_seg) - (char*)ws), st));
   {
-    const long long work = std::max<long long>(std::max(in.n_wave_t, nW), in.n);
-    const int g = (int)std::min<long long>((work + 255) / 256, (long long)sm_count() * 8);
-    const int need = (std::max(in.n_wave_t, nW) + 255) / 256;
-    node_setup_kernel<<<std::max(g, need), 256, 0, st>>>(in.ssp_wave_z, nW, in.wave_t,
-                                                         in.n_wave_t, in.vel, in.vel_stride,
-                                                         in.vel_comp, in.n, dust_e, L.ctrl);
-    RUBIX_LAUNCH_CHECK("node_setup_kernel");
-  }
-  const int kpad = kpad_of(nW);
-  {
-    node_tables_kernel<<<n_templ + kWeightBlocks, kPrefixThreads, 0, st>>>(
-        in.ssp_flux, n_templ, nW, in.ssp_wave_z, in.wave_t, in.n_wave_t, L.prefix, L.h, kpad,
-        L.ctrl);
-    RUBIX_LAUNCH_CHECK("node_tables_kernel");
-    node_table_product_kernel<<<dim3((n_templ + 31) / 32, kAlphaTiles), 128, 0, st>>>(
-        L.h, kpad, in.ssp_flux, n_templ, nW, in.wave_t, in.n_wave_t, dust_e != nullptr,
-        L.ctrl, L.H);
-    RUBIX_LAUNCH_CHECK("node_table_product_kernel");
+    const int rc = node_build_tables(in, dust_e, L.prefix, L.h, L.H, L.ctrl, st);
+    if (rc != RUBIX_OK) return rc;
   }
   {
     const int g = (int)std::min<long long>((in.n_seg + 255) / 256, (long long)sm_count() * 8);
@@ -1525,10 +1003,10 @@ int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* l
   }
   // The flagged spaxels, if any, in the region that the slices no longer need.
   Carve c(static_cast<char*>(ws) + L.shared_off);
-  *fb = carve_fallback(c, in);
+  *fb = carve_fallback(c, in, false);
   const int blocks = sm_count() * 8;
   node_fallback_kernel<<<blocks, 256, 0, st>>>(in, *fb, L.prefix, L.flags, L.ctrl,
-                                               static_cast<CubeCtrl*>(ws));
+                                               static_cast<CubeCtrl*>(ws), false);
   RUBIX_LAUNCH_CHECK("node_fallback_kernel");
   return RUBIX_OK;
 }

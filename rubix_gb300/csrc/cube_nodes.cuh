@@ -34,6 +34,15 @@ bool cube_nodes_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, siz
 
 // Kernels that cube_nodes_forward launches.
 int cube_nodes_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t bytes);
+// The adjoint of cube_nodes_forward without dust (cube_nodes_bwd.cu): grads are dL/dmass,
+// dL/dZ, dL/dage and dL/dv_los (zeroed by the caller, null where not wanted).
+int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_stride,
+                        float* const* grads, void* ws, size_t ws_bytes, NodeFallback* fb,
+                        cudaStream_t st);
+bool cube_nodes_bwd_supported(int nZ, int nA, int nW, int n_t);
+size_t cube_nodes_bwd_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t);
+bool cube_nodes_bwd_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, size_t bytes);
+int cube_nodes_bwd_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t bytes);
 // Workspace of the path without it (accumulate.cu).
 size_t cube_general_workspace(int64_t n, int32_t n_segments, int32_t n_wave_t, int32_t n_met,
                               int32_t n_age, int32_t n_wave);

@@ -253,8 +253,8 @@ def cube_backward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, 
                   _ptr(dust_exponent), _ptr(perm), _ptr(seg_offsets), int(n_segments), n,
                   _ptr(adj), adj.stride(0), *[_ptr(g) for g in grads], _ptr(ws), ws.numel(),
                   _stream(dev))
-    # setup, corner table, prefix, count, scans (one launch), fill, adjoint (+ gather)
-    _count((7 + (1 if n > 0 else 0)) if (n_segments > 0 and n > 0) else 0)
+    _count(_lib.query("rubix_cube_bwd_launches", n, int(n_segments), L, nz, na, nw,
+                      0 if dust_av is None else 1, ws.numel()))
     return tuple(grads)
 
 
