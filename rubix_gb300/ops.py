@@ -44,7 +44,7 @@ def _count(k: int) -> None:
 
 def _sort_passes(n_segments: int) -> int:
     bits = max(1, int(n_segments).bit_length())
-    return (bits + 7) // 8
+    return (bits + 8) // 9
 
 
 def _stream(dev: torch.device) -> int:
@@ -118,7 +118,7 @@ def spaxel_sort(idx: torch.Tensor, n_segments: int, keep: torch.Tensor | None = 
     ws = workspace(nbytes, dev)
     _lib.call("rubix_spaxel_sort", _ptr(idx), _ptr(keep), n, int(n_segments), _ptr(perm),
               _ptr(offs), _ptr(ws), ws.numel(), _stream(dev))
-    _count(2 + 3 * _sort_passes(n_segments) if n > 0 else 0)
+    _count(1 + 3 * _sort_passes(n_segments) if n > 0 else 0)
     return perm, offs
 
 
