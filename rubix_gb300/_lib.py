@@ -196,7 +196,7 @@ def lib():
 
 def call(name: str, *args) -> None:
     """Call a status-returning entry point and raise RubixError on failure."""
-    h = lib()
+    h = _lib or lib()
     rc = getattr(h, name)(*args)
     if rc != RUBIX_OK:
         msg = h.rubix_last_error()
@@ -204,4 +204,4 @@ def call(name: str, *args) -> None:
 
 
 def query(name: str, *args) -> int:
-    return int(getattr(lib(), name)(*args))
+    return int(getattr(_lib or lib(), name)(*args))

@@ -117,9 +117,9 @@ class IFURenderer:
     # -------------------------------------------------------------- steps
     def assign(self, coords):
         coords = _dev(coords, self.device)
-        idx = ops.spaxel_assign(coords, self.edges)
-        mask = ops.aperture_mask(coords, self.edges) if self.apply_filter else None
-        return idx, mask
+        if self.apply_filter:
+            return ops.assign_and_mask(coords, self.edges)
+        return ops.spaxel_assign(coords, self.edges), None
 
     def sort(self, idx, mask=None):
         return ops.spaxel_sort(idx, self.sbin * self.sbin, mask)

@@ -879,11 +879,9 @@ int launch_main_t(const MainArgs& args, size_t smem, cudaStream_t st) {
   if (e != cudaSuccess)
     return set_error(RUBIX_E_CUDA, "cudaFuncSetAttribute(cube_main_kernel): %s",
                      cudaGetErrorString(e));
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cube_main_kernel<R, kDust, kStaged>,
-                                                    kAccThreads,
-                                                    smem);
-  if (e != cudaSuccess || per_sm < 1)
+  const int per_sm = blocks_per_sm(
+      reinterpret_cast<const void*>(cube_main_kernel<R, kDust, kStaged>), kAccThreads, smem);
+  if (per_sm < 1)
     return set_error(RUBIX_E_UNSUPPORTED,
                      "cube_main_kernel does not fit on an SM with %zu bytes of shared memory",
                      smem);
@@ -940,8 +938,8 @@ extern "C" int rubix_cube_fwd_launches(int64_t n, int32_t n_segments, int32_t n_
   if (!general && n > 0 && cube_nodes_supported(n_met, n_age, n_wave, n_wave_t) &&
       cube_nodes_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes))
     return cube_nodes_launches(n, n_segments, n_met, n_age, n_wave, workspace_bytes) + 1;
-  // setup, corner table, prefix, count, scans (one launch), fill, main (+ gather)
-  return 7 + (n > 0 ? 1 : 0);
+  // grid tables, items (count, scans and fill, or one launch), main (+ gather)
+  return (n_segments <= kItemsOneBlock ? 3 : 5) + (n > 0 ? 1 : 0);
 }
 
 namespace rubix {

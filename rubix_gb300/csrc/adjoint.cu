@@ -547,10 +547,9 @@ int launch_adjoint_t(const AdjArgs& args, size_t smem, cudaStream_t st) {
   if (e != cudaSuccess)
     return set_error(RUBIX_E_CUDA, "cudaFuncSetAttribute(cube_adjoint_kernel): %s",
                      cudaGetErrorString(e));
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cube_adjoint_kernel<R, kDust>,
-                                                    kAdjThreads, smem);
-  if (e != cudaSuccess || per_sm < 1)
+  const int per_sm = blocks_per_sm(
+      reinterpret_cast<const void*>(cube_adjoint_kernel<R, kDust>), kAdjThreads, smem);
+  if (per_sm < 1)
     return set_error(RUBIX_E_UNSUPPORTED,
                      "cube_adjoint_kernel does not fit on an SM with %zu bytes of shared memory",
                      smem);
@@ -586,8 +585,8 @@ extern "C" int rubix_cube_bwd_launches(int64_t n, int32_t n_segments, int32_t n_
   if (!dust && cube_nodes_bwd_supported(n_met, n_age, n_wave, n_wave_t) &&
       cube_nodes_bwd_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes))
     return cube_nodes_bwd_launches(n, n_segments, n_met, n_age, n_wave, workspace_bytes) + 1;
-  // setup, corner table, prefix, gather, count, scans (one launch), fill, adjoint
-  return 8;
+  // grid tables, gather, items (count, scans and fill, or one launch), adjoint
+  return n_segments <= kItemsOneBlock ? 4 : 6;
 }
 
 namespace rubix {
@@ -615,8 +614,13 @@ int cube_bwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // every gradient entry is written: zeros for particles outside the sorted set
   float* grads[5] = {grad_mass, grad_metallicity, grad_age, grad_vlos, grad_av};
-  for (float* g : grads)
-    if (g && n > 0) RUBIX_CUDA_TRY(cudaMemsetAsync(g, 0, sizeof(float) * (size_t)n, st));
+  for (int i = 0; i < 5 && n > 0;) {
+    int j = i + 1;  // arrays that follow one another in memory: one memset
+    while (grads[i] && j < 5 && grads[j] == grads[i] + (size_t)(j - i) * n) ++j;
+    if (grads[i])
+      RUBIX_CUDA_TRY(cudaMemsetAsync(grads[i], 0, sizeof(float) * (size_t)n * (j - i), st));
+    i = j;
+  }
   if (n_segments == 0 || n == 0) return RUBIX_OK;
   RUBIX_REQUIRE(ssp_flux && ssp_metallicity && ssp_age && ssp_wave_z && wave_t && seg_offsets &&
                     adj && mass && metallicity && age && velocity && perm,

@@ -32,6 +32,34 @@ int sm_count() {
   return cached[dev];
 }
 
+int blocks_per_sm(const void* kernel, int threads, size_t smem) {
+  struct Entry {
+    int dev, threads, blocks;
+    const void* kernel;
+    size_t smem;
+  };
+  constexpr int kMax = 256;
+  static std::mutex mu;
+  static Entry cached[kMax];
+  static int count = 0;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    for (int i = 0; i < count; ++i) {
+      const Entry& e = cached[i];
+      if (e.dev == dev && e.threads == threads && e.kernel == kernel && e.smem == smem)
+        return e.blocks;
+    }
+  }
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess)
+    return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  if (n > 0 && count < kMax) cached[count++] = Entry{dev, threads, n, kernel, smem};
+  return n;
+}
+
 }  // namespace rubix
 
 extern "C" int rubix_abi_version(void) { return RUBIX_ABI_VERSION; }

@@ -60,6 +60,10 @@ struct Carve {
 
 int sm_count();  // cached multiprocessor count of the current device
 
+// Blocks of a kernel that fit on an SM of the current device (0 if none or on an error): the
+// occupancy query, whose answer depends on these arguments alone, made once for each.
+int blocks_per_sm(const void* kernel, int threads, size_t smem);
+
 constexpr double kSpeedOfLight = 299792.458;  // km/s, rubix_config.yml:8
 constexpr float kFltMax = 3.402823466e+38f;
 

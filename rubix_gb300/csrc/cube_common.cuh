@@ -21,7 +21,7 @@ struct CubeCtrl {
   int next_item;
   int n_items;
   int error;               // 1: a TMA wait timed out
-  unsigned dz_min_bits;    // min SSP spacing near the telescope range (float bits)
+  unsigned dz_min_inv;     // min SSP spacing near the telescope range (inverted float bits)
   unsigned dt_max_bits;    // max telescope bin width (float bits)
   float bmax;              // |B| limit: (vmax / c) / h
   double lnq0;             // log of the lowest wavelength covered by bucket 0
@@ -118,15 +118,13 @@ __device__ __forceinline__ int2 bucket_entry(const float* __restrict__ wave_z, i
 
 // Bucket table over log(q), per-wavelength bucket coordinates A_t, and the spacing
 // extrema that decide whether the one-step walk is exact.  Any number of blocks;
-// ctrl->dz_min_bits / dt_max_bits must be preset to 0xffffffff / 0.
-__global__ void cube_setup_kernel(const float* __restrict__ wave_z, int n_wave,
+// ctrl must be preset to 0.
+__device__ __forceinline__ void cube_setup(const float* __restrict__ wave_z, int n_wave,
                                   const float* __restrict__ wave_t, int n_t,
                                   CubeCtrl* __restrict__ ctrl, float* __restrict__ At,
-                                  int2* __restrict__ bucket) {
+                                  int2* __restrict__ bucket, int gtid, int gsz) {
   double lnq0, h;
   bucket_params(wave_t, n_t, lnq0, h);
-  const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int gsz = gridDim.x * blockDim.x;
   if (gtid == 0) {
     ctrl->next_item = 0;
     ctrl->error = 0;
@@ -150,7 +148,7 @@ __global__ void cube_setup_kernel(const float* __restrict__ wave_z, int n_wave,
     if (b >= qlo && a <= qhi) {
       float d = wave_z[k + 1] - wave_z[k];
       if (!(d > 0.f)) d = 0.f;
-      atomicMin(&ctrl->dz_min_bits, __float_as_uint(d));
+      atomicMax(&ctrl->dz_min_inv, ~__float_as_uint(d));
     }
   }
   for (int b = gtid; b < kBuckets; b += gsz) bucket[b] = bucket_entry(wave_z, n_wave, lnq0, h, b);
@@ -159,10 +157,10 @@ __global__ void cube_setup_kernel(const float* __restrict__ wave_z, int n_wave,
 // Corner table: ct[(iz*(nA-1) + ia)*nW + k] = (F[iz][ia][k], F[iz+1][ia][k],
 // F[iz][ia+1][k], F[iz+1][ia+1][k]).
 __device__ __forceinline__ void corner_table(const float* __restrict__ flux, int nZ, int nA,
-                                             int nW, float4* __restrict__ ct) {
+                                             int nW, float4* __restrict__ ct, long long first,
+                                             long long step) {
   const long long total = (long long)(nZ - 1) * (nA - 1) * nW;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
+  for (long long i = first; i < total; i += step) {
     const long long cell = i / nW;
     const int k = (int)(i - cell * nW);
     const int iz = (int)(cell / (nA - 1)), ia = (int)(cell - (long long)iz * (nA - 1));
@@ -170,11 +168,6 @@ __device__ __forceinline__ void corner_table(const float* __restrict__ flux, int
     const long long b10 = b00 + (long long)nA * nW;
     ct[i] = make_float4(flux[b00], flux[b10], flux[b00 + nW], flux[b10 + nW]);
   }
-}
-
-__global__ void cube_corner_table_kernel(const float* __restrict__ flux, int nZ, int nA,
-                                         int nW, float4* __restrict__ ct) {
-  corner_table(flux, nZ, nA, nW, ct);
 }
 
 // prefix[r][k] = sum_{k'=1..k} F[r][k'] * (lambda_z,k' - lambda_z,k'-1) for every SSP row
@@ -217,10 +210,26 @@ __device__ __forceinline__ void prefix_row(const float* __restrict__ flux, int r
   __syncthreads();  // s_warp is reused by the next row
 }
 
-__global__ void __launch_bounds__(kPrefixThreads) cube_prefix_kernel(
-    const float* __restrict__ flux, int rows, int nW, const float* __restrict__ wave_z,
-    double* __restrict__ prefix) {
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) prefix_row(flux, r, nW, wave_z, prefix);
+// The setup passes over the grids in one launch: the first n_setup blocks the bucket table and
+// the spacing extrema, the next n_corner the corner table, the others the prefix sums.
+__global__ void __launch_bounds__(kPrefixThreads) cube_tables_kernel(
+    const float* __restrict__ flux, int nZ, int nA, int nW, const float* __restrict__ wave_z,
+    const float* __restrict__ wave_t, int n_t, CubeCtrl* __restrict__ ctrl,
+    float* __restrict__ At, int2* __restrict__ bucket, float4* __restrict__ ct,
+    double* __restrict__ prefix, int n_setup, int n_corner) {
+  const int b = blockIdx.x;
+  if (b < n_setup) {
+    cube_setup(wave_z, nW, wave_t, n_t, ctrl, At, bucket, b * kPrefixThreads + threadIdx.x,
+               n_setup * kPrefixThreads);
+  } else if (b < n_setup + n_corner) {
+    corner_table(flux, nZ, nA, nW, ct,
+                 (long long)(b - n_setup) * kPrefixThreads + threadIdx.x,
+                 (long long)n_corner * kPrefixThreads);
+  } else {
+    const int rows = nZ * nA;
+    for (int r = b - n_setup - n_corner; r < rows; r += gridDim.x - n_setup - n_corner)
+      prefix_row(flux, r, nW, wave_z, prefix);
+  }
 }
 
 // dz, dt: smallest SSP spacing near the telescope range and widest telescope bin.
@@ -313,15 +322,15 @@ __global__ void cube_gather_kernel(const float* __restrict__ mass, const float* 
                                    const float* __restrict__ av, float alo, float ahi) {
   gather_records(mass, met, age, vel, vel_stride, vel_comp, perm, seg_off, n_seg, n, zg, nZ, ag,
                  nA, wave_z, n_wave, wave_t, n_t, prefix, ctrl->inv_h, ctrl->bmax,
-                 __uint_as_float(ctrl->dz_min_bits), __uint_as_float(ctrl->dt_max_bits), rec,
+                 __uint_as_float(~ctrl->dz_min_inv), __uint_as_float(ctrl->dt_max_bits), rec,
                  with_grad, av, alo, ahi);
 }
 
 // Per spaxel: chunk count.  Multi-chunk spaxels get one item (and partial slot) per
 // chunk; single-chunk spaxels are split into a "big" and a "small" class.
-__global__ void cube_count_kernel(const int* __restrict__ seg_off, int n_seg, int chunk,
-                                  int big_item, int* __restrict__ slot_cnt,
-                                  int* __restrict__ big_cnt, int* __restrict__ small_cnt) {
+__device__ __forceinline__ void cube_count(const int* seg_off, int n_seg, int chunk,
+                                           int big_item, int* slot_cnt, int* big_cnt,
+                                           int* small_cnt) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += gridDim.x * blockDim.x) {
     const int cnt = seg_off[s + 1] - seg_off[s];
     const int nch = cnt <= chunk ? 1 : (cnt + chunk - 1) / chunk;
@@ -331,13 +340,17 @@ __global__ void cube_count_kernel(const int* __restrict__ seg_off, int n_seg, in
   }
 }
 
+__global__ void cube_count_kernel(const int* seg_off, int n_seg, int chunk, int big_item,
+                                  int* slot_cnt, int* big_cnt, int* small_cnt) {
+  cube_count(seg_off, n_seg, chunk, big_item, slot_cnt, big_cnt, small_cnt);
+}
+
 // Item order: chunks of multi-chunk spaxels (item index = partial slot), then big
 // single-chunk spaxels, then the rest.
-__global__ void cube_fill_items_kernel(const int* __restrict__ seg_off, int n_seg, int chunk,
-                                       int big_item, const int* __restrict__ slot_start,
-                                       const int* __restrict__ big_start,
-                                       const int* __restrict__ small_start,
-                                       int2* __restrict__ items, CubeCtrl* __restrict__ ctrl) {
+__device__ __forceinline__ void cube_fill_items(const int* seg_off, int n_seg, int chunk,
+                                                int big_item, const int* slot_start,
+                                                const int* big_start, const int* small_start,
+                                                int2* items, CubeCtrl* ctrl) {
   const int total_slots = slot_start[n_seg];
   const int total_big = big_start[n_seg];
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += gridDim.x * blockDim.x) {
@@ -353,6 +366,13 @@ __global__ void cube_fill_items_kernel(const int* __restrict__ seg_off, int n_se
   }
   if (blockIdx.x == 0 && threadIdx.x == 0)
     ctrl->n_items = total_slots + total_big + small_start[n_seg];
+}
+
+__global__ void cube_fill_items_kernel(const int* seg_off, int n_seg, int chunk, int big_item,
+                                       const int* slot_start, const int* big_start,
+                                       const int* small_start, int2* items, CubeCtrl* ctrl) {
+  cube_fill_items(seg_off, n_seg, chunk, big_item, slot_start, big_start, small_start, items,
+                  ctrl);
 }
 
 struct CubeLayout {
@@ -378,6 +398,7 @@ CubeLayout carve_cube(void* ws, long long n, int n_seg, int n_t, int nZ, int nA,
   Carve c(ws);
   CubeLayout L;
   L.ctrl = c.take<CubeCtrl>(1);
+  L.done = c.take<int>((size_t)n_seg);  // zeroed together with ctrl
   L.At = c.take<float>((size_t)n_t);
   L.bucket = c.take<int2>(kBuckets);
   L.ct = c.take<float4>((size_t)(nZ > 1 ? nZ - 1 : 0) * (nA > 1 ? nA - 1 : 0) * nW);
@@ -387,36 +408,44 @@ CubeLayout carve_cube(void* ws, long long n, int n_seg, int n_t, int nZ, int nA,
   L.big_cnt = c.take<int>((size_t)n_seg + 1);
   L.small_cnt = c.take<int>((size_t)n_seg + 1);
   L.items = c.take<int2>((size_t)(max_slots(n, chunk) + n_seg));
-  L.done = c.take<int>((size_t)n_seg);
   L.partials = c.take<float>((size_t)max_slots(n, chunk) * n_t);
   L.bytes = c.off;
   return L;
 }
 
-// Launches the setup passes into the carved workspace: bucket table, corner table,
-// prefix sums, particle records (with dT/dZ, dT/dage when with_grad) and the work-item
-// list.  Six to eight kernels plus three small memsets on stream st.
+// Work items of up to 8192 spaxels by one block: count, scans and fill in one launch.
+constexpr int kItemsOneBlock = 8192;
+__global__ void __launch_bounds__(1024) cube_items_kernel(const int* seg_off, int n_seg, int chunk,
+                                                          int big_item, int* slot_cnt,
+                                                          int* big_cnt, int* small_cnt,
+                                                          int2* items, CubeCtrl* ctrl) {
+  cube_count(seg_off, n_seg, chunk, big_item, slot_cnt, big_cnt, small_cnt);
+  __syncthreads();
+  scan_exclusive_block(slot_cnt, n_seg, 1);
+  scan_exclusive_block(big_cnt, n_seg, 1);
+  scan_exclusive_block(small_cnt, n_seg, 1);
+  __syncthreads();
+  cube_fill_items(seg_off, n_seg, chunk, big_item, slot_cnt, big_cnt, small_cnt, items, ctrl);
+}
+
+// Launches the setup passes into the carved workspace: bucket table, corner table and
+// prefix sums (one launch), particle records (with dT/dZ, dT/dage when with_grad) and the
+// work-item list (one launch up to kItemsOneBlock spaxels, else three), after one memset.
 inline int cube_prepare(const CubeInputs& in, const CubeLayout& L, const CubeTuning& tune,
                         bool with_grad, cudaStream_t st) {
-  RUBIX_CUDA_TRY(cudaMemsetAsync(&L.ctrl->dz_min_bits, 0xff, sizeof(unsigned), st));
-  RUBIX_CUDA_TRY(cudaMemsetAsync(&L.ctrl->dt_max_bits, 0, sizeof(unsigned), st));
+  RUBIX_CUDA_TRY(cudaMemsetAsync(L.ctrl, 0, (size_t)((char*)(L.done + in.n_seg) - (char*)L.ctrl),
+                                 st));
   {
     const int work = std::max(std::max(in.n_wave_t, in.n_wave), kBuckets);
-    cube_setup_kernel<<<div_up(work, 128), 128, 0, st>>>(in.ssp_wave_z, in.n_wave, in.wave_t,
-                                                         in.n_wave_t, L.ctrl, L.At, L.bucket);
-    RUBIX_LAUNCH_CHECK("cube_setup_kernel");
-  }
-  {
+    const int n_setup = div_up(work, kPrefixThreads);
     const long long total = (long long)(in.n_met - 1) * (in.n_age - 1) * in.n_wave;
-    const int g = (int)std::min<long long>((total + 255) / 256, (long long)sm_count() * 8);
-    cube_corner_table_kernel<<<g, 256, 0, st>>>(in.ssp_flux, in.n_met, in.n_age, in.n_wave,
-                                                L.ct);
-    RUBIX_LAUNCH_CHECK("cube_corner_table_kernel");
-    const int rows = in.n_met * in.n_age;
-    const int pg = std::min(rows, sm_count() * 16);
-    cube_prefix_kernel<<<pg, kPrefixThreads, 0, st>>>(in.ssp_flux, rows, in.n_wave,
-                                                      in.ssp_wave_z, L.prefix);
-    RUBIX_LAUNCH_CHECK("cube_prefix_kernel");
+    const int n_corner = (int)std::min<long long>((total + kPrefixThreads - 1) / kPrefixThreads,
+                                                  (long long)sm_count() * 16);
+    const int rows = std::min(in.n_met * in.n_age, sm_count() * 16);
+    cube_tables_kernel<<<n_setup + n_corner + rows, kPrefixThreads, 0, st>>>(
+        in.ssp_flux, in.n_met, in.n_age, in.n_wave, in.ssp_wave_z, in.wave_t, in.n_wave_t, L.ctrl,
+        L.At, L.bucket, L.ct, L.prefix, n_setup, n_corner);
+    RUBIX_LAUNCH_CHECK("cube_tables_kernel");
   }
   if (in.n > 0) {
     const int g = (int)std::min<long long>((in.n + 255) / 256, (long long)sm_count() * 8);
@@ -429,7 +458,11 @@ inline int cube_prepare(const CubeInputs& in, const CubeLayout& L, const CubeTun
                                           (float)std::exp(kVmaxKms / kSpeedOfLight));
     RUBIX_LAUNCH_CHECK("cube_gather_kernel");
   }
-  {
+  if (in.n_seg <= kItemsOneBlock) {
+    cube_items_kernel<<<1, 1024, 0, st>>>(in.seg_off, in.n_seg, tune.chunk, tune.big_item,
+                                          L.slot_cnt, L.big_cnt, L.small_cnt, L.items, L.ctrl);
+    RUBIX_LAUNCH_CHECK("cube_items_kernel");
+  } else {
     const int g = (int)std::min<long long>((in.n_seg + 255) / 256, (long long)sm_count() * 8);
     cube_count_kernel<<<g, 256, 0, st>>>(in.seg_off, in.n_seg, tune.chunk, tune.big_item,
                                          L.slot_cnt, L.big_cnt, L.small_cnt);
@@ -440,7 +473,6 @@ inline int cube_prepare(const CubeInputs& in, const CubeLayout& L, const CubeTun
                                               tune.big_item, L.slot_cnt, L.big_cnt,
                                               L.small_cnt, L.items, L.ctrl);
     RUBIX_LAUNCH_CHECK("cube_fill_items_kernel");
-    RUBIX_CUDA_TRY(cudaMemsetAsync(L.done, 0, sizeof(int) * (size_t)in.n_seg, st));
   }
   return RUBIX_OK;
 }

@@ -46,9 +46,8 @@ constexpr int kItem = 4 * kSub;  // particles of a work item
 
 // Work items: ranges of up to kItem particles of one spaxel; empty spaxels have none.
 // Spaxels of several items first (item index = row), then those with many particles.
-__global__ void node_count_kernel(const int* __restrict__ seg_off, int n_seg, int big,
-                                  int* __restrict__ multi, int* __restrict__ large,
-                                  int* __restrict__ small) {
+__device__ __forceinline__ void node_count(const int* seg_off, int n_seg, int big, int* multi,
+                                           int* large, int* small) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += gridDim.x * blockDim.x) {
     const int cnt = seg_off[s + 1] - seg_off[s];
     multi[s] = cnt > kItem ? (cnt + kItem - 1) / kItem : 0;
@@ -57,21 +56,22 @@ __global__ void node_count_kernel(const int* __restrict__ seg_off, int n_seg, in
   }
 }
 
+__global__ void node_count_kernel(const int* seg_off, int n_seg, int big, int* multi, int* large,
+                                  int* small) {
+  node_count(seg_off, n_seg, big, multi, large, small);
+}
+
 // Item index of chunk 0 of a spaxel (its chunks follow one another).
-__device__ __forceinline__ int first_item(int s, int cnt, int big, int n_seg,
-                                          const int* __restrict__ multi,
-                                          const int* __restrict__ large,
-                                          const int* __restrict__ small) {
+__device__ __forceinline__ int first_item(int s, int cnt, int big, int n_seg, const int* multi,
+                                          const int* large, const int* small) {
   if (cnt > kItem) return multi[s];
   if (cnt >= big) return multi[n_seg] + large[s];
   return multi[n_seg] + large[n_seg] + small[s];
 }
 
-__global__ void node_fill_items_kernel(const int* __restrict__ seg_off, int n_seg, int big,
-                                       const int* __restrict__ multi,
-                                       const int* __restrict__ large,
-                                       const int* __restrict__ small, int2* __restrict__ items,
-                                       NodeCtrl* __restrict__ ctrl) {
+__device__ __forceinline__ void node_fill_items(const int* seg_off, int n_seg, int big,
+                                                const int* multi, const int* large,
+                                                const int* small, int2* items, NodeCtrl* ctrl) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += gridDim.x * blockDim.x) {
     const int cnt = seg_off[s + 1] - seg_off[s];
     if (cnt == 0) continue;
@@ -82,6 +82,25 @@ __global__ void node_fill_items_kernel(const int* __restrict__ seg_off, int n_se
     ctrl->n_multi = multi[n_seg];
     ctrl->n_items = multi[n_seg] + large[n_seg] + small[n_seg];
   }
+}
+
+__global__ void node_fill_items_kernel(const int* seg_off, int n_seg, int big, const int* multi,
+                                       const int* large, const int* small, int2* items,
+                                       NodeCtrl* ctrl) {
+  node_fill_items(seg_off, n_seg, big, multi, large, small, items, ctrl);
+}
+
+// All three steps by one block, up to kItemsOneBlock spaxels.
+__global__ void __launch_bounds__(1024) node_items_kernel(const int* seg_off, int n_seg, int big,
+                                                          int* multi, int* large, int* small,
+                                                          int2* items, NodeCtrl* ctrl) {
+  node_count(seg_off, n_seg, big, multi, large, small);
+  __syncthreads();
+  scan_exclusive_block(multi, n_seg, 1);
+  scan_exclusive_block(large, n_seg, 1);
+  scan_exclusive_block(small, n_seg, 1);
+  __syncthreads();
+  node_fill_items(seg_off, n_seg, big, multi, large, small, items, ctrl);
 }
 
 struct GatherArgs {
@@ -908,7 +927,7 @@ int cube_nodes_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t b
   const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
   const long long fit = (long long)((bytes - L.fixed) / row_bytes(nW)) - multi_row_count(n);
   const long long wave = std::min<long long>(n_seg, fit);
-  return 8 + 2 * (int)((n_seg + wave - 1) / wave);
+  return (n_seg <= kItemsOneBlock ? 6 : 8) + 2 * (int)((n_seg + wave - 1) / wave);
 }
 
 int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* lsf_taps, int n_lsf, int lsf_crop,
@@ -932,7 +951,11 @@ int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* l
     const int rc = node_build_tables(in, dust_e, L.prefix, L.h, L.H, L.ctrl, st);
     if (rc != RUBIX_OK) return rc;
   }
-  {
+  if (in.n_seg <= kItemsOneBlock) {
+    node_items_kernel<<<1, 1024, 0, st>>>(in.seg_off, in.n_seg, big_item, L.multi, L.large,
+                                          L.small, L.items, L.ctrl);
+    RUBIX_LAUNCH_CHECK("node_items_kernel");
+  } else {
     const int g = (int)std::min<long long>((in.n_seg + 255) / 256, (long long)sm_count() * 8);
     node_count_kernel<<<g, 256, 0, st>>>(in.seg_off, in.n_seg, big_item, L.multi, L.large,
                                          L.small);

@@ -42,21 +42,37 @@ struct __align__(16) AdjFinal {
   float4 b;  // 1 / dZ, 1 / dage of the cell, mass, index of the particle (bits)
 };
 
-__global__ void node_adj_count_kernel(const int* __restrict__ seg_off, int n_seg,
-                                      int* __restrict__ chunks) {
+__device__ __forceinline__ void adj_count(const int* seg_off, int n_seg, int* chunks) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += gridDim.x * blockDim.x)
     chunks[s] = (seg_off[s + 1] - seg_off[s] + kAdjItem - 1) / kAdjItem;
 }
 
 // Items in the order of their particles, so that a wave of particles is a range of items.
-__global__ void node_adj_fill_kernel(const int* __restrict__ seg_off, int n_seg,
-                                     const int* __restrict__ chunks, int2* __restrict__ items,
-                                     NodeCtrl* __restrict__ ctrl) {
+__device__ __forceinline__ void adj_fill(int n_seg, const int* chunks, int2* items,
+                                         NodeCtrl* ctrl) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += gridDim.x * blockDim.x) {
     const int n = chunks[s + 1] - chunks[s];
     for (int c = 0; c < n; ++c) items[chunks[s] + c] = make_int2(s, c);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->n_items = chunks[n_seg];
+}
+
+__global__ void node_adj_count_kernel(const int* seg_off, int n_seg, int* chunks) {
+  adj_count(seg_off, n_seg, chunks);
+}
+__global__ void node_adj_fill_kernel(int n_seg, const int* chunks, int2* items, NodeCtrl* ctrl) {
+  adj_fill(n_seg, chunks, items, ctrl);
+}
+
+// All three steps by one block, up to kItemsOneBlock spaxels.
+__global__ void __launch_bounds__(1024) node_adj_items_kernel(const int* seg_off, int n_seg,
+                                                              int* chunks, int2* items,
+                                                              NodeCtrl* ctrl) {
+  adj_count(seg_off, n_seg, chunks);
+  __syncthreads();
+  scan_exclusive_block(chunks, n_seg, 1);
+  __syncthreads();
+  adj_fill(n_seg, chunks, items, ctrl);
 }
 
 struct AdjGatherArgs {
@@ -627,7 +643,7 @@ bool cube_nodes_bwd_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t,
 int cube_nodes_bwd_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t bytes) {
   const AdjNodeLayout L = carve_adj(nullptr, n, n_seg, nZ, nA, nW);
   const long long per = std::min(n, part_particles(bytes - L.fixed, nW));
-  return 8 + 2 * (int)((n + per - 1) / per);
+  return (n_seg <= kItemsOneBlock ? 6 : 8) + 2 * (int)((n + per - 1) / per);
 }
 
 int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_stride,
@@ -640,13 +656,16 @@ int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_st
     const int rc = node_build_tables(in, nullptr, L.prefix, L.h, L.H, L.ctrl, st);
     if (rc != RUBIX_OK) return rc;
   }
-  {
+  if (in.n_seg <= kItemsOneBlock) {
+    node_adj_items_kernel<<<1, 1024, 0, st>>>(in.seg_off, in.n_seg, L.chunks, L.items, L.ctrl);
+    RUBIX_LAUNCH_CHECK("node_adj_items_kernel");
+  } else {
     const int g = (int)std::min<long long>((in.n_seg + 255) / 256, (long long)sm_count() * 8);
     node_adj_count_kernel<<<g, 256, 0, st>>>(in.seg_off, in.n_seg, L.chunks);
     RUBIX_LAUNCH_CHECK("node_adj_count_kernel");
     scan_exclusive_1block<<<1, 1024, 0, st>>>(L.chunks, in.n_seg, 1);
     RUBIX_LAUNCH_CHECK("scan_exclusive_1block");
-    node_adj_fill_kernel<<<g, 256, 0, st>>>(in.seg_off, in.n_seg, L.chunks, L.items, L.ctrl);
+    node_adj_fill_kernel<<<g, 256, 0, st>>>(in.n_seg, L.chunks, L.items, L.ctrl);
     RUBIX_LAUNCH_CHECK("node_adj_fill_kernel");
   }
   const int blocks =

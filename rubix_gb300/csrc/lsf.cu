@@ -248,9 +248,8 @@ int launch_row(const LsfArgs& a, cudaStream_t st) {
   if (e != cudaSuccess)
     return set_error(RUBIX_E_CUDA, "cudaFuncSetAttribute(lsf_row_kernel): %s",
                      cudaGetErrorString(e));
-  int per_sm = 0;
-  RUBIX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lsf_row_kernel<KC>,
-                                                               kLsfRowThreads, smem));
+  const int per_sm =
+      blocks_per_sm(reinterpret_cast<const void*>(lsf_row_kernel<KC>), kLsfRowThreads, smem);
   const long long grid = std::min<long long>(a.rows, (long long)sm_count() * std::max(per_sm, 1));
   lsf_row_kernel<KC><<<(int)grid, kLsfRowThreads, smem, st>>>(a);
   RUBIX_LAUNCH_CHECK("lsf_row_kernel");

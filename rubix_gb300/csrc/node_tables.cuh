@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(256) node_fallback_kernel(CubeInputs in, NodeF
       __syncthreads();
     }
   }
-  corner_table(in.ssp_flux, in.n_met, in.n_age, in.n_wave, f.ct);
+  corner_table(in.ssp_flux, in.n_met, in.n_age, in.n_wave, f.ct, gtid, gsz);
   gather_records(in.mass, in.met, in.age, in.vel, in.vel_stride, in.vel_comp, in.perm,
                  in.seg_off, in.n_seg, in.n, in.ssp_met, in.n_met, in.ssp_age, in.n_age,
                  in.ssp_wave_z, in.n_wave, in.wave_t, in.n_wave_t, prefix, 1.0 / h,

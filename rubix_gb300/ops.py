@@ -9,6 +9,9 @@ has a CPU path.
 
 from __future__ import annotations
 
+import ctypes
+import functools
+
 import numpy as np
 import torch
 
@@ -42,13 +45,22 @@ def _count(k: int) -> None:
     LAUNCHES["count"] += int(k)
 
 
+@functools.lru_cache(maxsize=4096)
+def _launches(name: str, *sizes: int) -> int:
+    """Kernels of one call, a function of its sizes alone."""
+    return _lib.query(name, *sizes)
+
+
 def _sort_passes(n_segments: int) -> int:
     bits = max(1, int(n_segments).bit_length())
     return (bits + 8) // 9
 
 
 def _stream(dev: torch.device) -> int:
-    return torch.cuda.current_stream(dev).cuda_stream
+    """The current stream's handle, without building the Stream object (10 us a call on a
+    Grace core, more than the kernel launches of a small step)."""
+    i = dev.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
 
 def _check_cuda(name: str, t: torch.Tensor, dtype=None) -> None:
@@ -101,6 +113,21 @@ def spaxel_assign(coords: torch.Tensor, edges: torch.Tensor) -> torch.Tensor:
               edges.numel(), _ptr(out), _stream(coords.device))
     _count(1 if n > 0 else 0)
     return out
+
+
+def assign_and_mask(coords: torch.Tensor, edges: torch.Tensor):
+    """(spaxel_assign, aperture_mask) of [n, 3] coordinates in one launch, the same values."""
+    coords = _contig("coords", coords, torch.float32)
+    if coords.dim() != 2 or coords.shape[1] != 3:
+        return spaxel_assign(coords, edges), aperture_mask(coords, edges)
+    edges = _contig("edges", edges, torch.float32)
+    n, dev = coords.shape[0], coords.device
+    idx = torch.empty(n, dtype=torch.int32, device=dev)
+    mask = torch.empty(n, dtype=torch.uint8, device=dev)
+    _lib.call("rubix_orient_filter_assign", _ptr(coords), None, n, None, None, None, _ptr(edges),
+              edges.numel(), 0, None, None, None, _ptr(mask), _ptr(idx), _stream(dev))
+    _count(1 if n > 0 else 0)
+    return idx, mask
 
 
 def spaxel_sort(idx: torch.Tensor, n_segments: int, keep: torch.Tensor | None = None):
@@ -190,11 +217,9 @@ def cube_forward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, m
     else:
         _lib.call("rubix_cube_fwd_dust", *ssp_args, *star_args, _ptr(dust_av),
                   _ptr(dust_exponent), *out_args)
-    _count(_lib.query("rubix_cube_fwd_launches", n, int(n_segments), L, nz, na, nw,
+    _count(_launches("rubix_cube_fwd_launches", n, int(n_segments), L, nz, na, nw,
                       1 if general else 0, ws.numel()))
     if check and n_segments > 0:
-        import ctypes
-
         err = ctypes.c_int(0)
         _lib.call("rubix_cube_status", _ptr(ws), ctypes.byref(err), _stream(dev))
     return out
@@ -230,7 +255,8 @@ def cube_backward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, 
     dev = mass.device
     if av_grad and dust_av is None:
         raise ValueError("av_grad needs dust_av and dust_exponent")
-    grads = [torch.empty(n, dtype=torch.float32, device=dev) for _ in range(5 if av_grad else 4)]
+    # one buffer: the library clears rows that follow one another with one memset
+    grads = torch.empty((5 if av_grad else 4, n), dtype=torch.float32, device=dev).unbind(0)
     nbytes = _lib.query("rubix_cube_bwd_workspace_size", n, int(n_segments), L, nz, na, nw)
     ws = workspace(nbytes, dev)
     if (dust_av is None) != (dust_exponent is None):
@@ -253,7 +279,7 @@ def cube_backward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, 
                   _ptr(dust_exponent), _ptr(perm), _ptr(seg_offsets), int(n_segments), n,
                   _ptr(adj), adj.stride(0), *[_ptr(g) for g in grads], _ptr(ws), ws.numel(),
                   _stream(dev))
-    _count(_lib.query("rubix_cube_bwd_launches", n, int(n_segments), L, nz, na, nw,
+    _count(_launches("rubix_cube_bwd_launches", n, int(n_segments), L, nz, na, nw,
                       0 if dust_av is None else 1, ws.numel()))
     return tuple(grads)
 
@@ -363,8 +389,6 @@ def orient_filter_assign(coords, velocity, matrix, edges, fields=(), mask=True,
     (host) or None; fields: float32 tensors with n rows, copied with the particles
     outside the aperture set to 0.  Returns (coords_out, velocity_out, fields_out, mask
     uint8 or None, idx int32); without ``matrix`` coords_out / velocity_out are None."""
-    import ctypes
-
     coords = _contig("coords", coords, torch.float32)
     n = coords.shape[0]
     if coords.dim() != 2 or coords.shape[1] != 3:
@@ -457,8 +481,6 @@ def apply_noise_(cube: torch.Tensor, signal_to_noise: float, distribution: str =
 
 def philox4x32_10(counter, key) -> list:
     """One Philox4x32-10 block computed by the library on the host (no GPU needed)."""
-    import ctypes
-
     c = (ctypes.c_uint32 * 4)(*[int(x) & 0xFFFFFFFF for x in counter])
     k = (ctypes.c_uint32 * 2)(*[int(x) & 0xFFFFFFFF for x in key])
     o = (ctypes.c_uint32 * 4)()
@@ -504,8 +526,6 @@ def psf_forward(cube: torch.Tensor, taps_y, taps_x=None, out=None) -> torch.Tens
 def psf_status(device=None) -> int:
     """Device error word of the TMA-staged PSF: 1 if a staged-row wait ran out since the
     last read (reading clears it), else 0.  Synchronises the current stream."""
-    import ctypes
-
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else device
     v = ctypes.c_int(0)
     _lib.lib().rubix_psf_status(ctypes.byref(v), _stream(dev))
