@@ -549,6 +549,141 @@ __global__ void __launch_bounds__(kPsfThreads, 2)
   }
 }
 
+// The strip with 64 wavelengths, for spaxel strides that rule the tiled copies out: a lane owns
+// two neighbouring wavelengths as a packed pair and kPairXB x positions, so both passes run
+// packed FMAs on operands that are pairs as they come (8-byte shared loads), for equal x and y
+// taps of up to 15 (one set of tap pairs in registers).  512 threads, one block an SM, rows
+// staged by 4-byte copies whose addresses and sizes are fixed but for the row.  Same products
+// and order per output as psf_reg_body: bit-identical.  150 x 150 x 3721, 15 taps: 207 us
+// where psf_reg2_kernel took 264 (one read and one write at the copy rate: 98); bound by
+// latency and issue (a barrier a row, 16 warps).  Staged by TMA it is no faster than
+// psf_tma_kernel (206 against 199 us), which keeps the aligned strides.
+constexpr int kPairXB = 2;
+constexpr int kPairThreads = 32 * kPsfTileX / kPairXB;
+constexpr int kPairTileL = 64;
+constexpr int kPairStages = 8;
+constexpr int kPairMaxTaps = 15;
+
+template <int M>
+constexpr size_t psf_pair_smem() {
+  return (size_t)kPairStages * (kPsfTileX + M - 1) * kPairTileL * sizeof(float);
+}
+
+template <int M>
+__global__ void __launch_bounds__(kPairThreads, 1) psf_pair_kernel(PsfArgs a) {
+  constexpr int W = kPsfTileX + M - 1;  // staged row width
+  constexpr int kRow = W * kPairTileL;
+  constexpr int kS = kPairStages;
+  constexpr int PER = (kRow + kPairThreads - 1) / kPairThreads;
+  extern __shared__ __align__(128) float s_pair[];  // [kS][kRow]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ny = a.ny, nx = a.nx, nl = a.nl, oy = a.oy;
+  const int x0 = blockIdx.x * kPsfTileX, l0 = blockIdx.y * kPairTileL;
+  const int l = l0 + 2 * lane, x = x0 + warp * kPairXB;
+  const int xsrc0 = x0 - (M - 1) + a.ox;
+  const int total = ny + oy;
+  // this thread's copies of a row: offsets from the row (0 where nothing is read) and sizes as
+  // bits 2, 3, .. (4 bytes or none)
+  unsigned off[PER], size = 0u;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int q = tid + k * kPairThreads;
+    const int xg = xsrc0 + q / kPairTileL, lg = l0 + q % kPairTileL;
+    const bool ok = q < kRow && xg >= 0 && xg < nx && lg < nl;
+    off[k] = ok ? (unsigned)((long long)xg * a.sin + lg) : 0u;
+    size |= ok ? (4u << k) : 0u;
+  }
+  const unsigned s0 = static_cast<unsigned>(__cvta_generic_to_shared(s_pair)) + 4u * tid;
+  const long long row_in = (long long)nx * a.sin;
+  const float* src = a.in;  // row of the next copies (the first again below the cube)
+  auto issue_row = [&](int r, int slot) {
+    if (r < total) {
+      const unsigned sz = r < ny ? size : 0u;
+      const unsigned dst = s0 + 4u * kRow * slot;
+#pragma unroll
+      for (int k = 0; k < PER; ++k)
+        if ((k + 1) * kPairThreads <= kRow || tid + k * kPairThreads < kRow)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
+                           dst + 4u * kPairThreads * k),
+                       "l"(src + off[k]), "r"((sz >> k) & 4u)
+                       : "memory");
+      if (r + 1 < ny) src += row_in;
+    }
+    cp_async_commit();
+  };
+  for (int r = 0; r < kS - 1; ++r) issue_row(r, r);
+  float2 win[M][kPairXB];
+#pragma unroll
+  for (int i = 0; i < M; ++i)
+#pragma unroll
+    for (int j = 0; j < kPairXB; ++j) win[i][j] = make_float2(0.f, 0.f);
+  // the taps as pairs, opaque to the compiler so that it keeps them (see psf_tma_kernel)
+  float2 tp[M];
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    unsigned long long v;
+    const float t = a.ty_dev ? a.ty_dev[i] : a.ty[i];
+    asm volatile("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(t));
+    tp[i] = *reinterpret_cast<const float2*>(&v);
+  }
+  const float* col = s_pair + warp * kPairXB * kPairTileL + 2 * lane;
+  // the outputs of this thread: row r - oy, columns x and x + 1, wavelengths l and l + 1
+  bool in[kPairXB][2];
+#pragma unroll
+  for (int j = 0; j < kPairXB; ++j) {
+    in[j][0] = x + j < nx && l < nl;
+    in[j][1] = x + j < nx && l + 1 < nl;
+  }
+  float* o0 = a.out + ((long long)-oy * nx + x) * a.sout + l;
+  float* o1 = o0 + a.sout;
+  const long long row_out = (long long)nx * a.sout;
+  int slot = 0;
+  for (int r0 = 0; r0 < total; r0 += M) {
+#pragma unroll
+    for (int jj = 0; jj < M; ++jj) {
+      const int r = r0 + jj;
+      if (r >= total) break;
+      cp_async_wait<kS - 2>();  // row r has landed (this thread's copies)
+      __syncthreads();          // ... and every thread's; row r - 1 is consumed
+      issue_row(r + kS - 1, slot == 0 ? kS - 1 : slot - 1);
+      // x-pass: inputs from the last to the first, so that each output takes its taps in
+      // order (output j of tap i reads input j + M - 1 - i)
+      const float* row = col + slot * kRow;
+      float2 h[kPairXB];
+#pragma unroll
+      for (int j = 0; j < kPairXB; ++j) h[j] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int q = kPairXB + M - 2; q >= 0; --q) {
+        const float2 v = *reinterpret_cast<const float2*>(row + q * kPairTileL);
+#pragma unroll
+        for (int j = 0; j < kPairXB; ++j) {
+          const int i = j + M - 1 - q;
+          if (i >= 0 && i < M) h[j] = __ffma2_rn(tp[i], v, h[j]);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kPairXB; ++j) win[jj][j] = h[j];
+      if (r >= oy) {
+        float2 y[kPairXB];
+#pragma unroll
+        for (int j = 0; j < kPairXB; ++j) {
+          y[j] = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int i = 0; i < M; ++i) y[j] = __ffma2_rn(tp[i], win[(jj - i + M) % M][j], y[j]);
+        }
+        if (in[0][0]) o0[0] = y[0].x;
+        if (in[0][1]) o0[1] = y[0].y;
+        if (in[1][0]) o1[0] = y[1].x;
+        if (in[1][1]) o1[1] = y[1].y;
+      }
+      o0 += row_out;
+      o1 += row_out;
+      slot = slot + 1 == kS ? 0 : slot + 1;
+    }
+  }
+  cp_async_wait<0>();
+}
+
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                    const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                    const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -568,26 +703,54 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
+// The tensor map of one staged row, when the input allows tiled copies (16-byte aligned base,
+// spaxel stride a multiple of 4 floats).
+template <int M>
+bool psf_map(const PsfArgs& a, int tile_l, CUtensorMap* map) {
+  if (a.sin % 4 != 0 || (reinterpret_cast<uintptr_t>(a.in) & 15) != 0) return false;
+  const EncodeTiledFn enc = encode_tiled();
+  if (enc == nullptr) return false;
+  constexpr int W = kPsfTileX + M - 1;
+  const cuuint64_t dims[3] = {(cuuint64_t)a.nl, (cuuint64_t)a.nx, (cuuint64_t)a.ny};
+  const cuuint64_t strides[2] = {(cuuint64_t)a.sin * sizeof(float),
+                                 (cuuint64_t)a.nx * (cuuint64_t)a.sin * sizeof(float)};
+  const cuuint32_t box[3] = {(cuuint32_t)tile_l, (cuuint32_t)W, 1};
+  const cuuint32_t elem[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(a.in), dims, strides,
+             box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The packed-pair kernel: no tiled copies, equal taps, and enough strips for a block on every
+// SM (smaller cubes fill the chip better with the 32-wavelength strips).
+template <int M>
+bool launch_psf_pair(const PsfArgs& a, cudaStream_t st, int* rc) {
+  if (a.sin % 4 == 0 && (reinterpret_cast<uintptr_t>(a.in) & 15) == 0) return false;
+  const dim3 grid(div_up(a.nx, kPsfTileX), div_up(a.nl, kPairTileL));
+  if ((long long)grid.x * grid.y < sm_count()) return false;
+  if (a.ty_dev ? a.ty_dev != a.tx_dev : !std::equal(a.ty, a.ty + M, a.tx)) return false;
+  const size_t smem = psf_pair_smem<M>();
+  const cudaError_t e = cudaFuncSetAttribute(
+      psf_pair_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) {
+    *rc = set_error(RUBIX_E_CUDA, "cudaFuncSetAttribute(psf_pair_kernel): %s",
+                    cudaGetErrorString(e));
+    return true;
+  }
+  psf_pair_kernel<M><<<grid, kPairThreads, smem, st>>>(a);
+  *rc = RUBIX_OK;
+  return true;
+}
+
 // The TMA-staged kernel when the input allows tiled copies (16-byte aligned base, spaxel
 // stride a multiple of 4 floats); false (nothing launched) otherwise.  With `w` the dot
 // mode (device taps) into *dot_out.
 template <int M>
 bool launch_psf_tma(const PsfArgs& a, cudaStream_t st, const float* w = nullptr,
                     FusedDotScratch* dot_ws = nullptr, double* dot_out = nullptr) {
-  if (a.sin % 4 != 0 || (reinterpret_cast<uintptr_t>(a.in) & 15) != 0) return false;
-  const EncodeTiledFn enc = encode_tiled();
-  if (enc == nullptr) return false;
-  constexpr int W = kPsfTileX + M - 1;
   CUtensorMap map;
-  const cuuint64_t dims[3] = {(cuuint64_t)a.nl, (cuuint64_t)a.nx, (cuuint64_t)a.ny};
-  const cuuint64_t strides[2] = {(cuuint64_t)a.sin * sizeof(float),
-                                 (cuuint64_t)a.nx * (cuuint64_t)a.sin * sizeof(float)};
-  const cuuint32_t box[3] = {(cuuint32_t)kPsfTileL, (cuuint32_t)W, 1};
-  const cuuint32_t elem[3] = {1, 1, 1};
-  if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(a.in), dims, strides, box,
-          elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return false;
+  if (!psf_map<M>(a, kPsfTileL, &map)) return false;
   dim3 grid(div_up(a.nx, kPsfTileX), div_up(a.nl, kPsfTileL));
   if (w != nullptr)
     psf_tma_kernel<M, true, true><<<grid, kPsfThreads, 0, st>>>(map, a, w, dot_ws, dot_out);
@@ -634,6 +797,14 @@ __global__ void __launch_bounds__(kPsfThreads) ragged_psf_kernel(RaggedPsfArgs a
 template <int M>
 int launch_psf_reg(const PsfArgs& a, cudaStream_t st) {
   dim3 grid(div_up(a.nx, kPsfTileX), div_up(a.nl, kPsfTileL));
+  if constexpr (M <= kPairMaxTaps) {
+    int rc = RUBIX_OK;
+    if (launch_psf_pair<M>(a, st, &rc)) {
+      if (rc != RUBIX_OK) return rc;
+      RUBIX_LAUNCH_CHECK("psf_pair_kernel");
+      return RUBIX_OK;
+    }
+  }
   // rows staged by TMA where the stride allows (up to 17 taps, where the window and the
   // tap pairs stay in registers), host or device taps
   if (M <= 17 && launch_psf_tma<(M <= 17 ? M : 17)>(a, st)) {
