@@ -262,6 +262,8 @@ __global__ void __launch_bounds__(kPrefixThreads) node_tables_kernel(
 // H[i][c] = sum_k h[i][k] F[c][k]: 64 alpha rows x 32 templates per block of 128 threads,
 // 4 x 4 per thread, 32 nodes staged at a time.  Sums of 32 products are added with Kahan's
 // compensation: a plain float32 sum over ~740 nodes would be 5e-7 off, this one is 1e-8.
+// 106 us at 10^7 particles (800 alpha rows x 1302 templates; 129 with padded tiles, whose
+// transposing stores fell in 8 banks).
 // Bound by FMA issue: 1 GFMA for 1025 rows of a 1326-template grid, 40 TFMA/s on the chip.
 __global__ void __launch_bounds__(128) node_table_product_kernel(
     const float* __restrict__ h, int kpad, const float* __restrict__ flux, int n_templ,
@@ -274,8 +276,10 @@ __global__ void __launch_bounds__(128) node_table_product_kernel(
   if (!p.ok) return;
   const int k_last = min(n_wave - ctrl->k_last_inv, n_wave - 1);
   const int K = min(k_last - p.k_first + 1, kpad);
-  __shared__ float sa[2][BK][BM + 4];
-  __shared__ float sb[2][BK][BN + 4];
+  // columns permuted by the node (column ^ 4 (k / 4 mod 8)): the transposing stores of a warp
+  // fall in 32 banks and the 16-byte loads stay whole
+  __shared__ __align__(16) float sa[2][BK][BM];
+  __shared__ __align__(16) float sb[2][BK][BN];
   const int tid = threadIdx.x;
   const int r0 = tile * BM, c0 = blockIdx.x * BN;
   const int tr = (tid >> 3) * 4, tc = (tid & 7) * 4;
@@ -297,13 +301,14 @@ __global__ void __launch_bounds__(128) node_table_product_kernel(
   auto store = [&](int buf) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      sa[buf][lk][lr + 16 * i] = ra[i].x;
-      sa[buf][lk + 1][lr + 16 * i] = ra[i].y;
-      sa[buf][lk + 2][lr + 16 * i] = ra[i].z;
-      sa[buf][lk + 3][lr + 16 * i] = ra[i].w;
+      const int col = (lr + 16 * i) ^ lk;  // lk = 4 (k / 4)
+      sa[buf][lk][col] = ra[i].x;
+      sa[buf][lk + 1][col] = ra[i].y;
+      sa[buf][lk + 2][col] = ra[i].z;
+      sa[buf][lk + 3][col] = ra[i].w;
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) sb[buf][lane][warp * 8 + j] = rb[j];
+    for (int j = 0; j < 8; ++j) sb[buf][lane][(warp * 8 + j) ^ (lane & 28)] = rb[j];
   };
   float sum[4][4], comp[4][4];
 #pragma unroll
@@ -319,8 +324,8 @@ __global__ void __launch_bounds__(128) node_table_product_kernel(
     float acc[4][4];
 #pragma unroll
     for (int k = 0; k < BK; ++k) {
-      const float4 a = *reinterpret_cast<const float4*>(&sa[s & 1][k][tr]);
-      const float4 b = *reinterpret_cast<const float4*>(&sb[s & 1][k][tc]);
+      const float4 a = *reinterpret_cast<const float4*>(&sa[s & 1][k][tr ^ (k & 28)]);
+      const float4 b = *reinterpret_cast<const float4*>(&sb[s & 1][k][tc ^ (k & 28)]);
       const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -345,6 +350,26 @@ __global__ void __launch_bounds__(128) node_table_product_kernel(
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (c0 + tc + j < n_templ) H[(long long)(r0 + tr + i) * n_templ + c0 + tc + j] = sum[i][j];
+}
+
+// Last SSP wavelength k with lambda'_k <= x (-1: none), on an ascending grid (where it is not,
+// the plan flags every spaxel): a linear guess, right to one node on a uniform grid, else the
+// search, whose ten dependent loads a block waited for (node_gather_kernel 194 -> 173 us at
+// 10^6 particles, 10.5 -> 7.8 at 2000; the adjoint's gather alike).
+__device__ __forceinline__ int last_below(const float* __restrict__ wz, int n, float alpha,
+                                          float x) {
+  if (n < 2) return count_le_scaled(wz, n, alpha, x) - 1;
+  const float z0 = wz[0], inv = (float)(n - 1) / (wz[n - 1] - z0);
+  const int k = (int)fminf(fmaxf((x / alpha - z0) * inv, 0.f), (float)(n - 2));
+  const float a = __fmul_rn(wz[k], alpha), b = __fmul_rn(wz[k + 1], alpha);
+  if (x < a) {
+    if (k > 0 && __fmul_rn(wz[k - 1], alpha) <= x) return k - 1;
+  } else if (x < b) {
+    return k;
+  } else if (k + 2 < n && x < __fmul_rn(wz[k + 2], alpha)) {
+    return k + 1;
+  }
+  return count_le_scaled(wz, n, alpha, x) - 1;
 }
 
 // One particle on the tables: the corner weights, T (and, for the gradients, its corner
@@ -388,8 +413,8 @@ __device__ __forceinline__ NodeParticle node_particle(const CubeInputs& in,
   p.dag = in.ssp_age[ia] - in.ssp_age[ia - 1];
   p.tz = p.dzg == 0.f ? 0.f : (Z - in.ssp_met[iz - 1]) / p.dzg;
   p.ta = p.dag == 0.f ? 0.f : (A - in.ssp_age[ia - 1]) / p.dag;
-  const int ks = count_le_scaled(in.ssp_wave_z, in.n_wave, p.alpha, x0) - 1;
-  const int ke = count_le_scaled(in.ssp_wave_z, in.n_wave, p.alpha, x1) - 1;
+  const int ks = last_below(in.ssp_wave_z, in.n_wave, p.alpha, x0);
+  const int ke = last_below(in.ssp_wave_z, in.n_wave, p.alpha, x1);
   p.row = (iz - 1) * in.n_age + (ia - 1);
   if (ks < 0 || ke + 1 > in.n_wave - 1) {
     p.bad = true;
