@@ -23,8 +23,6 @@ constexpr float kAlphaMax = 2040.f * kAlphaStep;       // |alpha - 1| covered (2
 constexpr int kAlphaTile = 64;                         // rows computed together
 constexpr int kAlphaTiles = 2 * kAlphaHalf / kAlphaTile + 1;
 constexpr int kAlphaRows = kAlphaTiles * kAlphaTile;
-constexpr int kNodeWarps = 20;
-constexpr int kNodeThreads = 32 * kNodeWarps;
 constexpr int kStage = 33;       // staged records of a warp: 32 and one of weight zero
 constexpr int kRuns = 4;
 constexpr int kDustMost = 8;     // samples between two nodes that a lane holds with dust
