@@ -132,18 +132,19 @@ def flops_per_particle_lambda(w):
     return 7.4 + 11.0 * n_e / float(w.wave_t.size)
 
 
-def profile_file(workload):
-    """The committed ncu summary of the main kernel on this workload's spaxel grid."""
-    return os.path.join(ROOT, "profiles", f"cube_fwd_{workload}.txt")
+def profile_file(workload, path="cube"):
+    """The committed ncu summary of rubix_cube_fwd on this workload's spaxel grid: the
+    general path's main kernel ("cube") or the kernels of the node path ("node")."""
+    return os.path.join(ROOT, "profiles", f"{path}_fwd_{workload}.txt")
 
 
-def _profile_per_launch(n_particles, total_key, fixed_key, workload="ifu"):
-    """A per-launch count of the main kernel from the committed ncu summary of the
+def _profile_per_launch(n_particles, total_key, fixed_key, workload="ifu", path="cube"):
+    """A per-launch count of rubix_cube_fwd from the committed ncu summary of the
     workload (fixed part + per-particle part), scaled to the particle count of this run;
     None when no summary exists for the workload's grid."""
     try:
         vals = {}
-        with open(profile_file(workload)) as f:
+        with open(profile_file(workload, path)) as f:
             for line in f:
                 if ":" in line and not line.startswith("#"):
                     k, v = line.split(":", 1)
@@ -156,15 +157,16 @@ def _profile_per_launch(n_particles, total_key, fixed_key, workload="ifu"):
         return None
 
 
-def traffic_per_launch(n_particles, workload="ifu"):
-    """DRAM bytes per rubix_cube_fwd main-kernel launch (ncu, scaled to the run)."""
-    return _profile_per_launch(n_particles, "dram_bytes_per_launch", "fixed_bytes", workload)
+def traffic_per_launch(n_particles, workload="ifu", path="cube"):
+    """DRAM bytes per rubix_cube_fwd (ncu, scaled to the run)."""
+    return _profile_per_launch(n_particles, "dram_bytes_per_launch", "fixed_bytes", workload,
+                               path)
 
 
-def instructions_per_launch(n_particles, workload="ifu"):
-    """Warp instructions per main-kernel launch (ncu smsp__inst_executed.sum, scaled)."""
+def instructions_per_launch(n_particles, workload="ifu", path="cube"):
+    """Warp instructions per rubix_cube_fwd (ncu smsp__inst_executed.sum, scaled)."""
     return _profile_per_launch(n_particles, "warp_instructions_per_launch",
-                               "fixed_warp_instructions", workload)
+                               "fixed_warp_instructions", workload, path)
 
 
 class ClockSampler:
@@ -1146,18 +1148,20 @@ def main():
     alg_bytes = 20 * N + flux_bytes + S2 * L * 4   # particle fields + perm, SSP flux, cube write
     cube_avg_s = statistics.mean(cube_ms) * 1e-3
     achieved = alg_bytes / cube_avg_s / 1e9
-    traffic = traffic_per_launch(N, w.name)
+    traffic = traffic_per_launch(N, w.name, "node") if not dusty else None
     fpl = flops_per_particle_lambda(w)
     fp32_peak = fp32_peak_tflops(dev)
     fp32_achieved = fpl * N * L / cube_avg_s / 1e12
     compute = {"fp32_peak_tflops": fp32_peak, "peak_source": "measured FMA-chain probe "
                "(bench_fma_probe.cu)", "achieved_tflops": fp32_achieved,
                "frac": fp32_achieved / fp32_peak if fp32_peak else None,
-               "flops_per_particle_lambda": fpl}
-    # instruction issue, the resource the main kernel is bound by: warp instructions per
+               "flops_per_particle_lambda": fpl,
+               "flops": "of the evaluation at every wavelength (general path); the node "
+                        "path that runs here needs fewer, so frac is an equivalent rate"}
+    # instruction issue, the resource the kernels are bound by first: warp instructions per
     # launch (ncu count, scaled to N) over the launch time, against one instruction per
     # cycle per scheduler (4 per SM) at the SM clock sampled during the timed region
-    insts = instructions_per_launch(N, w.name) if not dusty else None  # dust-free kernel
+    insts = instructions_per_launch(N, w.name, "node") if not dusty else None
     issue = None
     if insts:
         sm_mhz = (clocks or {}).get("sm_mhz") or (clocks or {}).get("sm_max_mhz") or 2070.0
@@ -1165,7 +1169,7 @@ def main():
         peak_issue = n_sm * 4 * sm_mhz * 1e6
         issue = {"warp_instructions_per_launch": insts, "achieved_per_s": insts / cube_avg_s,
                  "peak_per_s": peak_issue, "frac": insts / cube_avg_s / peak_issue,
-                 "source": f"smsp__inst_executed.sum of profiles/cube_fwd_{w.name}.txt scaled to "
+                 "source": f"smsp__inst_executed.sum of profiles/node_fwd_{w.name}.txt scaled to "
                            f"{N} particles; peak = {n_sm} SMs x 4 schedulers x 1 warp "
                            f"instruction per cycle at {sm_mhz:.0f} MHz"}
     roofline = {"kernel": "rubix_cube_fwd (fused lookup/mass/Doppler/resample/accumulate)",

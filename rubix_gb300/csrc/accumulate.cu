@@ -2,6 +2,12 @@
 // Doppler shift, flux-conserving resampling onto the telescope grid and the
 // per-spaxel accumulation of the datacube.
 //
+// This file is the general path: any SSP and telescope grid, any particle.  Where
+// cube_nodes.cu applies, rubix_cube_fwd and rubix_cube_fwd_dust sum over SSP nodes there
+// instead (2.5 to 3.6 times as fast) and only spaxels with a particle that it leaves out
+// (hypervelocity, outside the tables) come here; rubix_cube_fwd_general takes this path
+// for everything.
+//
 // Work decomposition
 //   * Setup passes (a few microseconds): a bucket table over log wavelength, the
 //     "corner table" holding, for every (metallicity, age) cell of the SSP grid and

@@ -14,6 +14,9 @@
 // These are the derivatives of the forward formulas with the float32 bracket choices
 // and the in-range mask held fixed, as an automatic differentiation of them gives.
 //
+// This file is the general path; where cube_nodes_bwd.cu applies, the dust-free adjoint is
+// summed over SSP nodes there and only the particles that it leaves out come here.
+//
 // Same decomposition as the forward kernel (persistent blocks pulling spaxel chunks,
 // TMA-staged corner-table segments, per-particle rows built in shared memory, thread i
 // owning R consecutive telescope wavelengths), one particle per step: each thread

@@ -15,7 +15,7 @@
 //
 // Measured (one GB300): 2 10^5 particles, 50 x 50 x 3721, 221 x 6 x 1221 templates: this
 // adjoint 0.82 ms with its tables (the slice kernel 0.59) against 1.43 ms of the general one,
-// a whole fit step 2.82 -> 2.20 ms; eight ragged galaxies (7 10^5 particles) 8.53 -> 6.14 ms.
+// a whole fit step 2.82 -> 2.15 ms; eight ragged galaxies (7 10^5 particles) 8.53 -> 6.10 ms.
 // The slice kernel is bound by issue (0.68 per cycle) and shared-memory wavefronts (60 %).
 // Relative 2-norm errors against float64 as the general path's (3.5e-7).
 //
