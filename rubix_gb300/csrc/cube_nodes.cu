@@ -769,16 +769,37 @@ __global__ void __launch_bounds__(kMergeThreads) node_merge_kernel(MergeArgs a) 
     wave_range(a.ctrl, a.wave, wave_items, i0, i1);
   }
   const int n_multi = a.ctrl->n_multi;
-  for (int s = blockIdx.x; s < a.n_seg; s += gridDim.x) {
-    const int cnt = a.seg_off[s + 1] - a.seg_off[s];
+  if (a.wave > 0 && i0 >= i1) return;
+  // The block's spaxels kMergeThreads at a time, one looked up per thread: a lookup is a chain
+  // of three loads, about 1 us a spaxel when the block waited for each (this kernel 180 ->
+  // 144 us at 22 500 spaxels, 1124 -> 915 at 90 000 and 10^7 particles).
+  __shared__ int s_cnt[kMergeThreads], s_it[kMergeThreads];
+  for (int b = 0, s = blockIdx.x; s < a.n_seg; ++b, s += gridDim.x) {
+    if (b % kMergeThreads == 0) {
+      const long long mine = s + (long long)tid * gridDim.x;
+      int n = -1, it = 0;  // -1: nothing to do
+      if (mine < a.n_seg) {
+        n = a.seg_off[mine + 1] - a.seg_off[mine];
+        if (n == 0) {
+          if (a.wave != 0) n = -1;
+        } else {
+          it = first_item((int)mine, n, a.big, a.n_seg, a.multi, a.large, a.small);
+          if (it < i0 || it >= i1 || a.flags[mine]) n = -1;
+        }
+      }
+      __syncthreads();  // the last batch is done with the lists
+      s_cnt[tid] = n;
+      s_it[tid] = it;
+      __syncthreads();
+    }
+    const int cnt = s_cnt[b % kMergeThreads];
+    if (cnt < 0) continue;
     float* out = a.cube + (long long)s * a.stride;
     if (cnt == 0) {
-      if (a.wave == 0)
-        for (int t = tid; t < n_t; t += kMergeThreads) out[t] = 0.f;
+      for (int t = tid; t < n_t; t += kMergeThreads) out[t] = 0.f;
       continue;
     }
-    const int it0 = first_item(s, cnt, a.big, a.n_seg, a.multi, a.large, a.small);
-    if (it0 < i0 || it0 >= i1 || a.flags[s]) continue;
+    const int it0 = s_it[b % kMergeThreads];
     const int chunks = (cnt + kItem - 1) / kItem;
     for (int i = tid; i < pad; i += kMergeThreads) s_spec[i] = 0.f;
     if (chunks > 1)
