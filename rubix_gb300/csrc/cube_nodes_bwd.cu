@@ -186,7 +186,7 @@ struct AdjSliceArgs {
 // A warp's item on one slice, two nodes per lane and two particles at a time (16 lanes each).
 // Lane (g, i) owns node 2 i + g when samples are summed; every lane then holds both nodes'.
 struct AdjItem {
-  static constexpr int NPL = 2, LPG = 16;
+  static constexpr int LPG = 16;
   const SliceShared& sh;
   const float* dx;  // window: dlambda of every sample, 0 outside the telescope grid
   const int lane, i, g, own, nxt_lane;

@@ -109,13 +109,6 @@ constexpr int kLsfOut = 12;
 constexpr int kLsfRowThreads = 320;  // 320 * 12 = 3840 outputs at a time
 constexpr int kLsfPre = 13;           // rows of up to 13 * 320 staged floats
 
-__device__ __forceinline__ void cp_async_word(float* dst, const float* src, bool valid) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  const int n = valid ? 4 : 0;  // 0: zero-fill, nothing read
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(n)
-               : "memory");
-}
-
 // Floats of one staged row: the last group's window ends 4 KC past a multiple of 12.
 __host__ __device__ constexpr int lsf_row_floats(int n, int KC) {
   return (n + kLsfOut - 1) / kLsfOut * kLsfOut + 4 * KC;
