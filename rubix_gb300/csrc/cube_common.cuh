@@ -180,8 +180,9 @@ constexpr int kPrefixThreads = 128;
 
 // Per SSP row r: prefix[r][k] = sum_{j=1..k} F[r][j] (lambda_z[j] - lambda_z[j-1]) in
 // float64.  One block per row: each thread sums a run of consecutive entries, a block
-// scan of the run totals gives each run's offset, and the run is written out.
-__device__ __forceinline__ void prefix_row(const float* __restrict__ flux, int r, int nW,
+// scan of the run totals gives each run's offset, and the run is written out.  Returns the row's
+// total.
+__device__ __forceinline__ double prefix_row(const float* __restrict__ flux, int r, int nW,
                                            const float* __restrict__ wave_z,
                                            double* __restrict__ prefix) {
   __shared__ double s_warp[kPrefixThreads / 32];
@@ -203,11 +204,14 @@ __device__ __forceinline__ void prefix_row(const float* __restrict__ flux, int r
   __syncthreads();
   double run = x - sum;
   for (int w = 0; w < warp; ++w) run += s_warp[w];
+  double total = 0.0;
+  for (int w = 0; w < kPrefixThreads / 32; ++w) total += s_warp[w];
   for (int k = k0; k < k1; ++k) {
     if (k >= 1) run += (double)f[k] * (double)(wave_z[k] - wave_z[k - 1]);
     o[k] = run;
   }
   __syncthreads();  // s_warp is reused by the next row
+  return total;
 }
 
 // The setup passes over the grids in one launch: the first n_setup blocks the bucket table and

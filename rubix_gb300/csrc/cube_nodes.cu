@@ -11,8 +11,10 @@
 //     the four corners c, and H_c(alpha) is smooth in alpha.  H is tabulated at
 //     alpha_i = 1 + i 2^-18 (1.1 km/s apart, exact in float32) for every template by one
 //     small matrix product and interpolated linearly: 2e-8 of T' rms on the synthetic
-//     templates (lines of 45 % depth, 2-8 A wide), below float32 rounding.  beta is then
-//     known before any spectrum is formed.
+//     templates (lines of 45 % depth, 2-8 A wide), below float32 rounding.  The error grows
+//     with a template's kinks; it is bounded template by template, and a particle of a rougher
+//     one (emission lines) has its T' summed on its own grid.  beta is then known before any
+//     spectrum is formed.
 //   * Inside one SSP interval the particle's spectrum is A + B (x - x_j).  A lane owns an
 //     SSP node; while alpha moves by less than one telescope bin the samples strictly
 //     between two nodes stay the same, so the lane sums (A, B) of its interval over all
@@ -118,6 +120,7 @@ struct GatherArgs {
   float* rec_av;  // dust only
   int* flags;
   int4* desc;
+  int2* rough;  // records of rough particles, and their spaxels
 };
 
 // Largest dust transmission that a column lets through (2^(e A_V) over all wavelengths).
@@ -127,10 +130,26 @@ __device__ __forceinline__ float dust_top(const GatherArgs& a, float av) {
   return isfinite(av) ? exp2f(fmaxf(up, 0.f)) : kFltMax;
 }
 
+// The record of a particle (beta times the corner weights); true: its spaxel is left to the
+// general kernel.
+__device__ __forceinline__ bool node_record(const GatherArgs& a, const NodeParticle& q,
+                                            long long i, float av, float4& w) {
+  const float mass = a.in.mass[i];
+  const float beta = mass != 0.f ? mass * (q.T / q.Tp) : 0.f;
+  const float top = fabsf(beta) * __uint_as_float(a.ctrl->fmax);  // without dust dust_top is 1
+  // what the general kernel treats specially, or what may leave float32's range; a
+  // particle outside the templates has no spectrum unless 0 times its mass or its
+  // transmission is not 0
+  if (q.outside && !q.bad) return !isfinite(mass) || !(dust_top(a, av) < 1e30f);
+  w = make_float4(beta * q.w[0], beta * q.w[1], beta * q.w[2], beta * q.w[3]);
+  return q.bad || !(top * dust_top(a, av) < 1e30f) || (beta != 0.f && !(top > 1e-25f));
+}
+
 // One block per work item: the record of each particle (beta times the four corner
 // weights; alpha and the byte offset of its first corner row in the slice table), sorted
 // by alpha within runs of kSub (ties by input order: the order is a function of the
 // spaxel's particles alone).  Latency-bound on the gathers through the permutation.
+// A particle of a rough template leaves what node_rough_kernel needs in the record's place.
 __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
   __shared__ __align__(16) unsigned s_key[kSub];
   __shared__ float s_lo[kSub / 32], s_hi[kSub / 32];
@@ -142,7 +161,6 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
   if (tid == 0) s_plan = node_plan(a.ctrl, in.n_wave, x1, a.rec_av != nullptr);
   __syncthreads();
   const NodePlan plan = s_plan;
-  const float fmax = __uint_as_float(a.ctrl->fmax);
   const int n_items = a.ctrl->n_items;
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const int2 it = a.items[item];
@@ -157,36 +175,30 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
       float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
       float alpha = 1.f, av = 0.f;
       int row = 0;
-      bool bad = false;
+      bool rough = false;
       if (tid < m) {
         const long long i = in.perm[j0 + tid];
         const NodeParticle q = node_particle(in, a.prefix, a.H, i);
-        const float mass = in.mass[i];
         if (a.rec_av) av = in.av[i];
         alpha = q.alpha;
         row = q.row;
-        const float beta = mass != 0.f ? mass * (q.T / q.Tp) : 0.f;
-        const float top = fabsf(beta) * fmax;  // without dust dust_top is 1
-        // what the general kernel treats specially, or what may leave float32's range; a
-        // particle outside the templates has no spectrum unless 0 times its mass or its
-        // transmission is not 0
-        if (q.outside && !q.bad) {
-          bad = !isfinite(mass) || !(dust_top(a, av) < 1e30f);
-        } else {
-          bad = q.bad || !(top * dust_top(a, av) < 1e30f) || (beta != 0.f && !(top > 1e-25f));
-          w = make_float4(beta * q.w[0], beta * q.w[1], beta * q.w[2], beta * q.w[3]);
+        rough = q.rough;
+        if (rough) {
+          w = make_float4(q.tz, q.ta, q.T, __int_as_float((int)i));
+        } else if (node_record(a, q, i, av, w)) {
+          s_flag = 1;
         }
       }
-      if (bad) s_flag = 1;
       s_key[tid] = tid < m ? __float_as_uint(alpha) : 0xffffffffu;
       __syncthreads();
       if (tid < m) {
         amin = fminf(amin, alpha);
         amax = fmaxf(amax, alpha);
-        const int rank = run_rank(s_key, m, tid);
-        a.rec_w[j0 + rank] = w;
-        a.rec_a[j0 + rank] = make_float2(alpha, __int_as_float(row * 128));
-        if (a.rec_av) a.rec_av[j0 + rank] = av;
+        const int at = j0 + run_rank(s_key, m, tid);
+        a.rec_w[at] = w;
+        a.rec_a[at] = make_float2(alpha, __int_as_float(row * 128));
+        if (a.rec_av) a.rec_av[at] = av;
+        if (rough) a.rough[rough_place(a.ctrl)] = make_int2(at, it.x);
       }
       __syncthreads();
     }
@@ -213,6 +225,44 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
       }
     }
     __syncthreads();
+  }
+}
+
+// The records of rough particles, a warp each.  Bound by latency and issue together, about 1000
+// instructions a particle: 2.0 ms for 10^6 particles of 740 nodes (all of them rough: forward
+// 1.94 -> 4.0 ms, where the general path takes 4.05), with two blocks an SM and two rounds of
+// nodes in flight; 2.2 with one, 2.0 with three blocks or four rounds.  One warp summed a
+// whole sorted run's in the gather before: 18 ms.
+__global__ void __launch_bounds__(kRoughThreads, kRoughBlocks) node_rough_kernel(GatherArgs a) {
+  const int n = a.ctrl->n_rough;
+  if (n == 0) return;
+  extern __shared__ __align__(16) float4 s_tab4[];
+  __shared__ NodePlan s_plan;
+  const CubeInputs& in = a.in;
+  if (threadIdx.x == 0)
+    s_plan = node_plan(a.ctrl, in.n_wave, in.wave_t[in.n_wave_t - 1], a.rec_av != nullptr);
+  const bool even = sample_table(in.wave_t, in.n_wave_t, s_tab4);
+  const NodePlan plan = s_plan;
+  for (int e = (blockIdx.x * kRoughThreads + threadIdx.x) >> 5; e < n;
+       e += gridDim.x * (kRoughThreads / 32)) {
+    const int2 at = a.rough[e];
+    const float4 rec = a.rec_w[at.x];
+    NodeParticle q;
+    corner_weights(rec.x, rec.y, q.w);
+    q.T = rec.z;
+    q.Tp = rough_tprime(in, plan, s_tab4, even, a.rec_a[at.x], q.w);
+    q.outside = false;
+    q.bad = bad_scale(q.T, q.Tp);
+    const long long i = __float_as_int(rec.w);
+    float4 w;
+    const bool bad = node_record(a, q, i, a.rec_av ? in.av[i] : 0.f, w);
+    if ((threadIdx.x & 31) == 0) {
+      a.rec_w[at.x] = w;
+      if (bad) {
+        a.flags[at.y] = 1;
+        a.ctrl->flagged = 1;
+      }
+    }
   }
 }
 
@@ -893,9 +943,11 @@ struct NodeLayout {
   // not used before the last merge by the fallback, nor after it by the slices
   float* h;
   float* H;
+  float* rough_of;
   float4* rec_w;
   float2* rec_a;
   float* rec_av;
+  int2* rough;
   float* rows;
   int2* row_pos;
   size_t shared_off, fixed;  // start of the shared region; bytes without rows
@@ -916,9 +968,11 @@ NodeLayout carve_nodes(void* ws, long long n, int n_seg, int nZ, int nA, int nW)
   L.shared_off = c.off;
   L.h = c.take<float>((size_t)kAlphaRows * kpad_of(nW));
   L.H = c.take<float>((size_t)kAlphaRows * nZ * nA);
+  L.rough_of = c.take<float>((size_t)nZ * nA);
   L.rec_w = c.take<float4>((size_t)n);
   L.rec_a = c.take<float2>((size_t)n);
   L.rec_av = c.take<float>((size_t)n);
+  L.rough = c.take<int2>((size_t)n);
   L.fixed = c.off;
   L.rows = nullptr;
   L.row_pos = nullptr;
@@ -955,7 +1009,7 @@ int cube_nodes_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t b
   const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
   const long long fit = (long long)((bytes - L.fixed) / row_bytes(nW)) - multi_row_count(n);
   const long long wave = std::min<long long>(n_seg, fit);
-  return (n_seg <= kItemsOneBlock ? 6 : 8) + 2 * (int)((n_seg + wave - 1) / wave);
+  return (n_seg <= kItemsOneBlock ? 7 : 9) + 2 * (int)((n_seg + wave - 1) / wave);
 }
 
 int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* lsf_taps, int n_lsf, int lsf_crop,
@@ -976,7 +1030,7 @@ int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* l
   // control block, counters and flags are contiguous
   RUBIX_CUDA_TRY(cudaMemsetAsync(ws, 0, (size_t)((char*)(L.flags + in.n_seg) - (char*)ws), st));
   {
-    const int rc = node_build_tables(in, dust_e, L.prefix, L.h, L.H, L.ctrl, st);
+    const int rc = node_build_tables(in, dust_e, L.prefix, L.h, L.H, L.rough_of, L.ctrl, st);
     if (rc != RUBIX_OK) return rc;
   }
   if (in.n_seg <= kItemsOneBlock) {
@@ -997,10 +1051,15 @@ int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* l
   const long long items_max = multi_rows + std::min<long long>(in.n_seg, in.n);
   {
     GatherArgs g{in, L.prefix, L.H, L.ctrl, L.items, L.rec_w, L.rec_a,
-                 dust_e ? L.rec_av : nullptr, L.flags, L.desc};
+                 dust_e ? L.rec_av : nullptr, L.flags, L.desc, L.rough};
     const int blocks = (int)std::min<long long>(items_max, (long long)sm_count() * 8);
     node_gather_kernel<<<blocks, kSub, 0, st>>>(g);
     RUBIX_LAUNCH_CHECK("node_gather_kernel");
+    const size_t smem = rough_smem(in.n_wave_t);
+    RUBIX_CUDA_TRY(cudaFuncSetAttribute(node_rough_kernel,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    node_rough_kernel<<<rough_blocks(in.n), kRoughThreads, smem, st>>>(g);
+    RUBIX_LAUNCH_CHECK("node_rough_kernel");
   }
   const size_t smem = slice_smem(n_templ);
   const auto slice_kernel = dust_e ? node_slice_kernel<true> : node_slice_kernel<false>;

@@ -86,9 +86,11 @@ struct AdjGatherArgs {
   AdjFinal* fin;
   int* flags;
   int4* desc;  // first record, records, smallest and largest alpha
+  int* rough;  // records of rough particles
 };
 
-// One block per work item, as node_gather_kernel, without beta.
+// One block per work item, as node_gather_kernel, without beta.  T' of a rough particle holds
+// its spaxel until it is summed.
 __global__ void __launch_bounds__(kSub) node_adj_gather_kernel(AdjGatherArgs a) {
   __shared__ __align__(16) unsigned s_key[kSub];
   __shared__ unsigned s_lo, s_hi;
@@ -140,6 +142,10 @@ __global__ void __launch_bounds__(kSub) node_adj_gather_kernel(AdjGatherArgs a) 
       a.fin[j] = f;
       a.rec_w[j] = make_float2(tz, ta);
       a.rec_a[j] = make_float2(q.alpha, __int_as_float(q.row * 128));
+      if (q.rough) {
+        a.fin[j].a.y = __int_as_float(it.x);
+        a.rough[rough_place(a.ctrl)] = j;
+      }
     }
     __syncthreads();
     if (tid == 0) {
@@ -151,6 +157,35 @@ __global__ void __launch_bounds__(kSub) node_adj_gather_kernel(AdjGatherArgs a) 
       }
     }
     __syncthreads();
+  }
+}
+
+// T' of rough particles, a warp each (as node_rough_kernel).
+__global__ void __launch_bounds__(kRoughThreads, kRoughBlocks) node_adj_rough_kernel(AdjGatherArgs a) {
+  const int n = a.ctrl->n_rough;
+  if (n == 0) return;
+  extern __shared__ __align__(16) float4 s_tab4[];
+  __shared__ NodePlan s_plan;
+  const CubeInputs& in = a.in;
+  if (threadIdx.x == 0)
+    s_plan = node_plan(a.ctrl, in.n_wave, in.wave_t[in.n_wave_t - 1], false);
+  const bool even = sample_table(in.wave_t, in.n_wave_t, s_tab4);
+  const NodePlan plan = s_plan;
+  for (int e = (blockIdx.x * kRoughThreads + threadIdx.x) >> 5; e < n;
+       e += gridDim.x * (kRoughThreads / 32)) {
+    const int j = a.rough[e];
+    const float4 f = a.fin[j].a;
+    const float2 z = a.rec_w[j];
+    float w[4];
+    corner_weights(z.x, z.y, w);
+    const float Tp = rough_tprime(in, plan, s_tab4, even, a.rec_a[j], w);
+    if ((threadIdx.x & 31) == 0) {
+      a.fin[j].a.y = Tp;
+      if (bad_scale(f.x, Tp)) {
+        a.flags[__float_as_int(f.y)] = 1;
+        a.ctrl->flagged = 1;
+      }
+    }
   }
 }
 
@@ -574,10 +609,11 @@ struct AdjNodeLayout {
   int2* items;
   int4* desc;
   double* prefix;
-  float *h, *H;
+  float *h, *H, *rough_of;
   float2* rec_w;  // place in the cell: tz, ta
   float2* rec_a;
   AdjFinal* fin;
+  int* rough;
   float* part;
   size_t shared_off, fixed;
 };
@@ -597,9 +633,11 @@ AdjNodeLayout carve_adj(void* ws, long long n, int n_seg, int nZ, int nA, int nW
   L.shared_off = c.off;
   L.h = c.take<float>((size_t)kAlphaRows * kpad_of(nW));
   L.H = c.take<float>((size_t)kAlphaRows * nZ * nA);
+  L.rough_of = c.take<float>((size_t)nZ * nA);
   L.rec_w = c.take<float2>((size_t)n);
   L.rec_a = c.take<float2>((size_t)n);
   L.fin = c.take<AdjFinal>((size_t)n);
+  L.rough = c.take<int>((size_t)n);
   L.fixed = c.off;
   L.part = ws ? reinterpret_cast<float*>(static_cast<char*>(ws) + L.fixed) : nullptr;
   return L;
@@ -643,7 +681,7 @@ bool cube_nodes_bwd_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t,
 int cube_nodes_bwd_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t bytes) {
   const AdjNodeLayout L = carve_adj(nullptr, n, n_seg, nZ, nA, nW);
   const long long per = std::min(n, part_particles(bytes - L.fixed, nW));
-  return (n_seg <= kItemsOneBlock ? 6 : 8) + 2 * (int)((n + per - 1) / per);
+  return (n_seg <= kItemsOneBlock ? 7 : 9) + 2 * (int)((n + per - 1) / per);
 }
 
 int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_stride,
@@ -653,7 +691,7 @@ int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_st
   const int n_templ = in.n_met * in.n_age, nW = in.n_wave;
   RUBIX_CUDA_TRY(cudaMemsetAsync(ws, 0, (size_t)((char*)(L.flags + in.n_seg) - (char*)ws), st));
   {
-    const int rc = node_build_tables(in, nullptr, L.prefix, L.h, L.H, L.ctrl, st);
+    const int rc = node_build_tables(in, nullptr, L.prefix, L.h, L.H, L.rough_of, L.ctrl, st);
     if (rc != RUBIX_OK) return rc;
   }
   if (in.n_seg <= kItemsOneBlock) {
@@ -671,10 +709,15 @@ int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_st
   const int blocks =
       (int)std::min<long long>(adj_items_max(in.n, in.n_seg), (long long)sm_count() * 8);
   {
-    const AdjGatherArgs g{in,      L.prefix, L.H,     L.ctrl,  L.items,
-                          L.rec_w, L.rec_a,  L.fin,   L.flags, L.desc};
+    const AdjGatherArgs g{in,      L.prefix, L.H,   L.ctrl, L.items,
+                          L.rec_w, L.rec_a,  L.fin, L.flags, L.desc, L.rough};
     node_adj_gather_kernel<<<blocks, kSub, 0, st>>>(g);
     RUBIX_LAUNCH_CHECK("node_adj_gather_kernel");
+    const size_t smem = rough_smem(in.n_wave_t);
+    RUBIX_CUDA_TRY(cudaFuncSetAttribute(node_adj_rough_kernel,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    node_adj_rough_kernel<<<rough_blocks(in.n), kRoughThreads, smem, st>>>(g);
+    RUBIX_LAUNCH_CHECK("node_adj_rough_kernel");
   }
   const long long per = std::min(in.n, part_particles(ws_bytes - L.fixed, nW));
   const int waves = (int)((in.n + per - 1) / per);

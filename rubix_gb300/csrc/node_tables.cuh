@@ -37,6 +37,7 @@ struct NodeCtrl {
   int k_first;                  // 1 + node below the telescope range at any alpha
   int k_last_inv;               // n_wave - node above it
   unsigned fmax;                // bits of max |flux| (above inf: NaN)
+  int n_rough;                  // particles in the list of rough ones
   int n_items, n_multi;         // work items with particles; those of several-item spaxels
   int next[kMaxWaves][kMaxSlices];
 };
@@ -52,7 +53,7 @@ __host__ __device__ inline int max_slices_of(int n_wave) {
 
 struct NodePlan {
   int ok;
-  int k_first, n_own, n_slices;  // first node, nodes of a slice
+  int k_first, k_last, n_own, n_slices;  // first and last node, nodes of a slice, slices
   int w;                         // samples that a node may cross within a group of particles
   float dt_min, window;          // samples that an item's alpha range may span
   int most;                      // samples between two nodes at most
@@ -65,7 +66,7 @@ __device__ __forceinline__ NodePlan node_plan(const NodeCtrl* c, int n_wave, flo
   const float dz = __uint_as_float(~c->dz_inv), dt = __uint_as_float(~c->dt_inv);
   const float dtm = __uint_as_float(c->dt_max), fm = __uint_as_float(c->fmax);
   p.k_first = max(c->k_first - 1, 0);
-  const int k_last = min(n_wave - c->k_last_inv, n_wave - 1);
+  const int k_last = p.k_last = min(n_wave - c->k_last_inv, n_wave - 1);
   p.dt_min = dt;
   p.ok = 0;
   p.n_own = 0;
@@ -211,29 +212,73 @@ __device__ __forceinline__ float2 interval_weights(const float* __restrict__ wz,
 
 constexpr int kWeightBlocks = 1024;
 
-// Per template: float64 prefix sums (block b < rows, as cube_prefix_kernel) and max |F|.
+// Largest roughness that the table is read with, relative to T': its error is then below 6e-7,
+// 1e-7 rms, the size of float32's own in a sum of 3721 products.  The synthetic templates
+// (absorption lines of 2 to 8 A) have up to 4.4e-7, 7.5e-7 on the 700 bluest samples; noise of
+// 10 % from node to node has 1.4e-6, emission lines of 100 A equivalent width 1e-5.
+constexpr float kRoughLimit = 1e-6f;
+
+// How far the interpolated T' of a template may be from the sum on its shifted grid, for
+// kRoughLimit.  T'(alpha) has a kink where a node passes a sample (bin width times the jump
+// of the template's slope at the node), of which linear interpolation over one alpha step cuts
+// off at most a quarter step; and the table's nodes are not rounded to float32, which moves a
+// node by up to lambda 2^-24 and T' by that times the mean step of the flux beside it.  Both
+// have either sign from node to node: the root of the sum of the squares over the nodes in
+// range.  Against float64 (templates with noise, absorption lines, emission lines of 1.5 and
+// 3 A, a single node; 400 velocities each) the largest error is 0.38 to 0.62 of this on 1.25 A
+// samples, 0.14 on 5 A ones, the rms error 0.03 to 0.14 of it.
+__device__ __forceinline__ float node_roughness(const float* __restrict__ f,
+                                                const float* __restrict__ wz, int k, float dt_max,
+                                                float scale) {
+  const float z = wz[k], f1 = f[k], up = (f[k + 1] - f1) * scale, dn = (f1 - f[k - 1]) * scale;
+  const float jump = __fdividef(up, wz[k + 1] - z) - __fdividef(dn, z - wz[k - 1]);
+  const float kink = dt_max * z * (0.25f * kAlphaStep) * jump;
+  const float round = z * 5.9604645e-8f * (0.5f * (fabsf(up) + fabsf(dn)));
+  return fmaf(kink, kink, round * round);
+}
+
+// Per template (block b < rows): float64 prefix sums, max |F| and the roughness.
 // The remaining blocks: the resampling weights of T' at alpha_i, h_k = sum_t dlambda_t
 // hat_k(x_t) with hat_k the hat function of node k, one alpha row of a used tile at a time.
 // Nodes are stored from k_first on, kpad to a row, zero beyond the last.
 __global__ void __launch_bounds__(kPrefixThreads) node_tables_kernel(
     const float* __restrict__ flux, int rows, int n_wave, const float* __restrict__ wz,
     const float* __restrict__ wt, int n_t, double* __restrict__ prefix, float* __restrict__ h,
-    int kpad, NodeCtrl* __restrict__ ctrl) {
+    int kpad, float* __restrict__ rough, NodeCtrl* __restrict__ ctrl) {
+  // the grid's node range (fmax, still being formed, only decides whether it is used)
+  const int k_first = max(ctrl->k_first - 1, 0);
+  const int k_last = min(n_wave - ctrl->k_last_inv, n_wave - 1);
   if ((int)blockIdx.x < rows) {
-    prefix_row(flux, blockIdx.x, n_wave, wz, prefix);
+    const double total = prefix_row(flux, blockIdx.x, n_wave, wz, prefix);
+    __shared__ float s_sum[kPrefixThreads / 32];
     const float* f = flux + (long long)blockIdx.x * n_wave;
+    const float dt_max = __uint_as_float(ctrl->dt_max);
+    // squares of fluxes in any unit: relative to the total (0: any value is rough)
+    const float scale = (float)(1.0 / fmax(fabs(total), 1e-37));
     unsigned m = 0u;
-    for (int k = threadIdx.x; k < n_wave; k += kPrefixThreads)
+    float sum = 0.f;
+    for (int k = threadIdx.x; k < n_wave; k += kPrefixThreads) {
       m = max(m, __float_as_uint(f[k]) & 0x7fffffffu);
+      if (k >= max(k_first, 1) && k <= min(k_last, n_wave - 2))
+        sum += node_roughness(f, wz, k, dt_max, scale);
+    }
     m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) atomicMax(&ctrl->fmax, m);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(&ctrl->fmax, m);
+      s_sum[threadIdx.x >> 5] = sum;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < kPrefixThreads / 32; ++w) sum += s_sum[w];
+      rough[blockIdx.x] = sqrtf(sum) / scale;
+    }
     return;
   }
   __shared__ float s_rise[kPrefixThreads + 1];
   const int tid = threadIdx.x;
-  // the grid's node range (fmax, still being formed, only decides whether it is used)
-  const int k_first = max(ctrl->k_first - 1, 0);
-  const int count = min(n_wave - ctrl->k_last_inv, n_wave - 1) - k_first + 1;
+  const int count = k_last - k_first + 1;
   const float x0 = wt[0], inv = (float)(n_t - 1) / (wt[n_t - 1] - x0);
   for (int u = blockIdx.x - rows;; u += kWeightBlocks) {
     // row u of the used tiles
@@ -260,20 +305,20 @@ __global__ void __launch_bounds__(kPrefixThreads) node_tables_kernel(
 // H[i][c] = sum_k h[i][k] F[c][k]: 64 alpha rows x 32 templates per block of 128 threads,
 // 4 x 4 per thread, 32 nodes staged at a time.  Sums of 32 products are added with Kahan's
 // compensation: a plain float32 sum over ~740 nodes would be 5e-7 off, this one is 1e-8.
+// NaN for a template too rough to be read from the table.
 // 106 us at 10^7 particles (800 alpha rows x 1302 templates; 129 with padded tiles, whose
 // transposing stores fell in 8 banks).
 // Bound by FMA issue: 1 GFMA for 1025 rows of a 1326-template grid, 40 TFMA/s on the chip.
 __global__ void __launch_bounds__(128) node_table_product_kernel(
     const float* __restrict__ h, int kpad, const float* __restrict__ flux, int n_templ,
     int n_wave, const float* __restrict__ wt, int n_t, bool dust,
-    const NodeCtrl* __restrict__ ctrl, float* __restrict__ H) {
+    const float* __restrict__ rough, const NodeCtrl* __restrict__ ctrl, float* __restrict__ H) {
   constexpr int BK = 32, BM = kAlphaTile, BN = 32;
   const int tile = blockIdx.y;
   if (!tile_used(ctrl, tile)) return;
   const NodePlan p = node_plan(ctrl, n_wave, wt[n_t - 1], dust);
   if (!p.ok) return;
-  const int k_last = min(n_wave - ctrl->k_last_inv, n_wave - 1);
-  const int K = min(k_last - p.k_first + 1, kpad);
+  const int K = min(p.k_last - p.k_first + 1, kpad);
   // columns permuted by the node (column ^ 4 (k / 4 mod 8)): the transposing stores of a warp
   // fall in 32 banks and the 16-byte loads stay whole
   __shared__ __align__(16) float sa[2][BK][BM];
@@ -344,10 +389,14 @@ __global__ void __launch_bounds__(128) node_table_product_kernel(
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int j = 0; j < 4; ++j) {
+    if (c0 + tc + j >= n_templ) continue;
+    const float e = rough[c0 + tc + j];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (c0 + tc + j < n_templ) H[(long long)(r0 + tr + i) * n_templ + c0 + tc + j] = sum[i][j];
+    for (int i = 0; i < 4; ++i)
+      H[(long long)(r0 + tr + i) * n_templ + c0 + tc + j] =
+          e <= kRoughLimit * fabsf(sum[i][j]) ? sum[i][j] : __int_as_float(0x7fffffff);
+  }
 }
 
 // Last SSP wavelength k with lambda'_k <= x (-1: none), on an ascending grid (where it is not,
@@ -370,6 +419,114 @@ __device__ __forceinline__ int last_below(const float* __restrict__ wz, int n, f
   return count_le_scaled(wz, n, alpha, x) - 1;
 }
 
+// 1 / x by the hardware's reciprocal (relative error about 2^-23); x is a positive normal.
+__device__ __forceinline__ float fast_rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+constexpr int kRoughThreads = 512;
+constexpr int kRoughBlocks = 2;  // per SM
+constexpr int kRoughUnroll = 2;
+
+// Samples before each sample, for sums over the samples of an interval: entry t holds
+// (x_{t-1}, sum_{q < t} dx_q x_q as a float pair, x_t), t = 0 .. n_t, with dx_0 = 0.
+// Returns whether a linear guess of a sample's place is right to half a sample everywhere.
+__device__ __forceinline__ bool sample_table(const float* __restrict__ wt, int n_t, float4* tab) {
+  __shared__ double s_warp[kRoughThreads / 32];
+  const int per = (n_t + kRoughThreads) / kRoughThreads, tid = threadIdx.x;
+  const int t0 = min(tid * per, n_t + 1), t1 = min(t0 + per, n_t + 1);
+  const float x0 = wt[0], inv = (float)(n_t - 1) / (wt[n_t - 1] - x0);
+  auto term = [&](int q) {
+    return q >= 1 && q < n_t ? (double)(wt[q] - wt[q - 1]) * (double)wt[q] : 0.0;
+  };
+  double sum = 0.0;
+  bool even = true;
+  for (int t = t0; t < t1; ++t) {
+    sum += term(t);
+    if (t < n_t) even = even && fabsf((wt[t] - x0) * inv - (float)t) <= 0.5f;
+  }
+  double run = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const double y = __shfl_up_sync(0xffffffffu, run, d);
+    if ((tid & 31) >= d) run += y;
+  }
+  if ((tid & 31) == 31) s_warp[tid >> 5] = run;
+  __syncthreads();
+  run -= sum;
+  for (int w = 0; w < (tid >> 5); ++w) run += s_warp[w];
+  for (int t = t0; t < t1; ++t) {
+    const float hi = (float)run;
+    tab[t] = make_float4(wt[max(t - 1, 0)], hi, (float)(run - (double)hi),
+                         t < n_t ? wt[t] : kFltMax);
+    run += term(t);
+  }
+  return __syncthreads_and(even);
+}
+
+size_t rough_smem(int n_t) { return sizeof(float4) * (size_t)(n_t + 1); }
+
+// Entry of the first sample >= a.  Even samples: a linear guess, corrected by one; else a search.
+template <bool kEven>
+__device__ __forceinline__ float4 first_sample(const float4* tab, int n_t, float a, float x0,
+                                               float inv) {
+  if constexpr (kEven) {
+    const int t = min(max((int)((a - x0) * inv), 0), n_t - 1) + 1;
+    float4 e = tab[t];
+    const bool before = !(e.x < a), after = e.w < a;
+    if (before || after) e = tab[before ? t - 1 : t + 1];
+    return e;
+  } else {
+    int lo = 0, hi = n_t;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (tab[mid].w < a) lo = mid + 1; else hi = mid;
+    }
+    return tab[lo];
+  }
+}
+
+// T' of one particle summed over its own shifted nodes by a warp, a lane per node (31 intervals
+// at a time): what the general kernel sums, without the table.  An interval's samples enter by
+// differences of the sample table: the sum of dx, exact, and that of dx (x - a), whose
+// large parts cancel exactly in the product-sum.
+template <bool kEven>
+__device__ __forceinline__ float direct_tprime(const float* __restrict__ f, int n_age, int n_wave,
+                                               const float* __restrict__ wz, const float4* tab,
+                                               int n_t, int k_first, int k_last, float alpha,
+                                               const float (&w)[4]) {
+  const int lane = threadIdx.x & 31;
+  const float* f1 = f + (long long)n_age * n_wave;  // corners 00, 10, 01, 11
+  const float* f2 = f + n_wave;
+  const float* f3 = f1 + n_wave;
+  const float x0 = tab[0].w, inv = (float)(n_t - 1) / (tab[n_t].x - x0);
+  float sum = 0.f;
+  constexpr int kUnroll = kEven ? kRoughUnroll : 1;
+#pragma unroll kUnroll
+  for (int k0 = k_first; k0 < k_last; k0 += 31) {
+    const int k = min(k0 + lane, k_last);
+    const float a = __fmul_rn(wz[k], alpha);
+    float G = w[0] * f[k];
+    G = fmaf(w[1], f1[k], G);
+    G = fmaf(w[2], f2[k], G);
+    G = fmaf(w[3], f3[k], G);
+    const float4 e = first_sample<kEven>(tab, n_t, a, x0, inv);
+    const float b = __shfl_down_sync(0xffffffffu, a, 1);
+    const float G1 = __shfl_down_sync(0xffffffffu, G, 1);
+    const float s0 = __shfl_down_sync(0xffffffffu, e.x, 1) - e.x;
+    const float hi = __shfl_down_sync(0xffffffffu, e.y, 1) - e.y;
+    const float lo = __shfl_down_sync(0xffffffffu, e.z, 1) - e.z;
+    const float s1 = fmaf(-a, s0, hi) + lo;
+    // past the last node nothing is added: a == b there
+    if (lane < 31 && k0 + lane < k_last) sum += fmaf(s1 * fast_rcp(b - a), G1 - G, s0 * G);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  return sum;
+}
+
 // One particle on the tables: the corner weights, T (and, for the gradients, its corner
 // values), T', and whether the general kernel has to take it.
 struct NodeParticle {
@@ -379,7 +536,21 @@ struct NodeParticle {
   float tz, ta, dzg, dag;
   int row;         // template 00
   bool outside, bad;
+  bool rough;      // T' is not in the table (NaN): to be summed directly
 };
+
+__device__ __forceinline__ void corner_weights(float tz, float ta, float (&w)[4]) {
+  w[0] = (1.f - tz) * (1.f - ta);
+  w[1] = tz * (1.f - ta);
+  w[2] = (1.f - tz) * ta;
+  w[3] = tz * ta;
+}
+
+// Whether T / T' is unusual and left to the general kernel.
+__device__ __forceinline__ bool bad_scale(float T, float Tp) {
+  const float sc = T / Tp;
+  return !(sc > 0.25f && sc < 4.f);
+}
 
 __device__ __forceinline__ NodeParticle node_particle(const CubeInputs& in,
                                                       const double* __restrict__ prefix,
@@ -391,7 +562,7 @@ __device__ __forceinline__ NodeParticle node_particle(const CubeInputs& in,
   p.alpha = doppler_factor(in.vel[i * in.vel_stride + in.vel_comp]);
   p.outside = (Z < in.ssp_met[0]) || (Z > in.ssp_met[in.n_met - 1]) || (A < in.ssp_age[0]) ||
               (A > in.ssp_age[in.n_age - 1]);
-  p.bad = false;
+  p.bad = p.rough = false;
   p.row = 0;
   p.T = p.Tp = p.tz = p.ta = p.dzg = p.dag = 0.f;
 #pragma unroll
@@ -418,10 +589,7 @@ __device__ __forceinline__ NodeParticle node_particle(const CubeInputs& in,
     p.bad = true;
     return p;
   }
-  p.w[0] = (1.f - p.tz) * (1.f - p.ta);
-  p.w[1] = p.tz * (1.f - p.ta);
-  p.w[2] = (1.f - p.tz) * p.ta;
-  p.w[3] = p.tz * p.ta;
+  corner_weights(p.tz, p.ta, p.w);
   const int rr[4] = {p.row, p.row + in.n_age, p.row + 1, p.row + in.n_age + 1};
   // T: in-range flux sum, entries ka..ke with x0 <= lambda'_k <= x1, k >= 1
   int ka = __fmul_rn(in.ssp_wave_z[ks], p.alpha) >= x0 ? ks : ks + 1;
@@ -439,9 +607,30 @@ __device__ __forceinline__ NodeParticle node_particle(const CubeInputs& in,
     p.Tp = fmaf(p.w[c], fmaf(fr, h1[rr[c]] - h0[rr[c]], h0[rr[c]]), p.Tp);
   }
   p.T *= p.alpha;
-  const float sc = p.T / p.Tp;
-  if (!(sc > 0.25f && sc < 4.f)) p.bad = true;
+  p.rough = isnan(p.Tp);
+  if (!p.rough && bad_scale(p.T, p.Tp)) p.bad = true;
   return p;
+}
+
+// A place in the list of rough particles, taken by the calling lanes of a warp together.
+__device__ __forceinline__ int rough_place(NodeCtrl* ctrl) {
+  const unsigned on = __activemask();
+  const int lane = threadIdx.x & 31, lead = __ffs(on) - 1;
+  int base = 0;
+  if (lane == lead) base = atomicAdd(&ctrl->n_rough, __popc(on));
+  return __shfl_sync(on, base, lead) + __popc(on & ((1u << lane) - 1u));
+}
+
+// T' of a rough particle by a warp: alpha and the byte offset of its corner row in the slice
+// table (as in the records), its corner weights.
+__device__ __forceinline__ float rough_tprime(const CubeInputs& in, const NodePlan& plan,
+                                              const float4* tab, bool even, float2 rec,
+                                              const float (&w)[4]) {
+  const float* f = in.ssp_flux + (long long)(__float_as_int(rec.y) / 128) * in.n_wave;
+  return even ? direct_tprime<true>(f, in.n_age, in.n_wave, in.ssp_wave_z, tab, in.n_wave_t,
+                                    plan.k_first, plan.k_last, rec.x, w)
+              : direct_tprime<false>(f, in.n_age, in.n_wave, in.ssp_wave_z, tab, in.n_wave_t,
+                                     plan.k_first, plan.k_last, rec.x, w);
 }
 
 // Rank of this thread's key (alpha's bits) among the m of the block's run, ties by place.
@@ -454,13 +643,6 @@ __device__ __forceinline__ int run_rank(const unsigned* s_key, int m, int tid) {
             (v.z < key || (v.z == key && q + 2 < tid)) + (v.w < key || (v.w == key && q + 3 < tid));
   }
   return rank;
-}
-
-// 1 / x by the hardware's reciprocal (relative error about 2^-23); x is a positive normal.
-__device__ __forceinline__ float fast_rcp(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
 }
 
 // The records that a warp has staged, one array per value: a step reads one word of NPL
@@ -523,12 +705,17 @@ __device__ __forceinline__ int busiest_slice(const int* next, int n_slices, int 
   return best;
 }
 
+int rough_blocks(long long n) {
+  return (int)std::min<long long>((n + kRoughThreads / 32 - 1) / (kRoughThreads / 32),
+                                  (long long)sm_count() * kRoughBlocks);
+}
+
 int kpad_of(int n_wave) { return (n_wave + 31) / 32 * 32; }
 
 // Grid extrema and used alpha rows, prefix sums and resampling weights, the T' table: three
 // launches.
 int node_build_tables(const CubeInputs& in, const float* dust_e, double* prefix, float* h,
-                      float* H, NodeCtrl* ctrl, cudaStream_t st) {
+                      float* H, float* rough, NodeCtrl* ctrl, cudaStream_t st) {
   const int n_templ = in.n_met * in.n_age, nW = in.n_wave, kpad = kpad_of(nW);
   const long long work = std::max<long long>(std::max(in.n_wave_t, nW), in.n);
   const int g = (int)std::min<long long>((work + 255) / 256, (long long)sm_count() * 8);
@@ -538,10 +725,10 @@ int node_build_tables(const CubeInputs& in, const float* dust_e, double* prefix,
                                                        dust_e, ctrl);
   RUBIX_LAUNCH_CHECK("node_setup_kernel");
   node_tables_kernel<<<n_templ + kWeightBlocks, kPrefixThreads, 0, st>>>(
-      in.ssp_flux, n_templ, nW, in.ssp_wave_z, in.wave_t, in.n_wave_t, prefix, h, kpad, ctrl);
+      in.ssp_flux, n_templ, nW, in.ssp_wave_z, in.wave_t, in.n_wave_t, prefix, h, kpad, rough, ctrl);
   RUBIX_LAUNCH_CHECK("node_tables_kernel");
   node_table_product_kernel<<<dim3((n_templ + 31) / 32, kAlphaTiles), 128, 0, st>>>(
-      h, kpad, in.ssp_flux, n_templ, nW, in.wave_t, in.n_wave_t, dust_e != nullptr, ctrl, H);
+      h, kpad, in.ssp_flux, n_templ, nW, in.wave_t, in.n_wave_t, dust_e != nullptr, rough, ctrl, H);
   RUBIX_LAUNCH_CHECK("node_table_product_kernel");
   return RUBIX_OK;
 }
