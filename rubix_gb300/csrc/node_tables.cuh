@@ -23,6 +23,7 @@ constexpr float kAlphaMax = 2040.f * kAlphaStep;       // |alpha - 1| covered (2
 constexpr int kAlphaTile = 64;                         // rows computed together
 constexpr int kAlphaTiles = 2 * kAlphaHalf / kAlphaTile + 1;
 constexpr int kAlphaRows = kAlphaTiles * kAlphaTile;
+static_assert(2040 + 4 < kAlphaHalf, "rows beside the limit exist");
 constexpr int kStage = 33;       // staged records of a warp: 32 and one of weight zero
 constexpr int kRuns = 4;
 constexpr int kDustMost = 8;     // samples between two nodes that a lane holds with dust
@@ -165,10 +166,11 @@ __global__ void __launch_bounds__(256) node_setup_kernel(
   __syncthreads();
   int last = -1;
   for (long long i = gtid; i < n; i += gsz) {
-    // alpha - 1 to ~1e-7: the rows on either side of it are marked
+    // alpha - 1 to ~1e-7: the rows on either side of it are marked, up to a row beyond the
+    // limit that node_particle checks on the rounded alpha
     const float z = vel[i * vel_stride + vel_comp] * (float)(1.0 / kSpeedOfLight);
     const float am1 = z * (1.f + 0.5f * z * (1.f + (1.f / 3.f) * z));
-    if (!(fabsf(am1) <= kAlphaMax)) continue;
+    if (!(fabsf(am1) <= kAlphaMax + kAlphaStep)) continue;
     const int r = (int)floorf(am1 * (float)(1 << kAlphaBits)) + kAlphaHalf;
     const int a = max(r - 1, 0) / kAlphaTile, b = min(r + 2, kAlphaRows - 1) / kAlphaTile;
     if (a != last) atomicOr(&s_mask[a >> 5], 1u << (a & 31));
