@@ -543,6 +543,20 @@ __global__ void __launch_bounds__(kAdjThreads, 2) cube_adjoint_kernel(AdjArgs a)
   }
 }
 
+// The caller's gradient arrays, any of them null, cleared in one launch (they are allocations of
+// their own, so no memset may span two, wherever they lie).
+__global__ void zero_grads_kernel(float* g0, float* g1, float* g2, float* g3, float* g4,
+                                  long long n) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    if (g0) g0[i] = 0.f;
+    if (g1) g1[i] = 0.f;
+    if (g2) g2[i] = 0.f;
+    if (g3) g3[i] = 0.f;
+    if (g4) g4[i] = 0.f;
+  }
+}
+
 template <int R, bool kDust>
 int launch_adjoint_t(const AdjArgs& args, size_t smem, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(cube_adjoint_kernel<R, kDust>,
@@ -587,9 +601,9 @@ extern "C" int rubix_cube_bwd_launches(int64_t n, int32_t n_segments, int32_t n_
   if (n_segments <= 0 || n <= 0) return 0;
   if (!dust && cube_nodes_bwd_supported(n_met, n_age, n_wave, n_wave_t) &&
       cube_nodes_bwd_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes))
-    return cube_nodes_bwd_launches(n, n_segments, n_met, n_age, n_wave, workspace_bytes) + 1;
-  // grid tables, gather, items (count, scans and fill, or one launch), adjoint
-  return n_segments <= kItemsOneBlock ? 4 : 6;
+    return cube_nodes_bwd_launches(n, n_segments, n_met, n_age, n_wave, workspace_bytes) + 2;
+  // zeros, grid tables, gather, items (count, scans and fill, or one launch), adjoint
+  return n_segments <= kItemsOneBlock ? 5 : 7;
 }
 
 namespace rubix {
@@ -617,12 +631,10 @@ int cube_bwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // every gradient entry is written: zeros for particles outside the sorted set
   float* grads[5] = {grad_mass, grad_metallicity, grad_age, grad_vlos, grad_av};
-  for (int i = 0; i < 5 && n > 0;) {
-    int j = i + 1;  // arrays that follow one another in memory: one memset
-    while (grads[i] && j < 5 && grads[j] == grads[i] + (size_t)(j - i) * n) ++j;
-    if (grads[i])
-      RUBIX_CUDA_TRY(cudaMemsetAsync(grads[i], 0, sizeof(float) * (size_t)n * (j - i), st));
-    i = j;
+  if (n > 0) {
+    const int g = (int)std::min<long long>((n + 255) / 256, (long long)sm_count() * 8);
+    zero_grads_kernel<<<g, 256, 0, st>>>(grads[0], grads[1], grads[2], grads[3], grads[4], n);
+    RUBIX_LAUNCH_CHECK("zero_grads_kernel");
   }
   if (n_segments == 0 || n == 0) return RUBIX_OK;
   RUBIX_REQUIRE(ssp_flux && ssp_metallicity && ssp_age && ssp_wave_z && wave_t && seg_offsets &&
