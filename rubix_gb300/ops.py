@@ -255,8 +255,7 @@ def cube_backward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, 
     dev = mass.device
     if av_grad and dust_av is None:
         raise ValueError("av_grad needs dust_av and dust_exponent")
-    # one buffer: the library clears rows that follow one another with one memset
-    grads = torch.empty((5 if av_grad else 4, n), dtype=torch.float32, device=dev).unbind(0)
+    grads = [torch.empty(n, dtype=torch.float32, device=dev) for _ in range(5 if av_grad else 4)]
     nbytes = _lib.query("rubix_cube_bwd_workspace_size", n, int(n_segments), L, nz, na, nw)
     ws = workspace(nbytes, dev)
     if (dust_av is None) != (dust_exponent is None):

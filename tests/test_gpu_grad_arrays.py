@@ -1,5 +1,5 @@
 """The gradient arrays of the adjoint are independent allocations: rubix_cube_bwd clears each by
-itself."""
+itself, and ops.cube_backward returns tensors that share nothing."""
 
 import ctypes
 
@@ -86,3 +86,19 @@ def test_unsorted_stars_have_zero_gradients(rubix_lib):
     args[11] = to_dev(np.array([0, 3, 3, 30], np.int32))
     for g in ops.cube_backward(*args):
         assert g[:30].abs().min() > 0 and not g[30:].any()
+
+
+def test_gradients_are_tensors_of_their_own(rubix_lib):
+    import torch
+
+    from rubix_gb300 import ops
+
+    prob = _problem([3, 0, 34])
+    grads = ops.cube_backward(*_args(prob, torch.ones(3, prob[2].size).cuda()))
+    assert len({g.untyped_storage().data_ptr() for g in grads}) == 4
+    versions = [g._version for g in grads]
+    grads[0].mul_(2.0)
+    assert [g._version for g in grads[1:]] == versions[1:]
+    scale = torch.ones((), device="cuda", requires_grad=True)
+    grads[1].mul_(scale)  # views of one unbind would refuse this
+    assert grads[1].requires_grad
