@@ -56,9 +56,12 @@ def _sort_passes(n_segments: int) -> int:
     return (bits + 8) // 9
 
 
-def _stream(dev: torch.device) -> int:
+def _stream(dev) -> int:
     """The current stream's handle, without building the Stream object (10 us a call on a
-    Grace core, more than the kernel launches of a small step)."""
+    Grace core, more than the kernel launches of a small step).  ``dev`` as for
+    ``torch.cuda.current_stream``: a device, its name, its index or None."""
+    if not isinstance(dev, torch.device):
+        dev = torch.device("cuda", dev) if isinstance(dev, int) else torch.device(dev or "cuda")
     i = dev.index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
