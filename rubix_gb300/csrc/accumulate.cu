@@ -934,7 +934,8 @@ extern "C" size_t rubix_cube_workspace_size(int64_t n, int32_t n_segments, int32
   if (n < 0 || n_segments < 0 || n_wave_t < 0 || n_met < 0 || n_age < 0 || n_wave < 0) return 0;
   const size_t general = rubix::cube_general_workspace(n, n_segments, n_wave_t, n_met, n_age, n_wave);
   if (n == 0 || !cube_nodes_supported(n_met, n_age, n_wave, n_wave_t)) return general;
-  return std::max(general, cube_nodes_bytes(n, n_segments, n_met, n_age, n_wave, n_wave_t));
+  return std::max(general, cube_nodes_bytes(n, n_segments, n_met, n_age, n_wave, n_wave_t,
+                                            cube_tuning_current().chunk));
 }
 
 extern "C" int rubix_cube_fwd_launches(int64_t n, int32_t n_segments, int32_t n_wave_t,
@@ -942,7 +943,8 @@ extern "C" int rubix_cube_fwd_launches(int64_t n, int32_t n_segments, int32_t n_
                                        int32_t general, size_t workspace_bytes) {
   if (n_segments <= 0) return 0;
   if (!general && n > 0 && cube_nodes_supported(n_met, n_age, n_wave, n_wave_t) &&
-      cube_nodes_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes))
+      cube_nodes_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, cube_tuning_current().chunk,
+                     workspace_bytes))
     return cube_nodes_launches(n, n_segments, n_met, n_age, n_wave, workspace_bytes) + 1;
   // grid tables, items (count, scans and fill, or one launch), main (+ gather)
   return (n_segments <= kItemsOneBlock ? 3 : 5) + (n > 0 ? 1 : 0);
@@ -1042,11 +1044,11 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
   MainArgs args;
   args.chunk = tune.chunk;
   if (nodes && n > 0 && cube_nodes_supported(n_met, n_age, n_wave, n_wave_t) &&
-      cube_nodes_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes)) {
+      cube_nodes_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, tune.chunk, workspace_bytes)) {
     NodeFallback fb;
     const int rc = cube_nodes_forward(in, dust_e2, lsf_taps, n_lsf_taps, lsf_crop,
-                                      tune.big_item, cube, spaxel_stride, workspace,
-                                      workspace_bytes, &fb, st);
+                                      tune, cube, spaxel_stride, workspace, workspace_bytes,
+                                      &fb, st);
     if (rc != RUBIX_OK) return rc;
     args.chunk = fb.chunk;
     L.At = fb.At;

@@ -592,7 +592,8 @@ extern "C" size_t rubix_cube_bwd_workspace_size(int64_t n, int32_t n_segments, i
   const size_t general =
       cube_general_workspace(n, n_segments, n_wave_t, n_met, n_age, n_wave);
   if (n == 0 || !cube_nodes_bwd_supported(n_met, n_age, n_wave, n_wave_t)) return general;
-  return std::max(general, cube_nodes_bwd_bytes(n, n_segments, n_met, n_age, n_wave, n_wave_t));
+  return std::max(general, cube_nodes_bwd_bytes(n, n_segments, n_met, n_age, n_wave, n_wave_t,
+                                                cube_tuning_current().chunk));
 }
 
 extern "C" int rubix_cube_bwd_launches(int64_t n, int32_t n_segments, int32_t n_wave_t,
@@ -600,7 +601,8 @@ extern "C" int rubix_cube_bwd_launches(int64_t n, int32_t n_segments, int32_t n_
                                        size_t workspace_bytes) {
   if (n_segments <= 0 || n <= 0) return 0;
   if (!dust && cube_nodes_bwd_supported(n_met, n_age, n_wave, n_wave_t) &&
-      cube_nodes_bwd_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes))
+      cube_nodes_bwd_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t,
+                         cube_tuning_current().chunk, workspace_bytes))
     return cube_nodes_bwd_launches(n, n_segments, n_met, n_age, n_wave, workspace_bytes) + 2;
   // zeros, grid tables, gather, items (count, scans and fill, or one launch), adjoint
   return n_segments <= kItemsOneBlock ? 5 : 7;
@@ -665,10 +667,11 @@ int cube_bwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
   AdjArgs args;
   args.chunk = tune.chunk;
   if (dust_e2 == nullptr && cube_nodes_bwd_supported(n_met, n_age, n_wave, n_wave_t) &&
-      cube_nodes_bwd_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, workspace_bytes)) {
+      cube_nodes_bwd_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, tune.chunk,
+                         workspace_bytes)) {
     NodeFallback fb;
     const int rc =
-        cube_nodes_backward(in, adj, adj_stride, grads, workspace, workspace_bytes, &fb, st);
+        cube_nodes_backward(in, adj, adj_stride, tune, grads, workspace, workspace_bytes, &fb, st);
     if (rc != RUBIX_OK) return rc;
     args.chunk = fb.chunk;
     L.At = fb.At;

@@ -236,22 +236,22 @@ __global__ void __launch_bounds__(kPrefixThreads) cube_tables_kernel(
   }
 }
 
+// Records of the sorted places first, first + step, .. below last.
 // dz, dt: smallest SSP spacing near the telescope range and widest telescope bin.
 __device__ __forceinline__ void gather_records(
     const float* __restrict__ mass, const float* __restrict__ met,
     const float* __restrict__ age, const float* __restrict__ vel, long long vel_stride,
     int vel_comp, const int* __restrict__ perm, const int* __restrict__ seg_off, int n_seg,
-    long long n, const float* __restrict__ zg, int nZ, const float* __restrict__ ag, int nA,
+    const float* __restrict__ zg, int nZ, const float* __restrict__ ag, int nA,
     const float* __restrict__ wave_z, int n_wave, const float* __restrict__ wave_t, int n_t,
     const double* __restrict__ prefix, double inv_h, float bmax, float dz, float dt,
     ParticleRec* __restrict__ rec, int with_grad, const float* __restrict__ av, float alo,
-    float ahi) {
+    float ahi, long long first, long long last, long long step) {
   const long long n_valid = seg_off[n_seg];
   const float t_lo = wave_t[0], t_hi = wave_t[n_t - 1];
   // lambda' spacing >= alpha*dz minus two float32 roundings of lambda' (|lambda'| < 2^14)
   const bool coarse_ok = dz * alo - 4.0e-3f > dt;
-  for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n && j < n_valid;
-       j += (long long)gridDim.x * blockDim.x) {
+  for (long long j = first; j < last && j < n_valid; j += step) {
     const long long i = perm[j];
     const float Z = met[i], A = age[i], m = mass[i];
     const float v = vel[i * vel_stride + vel_comp];
@@ -324,10 +324,11 @@ __global__ void cube_gather_kernel(const float* __restrict__ mass, const float* 
                                    const CubeCtrl* __restrict__ ctrl,
                                    ParticleRec* __restrict__ rec, int with_grad,
                                    const float* __restrict__ av, float alo, float ahi) {
-  gather_records(mass, met, age, vel, vel_stride, vel_comp, perm, seg_off, n_seg, n, zg, nZ, ag,
+  gather_records(mass, met, age, vel, vel_stride, vel_comp, perm, seg_off, n_seg, zg, nZ, ag,
                  nA, wave_z, n_wave, wave_t, n_t, prefix, ctrl->inv_h, ctrl->bmax,
                  __uint_as_float(~ctrl->dz_min_inv), __uint_as_float(ctrl->dt_max_bits), rec,
-                 with_grad, av, alo, ahi);
+                 with_grad, av, alo, ahi, blockIdx.x * (long long)blockDim.x + threadIdx.x, n,
+                 (long long)gridDim.x * blockDim.x);
 }
 
 // Per spaxel: chunk count.  Multi-chunk spaxels get one item (and partial slot) per

@@ -50,21 +50,21 @@ constexpr int kItem = 4 * kSub;  // particles of a work item
 template <bool kDust>
 constexpr int kNodeWarps = kDust ? 16 : 20;
 
-// Work items: ranges of up to kItem particles of one spaxel; empty spaxels have none.
-// Spaxels of several items first (item index = row), then those with many particles.
-__device__ __forceinline__ void node_count(const int* seg_off, int n_seg, int big, int* multi,
-                                           int* large, int* small) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += gridDim.x * blockDim.x) {
-    const int cnt = seg_off[s + 1] - seg_off[s];
+// Work items: ranges of up to kItem particles of one spaxel; empty and flagged spaxels have
+// none.  Spaxels of several items first (item index = row), then those with many particles.
+__device__ __forceinline__ void node_count(const CubeInputs& in, const NodeFlags& flags, bool dust,
+                                           int big, int* multi, int* large, int* small) {
+  screened_counts(in, flags, dust, kItem, [&](int s, int cnt) {
     multi[s] = cnt > kItem ? (cnt + kItem - 1) / kItem : 0;
     large[s] = (cnt <= kItem && cnt >= big) ? 1 : 0;
     small[s] = (cnt < big && cnt > 0) ? 1 : 0;
-  }
+  });
 }
 
-__global__ void node_count_kernel(const int* seg_off, int n_seg, int big, int* multi, int* large,
-                                  int* small) {
-  node_count(seg_off, n_seg, big, multi, large, small);
+__global__ void __launch_bounds__(256) node_count_kernel(CubeInputs in, NodeFlags flags, bool dust,
+                                                         int big, int* multi, int* large,
+                                                         int* small) {
+  node_count(in, flags, dust, big, multi, large, small);
 }
 
 // Item index of chunk 0 of a spaxel (its chunks follow one another).
@@ -75,12 +75,12 @@ __device__ __forceinline__ int first_item(int s, int cnt, int big, int n_seg, co
   return multi[n_seg] + large[n_seg] + small[s];
 }
 
-__device__ __forceinline__ void node_fill_items(const int* seg_off, int n_seg, int big,
-                                                const int* multi, const int* large,
+__device__ __forceinline__ void node_fill_items(const int* seg_off, const int* flags, int n_seg,
+                                                int big, const int* multi, const int* large,
                                                 const int* small, int2* items, NodeCtrl* ctrl) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += gridDim.x * blockDim.x) {
     const int cnt = seg_off[s + 1] - seg_off[s];
-    if (cnt == 0) continue;
+    if (cnt == 0 || flags[s]) continue;
     const int i0 = first_item(s, cnt, big, n_seg, multi, large, small);
     for (int c = 0; c * kItem < cnt; ++c) items[i0 + c] = make_int2(s, c);
   }
@@ -90,23 +90,24 @@ __device__ __forceinline__ void node_fill_items(const int* seg_off, int n_seg, i
   }
 }
 
-__global__ void node_fill_items_kernel(const int* seg_off, int n_seg, int big, const int* multi,
-                                       const int* large, const int* small, int2* items,
-                                       NodeCtrl* ctrl) {
-  node_fill_items(seg_off, n_seg, big, multi, large, small, items, ctrl);
+__global__ void node_fill_items_kernel(const int* seg_off, const int* flags, int n_seg, int big,
+                                       const int* multi, const int* large, const int* small,
+                                       int2* items, NodeCtrl* ctrl) {
+  node_fill_items(seg_off, flags, n_seg, big, multi, large, small, items, ctrl);
 }
 
-// All three steps by one block, up to kItemsOneBlock spaxels.
-__global__ void __launch_bounds__(1024) node_items_kernel(const int* seg_off, int n_seg, int big,
+// All three steps by one block, or the last two.
+__global__ void __launch_bounds__(1024) node_items_kernel(CubeInputs in, NodeFlags flags,
+                                                          bool count, bool dust, int big,
                                                           int* multi, int* large, int* small,
-                                                          int2* items, NodeCtrl* ctrl) {
-  node_count(seg_off, n_seg, big, multi, large, small);
+                                                          int2* items) {
+  if (count) node_count(in, flags, dust, big, multi, large, small);
   __syncthreads();
-  scan_exclusive_block(multi, n_seg, 1);
-  scan_exclusive_block(large, n_seg, 1);
-  scan_exclusive_block(small, n_seg, 1);
+  scan_exclusive_block(multi, in.n_seg, 1);
+  scan_exclusive_block(large, in.n_seg, 1);
+  scan_exclusive_block(small, in.n_seg, 1);
   __syncthreads();
-  node_fill_items(seg_off, n_seg, big, multi, large, small, items, ctrl);
+  node_fill_items(in.seg_off, flags.flags, in.n_seg, big, multi, large, small, items, flags.ctrl);
 }
 
 struct GatherArgs {
@@ -118,7 +119,7 @@ struct GatherArgs {
   float4* rec_w;
   float2* rec_a;
   float* rec_av;  // dust only
-  int* flags;
+  NodeFlags flags;
   int4* desc;
   int2* rough;  // records of rough particles, and their spaxels
 };
@@ -219,10 +220,7 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
       }
       a.desc[item] = make_int4(jb, je - jb, __float_as_int(amin), __float_as_int(amax));
       // the samples a node crosses within the item must fit the row
-      if (s_flag || (amax - amin) * x1 / (1.f - kAlphaMax) > plan.window * plan.dt_min) {
-        a.flags[it.x] = 1;
-        a.ctrl->flagged = 1;
-      }
+      if (s_flag || too_wide(plan, amin, amax, x1)) a.flags.leave(it.x);
     }
     __syncthreads();
   }
@@ -258,10 +256,7 @@ __global__ void __launch_bounds__(kRoughThreads, kRoughBlocks) node_rough_kernel
     const bool bad = node_record(a, q, i, a.rec_av ? in.av[i] : 0.f, w);
     if ((threadIdx.x & 31) == 0) {
       a.rec_w[at.x] = w;
-      if (bad) {
-        a.flags[at.y] = 1;
-        a.ctrl->flagged = 1;
-      }
+      if (bad) a.flags.leave(at.y);
     }
   }
 }
@@ -832,9 +827,11 @@ __global__ void __launch_bounds__(kMergeThreads) node_merge_kernel(MergeArgs a) 
         n = a.seg_off[mine + 1] - a.seg_off[mine];
         if (n == 0) {
           if (a.wave != 0) n = -1;
+        } else if (a.flags[mine]) {
+          n = -1;
         } else {
           it = first_item((int)mine, n, a.big, a.n_seg, a.multi, a.large, a.small);
-          if (it < i0 || it >= i1 || a.flags[mine]) n = -1;
+          if (it < i0 || it >= i1) n = -1;
         }
       }
       __syncthreads();  // the last batch is done with the lists
@@ -991,31 +988,34 @@ bool cube_nodes_supported(int nZ, int nA, int nW, int n_t) {
   return n_t >= 2 && nW >= 2 && slice_smem(nZ * nA) <= 227 * 1024;
 }
 
-size_t cube_nodes_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
+size_t cube_nodes_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk) {
   const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
   const long long wave = std::max(
       min_wave_items(n_seg), std::min<long long>(n_seg, (long long)(kRowBudget / row_bytes(nW))));
   return std::max(L.fixed + (size_t)(multi_row_count(n) + wave) * row_bytes(nW),
-                  L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, false));
+                  L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, chunk, false));
 }
 
-bool cube_nodes_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, size_t bytes) {
+bool cube_nodes_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk,
+                    size_t bytes) {
   const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
   return bytes >= L.fixed + (size_t)(multi_row_count(n) + min_wave_items(n_seg)) * row_bytes(nW) &&
-         bytes >= L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, false);
+         bytes >= L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, chunk, false);
 }
 
 int cube_nodes_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t bytes) {
   const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
   const long long fit = (long long)((bytes - L.fixed) / row_bytes(nW)) - multi_row_count(n);
   const long long wave = std::min<long long>(n_seg, fit);
-  return (n_seg <= kItemsOneBlock ? 7 : 9) + 2 * (int)((n_seg + wave - 1) / wave);
+  return 6 + items_launches(n_seg, n) + 2 * (int)((n_seg + wave - 1) / wave);
 }
 
 int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* lsf_taps, int n_lsf, int lsf_crop,
-                       int big_item, float* cube, long long stride, void* ws, size_t ws_bytes,
-                       NodeFallback* fb, cudaStream_t st) {
+                       const CubeTuning& tune, float* cube, long long stride, void* ws,
+                       size_t ws_bytes, NodeFallback* fb, cudaStream_t st) {
   NodeLayout L = carve_nodes(ws, in.n, in.n_seg, in.n_met, in.n_age, in.n_wave);
+  const int big_item = tune.big_item;
+  const NodeFlags flags{L.flags, L.ctrl, in.seg_off, tune.chunk, big_item};
   const int n_templ = in.n_met * in.n_age, nW = in.n_wave;
   const size_t rb = row_bytes(nW);
   const long long multi_rows = multi_row_count(in.n);
@@ -1030,28 +1030,37 @@ int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* l
   // control block, counters and flags are contiguous
   RUBIX_CUDA_TRY(cudaMemsetAsync(ws, 0, (size_t)((char*)(L.flags + in.n_seg) - (char*)ws), st));
   {
-    const int rc = node_build_tables(in, dust_e, L.prefix, L.h, L.H, L.rough_of, L.ctrl, st);
+    const int rc = node_setup(in, dust_e, L.ctrl, st);
     if (rc != RUBIX_OK) return rc;
   }
-  if (in.n_seg <= kItemsOneBlock) {
-    node_items_kernel<<<1, 1024, 0, st>>>(in.seg_off, in.n_seg, big_item, L.multi, L.large,
-                                          L.small, L.items, L.ctrl);
+  const bool dust = dust_e != nullptr;
+  const int steps = items_launches(in.n_seg, in.n);
+  const long long work = std::max<long long>(in.n_seg, in.n / 8);  // if screened, a warp a spaxel
+  const int g = (int)std::min<long long>((work + 255) / 256, (long long)sm_count() * 8);
+  if (steps > 1) {
+    node_count_kernel<<<g, 256, 0, st>>>(in, flags, dust, big_item, L.multi, L.large, L.small);
+    RUBIX_LAUNCH_CHECK("node_count_kernel");
+  }
+  if (steps < 3) {
+    node_items_kernel<<<1, 1024, 0, st>>>(in, flags, steps == 1, dust, big_item, L.multi, L.large,
+                                          L.small, L.items);
     RUBIX_LAUNCH_CHECK("node_items_kernel");
   } else {
-    const int g = (int)std::min<long long>((in.n_seg + 255) / 256, (long long)sm_count() * 8);
-    node_count_kernel<<<g, 256, 0, st>>>(in.seg_off, in.n_seg, big_item, L.multi, L.large,
-                                         L.small);
-    RUBIX_LAUNCH_CHECK("node_count_kernel");
     scan_exclusive_3<<<3, 1024, 0, st>>>(L.multi, L.large, L.small, in.n_seg);
     RUBIX_LAUNCH_CHECK("scan_exclusive_3");
-    node_fill_items_kernel<<<g, 256, 0, st>>>(in.seg_off, in.n_seg, big_item, L.multi, L.large,
-                                              L.small, L.items, L.ctrl);
+    node_fill_items_kernel<<<g, 256, 0, st>>>(in.seg_off, L.flags, in.n_seg, big_item, L.multi,
+                                              L.large, L.small, L.items, L.ctrl);
     RUBIX_LAUNCH_CHECK("node_fill_items_kernel");
+  }
+  {
+    const int rc = node_build_tables(in, dust_e, L.prefix, L.h, L.H, L.rough_of, L.ctrl,
+                                     static_cast<CubeCtrl*>(ws), st);
+    if (rc != RUBIX_OK) return rc;
   }
   const long long items_max = multi_rows + std::min<long long>(in.n_seg, in.n);
   {
     GatherArgs g{in, L.prefix, L.H, L.ctrl, L.items, L.rec_w, L.rec_a,
-                 dust_e ? L.rec_av : nullptr, L.flags, L.desc, L.rough};
+                 dust_e ? L.rec_av : nullptr, flags, L.desc, L.rough};
     const int blocks = (int)std::min<long long>(items_max, (long long)sm_count() * 8);
     node_gather_kernel<<<blocks, kSub, 0, st>>>(g);
     RUBIX_LAUNCH_CHECK("node_gather_kernel");
@@ -1113,10 +1122,9 @@ int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* l
   }
   // The flagged spaxels, if any, in the region that the slices no longer need.
   Carve c(static_cast<char*>(ws) + L.shared_off);
-  *fb = carve_fallback(c, in, false);
-  const int blocks = sm_count() * 8;
-  node_fallback_kernel<<<blocks, 256, 0, st>>>(in, *fb, L.prefix, L.flags, L.ctrl,
-                                               static_cast<CubeCtrl*>(ws), false);
+  *fb = carve_fallback(c, in, tune.chunk, false);
+  node_fallback_kernel<<<sm_count() * 8, 256, 0, st>>>(
+      in, *fb, L.prefix, flags, static_cast<CubeCtrl*>(ws), false);
   RUBIX_LAUNCH_CHECK("node_fallback_kernel");
   return RUBIX_OK;
 }

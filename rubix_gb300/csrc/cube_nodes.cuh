@@ -9,6 +9,7 @@ namespace rubix {
 // (their number in the workspace's CubeCtrl, 0 when none is flagged) and its inputs.
 struct NodeFallback {
   int chunk;
+  float alo, ahi;  // alpha at -kVmaxKms and kVmaxKms
   int2* items;  // items of several-chunk spaxels (item index = partial slot), then others
   int* slot_start;
   float* At;
@@ -20,28 +21,31 @@ struct NodeFallback {
 };
 
 // Runs the node path: the cube of every spaxel that is not flagged, and *fb for the rest.
-// dust_e: dust exponents per telescope wavelength (with in.av), or null.
+// dust_e: dust exponents per telescope wavelength (with in.av), or null.  tune: the work items
+// of the general kernel.
 int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* lsf_taps, int n_lsf, int lsf_crop,
-                       int big_item, float* cube, long long stride, void* ws, size_t ws_bytes,
-                       NodeFallback* fb, cudaStream_t st);
+                       const CubeTuning& tune, float* cube, long long stride, void* ws,
+                       size_t ws_bytes, NodeFallback* fb, cudaStream_t st);
 
 // Whether the host-side sizes qualify (the template slice fits shared memory).
 bool cube_nodes_supported(int nZ, int nA, int nW, int n_t);
 // Workspace of the node path, and whether a workspace of `bytes` holds it (with fewer rows
-// at a time in a smaller one).
-size_t cube_nodes_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t);
-bool cube_nodes_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, size_t bytes);
+// at a time in a smaller one); chunk: of the general kernel's work items.
+size_t cube_nodes_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk);
+bool cube_nodes_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk,
+                    size_t bytes);
 
 // Kernels that cube_nodes_forward launches.
 int cube_nodes_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t bytes);
 // The adjoint of cube_nodes_forward without dust (cube_nodes_bwd.cu): grads are dL/dmass,
 // dL/dZ, dL/dage and dL/dv_los (zeroed by the caller, null where not wanted).
 int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_stride,
-                        float* const* grads, void* ws, size_t ws_bytes, NodeFallback* fb,
+                        const CubeTuning& tune, float* const* grads, void* ws, size_t ws_bytes, NodeFallback* fb,
                         cudaStream_t st);
 bool cube_nodes_bwd_supported(int nZ, int nA, int nW, int n_t);
-size_t cube_nodes_bwd_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t);
-bool cube_nodes_bwd_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, size_t bytes);
+size_t cube_nodes_bwd_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk);
+bool cube_nodes_bwd_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk,
+                        size_t bytes);
 int cube_nodes_bwd_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t bytes);
 // Workspace of the path without it (accumulate.cu).
 size_t cube_general_workspace(int64_t n, int32_t n_segments, int32_t n_wave_t, int32_t n_met,

@@ -42,9 +42,11 @@ struct __align__(16) AdjFinal {
   float4 b;  // 1 / dZ, 1 / dage of the cell, mass, index of the particle (bits)
 };
 
-__device__ __forceinline__ void adj_count(const int* seg_off, int n_seg, int* chunks) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_seg; s += gridDim.x * blockDim.x)
-    chunks[s] = (seg_off[s + 1] - seg_off[s] + kAdjItem - 1) / kAdjItem;
+__device__ __forceinline__ void adj_count(const CubeInputs& in, const NodeFlags& flags,
+                                          int* chunks) {
+  screened_counts(in, flags, false, kAdjItem, [&](int s, int cnt) {
+    chunks[s] = (cnt + kAdjItem - 1) / kAdjItem;
+  });
 }
 
 // Items in the order of their particles, so that a wave of particles is a range of items.
@@ -57,22 +59,23 @@ __device__ __forceinline__ void adj_fill(int n_seg, const int* chunks, int2* ite
   if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->n_items = chunks[n_seg];
 }
 
-__global__ void node_adj_count_kernel(const int* seg_off, int n_seg, int* chunks) {
-  adj_count(seg_off, n_seg, chunks);
+__global__ void __launch_bounds__(256) node_adj_count_kernel(CubeInputs in, NodeFlags flags,
+                                                             int* chunks) {
+  adj_count(in, flags, chunks);
 }
 __global__ void node_adj_fill_kernel(int n_seg, const int* chunks, int2* items, NodeCtrl* ctrl) {
   adj_fill(n_seg, chunks, items, ctrl);
 }
 
-// All three steps by one block, up to kItemsOneBlock spaxels.
-__global__ void __launch_bounds__(1024) node_adj_items_kernel(const int* seg_off, int n_seg,
-                                                              int* chunks, int2* items,
-                                                              NodeCtrl* ctrl) {
-  adj_count(seg_off, n_seg, chunks);
+// All three steps by one block, or the last two.
+__global__ void __launch_bounds__(1024) node_adj_items_kernel(CubeInputs in, NodeFlags flags,
+                                                              bool count, int* chunks,
+                                                              int2* items) {
+  if (count) adj_count(in, flags, chunks);
   __syncthreads();
-  scan_exclusive_block(chunks, n_seg, 1);
+  scan_exclusive_block(chunks, in.n_seg, 1);
   __syncthreads();
-  adj_fill(n_seg, chunks, items, ctrl);
+  adj_fill(in.n_seg, chunks, items, flags.ctrl);
 }
 
 struct AdjGatherArgs {
@@ -84,7 +87,7 @@ struct AdjGatherArgs {
   float2* rec_w;  // place in the cell: tz, ta
   float2* rec_a;
   AdjFinal* fin;
-  int* flags;
+  NodeFlags flags;
   int4* desc;  // first record, records, smallest and largest alpha
   int* rough;  // records of rough particles
 };
@@ -151,10 +154,7 @@ __global__ void __launch_bounds__(kSub) node_adj_gather_kernel(AdjGatherArgs a) 
     if (tid == 0) {
       const float lo = __uint_as_float(s_lo), hi = __uint_as_float(s_hi);
       a.desc[item] = make_int4(jb, m, (int)s_lo, (int)s_hi);
-      if (s_flag || (hi - lo) * x1 / (1.f - kAlphaMax) > plan.window * plan.dt_min) {
-        a.flags[it.x] = 1;
-        a.ctrl->flagged = 1;
-      }
+      if (s_flag || too_wide(plan, lo, hi, x1)) a.flags.leave(it.x);
     }
     __syncthreads();
   }
@@ -181,10 +181,7 @@ __global__ void __launch_bounds__(kRoughThreads, kRoughBlocks) node_adj_rough_ke
     const float Tp = rough_tprime(in, plan, s_tab4, even, a.rec_a[j], w);
     if ((threadIdx.x & 31) == 0) {
       a.fin[j].a.y = Tp;
-      if (bad_scale(f.x, Tp)) {
-        a.flags[__float_as_int(f.y)] = 1;
-        a.ctrl->flagged = 1;
-      }
+      if (bad_scale(f.x, Tp)) a.flags.leave(__float_as_int(f.y));
     }
   }
 }
@@ -211,7 +208,7 @@ struct AdjSliceArgs {
   const float2* rec_a;
   const float* adj;
   long long adj_stride;
-  int* flags;
+  NodeFlags flags;
   float* part;  // [slice][kNodeSums][per + kAdjItem]
   NodeCtrl* ctrl;
   int wave;
@@ -403,10 +400,7 @@ __device__ __forceinline__ void adj_items(const AdjSliceArgs& a, const SliceShar
       bad |= !(fabsf(h) < h_max);
       sh.f[b] = h;
     }
-    if (bad) {
-      a.flags[it.x] = 1;
-      a.ctrl->flagged = 1;
-    }
+    if (bad) a.flags.leave(it.x);
     bool open = false;
     float a_lim = 0.f;
     for (int base = 0; base < np; base += 32) {
@@ -664,53 +658,64 @@ bool cube_nodes_bwd_supported(int nZ, int nA, int nW, int n_t) {
   return n_t >= 2 && nW >= 2 && adj_slice_smem(nZ * nA) <= 227 * 1024;
 }
 
-size_t cube_nodes_bwd_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
+size_t cube_nodes_bwd_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk) {
   const AdjNodeLayout L = carve_adj(nullptr, n, n_seg, nZ, nA, nW);
   const long long per =
       std::max(min_wave_particles(n), std::min(n, part_particles(kPartBudget, nW)));
   return std::max(L.fixed + part_bytes(per, nW),
-                  L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, true));
+                  L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, chunk, true));
 }
 
-bool cube_nodes_bwd_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, size_t bytes) {
+bool cube_nodes_bwd_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk,
+                        size_t bytes) {
   const AdjNodeLayout L = carve_adj(nullptr, n, n_seg, nZ, nA, nW);
   return bytes >= L.fixed + part_bytes(min_wave_particles(n), nW) &&
-         bytes >= L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, true);
+         bytes >= L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, chunk, true);
 }
 
 int cube_nodes_bwd_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t bytes) {
   const AdjNodeLayout L = carve_adj(nullptr, n, n_seg, nZ, nA, nW);
   const long long per = std::min(n, part_particles(bytes - L.fixed, nW));
-  return (n_seg <= kItemsOneBlock ? 7 : 9) + 2 * (int)((n + per - 1) / per);
+  return 6 + items_launches(n_seg, n) + 2 * (int)((n + per - 1) / per);
 }
 
 int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_stride,
-                        float* const* grads, void* ws, size_t ws_bytes, NodeFallback* fb,
-                        cudaStream_t st) {
+                        const CubeTuning& tune, float* const* grads, void* ws, size_t ws_bytes,
+                        NodeFallback* fb, cudaStream_t st) {
   const AdjNodeLayout L = carve_adj(ws, in.n, in.n_seg, in.n_met, in.n_age, in.n_wave);
+  const NodeFlags flags{L.flags, L.ctrl, in.seg_off, tune.chunk, tune.big_item};
   const int n_templ = in.n_met * in.n_age, nW = in.n_wave;
   RUBIX_CUDA_TRY(cudaMemsetAsync(ws, 0, (size_t)((char*)(L.flags + in.n_seg) - (char*)ws), st));
   {
-    const int rc = node_build_tables(in, nullptr, L.prefix, L.h, L.H, L.rough_of, L.ctrl, st);
+    const int rc = node_setup(in, nullptr, L.ctrl, st);
     if (rc != RUBIX_OK) return rc;
   }
-  if (in.n_seg <= kItemsOneBlock) {
-    node_adj_items_kernel<<<1, 1024, 0, st>>>(in.seg_off, in.n_seg, L.chunks, L.items, L.ctrl);
+  const int steps = items_launches(in.n_seg, in.n);
+  const long long work = std::max<long long>(in.n_seg, in.n / 8);  // if screened, a warp a spaxel
+  const int g = (int)std::min<long long>((work + 255) / 256, (long long)sm_count() * 8);
+  if (steps > 1) {
+    node_adj_count_kernel<<<g, 256, 0, st>>>(in, flags, L.chunks);
+    RUBIX_LAUNCH_CHECK("node_adj_count_kernel");
+  }
+  if (steps < 3) {
+    node_adj_items_kernel<<<1, 1024, 0, st>>>(in, flags, steps == 1, L.chunks, L.items);
     RUBIX_LAUNCH_CHECK("node_adj_items_kernel");
   } else {
-    const int g = (int)std::min<long long>((in.n_seg + 255) / 256, (long long)sm_count() * 8);
-    node_adj_count_kernel<<<g, 256, 0, st>>>(in.seg_off, in.n_seg, L.chunks);
-    RUBIX_LAUNCH_CHECK("node_adj_count_kernel");
     scan_exclusive_1block<<<1, 1024, 0, st>>>(L.chunks, in.n_seg, 1);
     RUBIX_LAUNCH_CHECK("scan_exclusive_1block");
     node_adj_fill_kernel<<<g, 256, 0, st>>>(in.n_seg, L.chunks, L.items, L.ctrl);
     RUBIX_LAUNCH_CHECK("node_adj_fill_kernel");
   }
+  {
+    const int rc = node_build_tables(in, nullptr, L.prefix, L.h, L.H, L.rough_of, L.ctrl,
+                                     static_cast<CubeCtrl*>(ws), st);
+    if (rc != RUBIX_OK) return rc;
+  }
   const int blocks =
       (int)std::min<long long>(adj_items_max(in.n, in.n_seg), (long long)sm_count() * 8);
   {
     const AdjGatherArgs g{in,      L.prefix, L.H,   L.ctrl, L.items,
-                          L.rec_w, L.rec_a,  L.fin, L.flags, L.desc, L.rough};
+                          L.rec_w, L.rec_a,  L.fin, flags, L.desc, L.rough};
     node_adj_gather_kernel<<<blocks, kSub, 0, st>>>(g);
     RUBIX_LAUNCH_CHECK("node_adj_gather_kernel");
     const size_t smem = rough_smem(in.n_wave_t);
@@ -727,7 +732,7 @@ int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_st
   for (int w = 0; w < waves; ++w) {
     const AdjSliceArgs a{in.ssp_flux, in.ssp_wave_z, in.wave_t, n_templ, in.n_age, nW,
                          in.n_wave_t, L.desc,        L.items,   L.rec_w, L.rec_a,  adj,
-                         adj_stride,  L.flags,       L.part,    L.ctrl,  w,        per};
+                         adj_stride,  flags,         L.part,    L.ctrl,  w,        per};
     node_adj_slice_kernel<<<sm_count(), kNodeAdjThreads, smem, st>>>(a);
     RUBIX_LAUNCH_CHECK("node_adj_slice_kernel");
     const AdjMergeArgs m{L.items, L.desc, L.fin, L.part,   L.flags,  L.ctrl,   in.wave_t, nW,
@@ -736,9 +741,9 @@ int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_st
     RUBIX_LAUNCH_CHECK("node_adj_merge_kernel");
   }
   Carve c(static_cast<char*>(ws) + L.shared_off);
-  *fb = carve_fallback(c, in, true);
-  node_fallback_kernel<<<sm_count() * 8, 256, 0, st>>>(in, *fb, L.prefix, L.flags, L.ctrl,
-                                                      static_cast<CubeCtrl*>(ws), true);
+  *fb = carve_fallback(c, in, tune.chunk, true);
+  node_fallback_kernel<<<sm_count() * 8, 256, 0, st>>>(
+      in, *fb, L.prefix, flags, static_cast<CubeCtrl*>(ws), true);
   RUBIX_LAUNCH_CHECK("node_fallback_kernel");
   return RUBIX_OK;
 }

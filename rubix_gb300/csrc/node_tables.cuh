@@ -18,20 +18,28 @@ constexpr int kMaxWaves = 64;
 constexpr int kSub = 256;        // particles sorted together
 constexpr int kAlphaBits = 18;
 constexpr float kAlphaStep = 1.0f / (1 << kAlphaBits);
-constexpr int kAlphaHalf = 2048;                       // alpha rows on either side of 1
 constexpr float kAlphaMax = 2040.f * kAlphaStep;       // |alpha - 1| covered (2333 km/s)
+// |alpha - 1| covered by the T' table (949 km/s): the few faster stars of a galaxy have their T'
+// summed directly, 2 ns each, where every tile of rows costs 4 us and 340 kB.
+constexpr int kAlphaHalf = 832;                        // alpha rows on either side of 1
+constexpr float kTableMax = 830.f * kAlphaStep;
 constexpr int kAlphaTile = 64;                         // rows computed together
 constexpr int kAlphaTiles = 2 * kAlphaHalf / kAlphaTile + 1;
 constexpr int kAlphaRows = kAlphaTiles * kAlphaTile;
-static_assert(2040 + 4 < kAlphaHalf, "rows beside the limit exist");
+static_assert(kAlphaTiles <= 32, "a word of tiles");
 constexpr int kStage = 33;       // staged records of a warp: 32 and one of weight zero
 constexpr int kRuns = 4;
 constexpr int kDustMost = 8;     // samples between two nodes that a lane holds with dust
 
 struct NodeCtrl {
-  int flagged;                  // some spaxel is left to cube_main_kernel
+  int flagged;                  // spaxels left to the general kernel
+  // their items by place in its list: of several-chunk spaxels, of large ones, of the rest
+  int left[3], listed[3];
   unsigned e_lo, e_hi;          // bits of max(-e), max(e) of the dust exponents, >= 0
-  unsigned tile_mask[(kAlphaTiles + 31) / 32];
+  unsigned tile_mask;           // tiles of alpha rows that some star needs
+  unsigned tile_sel;            // the same without the screened spaxels' stars
+  unsigned a_min_inv, a_max;    // ~bits, bits of the smallest and largest alpha, approximate
+  int fast, screened;           // a star beyond the table; flags set before the items
   unsigned dz_inv, dt_inv;      // ~bits of the smallest SSP / telescope spacing
   unsigned dz_max, dt_max;      // bits of the largest (3e38: not ascending)
   unsigned run_max[kRuns], run_min_inv[kRuns];  // extent of own_nodes(r) + 1, + 0 intervals
@@ -41,6 +49,36 @@ struct NodeCtrl {
   int n_rough;                  // particles in the list of rough ones
   int n_items, n_multi;         // work items with particles; those of several-item spaxels
   int next[kMaxWaves][kMaxSlices];
+};
+
+// A spaxel is left to the general kernel: its flag, and its items counted for that kernel's list
+// (work items of `chunk` particles as in cube_prepare).
+struct NodeFlags {
+  int* flags;
+  NodeCtrl* ctrl;
+  const int* seg_off;
+  int chunk, big;
+  // Place in the list's order and number of a spaxel's items.
+  __device__ __forceinline__ int place(int s, int& items) const {
+    const int cnt = seg_off[s + 1] - seg_off[s];
+    items = (cnt + chunk - 1) / chunk;
+    return items > 1 ? 0 : (cnt >= big ? 1 : 2);
+  }
+  __device__ __forceinline__ void leave(int s) const {
+    if (atomicExch(&flags[s], 1) != 0) return;
+    int items;
+    const int p = place(s, items);
+    atomicAdd(&ctrl->left[p], items);
+    ctrl->flagged = 1;
+  }
+  // The counts of spaxels that a block has flagged itself.
+  __device__ __forceinline__ void add(const int* s_left) const {
+    const int tid = threadIdx.x;
+    if (tid < 3 && s_left[tid] > 0) {
+      atomicAdd(&ctrl->left[tid], s_left[tid]);
+      ctrl->flagged = 1;
+    }
+  }
 };
 
 // A slice has 32, 16, 8 or 4 nodes; all but its first and last are its own.
@@ -119,6 +157,22 @@ __device__ __forceinline__ float x_ext(const float* __restrict__ wt, int n, int 
   return wt[t];
 }
 
+// alpha - 1 of a velocity, to 1e-7.
+__device__ __forceinline__ float approx_am1(float v) {
+  const float z = v * (float)(1.0 / kSpeedOfLight);
+  return z * (1.f + 0.5f * z * (1.f + (1.f / 3.f) * z));
+}
+
+// The tiles of alpha rows on either side of it, up to a row beyond the limit that node_particle
+// checks on the rounded alpha; false beyond.
+__device__ __forceinline__ bool alpha_tiles(float am1, int& a, int& b) {
+  if (!(fabsf(am1) <= kTableMax + kAlphaStep)) return false;
+  const int r = (int)floorf(am1 * (float)(1 << kAlphaBits)) + kAlphaHalf;
+  a = max(r - 1, 0) / kAlphaTile;
+  b = min(r + 2, kAlphaRows - 1) / kAlphaTile;
+  return true;
+}
+
 // Grid extrema, and the rows of alpha that the particles' velocities fall on.
 __global__ void __launch_bounds__(256) node_setup_kernel(
     const float* __restrict__ wz, int n_wave, const float* __restrict__ wt, int n_t,
@@ -161,29 +215,185 @@ __global__ void __launch_bounds__(256) node_setup_kernel(
       }
     }
   }
-  __shared__ unsigned s_mask[(kAlphaTiles + 31) / 32];
-  if (threadIdx.x < (kAlphaTiles + 31) / 32) s_mask[threadIdx.x] = 0u;
-  __syncthreads();
-  int last = -1;
-  for (long long i = gtid; i < n; i += gsz) {
-    // alpha - 1 to ~1e-7: the rows on either side of it are marked, up to a row beyond the
-    // limit that node_particle checks on the rounded alpha
-    const float z = vel[i * vel_stride + vel_comp] * (float)(1.0 / kSpeedOfLight);
-    const float am1 = z * (1.f + 0.5f * z * (1.f + (1.f / 3.f) * z));
-    if (!(fabsf(am1) <= kAlphaMax + kAlphaStep)) continue;
-    const int r = (int)floorf(am1 * (float)(1 << kAlphaBits)) + kAlphaHalf;
-    const int a = max(r - 1, 0) / kAlphaTile, b = min(r + 2, kAlphaRows - 1) / kAlphaTile;
-    if (a != last) atomicOr(&s_mask[a >> 5], 1u << (a & 31));
-    if (b != a) atomicOr(&s_mask[b >> 5], 1u << (b & 31));
-    last = a;
+  __shared__ unsigned s_mask, s_min_inv, s_max;
+  __shared__ int s_fast;
+  if (threadIdx.x == 0) {
+    s_mask = s_min_inv = s_max = 0u;
+    s_fast = 0;
   }
   __syncthreads();
-  if (threadIdx.x < (kAlphaTiles + 31) / 32 && s_mask[threadIdx.x])
-    atomicOr(&ctrl->tile_mask[threadIdx.x], s_mask[threadIdx.x]);
+  unsigned mask = 0u;
+  bool fast = false;
+  float amin = 2.f, amax = 0.f;
+  for (long long i = gtid; i < n; i += gsz) {
+    const float am1 = approx_am1(vel[i * vel_stride + vel_comp]);
+    fast = fast || !(fabsf(am1) <= kAlphaMax - kAlphaStep);
+    amin = fminf(amin, 1.f + am1);
+    amax = fmaxf(amax, 1.f + am1);
+    int a, b;
+    if (!alpha_tiles(am1, a, b)) continue;
+    mask |= (1u << a) | (1u << b);
+  }
+  mask = __reduce_or_sync(0xffffffffu, mask);
+  const unsigned lo_inv = __reduce_max_sync(0xffffffffu, ~__float_as_uint(amin));
+  const unsigned hi_bits = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&s_min_inv, lo_inv);
+    atomicMax(&s_max, hi_bits);
+    atomicOr(&s_mask, mask);
+  }
+  if (fast) s_fast = 1;
+  __syncthreads();
+  if (threadIdx.x == 0 && s_mask) atomicOr(&ctrl->tile_mask, s_mask);
+  if (threadIdx.x == 0) {
+    atomicMax(&ctrl->a_min_inv, s_min_inv);
+    atomicMax(&ctrl->a_max, s_max);
+    if (s_fast) ctrl->fast = 1;
+  }
 }
 
 __device__ __forceinline__ bool tile_used(const NodeCtrl* c, int tile) {
-  return (c->tile_mask[tile >> 5] >> (tile & 31)) & 1u;
+  return ((c->screened ? c->tile_sel : c->tile_mask) >> tile) & 1u;
+}
+
+// Whether the call's velocities may flag a spaxel: where no star is beyond the table and all of
+// them together fit an item's window, none is screened.
+__device__ __forceinline__ bool screen_wanted(const NodeCtrl* c, const NodePlan& p, float x1) {
+  const float spread = __uint_as_float(c->a_max) - __uint_as_float(~c->a_min_inv) + 1e-6f;
+  return !p.ok || c->fast || spread * x1 / (1.f - kAlphaMax) > p.window * p.dt_min;
+}
+
+// Whether an item's range of alpha is wider than the rows of its slices.
+__device__ __forceinline__ bool too_wide(const NodePlan& p, float amin, float amax, float x1) {
+  return (amax - amin) * x1 / (1.f - kAlphaMax) > p.window * p.dt_min;
+}
+
+// What the velocities of one item's stars say, by a warp: whether they flag their spaxel, and
+// the tiles of their alpha rows.  On alpha to 1e-7 in float32 (the exact one takes 64-bit
+// products, 0.7 ms for 2 10^5 stars on one SM), so it flags what is beyond the gather's conditions
+// by more than that and leaves the rest to them.
+__device__ __forceinline__ bool screen_item(const CubeInputs& in, const NodePlan& p, int jb,
+                                            int je, float x1, unsigned& mask) {
+  float lo = 1.f, hi = -1.f, far = 0.f;
+#pragma unroll 4
+  for (int j = jb + (threadIdx.x & 31); j < je; j += 32) {
+    const float am1 = approx_am1(in.vel[(long long)in.perm[j] * in.vel_stride + in.vel_comp]);
+    int a, b;
+    if (alpha_tiles(am1, a, b)) mask |= (1u << a) | (1u << b);
+    lo = fminf(lo, am1);
+    hi = fmaxf(hi, am1);
+    far = fmaxf(far, isnan(am1) ? 1.f : fabsf(am1));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    far = fmaxf(far, __shfl_xor_sync(0xffffffffu, far, o));
+  }
+  return far > kAlphaMax + kAlphaStep || too_wide(p, lo + 1e-6f, hi, x1);
+}
+
+// Particles of each spaxel that the node path renders, to count(s, particles), by the whole grid
+// and before there are work items.  Where velocities rule spaxels out, or the grids all of
+// them, they are flagged here and count nothing, and only the other stars' tiles are built:
+// with a dispersion of 1000 km/s, where nearly every spaxel is flagged, the table product
+// alone took 270 us.
+template <class F>
+__device__ __forceinline__ void screened_counts(const CubeInputs& in, const NodeFlags& flags,
+                                                bool dust, int item, F count) {
+  constexpr int kLarge = 256;  // stars of a spaxel that a whole block screens
+  __shared__ NodePlan s_plan;
+  __shared__ int s_left[3], s_large[32], s_large_n, s_flag;
+  __shared__ unsigned s_sel, s_mask;
+  const float x1 = in.wave_t[in.n_wave_t - 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+  const int gtid = blockIdx.x * blockDim.x + tid, gsz = gridDim.x * blockDim.x;
+  if (tid == 0) {
+    s_plan = node_plan(flags.ctrl, in.n_wave, x1, dust);
+    s_sel = 0u;
+  }
+  if (tid < 3) s_left[tid] = 0;
+  int own = gtid < in.n_seg ? in.seg_off[gtid + 1] - in.seg_off[gtid] : 0;  // loaded meanwhile
+  __syncthreads();
+  const NodePlan plan = s_plan;
+  const bool screen = screen_wanted(flags.ctrl, plan, x1);
+  auto leave = [&](int s) {
+    int items;
+    const int p = flags.place(s, items);
+    atomicAdd(&s_left[p], items);
+    flags.flags[s] = 1;
+    count(s, 0);
+  };
+  if (!screen || !plan.ok) {
+    for (int s = gtid; s < in.n_seg; s += gsz) {
+      if (s != gtid) own = in.seg_off[s + 1] - in.seg_off[s];
+      if (screen && own > 0) leave(s);
+      else count(s, own);
+    }
+  } else {
+    // a spaxel per warp, the large ones among them by the block together
+    if (gtid == 0) flags.ctrl->screened = 1;
+    for (int s0 = blockIdx.x * warps; s0 < in.n_seg; s0 += gridDim.x * warps) {
+      if (tid == 0) s_large_n = 0;
+      __syncthreads();
+      const int s = s0 + warp;
+      if (s < in.n_seg) {
+        const int jb = in.seg_off[s], je = in.seg_off[s + 1];
+        if (je - jb > kLarge) {
+          if (lane == 0) s_large[atomicAdd(&s_large_n, 1)] = s;
+        } else {
+          unsigned mask = 0u;
+          const bool flag = screen_item(in, plan, jb, je, x1, mask);
+          mask = __reduce_or_sync(0xffffffffu, mask);
+          if (lane == 0) {
+            if (flag) leave(s);
+            else count(s, je - jb);
+            if (!flag && mask) atomicOr(&s_sel, mask);
+          }
+        }
+      }
+      __syncthreads();
+      const int n_large = s_large_n;
+      for (int q = 0; q < n_large; ++q) {
+        if (tid == 0) {
+          s_flag = 0;
+          s_mask = 0u;
+        }
+        __syncthreads();
+        const int big = s_large[q], jb = in.seg_off[big], je = in.seg_off[big + 1];
+        unsigned mask = 0u;
+        bool flag = false;
+        for (int c = jb + warp * item; c < je; c += warps * item)
+          flag = screen_item(in, plan, c, min(c + item, je), x1, mask) || flag;
+        mask = __reduce_or_sync(0xffffffffu, mask);
+        if (lane == 0) {
+          if (flag) s_flag = 1;
+          atomicOr(&s_mask, mask);
+        }
+        __syncthreads();
+        if (tid == 0) {
+          if (s_flag) {
+            leave(big);
+          } else {
+            count(big, je - jb);
+            s_sel |= s_mask;
+          }
+        }
+        __syncthreads();
+      }
+    }
+  }
+  __syncthreads();
+  flags.add(s_left);
+  if (tid == 0 && s_sel) atomicOr(&flags.ctrl->tile_sel, s_sel);
+}
+
+// How the work items are made: up to kItemsOneBlock spaxels by one block, which counts their
+// stars too up to kCountOneBlock (one SM screens 2 10^5 stars in 0.4 ms); else in a launch each
+// for counts, scans and list.
+constexpr long long kCountOneBlock = 1 << 16;
+inline int items_launches(int n_seg, long long n) {
+  return n_seg > kItemsOneBlock ? 3 : (n > kCountOneBlock ? 2 : 1);
 }
 
 // The two resampling weights that interval [k, k + 1] gives its nodes at one alpha: the
@@ -246,8 +456,16 @@ __device__ __forceinline__ float node_roughness(const float* __restrict__ f,
 __global__ void __launch_bounds__(kPrefixThreads) node_tables_kernel(
     const float* __restrict__ flux, int rows, int n_wave, const float* __restrict__ wz,
     const float* __restrict__ wt, int n_t, double* __restrict__ prefix, float* __restrict__ h,
-    int kpad, float* __restrict__ rough, NodeCtrl* __restrict__ ctrl) {
-  // the grid's node range (fmax, still being formed, only decides whether it is used)
+    int kpad, float* __restrict__ rough, bool dust, NodeCtrl* __restrict__ ctrl,
+    CubeCtrl* __restrict__ cc) {
+  if ((int)blockIdx.x == rows + kWeightBlocks) {  // for the general kernel's tables
+    if (threadIdx.x == 0) {
+      bucket_params(wt, n_t, cc->lnq0, cc->h);
+      cc->inv_h = 1.0 / cc->h;
+      cc->bmax = (float)(kVmaxKms / kSpeedOfLight / cc->h);
+    }
+    return;
+  }
   const int k_first = max(ctrl->k_first - 1, 0);
   const int k_last = min(n_wave - ctrl->k_last_inv, n_wave - 1);
   if ((int)blockIdx.x < rows) {
@@ -278,6 +496,9 @@ __global__ void __launch_bounds__(kPrefixThreads) node_tables_kernel(
     }
     return;
   }
+  // nothing reads the weights of a grid that does not qualify (fmax, still being formed, can
+  // only rule it out)
+  if (!node_plan(ctrl, n_wave, wt[n_t - 1], dust).ok) return;
   __shared__ float s_rise[kPrefixThreads + 1];
   const int tid = threadIdx.x;
   const int count = k_last - k_first + 1;
@@ -599,6 +820,7 @@ __device__ __forceinline__ NodeParticle node_particle(const CubeInputs& in,
   const float u = (p.alpha - 1.f) * (float)(1 << kAlphaBits);  // exact
   const int r = (int)floorf(u) + kAlphaHalf;
   const float fr = u - floorf(u);
+  const bool tabled = fabsf(p.alpha - 1.f) <= kTableMax;
   const float* h0 = H + (long long)r * n_templ;
   const float* h1 = h0 + n_templ;
 #pragma unroll
@@ -606,10 +828,10 @@ __device__ __forceinline__ NodeParticle node_particle(const CubeInputs& in,
     const double* pf = prefix + (long long)rr[c] * in.n_wave;
     if (ka <= ke) p.dT[c] = pf[ke] - pf[ka - 1];
     p.T = fmaf(p.w[c], (float)p.dT[c], p.T);
-    p.Tp = fmaf(p.w[c], fmaf(fr, h1[rr[c]] - h0[rr[c]], h0[rr[c]]), p.Tp);
+    if (tabled) p.Tp = fmaf(p.w[c], fmaf(fr, h1[rr[c]] - h0[rr[c]], h0[rr[c]]), p.Tp);
   }
   p.T *= p.alpha;
-  p.rough = isnan(p.Tp);
+  p.rough = !tabled || isnan(p.Tp);
   if (!p.rough && bad_scale(p.T, p.Tp)) p.bad = true;
   return p;
 }
@@ -714,20 +936,25 @@ int rough_blocks(long long n) {
 
 int kpad_of(int n_wave) { return (n_wave + 31) / 32 * 32; }
 
-// Grid extrema and used alpha rows, prefix sums and resampling weights, the T' table: three
-// launches.
-int node_build_tables(const CubeInputs& in, const float* dust_e, double* prefix, float* h,
-                      float* H, float* rough, NodeCtrl* ctrl, cudaStream_t st) {
-  const int n_templ = in.n_met * in.n_age, nW = in.n_wave, kpad = kpad_of(nW);
-  const long long work = std::max<long long>(std::max(in.n_wave_t, nW), in.n);
+// Grid extrema and used alpha rows.
+int node_setup(const CubeInputs& in, const float* dust_e, NodeCtrl* ctrl, cudaStream_t st) {
+  const long long work = std::max<long long>(std::max(in.n_wave_t, in.n_wave), in.n);
   const int g = (int)std::min<long long>((work + 255) / 256, (long long)sm_count() * 8);
-  const int need = (std::max(in.n_wave_t, nW) + 255) / 256;
-  node_setup_kernel<<<std::max(g, need), 256, 0, st>>>(in.ssp_wave_z, nW, in.wave_t, in.n_wave_t,
-                                                       in.vel, in.vel_stride, in.vel_comp, in.n,
-                                                       dust_e, ctrl);
+  const int need = (std::max(in.n_wave_t, in.n_wave) + 255) / 256;
+  node_setup_kernel<<<std::max(g, need), 256, 0, st>>>(in.ssp_wave_z, in.n_wave, in.wave_t,
+                                                       in.n_wave_t, in.vel, in.vel_stride,
+                                                       in.vel_comp, in.n, dust_e, ctrl);
   RUBIX_LAUNCH_CHECK("node_setup_kernel");
-  node_tables_kernel<<<n_templ + kWeightBlocks, kPrefixThreads, 0, st>>>(
-      in.ssp_flux, n_templ, nW, in.ssp_wave_z, in.wave_t, in.n_wave_t, prefix, h, kpad, rough, ctrl);
+  return RUBIX_OK;
+}
+
+// Prefix sums and resampling weights, the T' table: two launches.
+int node_build_tables(const CubeInputs& in, const float* dust_e, double* prefix, float* h,
+                      float* H, float* rough, NodeCtrl* ctrl, CubeCtrl* cc, cudaStream_t st) {
+  const int n_templ = in.n_met * in.n_age, nW = in.n_wave, kpad = kpad_of(nW);
+  node_tables_kernel<<<n_templ + kWeightBlocks + 1, kPrefixThreads, 0, st>>>(
+      in.ssp_flux, n_templ, nW, in.ssp_wave_z, in.wave_t, in.n_wave_t, prefix, h, kpad, rough,
+      dust_e != nullptr, ctrl, cc);
   RUBIX_LAUNCH_CHECK("node_tables_kernel");
   node_table_product_kernel<<<dim3((n_templ + 31) / 32, kAlphaTiles), 128, 0, st>>>(
       h, kpad, in.ssp_flux, n_templ, nW, in.wave_t, in.n_wave_t, dust_e != nullptr, rough, ctrl, H);
@@ -737,7 +964,7 @@ int node_build_tables(const CubeInputs& in, const float* dust_e, double* prefix,
 
 // The workspace of what is left to the general kernels (grad: the adjoint's, which has no
 // partial spectra).
-NodeFallback carve_fallback(Carve& c, const CubeInputs& in, bool grad) {
+NodeFallback carve_fallback(Carve& c, const CubeInputs& in, int chunk, bool grad) {
   NodeFallback f{};
   f.At = c.take<float>((size_t)in.n_wave_t);
   f.bucket = c.take<int2>(kBuckets);
@@ -745,14 +972,16 @@ NodeFallback carve_fallback(Carve& c, const CubeInputs& in, bool grad) {
   f.rec = c.take<ParticleRec>((size_t)in.n);
   f.done = c.take<int>((size_t)in.n_seg);
   f.slot_start = c.take<int>((size_t)in.n_seg);
-  f.chunk = kMaxChunk;
-  f.items = c.take<int2>((size_t)max_slots(in.n, kMaxChunk) + in.n_seg);
+  f.chunk = chunk;
+  f.alo = (float)std::exp(-kVmaxKms / kSpeedOfLight);
+  f.ahi = (float)std::exp(kVmaxKms / kSpeedOfLight);
+  f.items = c.take<int2>((size_t)max_slots(in.n, chunk) + in.n_seg);
   if (!grad)
-    f.partials = c.take<float>((size_t)max_slots(in.n, kMaxChunk) * in.n_wave_t);
+    f.partials = c.take<float>((size_t)max_slots(in.n, chunk) * in.n_wave_t);
   return f;
 }
 
-size_t fallback_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t,
+size_t fallback_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk,
                       bool grad) {
   CubeInputs in{};
   in.n_met = nZ;
@@ -762,56 +991,64 @@ size_t fallback_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t,
   in.n_seg = n_seg;
   in.n = n;
   Carve c(nullptr);
-  carve_fallback(c, in, grad);
+  carve_fallback(c, in, chunk, grad);
   return c.off;
 }
 
-// What cube_main_kernel reads (cube_prepare's setup passes), when a spaxel is flagged.
+// What the general kernel reads (cube_prepare's setup passes), when a spaxel is flagged: the
+// tables over the grids, the flagged spaxels' items and the records of their particles.
 __global__ void __launch_bounds__(256) node_fallback_kernel(CubeInputs in, NodeFallback f,
                                                             const double* __restrict__ prefix,
-                                                            const int* __restrict__ flags,
-                                                            const NodeCtrl* __restrict__ nc,
+                                                            NodeFlags flags,
                                                             CubeCtrl* __restrict__ ctrl,
                                                             bool grad) {
+  const NodeCtrl* nc = flags.ctrl;
   if (!nc->flagged) return;
-  const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
-  double lnq0, h;
-  bucket_params(in.wave_t, in.n_wave_t, lnq0, h);
+  __shared__ int s_cnt[3], s_at[3];
+  const int tid = threadIdx.x;
+  const int gtid = blockIdx.x * 256 + tid, gsz = gridDim.x * 256;
+  const double lnq0 = ctrl->lnq0, h = ctrl->h;
   for (int t = gtid; t < in.n_wave_t; t += gsz)
     f.At[t] = (float)((log((double)in.wave_t[t]) - lnq0) / h);
   for (int b = gtid; b < kBuckets; b += gsz)
     f.bucket[b] = bucket_entry(in.ssp_wave_z, in.n_wave, lnq0, h, b);
-  if (blockIdx.x == 0) {
-    // the flagged spaxels' items: those of several chunks first
-    __shared__ int s_multi, s_single;
-    if (threadIdx.x == 0) s_multi = s_single = 0;
+  const int at1 = nc->left[0], at2 = at1 + nc->left[1];
+  if (gtid == 0) ctrl->n_items = at2 + nc->left[2];
+  // 256 spaxels at a time: places within the block, then the block's in the list
+  for (long long s0 = blockIdx.x * 256LL; s0 < in.n_seg; s0 += gsz) {
+    const long long s = s0 + tid;
+    const bool on = s < in.n_seg && flags.flags[s];
+    int n = 0, p = 0, at = 0;
+    if (on) p = flags.place((int)s, n);
     __syncthreads();
-    for (int pass = 0; pass < 2; ++pass) {
-      for (int s = threadIdx.x; s < in.n_seg; s += blockDim.x) {
-        if (!flags[s]) continue;
-        const int cnt = in.seg_off[s + 1] - in.seg_off[s];
-        const int nch = (cnt + f.chunk - 1) / f.chunk;
-        if ((nch > 1) != (pass == 0)) continue;
-        const int at = atomicAdd(pass == 0 ? &s_multi : &s_single, nch);
-        f.slot_start[s] = at;
-        f.done[s] = 0;
-        for (int c = 0; c < nch; ++c) f.items[at + c] = make_int2(s, c);
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        if (pass == 0) s_single = s_multi;
-        else ctrl->n_items = s_single;
-      }
-      __syncthreads();
+    if (tid < 3) s_cnt[tid] = 0;
+    __syncthreads();
+    if (on) at = atomicAdd(&s_cnt[p], n);
+    __syncthreads();
+    if (tid < 3 && s_cnt[tid] > 0) s_at[tid] = atomicAdd(&flags.ctrl->listed[tid], s_cnt[tid]);
+    __syncthreads();
+    if (on) {
+      at += s_at[p] + (p == 0 ? 0 : (p == 1 ? at1 : at2));
+      f.slot_start[s] = at;
+      f.done[s] = 0;
+      for (int c = 0; c < n; ++c) f.items[at + c] = make_int2((int)s, c);
     }
   }
   corner_table(in.ssp_flux, in.n_met, in.n_age, in.n_wave, f.ct, gtid, gsz);
-  gather_records(in.mass, in.met, in.age, in.vel, in.vel_stride, in.vel_comp, in.perm,
-                 in.seg_off, in.n_seg, in.n, in.ssp_met, in.n_met, in.ssp_age, in.n_age,
-                 in.ssp_wave_z, in.n_wave, in.wave_t, in.n_wave_t, prefix, 1.0 / h,
-                 (float)(kVmaxKms / kSpeedOfLight / h), __uint_as_float(~nc->dz_inv),
-                 __uint_as_float(nc->dt_max), f.rec, grad ? 1 : 0, in.av,
-                 (float)exp(-kVmaxKms / kSpeedOfLight), (float)exp(kVmaxKms / kSpeedOfLight));
+  const long long n_valid = in.seg_off[in.n_seg];
+  for (long long j = gtid; j < n_valid && j < in.n; j += gsz) {
+    int lo = 0, hi = in.n_seg - 1;  // the spaxel of place j: the last that starts at or before it
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (in.seg_off[mid] <= j) lo = mid; else hi = mid - 1;
+    }
+    if (!flags.flags[lo]) continue;
+    gather_records(in.mass, in.met, in.age, in.vel, in.vel_stride, in.vel_comp, in.perm,
+                   in.seg_off, in.n_seg, in.ssp_met, in.n_met, in.ssp_age, in.n_age,
+                   in.ssp_wave_z, in.n_wave, in.wave_t, in.n_wave_t, prefix, ctrl->inv_h,
+                   ctrl->bmax, __uint_as_float(~nc->dz_inv), __uint_as_float(nc->dt_max), f.rec,
+                   grad ? 1 : 0, in.av, f.alo, f.ahi, j, j + 1, 1);
+  }
 }
 
 }  // namespace
