@@ -109,12 +109,18 @@ RUBIX_API int rubix_spaxel_sort(const int32_t* idx, const uint8_t* keep, int64_t
 RUBIX_API size_t rubix_cube_workspace_size(int64_t n, int32_t n_segments, int32_t n_wave_t,
                                            int32_t n_met, int32_t n_age, int32_t n_wave);
 
-/* Kernels that rubix_cube_fwd and rubix_cube_fwd_dust (general = 0), or
- * rubix_cube_fwd_general (general = 1), launch for these sizes with a workspace of
+/* Whether rubix_cube_fwd and rubix_cube_fwd_dust sum over SSP nodes (1: where the grids also
+ * qualify and the workspace has the size queried above, or half of it) or take the general path
+ * (0), by the sizes: with few stars a spaxel, or few altogether, the general path is the faster. */
+RUBIX_API int rubix_cube_fwd_path(int64_t n, int32_t n_segments, int32_t n_wave_t, int32_t n_met,
+                                  int32_t n_age, int32_t n_wave);
+
+/* Kernels that rubix_cube_fwd and rubix_cube_fwd_dust (path = 0), rubix_cube_fwd_general
+ * (path = 1) or rubix_cube_fwd_nodes (path = 2) launch for these sizes with a workspace of
  * workspace_bytes. */
 RUBIX_API int rubix_cube_fwd_launches(int64_t n, int32_t n_segments, int32_t n_wave_t,
                                       int32_t n_met, int32_t n_age, int32_t n_wave,
-                                      int32_t general, size_t workspace_bytes);
+                                      int32_t path, size_t workspace_bytes);
 
 /*
  * cube[s][0..n_wave_t) = sum over kept particles p of spaxel s of
@@ -143,17 +149,30 @@ RUBIX_API int rubix_cube_fwd(const float* ssp_flux, const float* ssp_metallicity
                    size_t workspace_bytes, void* stream);
 
 /*
- * rubix_cube_fwd (av and ext_exponent NULL) or rubix_cube_fwd_dust with every particle
- * evaluated at every telescope wavelength, as those themselves do where the template grid
- * does not qualify for sums over SSP nodes (csrc/cube_nodes.cu).  The results agree to
- * float32 rounding; this one keeps the summation order that float64 sums over the cube (the
- * gradients of the instrument widths) have been recorded with.
- * Workspace: rubix_cube_general_workspace_size.
+ * rubix_cube_fwd (av and ext_exponent NULL) or rubix_cube_fwd_dust by one path whatever
+ * rubix_cube_fwd_path says: every particle evaluated at every telescope wavelength
+ * (rubix_cube_fwd_general), or sums over SSP nodes (rubix_cube_fwd_nodes, csrc/cube_nodes.cu;
+ * still the general path where the grids do not qualify or the workspace is smaller than
+ * half of its query).  The results agree to float32 rounding.  A caller that
+ * renders parts of a batch by themselves gets the batch's bits by taking the batch's path.
  */
 RUBIX_API size_t rubix_cube_general_workspace_size(int64_t n, int32_t n_segments,
                                                    int32_t n_wave_t, int32_t n_met,
                                                    int32_t n_age, int32_t n_wave);
 RUBIX_API int rubix_cube_fwd_general(const float* ssp_flux, const float* ssp_metallicity,
+                   const float* ssp_age, const float* ssp_wave_z, int32_t n_met,
+                   int32_t n_age, int32_t n_wave, const float* wave_t, int32_t n_wave_t,
+                   const float* mass, const float* metallicity, const float* age,
+                   const float* velocity, int64_t vel_stride, int32_t vel_component,
+                   const float* av, const float* ext_exponent, const int32_t* perm,
+                   const int32_t* seg_offsets, int32_t n_segments, int64_t n,
+                   const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop,
+                   float* cube, int64_t spaxel_stride, void* workspace,
+                   size_t workspace_bytes, void* stream);
+RUBIX_API size_t rubix_cube_nodes_workspace_size(int64_t n, int32_t n_segments,
+                                                 int32_t n_wave_t, int32_t n_met,
+                                                 int32_t n_age, int32_t n_wave);
+RUBIX_API int rubix_cube_fwd_nodes(const float* ssp_flux, const float* ssp_metallicity,
                    const float* ssp_age, const float* ssp_wave_z, int32_t n_met,
                    int32_t n_age, int32_t n_wave, const float* wave_t, int32_t n_wave_t,
                    const float* mass, const float* metallicity, const float* age,

@@ -55,6 +55,14 @@ SIGNATURES = {
          _vp, _vp, _i32, _i64, _vp, _i32, _i32, _vp, _i64, _vp, _sz, _vp],
     ),
     "rubix_cube_general_workspace_size": (_sz, [_i64, _i32, _i32, _i32, _i32, _i32]),
+    "rubix_cube_fwd_nodes": (
+        _c.c_int,
+        [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp, _i32,
+         _vp, _vp, _vp, _vp, _i64, _i32, _vp, _vp,
+         _vp, _vp, _i32, _i64, _vp, _i32, _i32, _vp, _i64, _vp, _sz, _vp],
+    ),
+    "rubix_cube_nodes_workspace_size": (_sz, [_i64, _i32, _i32, _i32, _i32, _i32]),
+    "rubix_cube_fwd_path": (_c.c_int, [_i64, _i32, _i32, _i32, _i32, _i32]),
     "rubix_cube_fwd_dust": (
         _c.c_int,
         [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp, _i32,

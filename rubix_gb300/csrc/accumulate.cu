@@ -912,7 +912,7 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                   const float* metallicity, const float* age, const float* velocity,
                   int64_t vel_stride, int32_t vel_component, const int32_t* perm,
                   const int32_t* seg_offsets, int32_t n_segments, int64_t n,
-                  const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop, bool nodes,
+                  const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop, CubePath path,
                   const float* av, const float* dust_e2, float* cube, int64_t spaxel_stride,
                   void* workspace, size_t workspace_bytes, void* stream);
 
@@ -929,22 +929,72 @@ size_t rubix::cube_general_workspace(int64_t n, int32_t n_segments, int32_t n_wa
       .bytes;
 }
 
-extern "C" size_t rubix_cube_workspace_size(int64_t n, int32_t n_segments, int32_t n_wave_t,
-                                            int32_t n_met, int32_t n_age, int32_t n_wave) {
+// The node path costs a table of T' first (as many stars' worth as n0) and some steps for every
+// spaxel; the general path more for every star.  Where they meet was measured on four grids
+// (8 x 2 x 800 to 221 x 6 x 1221 and 50 x 5 x 1400 templates), 700 to 3721 samples and 16 to
+// 22 500 spaxels of 1 to 24 stars, node / general path in us:
+//   256 spaxels, 120 templates: 1 star 1.9, 6 stars 1.02, 16 stars 0.59; 1326 templates: 8 stars 1.09,
+//   10 stars 0.98; 64 spaxels cross at 10 (16), 16 at 24 (more than 24) stars: the table;
+//   22 500 spaxels, 3721 samples: 120 templates 1.23 at 4, 0.91 at 10; 1326: 1.46, 1.07;
+//   700 samples: 1.14, 0.72 and 1.25, 0.82.  Coarse templates (800, of 8 samples an interval)
+//   have twice the slices: 1.76 at 4, 1.24 at 13 stars.  Beyond about 1300 template wavelengths
+//   the general kernel has one block an SM: 0.93 at one star, 1.03 at 8 on 4000 spaxels.
+bool rubix::cube_nodes_worth(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
+  const double templates = (double)nZ * nA;
+  const double n0 = 470.0 + templates / 3.5;
+  double per = 3.0 + templates / 700.0;
+  if (n_seg > 2000) {
+    per = 3.5 + templates / 700.0 + n_t / 700.0;
+    if (n_t > 3.8 * nW) per *= 2.0;
+    const int pool = kPB * (nW + 2);  // one block of the general kernel on an SM, not two
+    if (smem_layout(nW, pool, pool).total > 113 * 1024) per = n_seg > 8192 ? 0.3 : per * 0.5;
+  }
+  return n >= n0 + per * n_seg;
+}
+
+extern "C" int rubix_cube_fwd_path(int64_t n, int32_t n_segments, int32_t n_wave_t, int32_t n_met,
+                                   int32_t n_age, int32_t n_wave) {
+  return n > 0 && n_segments > 0 && cube_nodes_supported(n_met, n_age, n_wave, n_wave_t) &&
+         cube_nodes_worth(n, n_segments, n_met, n_age, n_wave, n_wave_t);
+}
+
+extern "C" size_t rubix_cube_nodes_workspace_size(int64_t n, int32_t n_segments, int32_t n_wave_t,
+                                                  int32_t n_met, int32_t n_age, int32_t n_wave) {
   if (n < 0 || n_segments < 0 || n_wave_t < 0 || n_met < 0 || n_age < 0 || n_wave < 0) return 0;
-  const size_t general = rubix::cube_general_workspace(n, n_segments, n_wave_t, n_met, n_age, n_wave);
+  const size_t general =
+      rubix::cube_general_workspace(n, n_segments, n_wave_t, n_met, n_age, n_wave);
   if (n == 0 || !cube_nodes_supported(n_met, n_age, n_wave, n_wave_t)) return general;
   return std::max(general, cube_nodes_bytes(n, n_segments, n_met, n_age, n_wave, n_wave_t,
                                             cube_tuning_current().chunk));
 }
 
+extern "C" size_t rubix_cube_workspace_size(int64_t n, int32_t n_segments, int32_t n_wave_t,
+                                            int32_t n_met, int32_t n_age, int32_t n_wave) {
+  if (n < 0 || n_segments < 0 || n_wave_t < 0 || n_met < 0 || n_age < 0 || n_wave < 0) return 0;
+  return rubix_cube_fwd_path(n, n_segments, n_wave_t, n_met, n_age, n_wave)
+             ? rubix_cube_nodes_workspace_size(n, n_segments, n_wave_t, n_met, n_age, n_wave)
+             : rubix::cube_general_workspace(n, n_segments, n_wave_t, n_met, n_age, n_wave);
+}
+
+namespace rubix {
+namespace {
+
+bool takes_nodes(CubePath path, long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk,
+                 size_t bytes) {
+  return path != kPathGeneral && n > 0 && cube_nodes_supported(nZ, nA, nW, n_t) &&
+         (path == kPathNodes || cube_nodes_worth(n, n_seg, nZ, nA, nW, n_t)) &&
+         cube_nodes_fit(n, n_seg, nZ, nA, nW, n_t, chunk, bytes);
+}
+
+}  // namespace
+}  // namespace rubix
+
 extern "C" int rubix_cube_fwd_launches(int64_t n, int32_t n_segments, int32_t n_wave_t,
                                        int32_t n_met, int32_t n_age, int32_t n_wave,
-                                       int32_t general, size_t workspace_bytes) {
+                                       int32_t path, size_t workspace_bytes) {
   if (n_segments <= 0) return 0;
-  if (!general && n > 0 && cube_nodes_supported(n_met, n_age, n_wave, n_wave_t) &&
-      cube_nodes_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, cube_tuning_current().chunk,
-                     workspace_bytes))
+  if (takes_nodes(path == 1 ? kPathGeneral : (path == 2 ? kPathNodes : kPathAuto), n, n_segments,
+                  n_met, n_age, n_wave, n_wave_t, cube_tuning_current().chunk, workspace_bytes))
     return cube_nodes_launches(n, n_segments, n_met, n_age, n_wave, workspace_bytes) + 1;
   // grid tables, items (count, scans and fill, or one launch), main (+ gather)
   return (n_segments <= kItemsOneBlock ? 3 : 5) + (n > 0 ? 1 : 0);
@@ -999,7 +1049,7 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                   const float* metallicity, const float* age, const float* velocity,
                   int64_t vel_stride, int32_t vel_component, const int32_t* perm,
                   const int32_t* seg_offsets, int32_t n_segments, int64_t n,
-                  const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop, bool nodes,
+                  const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop, CubePath path,
                   const float* av, const float* dust_e2, float* cube, int64_t spaxel_stride,
                   void* workspace, size_t workspace_bytes, void* stream) {
   {
@@ -1043,8 +1093,8 @@ int cube_fwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                       vel_component, perm, seg_offsets, n_segments, n, av};
   MainArgs args;
   args.chunk = tune.chunk;
-  if (nodes && n > 0 && cube_nodes_supported(n_met, n_age, n_wave, n_wave_t) &&
-      cube_nodes_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, tune.chunk, workspace_bytes)) {
+  if (takes_nodes(path, n, n_segments, n_met, n_age, n_wave, n_wave_t, tune.chunk,
+                  workspace_bytes)) {
     NodeFallback fb;
     const int rc = cube_nodes_forward(in, dust_e2, lsf_taps, n_lsf_taps, lsf_crop,
                                       tune, cube, spaxel_stride, workspace, workspace_bytes,
@@ -1114,7 +1164,7 @@ int cube_fwd_named(const char* who, const float* ssp_flux, const float* ssp_meta
   return cube_fwd_impl(who, ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, n_met, n_age,
                        n_wave, wave_t, n_wave_t, mass, metallicity, age, velocity, vel_stride,
                        vel_component, perm, seg_offsets, n_segments, n, lsf_taps, n_lsf_taps,
-                       lsf_crop, true, nullptr, nullptr, cube, spaxel_stride, workspace,
+                       lsf_crop, kPathAuto, nullptr, nullptr, cube, spaxel_stride, workspace,
                        workspace_bytes, stream);
 }
 
@@ -1133,7 +1183,7 @@ extern "C" int rubix_cube_fwd(const float* ssp_flux, const float* ssp_metallicit
   return cube_fwd_impl("rubix_cube_fwd", ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, n_met,
                        n_age, n_wave, wave_t, n_wave_t, mass, metallicity, age, velocity,
                        vel_stride, vel_component, perm, seg_offsets, n_segments, n, lsf_taps,
-                       n_lsf_taps, lsf_crop, true, nullptr, nullptr, cube, spaxel_stride, workspace,
+                       n_lsf_taps, lsf_crop, kPathAuto, nullptr, nullptr, cube, spaxel_stride, workspace,
                        workspace_bytes, stream);
 }
 
@@ -1161,7 +1211,27 @@ extern "C" int rubix_cube_fwd_general(const float* ssp_flux, const float* ssp_me
   return cube_fwd_impl("rubix_cube_fwd_general", ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z,
                        n_met, n_age, n_wave, wave_t, n_wave_t, mass, metallicity, age, velocity,
                        vel_stride, vel_component, perm, seg_offsets, n_segments, n, lsf_taps,
-                       n_lsf_taps, lsf_crop, false, av, ext_exponent, cube, spaxel_stride,
+                       n_lsf_taps, lsf_crop, kPathGeneral, av, ext_exponent, cube, spaxel_stride,
+                       workspace, workspace_bytes, stream);
+}
+
+extern "C" int rubix_cube_fwd_nodes(const float* ssp_flux, const float* ssp_metallicity,
+                                    const float* ssp_age, const float* ssp_wave_z, int32_t n_met,
+                                    int32_t n_age, int32_t n_wave, const float* wave_t,
+                                    int32_t n_wave_t, const float* mass, const float* metallicity,
+                                    const float* age, const float* velocity, int64_t vel_stride,
+                                    int32_t vel_component, const float* av,
+                                    const float* ext_exponent, const int32_t* perm,
+                                    const int32_t* seg_offsets, int32_t n_segments, int64_t n,
+                                    const float* lsf_taps, int32_t n_lsf_taps, int32_t lsf_crop,
+                                    float* cube, int64_t spaxel_stride, void* workspace,
+                                    size_t workspace_bytes, void* stream) {
+  RUBIX_REQUIRE(n == 0 || (av != nullptr) == (ext_exponent != nullptr), RUBIX_E_INVALID,
+                "rubix_cube_fwd_nodes: A_V and extinction exponent go together");
+  return cube_fwd_impl("rubix_cube_fwd_nodes", ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z,
+                       n_met, n_age, n_wave, wave_t, n_wave_t, mass, metallicity, age, velocity,
+                       vel_stride, vel_component, perm, seg_offsets, n_segments, n, lsf_taps,
+                       n_lsf_taps, lsf_crop, kPathNodes, av, ext_exponent, cube, spaxel_stride,
                        workspace, workspace_bytes, stream);
 }
 
@@ -1181,7 +1251,7 @@ extern "C" int rubix_cube_fwd_dust(const float* ssp_flux, const float* ssp_metal
   return cube_fwd_impl("rubix_cube_fwd_dust", ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z,
                        n_met, n_age, n_wave, wave_t, n_wave_t, mass, metallicity, age, velocity,
                        vel_stride, vel_component, perm, seg_offsets, n_segments, n, lsf_taps,
-                       n_lsf_taps, lsf_crop, true, av, ext_exponent, cube, spaxel_stride, workspace,
+                       n_lsf_taps, lsf_crop, kPathAuto, av, ext_exponent, cube, spaxel_stride, workspace,
                        workspace_bytes, stream);
 }
 

@@ -586,12 +586,36 @@ int launch_adjoint(const AdjArgs& args, size_t smem, cudaStream_t st) {
 
 using namespace rubix;
 
+namespace rubix {
+namespace {
+
+// As cube_nodes_worth; the general adjoint costs more per star, and up to some 5000 spaxels it
+// waits on latency.  Node / general path: 256 spaxels, 120 templates 1.2 at 2 stars, 0.8 at 4, 0.33
+// at 16, 1326 templates 1.5, 0.96 (700 samples), 0.48; 22 500 spaxels, 3721 samples 1.5 to 1.75 at 4
+// stars, about 1 at 10; 700 samples 0.95 at 2.
+bool bwd_nodes_worth(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
+  const double templates = (double)nZ * nA;
+  double per = 1.8 + templates / 1900.0;
+  if (n_seg > 5000) per = 1.5 + n_t / 450.0;
+  if (n_seg > 5000 && n_t > 3.8 * nW) per *= 2.0;
+  return n >= 130.0 + templates / 11.0 + per * n_seg;
+}
+
+// Host-side choice of path for an adjoint without dust.
+bool bwd_nodes_path(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
+  return n > 0 && n_seg > 0 && cube_nodes_bwd_supported(nZ, nA, nW, n_t) &&
+         bwd_nodes_worth(n, n_seg, nZ, nA, nW, n_t);
+}
+
+}  // namespace
+}  // namespace rubix
+
 extern "C" size_t rubix_cube_bwd_workspace_size(int64_t n, int32_t n_segments, int32_t n_wave_t,
                                                 int32_t n_met, int32_t n_age, int32_t n_wave) {
   if (n < 0 || n_segments < 0 || n_wave_t < 0 || n_met < 0 || n_age < 0 || n_wave < 0) return 0;
   const size_t general =
       cube_general_workspace(n, n_segments, n_wave_t, n_met, n_age, n_wave);
-  if (n == 0 || !cube_nodes_bwd_supported(n_met, n_age, n_wave, n_wave_t)) return general;
+  if (!bwd_nodes_path(n, n_segments, n_met, n_age, n_wave, n_wave_t)) return general;
   return std::max(general, cube_nodes_bwd_bytes(n, n_segments, n_met, n_age, n_wave, n_wave_t,
                                                 cube_tuning_current().chunk));
 }
@@ -600,7 +624,7 @@ extern "C" int rubix_cube_bwd_launches(int64_t n, int32_t n_segments, int32_t n_
                                        int32_t n_met, int32_t n_age, int32_t n_wave, int32_t dust,
                                        size_t workspace_bytes) {
   if (n_segments <= 0 || n <= 0) return 0;
-  if (!dust && cube_nodes_bwd_supported(n_met, n_age, n_wave, n_wave_t) &&
+  if (!dust && bwd_nodes_path(n, n_segments, n_met, n_age, n_wave, n_wave_t) &&
       cube_nodes_bwd_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t,
                          cube_tuning_current().chunk, workspace_bytes))
     return cube_nodes_bwd_launches(n, n_segments, n_met, n_age, n_wave, workspace_bytes) + 2;
@@ -666,7 +690,7 @@ int cube_bwd_impl(const char* who, const float* ssp_flux, const float* ssp_metal
                       vel_component, perm, seg_offsets, n_segments, n, av};
   AdjArgs args;
   args.chunk = tune.chunk;
-  if (dust_e2 == nullptr && cube_nodes_bwd_supported(n_met, n_age, n_wave, n_wave_t) &&
+  if (dust_e2 == nullptr && bwd_nodes_path(n, n_segments, n_met, n_age, n_wave, n_wave_t) &&
       cube_nodes_bwd_fit(n, n_segments, n_met, n_age, n_wave, n_wave_t, tune.chunk,
                          workspace_bytes)) {
     NodeFallback fb;

@@ -96,12 +96,11 @@ __global__ void node_fill_items_kernel(const int* seg_off, const int* flags, int
   node_fill_items(seg_off, flags, n_seg, big, multi, large, small, items, ctrl);
 }
 
-// All three steps by one block, or the last two.
+// All three steps by one block.
 __global__ void __launch_bounds__(1024) node_items_kernel(CubeInputs in, NodeFlags flags,
-                                                          bool count, bool dust, int big,
-                                                          int* multi, int* large, int* small,
-                                                          int2* items) {
-  if (count) node_count(in, flags, dust, big, multi, large, small);
+                                                          bool dust, int big, int* multi,
+                                                          int* large, int* small, int2* items) {
+  node_count(in, flags, dust, big, multi, large, small);
   __syncthreads();
   scan_exclusive_block(multi, in.n_seg, 1);
   scan_exclusive_block(large, in.n_seg, 1);
@@ -988,18 +987,25 @@ bool cube_nodes_supported(int nZ, int nA, int nW, int n_t) {
   return n_t >= 2 && nW >= 2 && slice_smem(nZ * nA) <= 227 * 1024;
 }
 
+// Rows for the single-item spaxels of a wave: all of them, or what kRowBudget holds.
+namespace {
+long long full_wave(int n_seg, int nW) {
+  return std::max(min_wave_items(n_seg),
+                  std::min<long long>(n_seg, (long long)(kRowBudget / row_bytes(nW))));
+}
+}  // namespace
+
 size_t cube_nodes_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk) {
   const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
-  const long long wave = std::max(
-      min_wave_items(n_seg), std::min<long long>(n_seg, (long long)(kRowBudget / row_bytes(nW))));
-  return std::max(L.fixed + (size_t)(multi_row_count(n) + wave) * row_bytes(nW),
+  return std::max(L.fixed + (size_t)(multi_row_count(n) + full_wave(n_seg, nW)) * row_bytes(nW),
                   L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, chunk, false));
 }
 
 bool cube_nodes_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk,
                     size_t bytes) {
   const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
-  return bytes >= L.fixed + (size_t)(multi_row_count(n) + min_wave_items(n_seg)) * row_bytes(nW) &&
+  const long long wave = std::max(min_wave_items(n_seg), (full_wave(n_seg, nW) + 1) / 2);
+  return bytes >= L.fixed + (size_t)(multi_row_count(n) + wave) * row_bytes(nW) &&
          bytes >= L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, chunk, false);
 }
 
@@ -1007,7 +1013,7 @@ int cube_nodes_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t b
   const NodeLayout L = carve_nodes(nullptr, n, n_seg, nZ, nA, nW);
   const long long fit = (long long)((bytes - L.fixed) / row_bytes(nW)) - multi_row_count(n);
   const long long wave = std::min<long long>(n_seg, fit);
-  return 6 + items_launches(n_seg, n) + 2 * (int)((n_seg + wave - 1) / wave);
+  return (items_one_block(n_seg, n) ? 7 : 9) + 2 * (int)((n_seg + wave - 1) / wave);
 }
 
 int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* lsf_taps, int n_lsf, int lsf_crop,
@@ -1034,18 +1040,15 @@ int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* l
     if (rc != RUBIX_OK) return rc;
   }
   const bool dust = dust_e != nullptr;
-  const int steps = items_launches(in.n_seg, in.n);
-  const long long work = std::max<long long>(in.n_seg, in.n / 8);  // if screened, a warp a spaxel
-  const int g = (int)std::min<long long>((work + 255) / 256, (long long)sm_count() * 8);
-  if (steps > 1) {
-    node_count_kernel<<<g, 256, 0, st>>>(in, flags, dust, big_item, L.multi, L.large, L.small);
-    RUBIX_LAUNCH_CHECK("node_count_kernel");
-  }
-  if (steps < 3) {
-    node_items_kernel<<<1, 1024, 0, st>>>(in, flags, steps == 1, dust, big_item, L.multi, L.large,
-                                          L.small, L.items);
+  if (items_one_block(in.n_seg, in.n)) {
+    node_items_kernel<<<1, 1024, 0, st>>>(in, flags, dust, big_item, L.multi, L.large, L.small,
+                                          L.items);
     RUBIX_LAUNCH_CHECK("node_items_kernel");
   } else {
+    const long long work = std::max<long long>(in.n_seg, in.n / 8);  // if screened, a warp a spaxel
+    const int g = (int)std::min<long long>((work + 255) / 256, (long long)sm_count() * 8);
+    node_count_kernel<<<g, 256, 0, st>>>(in, flags, dust, big_item, L.multi, L.large, L.small);
+    RUBIX_LAUNCH_CHECK("node_count_kernel");
     scan_exclusive_3<<<3, 1024, 0, st>>>(L.multi, L.large, L.small, in.n_seg);
     RUBIX_LAUNCH_CHECK("scan_exclusive_3");
     node_fill_items_kernel<<<g, 256, 0, st>>>(in.seg_off, L.flags, in.n_seg, big_item, L.multi,

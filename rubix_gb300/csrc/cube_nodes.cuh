@@ -27,10 +27,15 @@ int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* l
                        const CubeTuning& tune, float* cube, long long stride, void* ws,
                        size_t ws_bytes, NodeFallback* fb, cudaStream_t st);
 
+// Which path a call takes by its sizes: kPathAuto the node path where it is the faster one.
+enum CubePath { kPathAuto, kPathGeneral, kPathNodes };
+bool cube_nodes_worth(long long n, int n_seg, int nZ, int nA, int nW, int n_t);
+
 // Whether the host-side sizes qualify (the template slice fits shared memory).
 bool cube_nodes_supported(int nZ, int nA, int nW, int n_t);
-// Workspace of the node path, and whether a workspace of `bytes` holds it (with fewer rows
-// at a time in a smaller one); chunk: of the general kernel's work items.
+// Workspace of the node path, and whether a workspace of `bytes` holds it (with as little as half
+// the rows at a time; with fewer, in more waves, it is slower than the general path);
+// chunk: of the general kernel's work items.
 size_t cube_nodes_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk);
 bool cube_nodes_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk,
                     size_t bytes);

@@ -67,11 +67,10 @@ __global__ void node_adj_fill_kernel(int n_seg, const int* chunks, int2* items, 
   adj_fill(n_seg, chunks, items, ctrl);
 }
 
-// All three steps by one block, or the last two.
+// All three steps by one block.
 __global__ void __launch_bounds__(1024) node_adj_items_kernel(CubeInputs in, NodeFlags flags,
-                                                              bool count, int* chunks,
-                                                              int2* items) {
-  if (count) adj_count(in, flags, chunks);
+                                                              int* chunks, int2* items) {
+  adj_count(in, flags, chunks);
   __syncthreads();
   scan_exclusive_block(chunks, in.n_seg, 1);
   __syncthreads();
@@ -658,25 +657,31 @@ bool cube_nodes_bwd_supported(int nZ, int nA, int nW, int n_t) {
   return n_t >= 2 && nW >= 2 && adj_slice_smem(nZ * nA) <= 227 * 1024;
 }
 
+namespace {
+// Particles of a wave: all of them, or what kPartBudget holds.
+long long full_wave_particles(long long n, int nW) {
+  return std::max(min_wave_particles(n), std::min(n, part_particles(kPartBudget, nW)));
+}
+}  // namespace
+
 size_t cube_nodes_bwd_bytes(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk) {
   const AdjNodeLayout L = carve_adj(nullptr, n, n_seg, nZ, nA, nW);
-  const long long per =
-      std::max(min_wave_particles(n), std::min(n, part_particles(kPartBudget, nW)));
-  return std::max(L.fixed + part_bytes(per, nW),
+  return std::max(L.fixed + part_bytes(full_wave_particles(n, nW), nW),
                   L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, chunk, true));
 }
 
 bool cube_nodes_bwd_fit(long long n, int n_seg, int nZ, int nA, int nW, int n_t, int chunk,
                         size_t bytes) {
   const AdjNodeLayout L = carve_adj(nullptr, n, n_seg, nZ, nA, nW);
-  return bytes >= L.fixed + part_bytes(min_wave_particles(n), nW) &&
+  const long long per = std::max(min_wave_particles(n), (full_wave_particles(n, nW) + 1) / 2);
+  return bytes >= L.fixed + part_bytes(per, nW) &&
          bytes >= L.shared_off + fallback_bytes(n, n_seg, nZ, nA, nW, n_t, chunk, true);
 }
 
 int cube_nodes_bwd_launches(long long n, int n_seg, int nZ, int nA, int nW, size_t bytes) {
   const AdjNodeLayout L = carve_adj(nullptr, n, n_seg, nZ, nA, nW);
   const long long per = std::min(n, part_particles(bytes - L.fixed, nW));
-  return 6 + items_launches(n_seg, n) + 2 * (int)((n + per - 1) / per);
+  return (items_one_block(n_seg, n) ? 7 : 9) + 2 * (int)((n + per - 1) / per);
 }
 
 int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_stride,
@@ -690,17 +695,14 @@ int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_st
     const int rc = node_setup(in, nullptr, L.ctrl, st);
     if (rc != RUBIX_OK) return rc;
   }
-  const int steps = items_launches(in.n_seg, in.n);
-  const long long work = std::max<long long>(in.n_seg, in.n / 8);  // if screened, a warp a spaxel
-  const int g = (int)std::min<long long>((work + 255) / 256, (long long)sm_count() * 8);
-  if (steps > 1) {
-    node_adj_count_kernel<<<g, 256, 0, st>>>(in, flags, L.chunks);
-    RUBIX_LAUNCH_CHECK("node_adj_count_kernel");
-  }
-  if (steps < 3) {
-    node_adj_items_kernel<<<1, 1024, 0, st>>>(in, flags, steps == 1, L.chunks, L.items);
+  if (items_one_block(in.n_seg, in.n)) {
+    node_adj_items_kernel<<<1, 1024, 0, st>>>(in, flags, L.chunks, L.items);
     RUBIX_LAUNCH_CHECK("node_adj_items_kernel");
   } else {
+    const long long work = std::max<long long>(in.n_seg, in.n / 8);  // if screened, a warp a spaxel
+    const int g = (int)std::min<long long>((work + 255) / 256, (long long)sm_count() * 8);
+    node_adj_count_kernel<<<g, 256, 0, st>>>(in, flags, L.chunks);
+    RUBIX_LAUNCH_CHECK("node_adj_count_kernel");
     scan_exclusive_1block<<<1, 1024, 0, st>>>(L.chunks, in.n_seg, 1);
     RUBIX_LAUNCH_CHECK("scan_exclusive_1block");
     node_adj_fill_kernel<<<g, 256, 0, st>>>(in.n_seg, L.chunks, L.items, L.ctrl);

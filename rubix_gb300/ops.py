@@ -155,7 +155,7 @@ def spaxel_sort(idx: torch.Tensor, n_segments: int, keep: torch.Tensor | None = 
 def cube_forward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, metallicity,
                  age, velocity, vel_component, perm, seg_offsets, n_segments, out=None,
                  lsf_taps=None, lsf_crop=0, check=False, dust_av=None, dust_exponent=None,
-                 general=False):
+                 general=False, sizes=None):
     """Fused lookup + mass + Doppler/resample + per-spaxel sum -> cube [n_segments, L].
 
     ``lsf_taps`` (optional) adds the LSF convolution along wavelength of every finished
@@ -163,7 +163,9 @@ def cube_forward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, m
     -0.4 log2(10) A(lambda)/A(V)) multiplies every resampled spectrum by its dust
     transmission before the sum.  ``general=True`` evaluates every particle at every
     wavelength (``rubix_cube_fwd_general``) instead of summing over SSP nodes where the
-    template grid allows that; the two agree to float32 rounding.  ``check=True`` synchronises the stream and raises if
+    template grid allows that; the two agree to float32 rounding.  ``sizes`` (particles,
+    spaxels): the path of a call of that size instead of this one's (``rubix_cube_fwd_path``),
+    for parts of a batch that are to have the batch's bits.  ``check=True`` synchronises the stream and raises if
     the kernel reported a device error (a timed-out shared-memory copy wait)."""
     ssp_flux = _contig("ssp_flux", ssp_flux, torch.float32)
     if ssp_flux.dim() != 3:
@@ -194,8 +196,13 @@ def cube_forward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, m
         if out.dim() != 2 or out.shape[0] != n_segments or out.shape[1] < L or out.stride(1) != 1:
             raise ValueError("out must be [n_segments, >=L] with unit stride along wavelength")
     lsf = None if lsf_taps is None else _host_taps(lsf_taps)
+    grid = (L, nz, na, nw)
+    if not general and sizes is not None:
+        general = not _lib.query("rubix_cube_fwd_path", int(sizes[0]), int(sizes[1]), *grid)
+    nodes = not general and sizes is not None
     nbytes = _lib.query("rubix_cube_general_workspace_size" if general
-                        else "rubix_cube_workspace_size", n, int(n_segments), L, nz, na, nw)
+                        else "rubix_cube_nodes_workspace_size" if nodes
+                        else "rubix_cube_workspace_size", n, int(n_segments), *grid)
     ws = workspace(nbytes, dev)
     lsf_args = (None if lsf is None else lsf.ctypes.data, 0 if lsf is None else lsf.size,
                 int(lsf_crop))
@@ -212,16 +219,16 @@ def cube_forward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, m
         dust_exponent = _contig("dust_exponent", dust_exponent, torch.float32).reshape(-1)
         if dust_av.numel() != n or dust_exponent.numel() != L:
             raise ValueError("dust_av must be [n] and dust_exponent [L]")
-    if general:
-        _lib.call("rubix_cube_fwd_general", *ssp_args, *star_args, _ptr(dust_av),
-                  _ptr(dust_exponent), *out_args)
+    if general or nodes:
+        _lib.call("rubix_cube_fwd_general" if general else "rubix_cube_fwd_nodes", *ssp_args,
+                  *star_args, _ptr(dust_av), _ptr(dust_exponent), *out_args)
     elif dust_av is None:
         _lib.call("rubix_cube_fwd", *ssp_args, *star_args, *out_args)
     else:
         _lib.call("rubix_cube_fwd_dust", *ssp_args, *star_args, _ptr(dust_av),
                   _ptr(dust_exponent), *out_args)
-    _count(_launches("rubix_cube_fwd_launches", n, int(n_segments), L, nz, na, nw,
-                      1 if general else 0, ws.numel()))
+    _count(_launches("rubix_cube_fwd_launches", n, int(n_segments), *grid,
+                     1 if general else 2 if nodes else 0, ws.numel()))
     if check and n_segments > 0:
         err = ctypes.c_int(0)
         _lib.call("rubix_cube_status", _ptr(ws), ctypes.byref(err), _stream(dev))

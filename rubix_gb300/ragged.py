@@ -304,7 +304,8 @@ def galaxy_edges(sbin: int, dist_z: float, spatial_res: float = 0.2) -> np.ndarr
 
 def render_per_galaxy(batch: RaggedBatch, coords, velocity, mass, metallicity, age):
     """The same batch rendered galaxy by galaxy with the single-galaxy launches (the
-    loop a ragged launch replaces); returns the concatenated [n_segments, L] cubes."""
+    loop a ragged launch replaces); returns the concatenated [n_segments, L] cubes, bit for
+    bit the batch's (each galaxy takes the path that the batch's size chooses)."""
     r = batch.r
     out = torch.empty((batch.n_segments, batch.L), dtype=torch.float32, device=batch.device)
     edges_d = batch.d_edges
@@ -321,7 +322,8 @@ def render_per_galaxy(batch: RaggedBatch, coords, velocity, mass, metallicity, a
         cube = ops.cube_forward(r.ssp_flux, r.ssp_metallicity, r.ssp_age, r.ssp_wave_z, r.wave_t,
                                 mass[p0:p1], metallicity[p0:p1], age[p0:p1], velocity[p0:p1],
                                 r.velocity_axis, perm, offs, S * S, lsf_taps=batch.lsf_t,
-                                lsf_crop=batch.lsf_crop)
+                                lsf_crop=batch.lsf_crop,
+                                sizes=(mass.shape[0], batch.n_segments))
         ops.psf_forward(cube.view(S, S, batch.L), batch.psf_t[g],
                         out=out[s0:s1].view(S, S, batch.L))
     return out

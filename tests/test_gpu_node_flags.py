@@ -4,6 +4,7 @@ rubix_cube_fwd_general renders them, whatever shares the call, with the caller's
 import numpy as np
 import pytest
 
+from node_path import force_nodes
 from test_gpu_nodes import TOL, _problem, _run
 from test_gpu_nodes_bwd import _check
 
@@ -53,7 +54,7 @@ def test_adjoint_of_flagged_spaxels(rubix_lib, which):
 
 @pytest.mark.parametrize("n_seg, per", [(40, 30), (9000, 5)])
 @pytest.mark.parametrize("sigma", [400.0, 1500.0])
-def test_wide_velocities(rubix_lib, n_seg, per, sigma):
+def test_wide_velocities(rubix_lib, monkeypatch, n_seg, per, sigma):
     """Some or nearly all spaxels ruled out by their velocities before there are work items; one
     block or several make those.  Slow stars' spaxels do not depend on the others."""
     rng = np.random.default_rng(4)
@@ -66,6 +67,7 @@ def test_wide_velocities(rubix_lib, n_seg, per, sigma):
         p["vel"] = np.where(np.repeat(slow, counts), rng.normal(0, 60.0, offs[-1]),
                             rng.normal(0, sigma, offs[-1]))
 
+    force_nodes(monkeypatch)
     prob = _problem(counts, ssp=(5, 3, 400), edit=edit)
     a, b = _run(rubix_lib, prob, False), _run(rubix_lib, prob, True)
     scale = np.maximum(np.abs(b).max(1, keepdims=True), 1e-30)

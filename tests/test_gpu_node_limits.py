@@ -42,7 +42,8 @@ def test_velocity_limit_alone(rubix_lib, monkeypatch, sign):
         star = [to_dev(np.repeat(p[k], n)) for k in ("mass", "metallicity", "age")]
         return ops.cube_forward(flux, met, age, wzd, wtd, *star, to_dev(vel), 0,
                                 to_dev(np.arange(n, dtype=np.int32)),
-                                to_dev(np.array([0, n], np.int32)), 1, general=general)
+                                to_dev(np.array([0, n], np.int32)), 1, general=general,
+                                sizes=None if general else (10**6, 1))
 
     for vel in around:
         render(2.0 * flux, np.array([sign * 2320.0], np.float32), False)  # leaves its tables
