@@ -51,18 +51,27 @@ __global__ void aperture_mask_kernel(const float* __restrict__ coords, long long
 }
 
 // spaxel_index on the block's edges.  On ascending edges the count of edges <= x does not
-// depend on how it is found: a linear guess, right to one edge on a uniform grid, takes 3 loads
-// where the search takes 9 for 301 edges (85 -> 49 us for 10^7 particles).
+// depend on how it is found: a linear guess, right to one edge on an even grid, takes 3 loads
+// where the search takes 9 for 301 edges (85 -> 49 us for 10^7 particles).  Edges that are not
+// even to half a step (the guess and the search: 168 us, the search alone 88), and few of them (5
+// edges: 86 and 45 us), are searched.
+constexpr int kGuessEdges = 24;
+
 struct EdgeBins {
   const float* e;
   const int n, nb;
-  const bool ascending;
+  const bool guess;
   const float e0, inv;
-  __device__ __forceinline__ EdgeBins(const float* e_, int n_, bool asc)
-      : e(e_), n(n_), nb(n_ - 1), ascending(asc), e0(e_[0]),
+  __device__ __forceinline__ EdgeBins(const float* e_, int n_, bool guess_)
+      : e(e_), n(n_), nb(n_ - 1), guess(guess_), e0(e_[0]),
         inv((float)(n_ - 1) / (e_[n_ - 1] - e_[0])) {}
+  // Whether edge i allows the guess.
+  static __device__ __forceinline__ bool even(const float* __restrict__ edges, int n, int i) {
+    const float v = edges[i], e0 = edges[0], inv = (float)(n - 1) / (edges[n - 1] - e0);
+    return fabsf((v - e0) * inv - (float)i) <= 0.5f && (i + 1 == n || v <= edges[i + 1]);
+  }
   __device__ __forceinline__ int bin(float x) const {
-    if (ascending) {
+    if (guess) {
       // clamped before the conversion: NaN becomes 0, a far x stays an index
       int c = (int)fminf(fmaxf((x - e0) * inv, 0.f), (float)(nb - 1)) + 1;
       c = min(c, nb);
@@ -82,14 +91,13 @@ __global__ void spaxel_assign_kernel(const float* __restrict__ coords, long long
   extern __shared__ float s_edges[];
   const bool in_smem = n_edges <= kMaxSmemEdges;
   const float* e = in_smem ? s_edges : edges;
-  bool ascending = true;
+  bool even = n_edges >= kGuessEdges;
   for (int i = threadIdx.x; i < n_edges; i += blockDim.x) {
-    const float v = edges[i];
-    if (in_smem) s_edges[i] = v;
-    if (i + 1 < n_edges) ascending = ascending && v <= edges[i + 1];
+    if (in_smem) s_edges[i] = edges[i];
+    even = even && EdgeBins::even(edges, n_edges, i);
   }
-  ascending = __syncthreads_and(ascending);
-  const EdgeBins bins(e, n_edges, ascending);
+  even = __syncthreads_and(even);
+  const EdgeBins bins(e, n_edges, even);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     idx_out[i] = bins.flat(coords[i * stride], coords[i * stride + 1]);
@@ -118,15 +126,14 @@ __global__ void frame_assign_kernel(const float* coords, const float* velocity, 
   __shared__ float s_lo, s_hi;
   const bool in_smem = n_edges <= kMaxSmemEdges;
   const float* e = in_smem ? s_edges : edges;
-  bool ascending = true;
+  bool even = n_edges >= kGuessEdges;
   for (int i = threadIdx.x; i < n_edges; i += blockDim.x) {
-    const float v = edges[i];
-    if (in_smem) s_edges[i] = v;
-    if (i + 1 < n_edges) ascending = ascending && v <= edges[i + 1];
+    if (in_smem) s_edges[i] = edges[i];
+    even = even && EdgeBins::even(edges, n_edges, i);
   }
   if (threadIdx.x < 32) edge_range(edges, n_edges, s_lo, s_hi);
-  ascending = __syncthreads_and(ascending);
-  const EdgeBins bins(e, n_edges, ascending);
+  even = __syncthreads_and(even);
+  const EdgeBins bins(e, n_edges, even);
   const float lo = s_lo, hi = s_hi;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
@@ -176,9 +183,11 @@ __global__ void seg_offsets_kernel(const unsigned* __restrict__ keys, long long 
   }
 }
 
-// The same by one binary search per segment: where there are fewer segments than half the
-// keys, and whatever the gaps between occupied segments (the pass over the keys writes a gap
-// with one thread: 98 us for a disk that leaves most of 90 000 spaxels empty, this 13 us).
+// The same by one binary search per segment, for many keys and segments: whatever the gaps
+// between occupied segments (the pass over the keys writes a gap with one thread: 98 us for a
+// disk of 10^7 stars that leaves most of 90 000 spaxels empty, this 13 us).  A chain of some 20
+// loads: for fewer keys or segments the pass is the faster one (10^5 keys of 3600 segments,
+// whole sort: 55.6 us with the search, 51.6 with the pass; 10^6 of 16 segments 37.4, 33.2).
 __global__ void seg_search_kernel(const unsigned* __restrict__ keys, int n, int n_segments,
                                   int* __restrict__ offsets) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s <= n_segments;
@@ -377,7 +386,7 @@ extern "C" int rubix_spaxel_sort(const int32_t* idx, const uint8_t* keep, int64_
     std::swap(kin, kout);
     vin = vout;
   }
-  if (n_segments < n / 2) {
+  if (n > (1 << 19) && n_segments >= 1024 && n_segments < n / 2) {
     seg_search_kernel<<<grid_for((long long)n_segments + 1, 256), 256, 0, st>>>(
         kin, (int)n, n_segments, seg_offsets_out);
     RUBIX_LAUNCH_CHECK("seg_search_kernel");
