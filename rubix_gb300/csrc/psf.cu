@@ -723,12 +723,17 @@ bool psf_map(const PsfArgs& a, int tile_l, CUtensorMap* map) {
 }
 
 // The packed-pair kernel: no tiled copies, equal taps, and enough strips for a block on every
-// SM (smaller cubes fill the chip better with the 32-wavelength strips).
+// SM (smaller cubes fill the chip better with the 32-wavelength strips).  One block an SM, so its
+// waves have to be full (250 x 250 x 1501, 9 taps, 192 strips: 258 us against 230 of
+// psf_reg2_kernel; 295 strips 159 against 181), and the strips of several waves long enough for
+// the copies in flight (20 x 1000 x 701, 5 taps: 33 against 29).
 template <int M>
 bool launch_psf_pair(const PsfArgs& a, cudaStream_t st, int* rc) {
   if (a.sin % 4 == 0 && (reinterpret_cast<uintptr_t>(a.in) & 15) == 0) return false;
   const dim3 grid(div_up(a.nx, kPsfTileX), div_up(a.nl, kPairTileL));
-  if ((long long)grid.x * grid.y < sm_count()) return false;
+  const long long strips = (long long)grid.x * grid.y, sms = sm_count();
+  if (strips < sms || 10 * strips < 7 * sms * ((strips + sms - 1) / sms)) return false;
+  if (a.ny < 32 && strips >= 2 * sms) return false;
   if (a.ty_dev ? a.ty_dev != a.tx_dev : !std::equal(a.ty, a.ty + M, a.tx)) return false;
   const size_t smem = psf_pair_smem<M>();
   const cudaError_t e = cudaFuncSetAttribute(
