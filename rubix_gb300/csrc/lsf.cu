@@ -2,8 +2,8 @@
 // the full convolution cropped to [crop, n + crop) (rubix/telescope/lsf/lsf.py:29-105).
 //
 // A block stages one spectrum in shared memory with K-1 zeros of halo.  Up to 28 taps a
-// thread produces 12 consecutive outputs (4 in the fused dot) from float4 loads of its
-// window; longer kernels take one output at a time.
+// thread produces 12 consecutive outputs (4 for short rows and in the fused dot) from float4
+// loads of its window; longer kernels take one output at a time.
 #include "common.cuh"
 #include "dot_reduce.cuh"
 
@@ -221,10 +221,23 @@ __global__ void __launch_bounds__(kLsfThreads) lsf_scalar_kernel(LsfArgs a) {
   }
 }
 
+// Whether lsf_row_kernel is the faster one: a row of n occupies n / 12 of its 320 threads, and of
+// the 4-output kernel's 256 n / 4, which short rows and few taps prefer.  22 500 rows, us of the
+// 4-output kernel / of this: 25 taps 37 / 77 at 300, 66 / 78 at 550, 81 / 79 at 600, 105 / 89 at
+// 960, 72 / 91 at 1000 and 81 / 91 at 1025 (one round of the other is full), 89 / 90 at 1060, 120 /
+// 94 at 1450; 13 taps 59 / 62 at 550, 73 / 64 at 600, 94 / 70 at 800; 9 taps 54 / 66 at 1000, 69 /
+// 70 at 1401, 74 / 72 at 1500.  A cube that stays in L2 (9000 rows): 25 taps at most 34 / 39 at
+// 1150, both the launch's time at 1350.
+bool lsf_row_pays(long long rows, int n, int KC) {
+  if (KC <= 3) return n > 1400;
+  if (KC > 4 && n <= 1300 && rows * n < 16'000'000) return false;
+  return n >= 600 && (n <= 980 || n > 1048);
+}
+
 template <int KC>
 int launch_row(const LsfArgs& a, cudaStream_t st) {
   const size_t smem = sizeof(float) * (size_t)lsf_row_floats(a.n, KC);
-  if (lsf_row_floats(a.n, KC) > kLsfPre * kLsfRowThreads) {  // a longer row
+  if (!lsf_row_pays(a.rows, a.n, KC) || lsf_row_floats(a.n, KC) > kLsfPre * kLsfRowThreads) {
     const size_t one = sizeof(float) * ((size_t)(a.n + 3) / 4 * 4 + KC * 4 + 4);
     cudaError_t e = cudaFuncSetAttribute(lsf_vec_kernel<KC>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one);
