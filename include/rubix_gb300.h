@@ -710,10 +710,12 @@ RUBIX_API int rubix_philox4x32_10(const uint32_t* counter4, const uint32_t* key2
 /* Tuning                                                                    */
 /* ------------------------------------------------------------------------- */
 /*
- * No counterpart in rubix.  Work-item shape of rubix_cube_fwd / rubix_cube_bwd on a
- * device: spaxels are processed in chunks of `chunk` particles (multiple of 32 in
- * [32, 256]; default 256) and single-chunk spaxels with at least `big_item` particles
- * are scheduled first (default 64).  Results do not depend on big_item; they depend
+ * No counterpart in rubix.  Work-item shape of the general cube kernels on a device
+ * (rubix_cube_fwd_general, the dusty adjoints, and rubix_cube_fwd / rubix_cube_bwd where they
+ * take the general path): spaxels are processed in chunks of `chunk` particles (multiple of
+ * 32 in [32, 256]; default 256) and single-chunk spaxels with at least `big_item` particles
+ * are scheduled first (default 64).  Sums over SSP nodes have work items of their own: only
+ * big_item orders them.  Results do not depend on big_item; those of the general kernels depend
  * on chunk only through the summation order of spaxels longer than one chunk.
  * Workspace sizes follow the tuning current at query time.  A per-device table
  * guarded by a mutex; set_(device, NULL) restores the defaults.

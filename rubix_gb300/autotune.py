@@ -1,13 +1,18 @@
-"""Autotuner for the work-item shape of the cube kernels.
+"""Autotuner for the work-item shape of the general cube kernels.
 
-The fused accumulate kernel and its adjoint process each spaxel in chunks of
+The general accumulate kernel and its adjoint process each spaxel in chunks of
 ``chunk`` particles and schedule large single-chunk spaxels first
-(``rubix_cube_tuning_set``).  The best chunk depends on how particles spread over
+(``rubix_cube_tuning_set``).  They run the forward of a differentiable render, the dusty
+adjoint, calls of few stars a spaxel, template grids that do not qualify for sums over SSP
+nodes and the spaxels that the node path leaves out; the node path itself has work items of
+its own and does not read the tuning.  The best chunk depends on how particles spread over
 spaxels (a 16x16 grid holding 1e6 particles wants different chunks from a
 150x150 grid holding 1e6), so ``autotune`` times a few candidates on the caller's
 own launch with CUDA events, keeps the fastest for the device and caches the choice
-by a caller-supplied key (for example the batch layout).  Results differ between
-chunk sizes only in the summation order of spaxels longer than one chunk.
+by a caller-supplied key (for example the batch layout).  Where no candidate is clearly
+faster than the first, as for a launch that takes the node path, the first is kept.
+Results differ between chunk sizes only in the summation order of spaxels longer than one
+chunk.
 """
 
 from __future__ import annotations
@@ -22,6 +27,9 @@ from . import _lib
 
 CANDIDATES: Tuple[Tuple[int, int], ...] = ((256, 64), (192, 64), (128, 64), (256, 16),
                                            (128, 16), (64, 16))
+
+# A candidate replaces the first only if it is faster by more than repeated timings differ.
+MARGIN = 0.02
 
 _cache: Dict[Hashable, Tuple[int, int]] = {}
 _lock = threading.Lock()
@@ -49,7 +57,7 @@ def set_tuning(device: int = 0, chunk: Optional[int] = None, big_item: int = 64)
 def autotune(run: Callable[[], object], key: Hashable, device: int = 0,
              candidates: Iterable[Tuple[int, int]] = CANDIDATES, repeats: int = 3) -> dict:
     """Time ``run()`` under each candidate (chunk, big_item), keep the fastest on
-    ``device`` and cache it under ``key``.  Returns {"best", "times_ms", "cached"}."""
+    ``device`` (the first unless another is faster by ``MARGIN``) and cache it under ``key``.  Returns {"best", "times_ms", "cached"}."""
     with _lock:
         if key in _cache:
             best = _cache[key]
@@ -71,7 +79,9 @@ def autotune(run: Callable[[], object], key: Hashable, device: int = 0,
                 torch.cuda.synchronize()
                 best_ms = min(best_ms, e0.elapsed_time(e1))
             times[cand] = best_ms
-    best = min(times, key=times.get)
+    first, best = next(iter(times)), min(times, key=times.get)
+    if times[best] > (1.0 - MARGIN) * times[first]:
+        best = first
     set_tuning(device, *best)
     with _lock:
         _cache[key] = best
