@@ -200,10 +200,19 @@ def cube_forward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, m
     if not general and sizes is not None:
         general = not _lib.query("rubix_cube_fwd_path", int(sizes[0]), int(sizes[1]), *grid)
     nodes = not general and sizes is not None
-    nbytes = _lib.query("rubix_cube_general_workspace_size" if general
-                        else "rubix_cube_nodes_workspace_size" if nodes
-                        else "rubix_cube_workspace_size", n, int(n_segments), *grid)
-    ws = workspace(nbytes, dev)
+
+    def scratch(name):
+        return workspace(_lib.query(name, n, int(n_segments), *grid), dev)
+
+    try:
+        ws = scratch("rubix_cube_general_workspace_size" if general
+                     else "rubix_cube_nodes_workspace_size" if nodes
+                     else "rubix_cube_workspace_size")
+    except torch.OutOfMemoryError:  # up to 2 GB more than the general path asks for
+        if general:
+            raise
+        general, nodes = True, False
+        ws = scratch("rubix_cube_general_workspace_size")
     lsf_args = (None if lsf is None else lsf.ctypes.data, 0 if lsf is None else lsf.size,
                 int(lsf_crop))
     if (dust_av is None) != (dust_exponent is None):
@@ -266,8 +275,11 @@ def cube_backward(ssp_flux, ssp_metallicity, ssp_age, ssp_wave_z, wave_t, mass, 
     if av_grad and dust_av is None:
         raise ValueError("av_grad needs dust_av and dust_exponent")
     grads = [torch.empty(n, dtype=torch.float32, device=dev) for _ in range(5 if av_grad else 4)]
-    nbytes = _lib.query("rubix_cube_bwd_workspace_size", n, int(n_segments), L, nz, na, nw)
-    ws = workspace(nbytes, dev)
+    work = (n, int(n_segments), L, nz, na, nw)
+    try:
+        ws = workspace(_lib.query("rubix_cube_bwd_workspace_size", *work), dev)
+    except torch.OutOfMemoryError:  # up to 2 GB more than the general path asks for
+        ws = workspace(_lib.query("rubix_cube_general_workspace_size", *work), dev)
     if (dust_av is None) != (dust_exponent is None):
         raise ValueError("dust_av and dust_exponent go together")
     if dust_av is None:
