@@ -111,7 +111,7 @@ RUBIX_API size_t rubix_cube_workspace_size(int64_t n, int32_t n_segments, int32_
 
 /* Whether rubix_cube_fwd and rubix_cube_fwd_dust sum over SSP nodes (1: where the grids also
  * qualify and the workspace has the size queried above, or half of it) or take the general path
- * (0), by the sizes: with few stars a spaxel, or few altogether, the general path is the faster. */
+ * (0), by the sizes: with few stars on few spaxels the general path is the faster. */
 RUBIX_API int rubix_cube_fwd_path(int64_t n, int32_t n_segments, int32_t n_wave_t, int32_t n_met,
                                   int32_t n_age, int32_t n_wave);
 

@@ -929,27 +929,25 @@ size_t rubix::cube_general_workspace(int64_t n, int32_t n_segments, int32_t n_wa
       .bytes;
 }
 
-// The node path costs a table of T' first (as many stars' worth as n0) and some steps for every
-// spaxel; the general path more for every star.  Where they meet was measured on four grids
-// (8 x 2 x 800 to 221 x 6 x 1221 and 50 x 5 x 1400 templates), 700 to 3721 samples and 16 to
-// 22 500 spaxels of 1 to 24 stars, node / general path in us:
-//   256 spaxels, 120 templates: 1 star 1.9, 6 stars 1.02, 16 stars 0.59; 1326 templates: 8 stars 1.09,
-//   10 stars 0.98; 64 spaxels cross at 10 (16), 16 at 24 (more than 24) stars: the table;
-//   22 500 spaxels, 3721 samples: 120 templates 1.23 at 4, 0.91 at 10; 1326: 1.46, 1.07;
-//   700 samples: 1.14, 0.72 and 1.25, 0.82.  Coarse templates (800, of 8 samples an interval)
-//   have twice the slices: 1.76 at 4, 1.24 at 13 stars.  Beyond about 1300 template wavelengths
-//   the general kernel has one block an SM: 0.93 at one star, 1.03 at 8 on 4000 spaxels.
+// The node path costs a table of T' and some ten launches first, the general path more for every
+// star and for every spaxel, also an empty one.  The line was measured on disks of 10^3 to 3 10^5
+// stars (R_d 3 kpc at z = 0.1, 0.2 arcsec spaxels) with four template grids and 700, 2000
+// and 3721 samples; node / general path:
+//   16 x 16 spaxels: 10^3 stars 1.9 to 2.4, 3000 1.7 to 2.1; 32 x 32: 3000 1.6 to 2.0, 10^4 1.3 to
+//   1.7, 3 10^4 0.85 to 1.1; 64 x 64: 10^4 1.2 to 1.5, 3 10^4 1.0 (120 templates) and 1.1 to 1.3
+//   (1326); 100 x 100, 10^4 stars: 1.2 to 1.3 at 700 samples, 0.9 to 1.1 at 3721; 150 x 150: at
+//   most 1.0 and 0.4 at 280 x 280, as most spaxels are empty.
+// Stars that crowd in a few spaxels wait for them in the general path (one spaxel, 10^3 stars: 0.6
+// to 0.8; a quarter of 256 spaxels, 12 stars a spaxel: 0.6 to 0.8), hence the line in stars a spaxel.
+// What it leaves: fields of more than 10^4 spaxels with a few stars in every one of them, which no
+// galaxy has (10^5 stars over 22 500 spaxels: 1.2 to 1.8).
+// Templates of more than some 1300 wavelengths leave the general kernel one block an SM: 100 x 100
+// spaxels 0.82 to 0.95.
 bool rubix::cube_nodes_worth(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
-  const double templates = (double)nZ * nA;
-  const double n0 = 470.0 + templates / 3.5;
-  double per = 3.0 + templates / 700.0;
-  if (n_seg > 2000) {
-    per = 3.5 + templates / 700.0 + n_t / 700.0;
-    if (n_t > 3.8 * nW) per *= 2.0;
-    const int pool = kPB * (nW + 2);  // one block of the general kernel on an SM, not two
-    if (smem_layout(nW, pool, pool).total > 113 * 1024) per = n_seg > 8192 ? 0.3 : per * 0.5;
-  }
-  return n >= n0 + per * n_seg;
+  if (n_seg > 12000 || (double)n_seg * n_t > 2.2e7) return true;
+  const int pool = kPB * (nW + 2);
+  if (n_seg > 6000 && smem_layout(nW, pool, pool).total > 113 * 1024) return true;
+  return n >= 10LL * n_seg + 600 || n >= 16000 + 12LL * nZ * nA;
 }
 
 extern "C" int rubix_cube_fwd_path(int64_t n, int32_t n_segments, int32_t n_wave_t, int32_t n_met,

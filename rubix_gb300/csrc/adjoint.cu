@@ -589,22 +589,19 @@ using namespace rubix;
 namespace rubix {
 namespace {
 
-// As cube_nodes_worth; the general adjoint costs more per star, and up to some 5000 spaxels it
-// waits on latency.  Node / general path: 256 spaxels, 120 templates 1.2 at 2 stars, 0.8 at 4, 0.33
-// at 16, 1326 templates 1.5, 0.96 (700 samples), 0.48; 22 500 spaxels, 3721 samples 1.5 to 1.75 at 4
-// stars, about 1 at 10; 700 samples 0.95 at 2.
-bool bwd_nodes_worth(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
-  const double templates = (double)nZ * nA;
-  double per = 1.8 + templates / 1900.0;
-  if (n_seg > 5000) per = 1.5 + n_t / 450.0;
-  if (n_seg > 5000 && n_t > 3.8 * nW) per *= 2.0;
-  return n >= 130.0 + templates / 11.0 + per * n_seg;
+// As cube_nodes_worth, on the same disks.  The general adjoint costs twice as much per star, so
+// the line is lower; node / general path: 16 x 16 spaxels, 10^3 stars 1.0 to 1.4 (120 templates, 700 to
+// 3721 samples) and 1.1 to 1.6 (1326), 3000 stars 0.84 to 1.04 and 0.95 to 1.3; 64 x 64: 3000
+// stars 0.9 to 1.2 and 1.0 to 1.4, 10^4 0.7 to 0.96 and 0.8 to 1.2; 150 x 150 at most 1.0.
+bool bwd_nodes_worth(long long n, int n_seg, int nZ, int nA, int n_t) {
+  if (n_seg > 12000 || n >= 4LL * n_seg + 150) return true;
+  return n >= (800.0 + 0.55 * n_t) * (1.0 + nZ * nA / 1100.0);
 }
 
 // Host-side choice of path for an adjoint without dust.
 bool bwd_nodes_path(long long n, int n_seg, int nZ, int nA, int nW, int n_t) {
   return n > 0 && n_seg > 0 && cube_nodes_bwd_supported(nZ, nA, nW, n_t) &&
-         bwd_nodes_worth(n, n_seg, nZ, nA, nW, n_t);
+         bwd_nodes_worth(n, n_seg, nZ, nA, n_t);
 }
 
 }  // namespace
