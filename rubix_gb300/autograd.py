@@ -106,8 +106,8 @@ class DatacubeFunction(torch.autograd.Function):
         r = renderer
         nseg = r.sbin * r.sbin
         dust_e = None if dust_av is None else r.dust_exponent
-        # the general path: the float64 sigma gradients are sums over this cube, and a
-        # recorded fit reproduces them bit for bit
+        # the general path for every size: the cube, and the float64 sums over it that give the
+        # sigma gradients, do not depend on the path that a call's sizes choose
         A = ops.cube_forward(r.ssp_flux, r.ssp_metallicity, r.ssp_age, r.ssp_wave_z, r.wave_t,
                              mass, metallicity, age, velocity, r.velocity_axis, perm,
                              seg_offsets, nseg, dust_av=dust_av, dust_exponent=dust_e,

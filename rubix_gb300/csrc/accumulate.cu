@@ -3,10 +3,10 @@
 // per-spaxel accumulation of the datacube.
 //
 // This file is the general path: any SSP and telescope grid, any particle.  Where
-// cube_nodes.cu applies, rubix_cube_fwd and rubix_cube_fwd_dust sum over SSP nodes there
-// instead (2.5 to 3.6 times as fast) and only spaxels with a particle that it leaves out
-// (hypervelocity, outside the tables) come here; rubix_cube_fwd_general takes this path
-// for everything.
+// cube_nodes.cu applies and the call is large enough (cube_nodes_worth), rubix_cube_fwd and
+// rubix_cube_fwd_dust sum over SSP nodes there instead (2.5 to 3.6 times as fast) and only
+// spaxels with a particle that it leaves out (hypervelocity, outside the tables) come here;
+// rubix_cube_fwd_general takes this path for everything.
 //
 // Work decomposition
 //   * Setup passes (a few microseconds): a bucket table over log wavelength, the
@@ -938,7 +938,8 @@ size_t rubix::cube_general_workspace(int64_t n, int32_t n_segments, int32_t n_wa
 //   (1326); 100 x 100, 10^4 stars: 1.2 to 1.3 at 700 samples, 0.9 to 1.1 at 3721; 150 x 150: at
 //   most 1.0 and 0.4 at 280 x 280, as most spaxels are empty.
 // Stars that crowd in a few spaxels wait for them in the general path (one spaxel, 10^3 stars: 0.6
-// to 0.8; a quarter of 256 spaxels, 12 stars a spaxel: 0.6 to 0.8), hence the line in stars a spaxel.
+// to 0.8; a quarter of 256 spaxels, 12 stars a spaxel: 0.6 to 0.8), hence the line in stars a
+// spaxel.
 // What it leaves: fields of more than 10^4 spaxels with a few stars in every one of them, which no
 // galaxy has (10^5 stars over 22 500 spaxels: 1.2 to 1.8).
 // Templates of more than some 1300 wavelengths leave the general kernel one block an SM: 100 x 100

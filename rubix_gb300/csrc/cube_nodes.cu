@@ -27,15 +27,17 @@
 // every sample (this file's slice kernel 8.4 ms of it, cube_main_kernel 38.5 ms); 10^6 on
 // 150 x 150, 1.71 ms against 4.46 ms.  Relative 2-norm error against float64 7.6e-8, as before.
 //
-// Stages (one launch each): grid extrema and the velocity range; prefix sums of the
-// templates and the resampling weights at alpha_i; H; the work-item list; records of
-// every item sorted by alpha; the slice kernel; the merge of the slices (and chunks) of a
-// spaxel with the optional LSF.  A spaxel with any particle that the tables do not cover
+// Stages: grid extrema and the velocity range; the work-item list, without the spaxels that
+// velocities rule out; prefix sums of the templates, their roughness and the resampling
+// weights at alpha_i; H; records of every item sorted by alpha, and those of rough
+// templates; the slice kernel; the merge of the slices (and chunks) of a spaxel with the
+// optional LSF.  A spaxel with any particle that the tables do not cover
 // (a shifted grid that does not span the telescope range, |v| above 2300 km/s, values
 // that are not finite or that may overflow) is flagged and left to cube_main_kernel, as
-// is everything when the grids themselves do not qualify.  Every decision depends on the
-// configuration and the spaxel's own particles only, so a spaxel's result does not depend
-// on what else is rendered with it.
+// is everything when the grids themselves do not qualify.  Within the path every decision
+// depends on the configuration and the spaxel's own particles only, so a spaxel's result does
+// not depend on what else is rendered with it; whether a call takes the path at all is chosen
+// by its sizes (cube_nodes_worth).
 #include "cube_nodes.cuh"
 #include "node_tables.cuh"
 
@@ -225,10 +227,11 @@ __global__ void __launch_bounds__(kSub) node_gather_kernel(GatherArgs a) {
   }
 }
 
-// The records of rough particles, a warp each.  Bound by latency and issue together, about 1000
-// instructions a particle: 2.0 ms for 10^6 particles of 740 nodes (all of them rough: forward
-// 1.94 -> 4.0 ms, where the general path takes 4.05), with two blocks an SM and two rounds of
-// nodes in flight; 2.2 with one, 2.0 with three blocks or four rounds.  One warp summed a
+// The records of rough particles, a warp each.  Bound by issue (0.63 per cycle) and shared-memory
+// wavefronts (69 %) together, about 1600 instructions a particle of 740 nodes: 2.0 ms for 10^6
+// (all of them rough: forward 1.94 -> 4.0 ms, where the general path takes 4.05), with two
+// blocks an SM and two rounds of nodes in flight; 2.2 with one, 2.0 with three blocks or four
+// rounds.  One warp summed a
 // whole sorted run's in the gather before: 18 ms.
 __global__ void __launch_bounds__(kRoughThreads, kRoughBlocks) node_rough_kernel(GatherArgs a) {
   const int n = a.ctrl->n_rough;

@@ -14,7 +14,8 @@ COARSE = (6, 20, 1000)
     (3000, 256, 3721, COARSE, 0), (10_000, 1024, 3721, FULL, 0), (10_000, 4096, 700, FULL, 0),
     (30_000, 4096, 3721, FULL, 0), (3000, 10_000, 700, FULL, 0),
     (1000, 1, 3721, FULL, 1), (30_000, 625, 3721, FULL, 1), (300_000, 4096, 3721, FULL, 1),
-    (3000, 10_000, 700, (5, 50, 1450), 1), (3000, 10_000, 3721, COARSE, 1), (1000, 40_000, 3721, COARSE, 1),
+    (3000, 10_000, 700, (5, 50, 1450), 1), (3000, 10_000, 3721, COARSE, 1),
+    (1000, 40_000, 3721, COARSE, 1),
     (100_000, 40_000, 700, FULL, 1), (1_000_000, 22_500, 3721, FULL, 1),
     (10_000_000, 90_000, 3721, FULL, 1), (333_337, 4489, 2049, (5, 53, 1447), 1),
 ])
