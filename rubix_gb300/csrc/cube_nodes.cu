@@ -23,9 +23,9 @@
 //     particles instead of once per particle.
 //
 // Measured (221 x 6 x 1221 templates, 3721 samples, LSF fused, one GB300): 10^7 particles on
-// 300 x 300 spaxels, whole render 12.4 ms against 40.2 ms with every particle evaluated at
+// 300 x 300 spaxels, whole render 12.3 ms against 40.2 ms with every particle evaluated at
 // every sample (this file's slice kernel 8.4 ms of it, cube_main_kernel 38.5 ms); 10^6 on
-// 150 x 150, 1.71 ms against 4.46 ms.  Relative 2-norm error against float64 7.6e-8, as before.
+// 150 x 150, 1.67 ms against 4.46 ms.  Relative 2-norm error against float64 7.6e-8, as before.
 //
 // Stages: grid extrema and the velocity range; the work-item list, without the spaxels that
 // velocities rule out; prefix sums of the templates, their roughness and the resampling
