@@ -1071,8 +1071,9 @@ int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* l
     node_gather_kernel<<<blocks, kSub, 0, st>>>(g);
     RUBIX_LAUNCH_CHECK("node_gather_kernel");
     const size_t smem = rough_smem(in.n_wave_t);
-    RUBIX_CUDA_TRY(cudaFuncSetAttribute(node_rough_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024)
+      RUBIX_CUDA_TRY(cudaFuncSetAttribute(
+          node_rough_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     node_rough_kernel<<<rough_blocks(in.n), kRoughThreads, smem, st>>>(g);
     RUBIX_LAUNCH_CHECK("node_rough_kernel");
   }
@@ -1111,9 +1112,8 @@ int cube_nodes_forward(const CubeInputs& in, const float* dust_e, const float* l
     const int blocks = (int)std::min<long long>(in.n_seg, (long long)sm_count() * 8);
     auto launch = [&](auto r) -> int {
       constexpr int R = decltype(r)::value;
+      // at most 33 KB: no opt-in
       const size_t ms = sizeof(float) * ((size_t)R * kMergeThreads + std::max(n_lsf, 0) + in.n_wave_t);
-      RUBIX_CUDA_TRY(cudaFuncSetAttribute(node_merge_kernel<R>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ms));
       node_merge_kernel<R><<<blocks, kMergeThreads, ms, st>>>(m);
       RUBIX_LAUNCH_CHECK("node_merge_kernel");
       return RUBIX_OK;

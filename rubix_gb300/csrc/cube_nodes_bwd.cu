@@ -721,8 +721,9 @@ int cube_nodes_backward(const CubeInputs& in, const float* adj, long long adj_st
     node_adj_gather_kernel<<<blocks, kSub, 0, st>>>(g);
     RUBIX_LAUNCH_CHECK("node_adj_gather_kernel");
     const size_t smem = rough_smem(in.n_wave_t);
-    RUBIX_CUDA_TRY(cudaFuncSetAttribute(node_adj_rough_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024)
+      RUBIX_CUDA_TRY(cudaFuncSetAttribute(
+          node_adj_rough_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     node_adj_rough_kernel<<<rough_blocks(in.n), kRoughThreads, smem, st>>>(g);
     RUBIX_LAUNCH_CHECK("node_adj_rough_kernel");
   }
